@@ -190,7 +190,7 @@ int upload_model(messi_ctx* ctx, messi_dataset* ds, const messi_model* m, bool p
     md->eig4 = (const double*)(base + o_eig4);
     if (pairs) {
         void* p;
-        if ((rc = ensure(ctx, kSlotP16, (size_t)c.C * ds->numnodes * 256 * sizeof(float), &p))) return rc;
+        if ((rc = ensure(ctx, kSlotP16, (size_t)c.C * ds->numnodes * kP16Floats * sizeof(float), &p))) return rc;
         md->P16 = (float*)p;
     }
     if (unpaired) {
@@ -602,6 +602,7 @@ int messi_dataset_create(messi_ctx* ctx, const messi_alignment* aln, int32_t max
     messi_dataset* ds = new (std::nothrow) messi_dataset();
     if (!ds) return fail(ctx, MESSI_ENOMEM, "dataset: host allocation");
     ds->ctx = ctx;
+    ds->fuse = ctx->prune_shape != 3;  // the tcgen05 form takes one node per launch tile
     std::string err;
     rc = build_plan(ds, aln, maxbasepairdistance, pairmask, &err);
     if (rc) {
@@ -627,9 +628,8 @@ int messi_dataset_destroy(messi_dataset* ds)
         }
         tune_forget(ctx, ds);
     }
-    void* bufs[] = {ds->d_bandidx, ds->d_lr, ds->d_leaf, ds->d_nodes, ds->d_tiles, ds->d_masks, ds->d_tree,
-                    ds->d_post, ds->d_arena_f, ds->d_arena_e, ds->d_mix, ds->d_mixlam, ds->d_leafnode,
-                    ds->d_leafmsg};
+    void* bufs[] = {ds->d_bandidx, ds->d_idx, ds->d_leaf, ds->d_segs, ds->d_steps, ds->d_tiles, ds->d_masks, ds->d_tree,
+                    ds->d_post, ds->d_arena_f, ds->d_arena_e, ds->d_mix, ds->d_mixlam, ds->d_leafnode};
     for (void* b : bufs)
         if (b) cudaFree(b);
     delete ds;
@@ -706,11 +706,11 @@ int messi_siterate_conditionals(messi_ctx* ctx, messi_dataset* ds, const messi_m
     // the root descriptor writes per-category values for this call only
     double* on = d_catll;
     double* off = nullptr;
-    const size_t field = offsetof(NodeDev, catll);
-    cudaError_t e = cudaMemcpyAsync((char*)ds->d_nodes + field, &on, sizeof(double*), cudaMemcpyHostToDevice, ctx->stream);
+    const size_t field = offsetof(SegDev, catll);
+    cudaError_t e = cudaMemcpyAsync((char*)ds->d_segs + field, &on, sizeof(double*), cudaMemcpyHostToDevice, ctx->stream);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "root descriptor");
     rc = run_pairs(ctx, ds, md.P16, md.pi16, md.logw, md.lam, C, md.cat.nlam, false);
-    e = cudaMemcpyAsync((char*)ds->d_nodes + field, &off, sizeof(double*), cudaMemcpyHostToDevice, ctx->stream);
+    e = cudaMemcpyAsync((char*)ds->d_segs + field, &off, sizeof(double*), cudaMemcpyHostToDevice, ctx->stream);
     if (rc) return rc;
     if (e != cudaSuccess) return cuda_fail(ctx, e, "root descriptor");
     void* pu;
@@ -1015,6 +1015,7 @@ int messi_structure_likelihood(messi_ctx* ctx, messi_dataset* ds, const messi_mo
         sub = new (std::nothrow) messi_dataset();
         if (!sub) return fail(ctx, MESSI_ENOMEM, "structure likelihood: host allocation");
         sub->ctx = ctx;
+        sub->fuse = ctx->prune_shape != 3;
         messi_alignment aln{ds->N, ds->L, ds->numnodes, ds->masks.data(), ds->children.data(), ds->seqindex.data()};
         std::string err;
         if ((rc = build_plan(sub, &aln, L - 1, nullptr, &err, &pairs, &pu))) {

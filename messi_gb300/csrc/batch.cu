@@ -45,13 +45,18 @@ struct messi_batch {
     struct Group {
         int a0 = 0, a1 = 0, H = 0;
         int64_t rows = 0, leaf0 = 0, leaf_rows = 0;
-        std::vector<int> tile_off, tile_cnt, rtile_off, rtile_cnt;
+        std::vector<SegLevel> levels, roots;  // by segment level: interior segments and root segments
     };
     std::vector<Group> groups;
     int64_t max_group_rows = 0, max_group_leaf_rows = 0;
     int2* d_tiles = nullptr;
-    NodeDev* d_nodes = nullptr;
-    std::vector<NodeDev> nodes_host;
+    // segments and steps of every alignment, concatenated
+    std::vector<int> seg_base, step_base;
+    int total_segs = 0, total_steps = 0;
+    SegDev* d_segs = nullptr;
+    StepDev* d_steps = nullptr;
+    std::vector<SegDev> segs_host;
+    std::vector<StepDev> steps_host;
     std::vector<int> desc_grp;  // model group the descriptors were written for
     float* d_arena_f = nullptr;
     int* d_arena_e = nullptr;
@@ -127,8 +132,8 @@ void destroy_batch(messi_batch* b)
     if (b->graph) cudaGraphExecDestroy(b->graph);
     for (messi_dataset* d : b->ds)
         if (d) messi_dataset_destroy(d);
-    void* bufs[] = {b->d_tiles, b->d_nodes, b->d_arena_f, b->d_arena_e, b->stage.p, b->P16.p, b->P4.p,
-                    b->d_leafrows, b->d_leafnode, b->d_leafmsg};
+    void* bufs[] = {b->d_tiles, b->d_segs, b->d_steps, b->d_arena_f, b->d_arena_e, b->stage.p, b->P16.p, b->P4.p,
+                    b->d_leafrows, b->d_leafnode};
     for (void* p : bufs)
         if (p) cudaFree(p);
     bandbatch_free(&b->bands);
@@ -143,7 +148,6 @@ int prepare_batch_arena(messi_ctx* ctx, messi_batch* b, int C)
     if (b->chunk != 0 && b->arena_C == C) return MESSI_OK;
     if (b->d_arena_f) cudaFree(b->d_arena_f);
     if (b->d_arena_e) cudaFree(b->d_arena_e);
-    if (b->d_leafmsg) cudaFree(b->d_leafmsg);
     b->d_arena_f = nullptr;
     b->d_arena_e = nullptr;
     b->d_leafmsg = nullptr;
@@ -155,11 +159,15 @@ int prepare_batch_arena(messi_ctx* ctx, messi_batch* b, int C)
     const int64_t rows = std::max<int64_t>(b->max_group_rows, 1);
     const int64_t leaf_rows = std::max<int64_t>(b->max_group_leaf_rows, 1);
     int chunk = C;
-    while (chunk > 1 && (size_t)chunk * (rows + leaf_rows) * row_bytes > freeb / 2) chunk = (chunk + 1) / 2;
-    cudaError_t e = cudaMalloc((void**)&b->d_arena_f, (size_t)chunk * rows * 16 * sizeof(float));
+    while (chunk > 1 && ((size_t)chunk * (rows + leaf_rows) * row_bytes > freeb / 2 ||
+                         chunk * (rows + leaf_rows) > (int64_t)UINT32_MAX))
+        chunk = (chunk + 1) / 2;
+    if (rows + leaf_rows > (int64_t)UINT32_MAX) return fail(ctx, MESSI_ENOMEM, "batch message arena: more than 2^32 rows");
+    // segment rows, then the leaf messages (which have no exponents)
+    cudaError_t e = cudaMalloc((void**)&b->d_arena_f, (size_t)chunk * (rows + leaf_rows) * 16 * sizeof(float));
     if (e == cudaSuccess) e = cudaMalloc((void**)&b->d_arena_e, (size_t)chunk * rows * sizeof(int));
-    if (e == cudaSuccess) e = cudaMalloc((void**)&b->d_leafmsg, (size_t)chunk * leaf_rows * 16 * sizeof(float));
     if (e != cudaSuccess) return cuda_fail(ctx, e, "batch message arena");
+    b->d_leafmsg = b->d_arena_f + (size_t)chunk * rows * 16;
     b->chunk = chunk;
     b->arena_C = C;
     b->desc_grp.clear();  // descriptors point into the old arena
@@ -169,17 +177,22 @@ int prepare_batch_arena(messi_ctx* ctx, messi_batch* b, int C)
 int write_descriptors(messi_ctx* ctx, messi_batch* b, const std::vector<int>& grp)
 {
     if (b->desc_grp == grp) return MESSI_OK;
-    b->nodes_host.assign(b->total_nodes, NodeDev{});
+    b->segs_host.assign(b->total_segs, SegDev{});
+    b->steps_host.assign(b->total_steps, StepDev{});
     const int64_t cs = std::max<int64_t>(b->max_group_rows, 1);
     for (const messi_batch::Group& gr : b->groups)
         for (int a = gr.a0; a < gr.a1; a++)
-            fill_node_descriptors(b->ds[a], b->d_arena_f, b->d_arena_e, b->row_base[a], cs, b->d_leafmsg,
-                                  b->leaf_base[a] - gr.leaf0, std::max<int64_t>(gr.leaf_rows, 1), b->node_base[a],
-                                  grp[a], b->nodes_host.data() + b->node_base[a]);
+            fill_descriptors(b->ds[a], b->d_arena_f, b->d_arena_e, b->row_base[a], cs,
+                             b->chunk * cs + b->leaf_base[a] - gr.leaf0, std::max<int64_t>(gr.leaf_rows, 1),
+                             b->node_base[a], grp[a], b->d_steps + b->step_base[a], b->segs_host.data() + b->seg_base[a],
+                             b->steps_host.data() + b->step_base[a]);
     b->gen++;
-    cudaError_t e = cudaMemcpyAsync(b->d_nodes, b->nodes_host.data(), sizeof(NodeDev) * b->total_nodes,
+    cudaError_t e = cudaMemcpyAsync(b->d_segs, b->segs_host.data(), sizeof(SegDev) * b->total_segs,
                                     cudaMemcpyHostToDevice, ctx->stream);
-    if (e != cudaSuccess) return cuda_fail(ctx, e, "batch node descriptors");
+    if (e == cudaSuccess)
+        e = cudaMemcpyAsync(b->d_steps, b->steps_host.data(), sizeof(StepDev) * b->total_steps,
+                            cudaMemcpyHostToDevice, ctx->stream);
+    if (e != cudaSuccess) return cuda_fail(ctx, e, "batch segment descriptors");
     // the host copy must outlive the asynchronous copy: keep it until the next call
     b->desc_grp = grp;
     return MESSI_OK;
@@ -226,28 +239,20 @@ int enqueue_batch(messi_ctx* ctx, messi_batch* b, const BatchStep& s)
         if ((rc = launch_baseline_batch(ctx, b->bands, 1.0))) return rc;
     }
     tune_mark(ctx, 0);
+    const int chunk = std::min(b->chunk, kCollectCategories);
     for (const messi_batch::Group& gr : b->groups) {
-        for (int c0 = 0; c0 < C; c0 += b->chunk) {
-            const int nc = std::min(b->chunk, C - c0);
+        for (int c0 = 0; c0 < C; c0 += chunk) {
+            const int nc = std::min(chunk, C - c0);
             if ((rc = launch_leaf_messages(ctx, b->d_leafrows + (size_t)gr.leaf0 * 16, b->d_leafnode + gr.leaf0,
                                            gr.leaf_rows, s.P, b->total_nodes, c0, nc, C, b->d_leafmsg)))
                 return rc;
             for (int lv = 1; lv <= gr.H; lv++) {
                 for (int root = 0; root < 2; root++) {
-                    const int nt = root ? gr.rtile_cnt[lv] : gr.tile_cnt[lv];
-                    if (nt == 0) continue;
-                    const int2* tl = b->d_tiles + (root ? gr.rtile_off[lv] : gr.tile_off[lv]);
-                    if (ctx->profiling) {
-                        double units = 0.0;
-                        for (int a = gr.a0; a < gr.a1; a++) {
-                            const messi_dataset* d = b->ds[a];
-                            if (lv > d->H || (root != 0) != (lv == d->H)) continue;
-                            for (int v : d->level_nodes[lv]) units += (double)d->nunique[v] * nc;
-                        }
-                        prof_begin(ctx, 0, units);
-                    }
-                    if ((rc = launch_prune_tiles(ctx, b->d_nodes, tl, nt, root != 0, s.P, b->total_nodes, c0, nc, C,
-                                                 s.pi16, s.logw, s.lam, false)))
+                    const SegLevel& sl = root ? gr.roots[lv] : gr.levels[lv];
+                    if (sl.tile_cnt == 0) continue;
+                    prof_begin(ctx, 0, sl.units * nc);
+                    if ((rc = launch_prune_level(ctx, b->d_segs, b->d_tiles, sl, root != 0, s.P, b->total_nodes, c0,
+                                                 nc, C, s.pi16, s.logw, s.lam, false)))
                         return rc;
                     prof_end(ctx);
                 }
@@ -327,6 +332,7 @@ int messi_batch_create(messi_ctx* ctx, int32_t n, const messi_alignment* alns, c
             messi_dataset* d = new (std::nothrow) messi_dataset();
             if (!d) { rcs[a] = MESSI_ENOMEM; errs[a] = "batch: host allocation"; continue; }
             d->ctx = ctx;
+            d->fuse = ctx->prune_shape != 3;
             b->ds[a] = d;
             const int W = maxbasepairdistance ? maxbasepairdistance[a] : alns[a].numcols - 1;
             rcs[a] = build_plan(d, &alns[a], W, nullptr, &errs[a]);
@@ -347,10 +353,16 @@ int messi_batch_create(messi_ctx* ctx, int32_t n, const messi_alignment* alns, c
     b->col_base.resize(n);
     b->row_base.resize(n);
     b->leaf_base.resize(n);
+    b->seg_base.resize(n);
+    b->step_base.resize(n);
     for (int a = 0; a < n; a++) {
         const messi_dataset* d = b->ds[a];
         b->leaf_base[a] = b->total_leaf_rows;
         b->total_leaf_rows += d->leaf_rows;
+        b->seg_base[a] = b->total_segs;
+        b->total_segs += (int)d->segs.size();
+        b->step_base[a] = b->total_steps;
+        b->total_steps += d->nsteps;
         b->node_base[a] = b->total_nodes;
         b->total_nodes += d->numnodes;
         b->col_base[a] = b->total_cols;
@@ -383,7 +395,7 @@ int messi_batch_create(messi_ctx* ctx, int32_t n, const messi_alignment* alns, c
                 b->row_base[a] = rows;  // group-local
                 rows += r;
                 lrows += l;
-                gr.H = std::max(gr.H, b->ds[a]->H);
+                gr.H = std::max(gr.H, b->ds[a]->SH);
                 a++;
             }
             gr.a1 = a;
@@ -396,34 +408,31 @@ int messi_batch_create(messi_ctx* ctx, int32_t n, const messi_alignment* alns, c
     }
     std::vector<int2> tiles;
     for (messi_batch::Group& gr : b->groups) {
-        gr.tile_off.assign(gr.H + 1, 0);
-        gr.tile_cnt.assign(gr.H + 1, 0);
-        gr.rtile_off.assign(gr.H + 1, 0);
-        gr.rtile_cnt.assign(gr.H + 1, 0);
-        for (int lv = 1; lv <= gr.H; lv++) {
-            gr.tile_off[lv] = (int)tiles.size();
-            for (int a = gr.a0; a < gr.a1; a++) {
-                const messi_dataset* d = b->ds[a];
-                if (lv >= d->H) continue;
-                for (int v : d->level_nodes[lv])
-                    for (int64_t s = 0; s < d->nunique[v]; s += kTile)
-                        tiles.push_back(make_int2(b->node_base[a] + v, (int)s));
+        gr.levels.assign(gr.H + 1, SegLevel{});
+        gr.roots.assign(gr.H + 1, SegLevel{});
+        for (int a = gr.a0; a < gr.a1; a++)
+            for (const Segment& sg : b->ds[a]->segs) level_add(sg.root == 0 ? &gr.roots[sg.level] : &gr.levels[sg.level], sg);
+        for (int lv = 1; lv <= gr.H; lv++)
+            for (int root = 0; root < 2; root++) {
+                SegLevel& sl = root ? gr.roots[lv] : gr.levels[lv];
+                level_shape(&sl, ctx->prune_shape != 3);
+                sl.tile_off = (int)tiles.size();
+                for (int a = gr.a0; a < gr.a1; a++) {
+                    const messi_dataset* d = b->ds[a];
+                    for (size_t g = 0; g < d->segs.size(); g++)
+                        if (d->segs[g].level == lv && (d->segs[g].root == 0) == (root != 0))
+                            for (int64_t s = 0; s < d->segs[g].n; s += 32 * sl.pg)
+                                tiles.push_back(make_int2(b->seg_base[a] + (int)g, (int)s));
+                }
+                sl.tile_cnt = (int)tiles.size() - sl.tile_off;
             }
-            gr.tile_cnt[lv] = (int)tiles.size() - gr.tile_off[lv];
-            gr.rtile_off[lv] = (int)tiles.size();
-            for (int a = gr.a0; a < gr.a1; a++) {
-                const messi_dataset* d = b->ds[a];
-                if (lv != d->H) continue;
-                for (int64_t s = 0; s < d->nunique[0]; s += kTile) tiles.push_back(make_int2(b->node_base[a], (int)s));
-            }
-            gr.rtile_cnt[lv] = (int)tiles.size() - gr.rtile_off[lv];
-        }
     }
     if (tiles.empty()) tiles.push_back(make_int2(0, 0));
     cudaError_t e = cudaMalloc((void**)&b->d_tiles, tiles.size() * sizeof(int2));
     if (e == cudaSuccess)
         e = cudaMemcpy(b->d_tiles, tiles.data(), tiles.size() * sizeof(int2), cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) e = cudaMalloc((void**)&b->d_nodes, sizeof(NodeDev) * std::max(1, b->total_nodes));
+    if (e == cudaSuccess) e = cudaMalloc((void**)&b->d_segs, sizeof(SegDev) * std::max(1, b->total_segs));
+    if (e == cudaSuccess) e = cudaMalloc((void**)&b->d_steps, sizeof(StepDev) * std::max(1, b->total_steps));
     {
         // leaf rows of all alignments and their global node ids
         const size_t R = (size_t)std::max<int64_t>(b->total_leaf_rows, 1);
@@ -572,7 +581,7 @@ int messi_batch_likelihood(messi_ctx* ctx, messi_batch* b, const messi_model* mo
     const void* old_P = b->P16.p;
     const void* old_P4 = b->P4.p;
     if (grow(b->stage, st.host.size(), &dev)) return fail(ctx, MESSI_ENOMEM, "batch model staging");
-    if (grow(b->P16, (size_t)C * b->total_nodes * 256 * sizeof(float), &pt))
+    if (grow(b->P16, (size_t)C * b->total_nodes * kP16Floats * sizeof(float), &pt))
         return fail(ctx, MESSI_ENOMEM, "batch transition matrices");
     if (grow(b->P4, (size_t)nsite * b->total_nodes * 16 * sizeof(double), &p4))
         return fail(ctx, MESSI_ENOMEM, "batch unpaired transition matrices");

@@ -46,30 +46,70 @@ struct Staged {
     }
 };
 
-// Per-internal-node descriptor of one pruning step (device resident).  Rows
-// are messages: the row a node sends to its parent is its partial likelihood
-// vector multiplied by its own branch's transition matrix, so a node update
-// is the elementwise product of its two children's messages followed by one
-// mat-vec (none at the root).
-struct NodeDev {
-    const int* li;     // [n] row of the left child for each unique pair
-    const int* ri;     // [n]
-    const float* lf;   // left child message rows (16 floats each)
-    const int* le;     // left child exponents (nullptr for leaves: exponent 0)
-    long long lcs;     // left child category stride in rows
-    const float* rf;
-    const int* re;
-    long long rcs;
-    float* of;         // output message rows (unused at the root)
-    int* oe;
-    long long ocs;
+// Pruning works on segments of the tree: a connected set of internal nodes
+// whose updates one warp does in registers for the pairs of the segment's top
+// node.  Rows in memory are messages: the row a segment sends upwards is the
+// partial likelihood vector of its top node multiplied by that node's own
+// branch matrix.  A segment's program is a list of steps, each of them one
+// gathered message row (of a leaf or of a segment below) or one popped message:
+//   kStepInit: the row becomes the running message (the first child of a node
+//              whose children are both gathered);
+//   otherwise: x = running message * row (or * popped message), then the
+//              mat-vec with the branch matrix of `self` (the dot with the root
+//              frequencies for kStepRoot), which becomes the running message;
+//   kStepPush: the running message is then set aside on the warp's stack.
+//   kStepLeaf: the gathered rows are a leaf's, whose exponents are 0.
+enum StepFlags { kStepGather = 1, kStepInit = 2, kStepPop = 4, kStepPush = 8, kStepRoot = 16, kStepLeaf = 32 };
+constexpr int kStepSlotShift = 8;   // flags >> 8: the step's gather slot
+// Message rows of leaves and segments share one buffer, so a step names its
+// table by a row number (32 bits: 2^32 rows are 256 GB).
+struct StepDev {
+    unsigned row;      // first row of the gathered table in category 0
+    unsigned cs;       // its category stride in rows
+    int self;          // node whose branch matrix multiplies the product
+    int flags;
+};
+static_assert(sizeof(StepDev) == 16, "a step is read as one 16-byte word");
+struct SegDev {
+    const StepDev* steps;
+    const int* idx;    // [tile of 32 pairs][nb][32] gathered rows; pair g + 8k of the tile at 4g + k
+    float* rows;       // message rows (16 floats each)
+    int* exps;         // and their exponents
+    unsigned out, ocs; // output rows: first row and category stride (unused at the root)
     double* mix;       // root only: [n] category mixture per unique root pair
     double* mixlam;    // root only: [kMaxLambda][n] per-lambda mixtures (nullable)
     double* catll;     // root only: [C][n] per-category log-likelihoods (nullable)
-    int n;             // unique pairs at this node
-    int self;          // this node's id (index of its branch's transition matrices)
+    int n;             // unique pairs of the segment's top node
+    int nsteps, nb, nmat;  // steps, gather slots, mat-vecs
     int grp;           // model group (index of the category tables pi16/logw)
     int pad;
+};
+
+// A segment as the plan holds it (steps in program order; `child` = the node
+// whose row a gathering step reads, -1 for a popped message).
+struct PlanStep {
+    int child, self, flags;
+};
+struct Segment {
+    int root = 0;
+    int64_t n = 0;
+    int nb = 0, nmat = 0, depth = 0, level = 0;
+    int64_t idx_off = 0;   // ints into d_idx
+    int64_t row_off = -1;  // arena row of the output (-1: the tree's root)
+    std::vector<PlanStep> steps;
+};
+// Limits of a segment: nodes (the gather indices of a warp's pairs stay in
+// shared memory, 128 bytes per slot) and set-aside messages (2 KB each per warp).
+constexpr int kSegMaxNodes = 40;
+constexpr int kSegMaxDepth = 3;
+// A launch over one level of segments: tiles (segment, first pair) of
+// 32 * pg pairs, and what its shared memory has to hold.
+struct SegLevel {
+    int tile_off = 0, tile_cnt = 0;
+    int pg = 4;            // pair groups (warps on different pairs) per CTA
+    int64_t warps = 0;     // 32-pair tiles of the level
+    int max_steps = 0, max_nb = 0, max_depth = 0;
+    double units = 0.0;    // node updates per category
 };
 
 // Discretised model categories built on the host for one call.
@@ -190,8 +230,8 @@ struct messi_ctx {
     // sequences) and their size (256, 512 or 1024 threads; 0 = by band size)
     int wave_ctas = 0;
     int wave_threads = 0;
-    // pair node-update pipeline (128-pair tiles): 0 = 2 stages x 4 CTAs/SM,
-    // 1 = 3 stages x 3 CTAs/SM, 2 = 2 stages x 3 CTAs/SM
+    // pruning launch shape: 0 = 32 pairs per warp, 20 warps/SM, 1 = 16
+    // warps/SM, 2 = 64 pairs per warp, 12 warps/SM, 3 = tcgen05 form
     int prune_shape = 0;
     // per-kernel event timing (messi_ctx_profile)
     bool profiling = false;
@@ -238,17 +278,21 @@ struct messi_dataset {
     int H = 0;                         // number of levels (root level)
     int64_t band_pairs = 0, nroot = 0, executed = 0, naive = 0, arena_rows = 0;
     std::vector<int64_t> nunique;      // per node
-    std::vector<int64_t> row_off;      // arena row offset per internal non-root node
-    std::vector<std::vector<int>> level_nodes;  // internal nodes per level (index = level)
-    std::vector<int> tile_off, tile_cnt;        // per level: offset/count into d_tiles
+    bool fuse = true;                  // false: every node its own segment
+    std::vector<messi::Segment> segs;  // segs[0]: the root's
+    std::vector<int> seg_of;           // segment whose top node this is, or -1
+    int SH = 0;                        // segment levels (the root segment's level)
+    std::vector<messi::SegLevel> seg_levels;    // [SH + 1]
+    int nsteps = 0;                    // steps of all segments
     int chunk = 0;                     // categories per pass (0 = arena not allocated yet)
     int arena_C = 0;                   // category count the arena was laid out for
     uint64_t arena_gen = 0;            // bumped whenever the arena and node descriptors are rewritten
     // device
     int* d_bandidx = nullptr;          // [L][W+1]
-    int* d_lr = nullptr;               // concatenated li/ri arrays
+    int* d_idx = nullptr;              // gather indices of all segments
     float* d_leaf = nullptr;           // concatenated leaf tables
-    messi::NodeDev* d_nodes = nullptr; // [numnodes]
+    messi::SegDev* d_segs = nullptr;   // [segments]
+    messi::StepDev* d_steps = nullptr; // [nsteps]
     int2* d_tiles = nullptr;
     uint8_t* d_masks = nullptr;        // [N][L]
     int* d_tree = nullptr;             // [numnodes][4]: child0, child1, seqindex, pad
@@ -257,14 +301,14 @@ struct messi_dataset {
     int* d_arena_e = nullptr;
     double* d_mix = nullptr;           // [nroot]
     double* d_mixlam = nullptr;        // [kMaxLambda][nroot]
-    std::vector<messi::NodeDev> nodes_host;
-    std::vector<int64_t> lr_off;       // per internal node offset into d_lr (li at off, ri at off+n)
+    std::vector<messi::SegDev> segs_host;
+    std::vector<messi::StepDev> steps_host;
     std::vector<int64_t> leaf_off;     // per leaf offset (rows) into d_leaf
     int64_t leaf_rows = 0;             // rows of d_leaf (unique pairs summed over the leaves)
     std::vector<float> leaf_host;      // [leaf_rows][16] host copy of d_leaf
     std::vector<int> leafnode_host;    // [leaf_rows] leaf node of each row
     int* d_leafnode = nullptr;         // device copy of leafnode_host
-    float* d_leafmsg = nullptr;        // [chunk][leaf_rows][16] leaf messages of the current pass
+    float* d_leafmsg = nullptr;        // [chunk][leaf_rows][16] leaf messages of the current pass (end of d_arena_f)
 };
 
 namespace messi {
@@ -310,20 +354,36 @@ int build_plan(messi_dataset* ds, const messi_alignment* aln, int W, const uint8
                const std::vector<int2>* pairs = nullptr, std::vector<int32_t>* pair_unique = nullptr);
 int allocate_arena(messi_dataset* ds, int C, std::string* err);
 
-// Node descriptors of one dataset whose message rows live at `arena_f/e` +
-// row_base rows, category stride `cstride` rows, and whose leaf messages live
-// at `leafmsg` + leaf_base rows, category stride `leaf_cstride` rows;
-// transition matrices of local node v are those of node node_base + v; model
-// group `grp`.
-void fill_node_descriptors(const messi_dataset* ds, float* arena_f, int* arena_e, int64_t row_base, int64_t cstride,
-                           float* leafmsg, int64_t leaf_base, int64_t leaf_cstride, int node_base, int grp,
-                           NodeDev* out);
+// Segment and step descriptors of one dataset.  Message rows live in `rows`
+// (exponents in `exps`): those of segments from row_base on with category
+// stride `cstride`, those of leaves from leaf_base on with category stride
+// `leaf_cstride`; transition matrices of local node v are those of node
+// node_base + v; model group `grp`; the steps are `d_steps` on the device.
+void fill_descriptors(const messi_dataset* ds, float* rows, int* exps, int64_t row_base, int64_t cstride,
+                      int64_t leaf_base, int64_t leaf_cstride, int node_base, int grp, const StepDev* d_steps,
+                      SegDev* segs, StepDev* steps);
+// Adds a segment to a level's launch, and picks the level's tile shape once all are in.
+void level_add(SegLevel* lv, const Segment& sg);
+void level_shape(SegLevel* lv, bool fuse);
+// Gather indices of every segment from the per-node child lists (prune.cu):
+// ops = for each segment [op_off[s], op_off[s+1]) in parent-before-child order.
+struct IdxOp {
+    long long list;  // child list (ints into d_lr)
+    int src, dst;    // local node the list is indexed by; local node (>= 0) or slot (~dst) it gives
+};
+struct IdxSeg {
+    long long out;   // ints into d_idx
+    int op0, op1, n, nb;
+};
+int launch_segment_indices(const IdxSeg* d_segs, const IdxOp* d_ops, int nseg, int64_t maxn, const int* d_lr, int* d_idx);
 
 // ---- pruning kernels (prune.cu) ----
+constexpr int kP16Floats = 512;  // floats of one 16 x 16 transition matrix (hi part, lo part)
+constexpr int kCollectCategories = 160;  // categories of one pass at most (a root CTA collects their values)
 // nodegrp: [numnodes] model group of each node, -1 for a root (nullptr: one
 // tree, root = node 0, group 0).  Category tables are [group][C][...].
-// d_P: FP32 matrices [C][numnodes][256] (the pruning kernel splits them into
-// TF32 hi/lo parts in registers).
+// d_P: matrices [C][numnodes][kP16Floats], each as TF32 hi and lo parts in
+// the pruning kernel's fragment order (p16_at); hi + lo is the FP32 entry exactly.
 int launch_build_P16(messi_ctx* ctx, const double* d_eig, const double* d_bl, const int* d_nodegrp, int numnodes,
                      int C, float* d_P);
 int launch_build_P4(messi_ctx* ctx, const double* d_eig4, const double* d_bl, const int* d_nodegrp, int numnodes,
@@ -333,8 +393,8 @@ int launch_build_P4(messi_ctx* ctx, const double* d_eig4, const double* d_bl, co
 // C categories.
 int launch_leaf_messages(messi_ctx* ctx, const float* d_rows, const int* d_rownode, int64_t R, const float* d_P,
                          int numnodes, int c0, int nc, int C, float* d_out);
-// The tensor-core node update over `nt` tiles of one level (root tiles when root).
-int launch_prune_tiles(messi_ctx* ctx, const NodeDev* d_nodes, const int2* d_tiles, int nt, bool root,
+// The segments of one level (the root segments when root) over categories c0 .. c0+nc-1.
+int launch_prune_level(messi_ctx* ctx, const SegDev* d_segs, const int2* d_tiles, const SegLevel& lv, bool root,
                        const float* d_P, int numnodes, int c0, int nc, int C, const float* d_pi16,
                        const double* d_logw, const int* d_lam, bool per_lambda);
 int run_pairs(messi_ctx* ctx, messi_dataset* ds, const float* d_P, const float* d_pi16, const double* d_logw,

@@ -1,6 +1,6 @@
 // plan.cpp -- per-dataset pair plan: column-pattern compression, unique pair
-// lists per tree node, child gather indices, level schedule and partial-buffer
-// arena layout.
+// lists per tree node, the tree's segments with their programs and gather
+// indices, level schedule and message arena layout.
 //
 // Semantics follow getindexdict (src/FelsensteinCUDA.jl:77-142) and
 // Dataset.subcolumnrefs (src/Dataset.jl:180-196): at node v two root pairs
@@ -10,6 +10,7 @@
 // once.  Results do not depend on the dedup, only the work does.
 #include <algorithm>
 #include <cstring>
+#include <functional>
 
 #include "internal.h"
 
@@ -48,6 +49,143 @@ struct KeyMap {
 };
 
 }  // namespace
+
+// ---------------------------------------------------------------------------
+// Segments.  A node whose unique pairs are nearly as many as its ancestor's
+// gains little from being computed once per unique pair: its rows would be
+// written and read back (68 bytes each way) to save few updates.  Such a node
+// joins its ancestor's segment and is recomputed in registers for each of the
+// segment's pairs.  A child joins when it has at least this share of the pairs
+// of the segment's top node (GB300, pruning of 64 x 1,000 / 30 x 9,000 / 100 x
+// 733 columns: 0.7: 5.80 / 19.5 / 6.08 ms, 0.6: 5.72 / 18.3 / 5.70, 0.5: 6.19 /
+// 19.5 / 6.38, 0.35: 6.80 / 24.3 / 7.15: below it the recomputed updates cost
+// more than the rows).
+// ---------------------------------------------------------------------------
+constexpr double kFuseShare = 0.6;
+
+struct SegBuilder {
+    messi_dataset* ds;
+    std::vector<char> in;      // node belongs to the segment being built
+    std::vector<int> need;     // set-aside messages its evaluation needs
+
+    bool internal(int v) const { return ds->children[2 * v] >= 0; }
+    // fused children of v, the one that needs more set-aside messages first
+    int fused(int v, int (&c)[2]) const
+    {
+        int k = 0;
+        for (int side = 0; side < 2; side++) {
+            const int w = ds->children[2 * v + side];
+            if (internal(w) && in[w]) c[k++] = w;
+        }
+        if (k == 2 && need[c[1]] > need[c[0]]) std::swap(c[0], c[1]);
+        return k;
+    }
+    void drop(int v)  // takes v's subtree out of the segment
+    {
+        in[v] = 0;
+        for (int side = 0; side < 2; side++) {
+            const int w = ds->children[2 * v + side];
+            if (internal(w) && in[w]) drop(w);
+        }
+    }
+    void emit(Segment& sg, int v, bool push)
+    {
+        int c[2];
+        const int k = fused(v, c);
+        const int flag = (v == 0 ? kStepRoot : 0) | (push ? kStepPush : 0);
+        if (k == 2) {
+            emit(sg, c[0], true);
+            emit(sg, c[1], false);
+            sg.steps.push_back({-1, v, flag | kStepPop});
+        } else {
+            int a = ds->children[2 * v], b = ds->children[2 * v + 1];
+            if (k == 1) {
+                emit(sg, c[0], false);
+                if (a == c[0]) a = b;
+            } else {
+                // the larger table first: its rows are asked for a step ahead
+                if (ds->nunique[b] > ds->nunique[a]) std::swap(a, b);
+                sg.steps.push_back({a, v, kStepGather | kStepInit | (sg.nb++ << kStepSlotShift)});
+                a = b;
+            }
+            sg.steps.push_back({a, v, flag | kStepGather | (sg.nb++ << kStepSlotShift)});
+        }
+        if (v != 0) sg.nmat++;
+    }
+
+    // Segment with top node r, then (recursively) the segments below it.
+    void build(int r0)
+    {
+        std::vector<int> todo{r0};
+        while (!todo.empty()) {
+            const int r = todo.back();
+            todo.pop_back();
+            // nodes, largest first, until the segment is full
+            std::vector<int> members{r}, cand;
+            in[r] = 1;
+            auto offer = [&](int v) {
+                for (int side = 0; side < 2; side++) {
+                    const int w = ds->children[2 * v + side];
+                    if (ds->fuse && internal(w) && (double)ds->nunique[w] >= kFuseShare * (double)ds->nunique[r])
+                        cand.push_back(w);
+                }
+            };
+            offer(r);
+            while (!cand.empty() && (int)members.size() < kSegMaxNodes) {
+                size_t best = 0;
+                for (size_t k = 1; k < cand.size(); k++)
+                    if (ds->nunique[cand[k]] > ds->nunique[cand[best]]) best = k;
+                const int v = cand[best];
+                cand.erase(cand.begin() + (long)best);
+                in[v] = 1;
+                members.push_back(v);
+                offer(v);
+            }
+            // children have larger numbers: descending order is bottom-up
+            std::sort(members.begin(), members.end(), std::greater<int>());
+            for (int v : members) {
+                if (!in[v]) continue;
+                int c[2];
+                int k = fused(v, c);
+                if (k == 2 && std::max(need[c[0]], 1 + need[c[1]]) > kSegMaxDepth) {
+                    // too many set-aside messages: the child with fewer pairs becomes a table
+                    const int w = ds->nunique[c[0]] < ds->nunique[c[1]] ? c[0] : c[1];
+                    drop(w);
+                    k = fused(v, c);
+                }
+                need[v] = (k == 2) ? std::max(need[c[0]], 1 + need[c[1]]) : (k == 1 ? need[c[0]] : 0);
+            }
+            Segment sg;
+            sg.root = r;
+            sg.n = ds->nunique[r];
+            sg.depth = need[r];
+            emit(sg, r, false);
+            ds->seg_of[r] = (int)ds->segs.size();
+            ds->segs.push_back(std::move(sg));
+            for (int v : members) {
+                if (!in[v]) continue;
+                for (int side = 0; side < 2; side++) {
+                    const int w = ds->children[2 * v + side];
+                    if (internal(w) && !in[w]) todo.push_back(w);
+                }
+            }
+            for (int v : members) in[v] = 0;
+        }
+    }
+};
+
+void level_add(SegLevel* lv, const Segment& sg)
+{
+    lv->warps += (sg.n + 31) / 32;
+    lv->max_steps = std::max(lv->max_steps, (int)sg.steps.size());
+    lv->max_nb = std::max(lv->max_nb, sg.nb);
+    lv->max_depth = std::max(lv->max_depth, sg.depth);
+    lv->units += (double)sg.n * (sg.nmat + (sg.root == 0 ? 1 : 0));
+}
+
+// Four pair groups per CTA where the level's pairs alone fill the GPU; below
+// that one pair group per CTA, whose warps share the categories (launch_prune_level).
+void level_shape(SegLevel* lv, bool fuse) { lv->pg = (lv->warps >= 4096 || !fuse) ? 4 : 1; }
 
 int build_plan(messi_dataset* ds, const messi_alignment* aln, int W, const uint8_t* pairmask, std::string* err,
                const std::vector<int2>* pairs, std::vector<int32_t>* pair_unique)
@@ -239,10 +377,32 @@ int build_plan(messi_dataset* ds, const messi_alignment* aln, int W, const uint8
         if (v != 0) { std::vector<int32_t>().swap(rep[v]); }
     }
 
-    // ---- statistics
+    // ---- segments, their levels (a segment's rows are read by one segment
+    // above it) and statistics
+    ds->segs.clear();
+    ds->seg_of.assign(nn, -1);
+    {
+        SegBuilder sb{ds, std::vector<char>(nn, 0), std::vector<int>(nn, 0)};
+        sb.build(0);
+    }
+    // a segment comes after the one that reads it: levels bottom-up in reverse order
+    std::vector<int> reader(ds->segs.size(), -1);
+    for (int g = (int)ds->segs.size() - 1; g >= 0; g--) {
+        Segment& sg = ds->segs[g];
+        for (const PlanStep& st : sg.steps)
+            if (st.child >= 0 && ds->seg_of[st.child] >= 0) {
+                const int below = ds->seg_of[st.child];
+                sg.level = std::max(sg.level, ds->segs[below].level);
+                reader[below] = g;
+            }
+        sg.level++;
+    }
+    ds->SH = ds->segs[0].level;
+    ds->seg_levels.assign(ds->SH + 1, SegLevel{});
+    for (const Segment& sg : ds->segs) level_add(&ds->seg_levels[sg.level], sg);
+    for (SegLevel& lv : ds->seg_levels) level_shape(&lv, ds->fuse);
     ds->executed = 0;
-    for (int v = 0; v < nn; v++)
-        if (ds->children[2 * v] >= 0) ds->executed += ds->nunique[v];
+    for (const SegLevel& lv : ds->seg_levels) ds->executed += (int64_t)lv.units;
     ds->naive = ds->band_pairs * (int64_t)(N - 1);
 
     // ---- leaf tables: row u = outer product of the two column masks
@@ -265,47 +425,76 @@ int build_plan(messi_dataset* ds, const messi_alignment* aln, int W, const uint8
         }
     }
 
-    // ---- arena layout over levels: a node's rows live from its level to its parent's
-    ds->row_off.assign(nn, -1);
-    ds->level_nodes.assign(ds->H + 1, {});
-    for (int v = 0; v < nn; v++)
-        if (ds->children[2 * v] >= 0) ds->level_nodes[ds->level[v]].push_back(v);
+    // ---- arena layout over levels: a segment's rows live from its level to its reader's
     {
-        struct Iv { int64_t off, len; int node; };
+        struct Iv { int64_t off, len; int last; };
         std::vector<Iv> live;
         int64_t peak = 0;
-        for (int lv = 1; lv <= ds->H; lv++) {
-            live.erase(std::remove_if(live.begin(), live.end(),
-                                      [&](const Iv& iv) { return ds->level[ds->parent[iv.node]] < lv; }),
+        for (int lv = 1; lv < ds->SH; lv++) {
+            live.erase(std::remove_if(live.begin(), live.end(), [&](const Iv& iv) { return iv.last < lv; }),
                        live.end());
-            for (int v : ds->level_nodes[lv]) {
-                if (v == 0) continue;  // the root writes mixtures, not rows
-                int64_t len = ds->nunique[v];
-                std::sort(live.begin(), live.end(), [](const Iv& a, const Iv& b) { return a.off < b.off; });
+            for (size_t g = 1; g < ds->segs.size(); g++) {  // the root (0) writes mixtures, not rows
+                Segment& sg = ds->segs[g];
+                if (sg.level != lv) continue;
+                std::sort(live.begin(), live.end(), [](const Iv& x, const Iv& y) { return x.off < y.off; });
                 int64_t pos = 0;
                 for (const Iv& iv : live) {
-                    if (iv.off - pos >= len) break;
+                    if (iv.off - pos >= sg.n) break;
                     pos = std::max(pos, iv.off + iv.len);
                 }
-                live.push_back({pos, len, v});
-                ds->row_off[v] = pos;
-                peak = std::max(peak, pos + len);
+                live.push_back({pos, sg.n, ds->segs[reader[g]].level});
+                sg.row_off = pos;
+                peak = std::max(peak, pos + sg.n);
             }
         }
         ds->arena_rows = std::max<int64_t>(peak, 1);
     }
 
+    // ---- gather indices: for every segment the child lists to follow from its
+    // top node down (composed on the device), parents before children
+    std::vector<IdxOp> idx_ops;
+    std::vector<IdxSeg> idx_segs;
+    std::vector<int64_t> lr_off(nn, -1);
+    int64_t lr_total = 0, idx_total = 0, max_seg_n = 0;
+    for (int v = 0; v < nn; v++)
+        if (ds->children[2 * v] >= 0) { lr_off[v] = lr_total; lr_total += 2 * ds->nunique[v]; }
+    {
+        std::vector<int> slot(nn, -1), local(nn, -1), inside;
+        ds->nsteps = 0;
+        for (Segment& sg : ds->segs) {
+            sg.idx_off = idx_total;
+            idx_total += ((sg.n + 31) / 32) * 32 * sg.nb;
+            max_seg_n = std::max(max_seg_n, sg.n);
+            ds->nsteps += (int)sg.steps.size();
+            IdxSeg is{sg.idx_off, (int)idx_ops.size(), 0, (int)sg.n, sg.nb};
+            inside.assign(1, sg.root);
+            for (const PlanStep& st : sg.steps) {
+                if (st.child >= 0) slot[st.child] = st.flags >> kStepSlotShift;
+                if (!(st.flags & kStepInit) && st.self != sg.root) inside.push_back(st.self);
+            }
+            std::sort(inside.begin(), inside.end());
+            for (size_t k = 0; k < inside.size(); k++) local[inside[k]] = (int)k;
+            for (int v : inside)
+                for (int side = 0; side < 2; side++) {
+                    const int c = ds->children[2 * v + side];
+                    idx_ops.push_back({lr_off[v] + side * ds->nunique[v], local[v], local[c] >= 0 ? local[c] : ~slot[c]});
+                }
+            for (int v : inside) local[v] = -1;
+            is.op1 = (int)idx_ops.size();
+            idx_segs.push_back(is);
+        }
+    }
+
     // ---- upload static device data
     cudaError_t e;
-    int64_t lr_total = 0;
-    ds->lr_off.assign(nn, -1);
-    for (int v = 0; v < nn; v++)
-        if (ds->children[2 * v] >= 0) { ds->lr_off[v] = lr_total; lr_total += 2 * ds->nunique[v]; }
+    int* d_lr = nullptr;
+    IdxOp* d_ops = nullptr;
+    IdxSeg* d_isegs = nullptr;
     std::vector<int32_t> lr((size_t)std::max<int64_t>(lr_total, 1));
     for (int v = 0; v < nn; v++)
         if (ds->children[2 * v] >= 0) {
-            std::copy(li[v].begin(), li[v].end(), lr.begin() + ds->lr_off[v]);
-            std::copy(ri[v].begin(), ri[v].end(), lr.begin() + ds->lr_off[v] + ds->nunique[v]);
+            std::copy(li[v].begin(), li[v].end(), lr.begin() + lr_off[v]);
+            std::copy(ri[v].begin(), ri[v].end(), lr.begin() + lr_off[v] + ds->nunique[v]);
         }
     std::vector<int> tree((size_t)nn * 4);
     for (int v = 0; v < nn; v++) {
@@ -320,7 +509,15 @@ int build_plan(messi_dataset* ds, const messi_alignment* aln, int W, const uint8
         if ((e = cudaMemcpy((dst), (src), (bytes), cudaMemcpyHostToDevice)) != cudaSuccess) goto cuda_error; \
     } while (0)
     UPLOAD(ds->d_bandidx, bandidx.data(), bandidx.size() * sizeof(int32_t));
-    UPLOAD(ds->d_lr, lr.data(), lr.size() * sizeof(int32_t));
+    UPLOAD(d_lr, lr.data(), lr.size() * sizeof(int32_t));
+    UPLOAD(d_ops, idx_ops.data(), idx_ops.size() * sizeof(IdxOp));
+    UPLOAD(d_isegs, idx_segs.data(), idx_segs.size() * sizeof(IdxSeg));
+    if ((e = cudaMalloc((void**)&ds->d_idx, (size_t)std::max<int64_t>(idx_total, 1) * sizeof(int))) != cudaSuccess)
+        goto cuda_error;
+    if (launch_segment_indices(d_isegs, d_ops, (int)idx_segs.size(), max_seg_n, d_lr, ds->d_idx)) {
+        e = cudaGetLastError();
+        goto cuda_error;
+    }
     UPLOAD(ds->d_leaf, leaf.data(), leaf.size() * sizeof(float));
     UPLOAD(ds->d_leafnode, ds->leafnode_host.data(), ds->leafnode_host.size() * sizeof(int));
     UPLOAD(ds->d_masks, ds->masks.data(), ds->masks.size());
@@ -335,71 +532,83 @@ int build_plan(messi_dataset* ds, const messi_alignment* aln, int W, const uint8
     {
         // tiles per level
         std::vector<int2> tiles;
-        ds->tile_off.assign(ds->H + 1, 0);
-        ds->tile_cnt.assign(ds->H + 1, 0);
-        for (int lv = 1; lv <= ds->H; lv++) {
-            ds->tile_off[lv] = (int)tiles.size();
-            for (int v : ds->level_nodes[lv])
-                for (int64_t b = 0; b < ds->nunique[v]; b += kTile) tiles.push_back(make_int2(v, (int)b));
-            ds->tile_cnt[lv] = (int)tiles.size() - ds->tile_off[lv];
+        for (int lv = 1; lv <= ds->SH; lv++) {
+            SegLevel& sl = ds->seg_levels[lv];
+            sl.tile_off = (int)tiles.size();
+            for (size_t g = 0; g < ds->segs.size(); g++)
+                if (ds->segs[g].level == lv)
+                    for (int64_t b = 0; b < ds->segs[g].n; b += 32 * sl.pg) tiles.push_back(make_int2((int)g, (int)b));
+            sl.tile_cnt = (int)tiles.size() - sl.tile_off;
         }
         if (tiles.empty()) tiles.push_back(make_int2(0, 0));
         if ((e = cudaMalloc((void**)&ds->d_tiles, tiles.size() * sizeof(int2))) != cudaSuccess) goto cuda_error;
         if ((e = cudaMemcpy(ds->d_tiles, tiles.data(), tiles.size() * sizeof(int2), cudaMemcpyHostToDevice)) !=
             cudaSuccess)
             goto cuda_error;
-        if ((e = cudaMalloc((void**)&ds->d_nodes, sizeof(NodeDev) * nn)) != cudaSuccess) goto cuda_error;
+        if ((e = cudaMalloc((void**)&ds->d_segs, sizeof(SegDev) * ds->segs.size())) != cudaSuccess) goto cuda_error;
+        if ((e = cudaMalloc((void**)&ds->d_steps, sizeof(StepDev) * std::max(1, ds->nsteps))) != cudaSuccess)
+            goto cuda_error;
     }
+    // the index kernel ran on the default stream: done before any context stream reads its output
+    if ((e = cudaStreamSynchronize(0)) != cudaSuccess) goto cuda_error;
+    cudaFree(d_lr);
+    cudaFree(d_ops);
+    cudaFree(d_isegs);
     return MESSI_OK;
 cuda_error:
+    cudaFree(d_lr);
+    cudaFree(d_ops);
+    cudaFree(d_isegs);
     *err = std::string("dataset upload: ") + cudaGetErrorString(e);
     return (e == cudaErrorMemoryAllocation) ? MESSI_ENOMEM : MESSI_ECUDA;
 }
 
-void fill_node_descriptors(const messi_dataset* ds, float* arena_f, int* arena_e, int64_t row_base, int64_t cstride,
-                           float* leafmsg, int64_t leaf_base, int64_t leaf_cstride, int node_base, int grp,
-                           NodeDev* out)
+void fill_descriptors(const messi_dataset* ds, float* rows, int* exps, int64_t row_base, int64_t cstride,
+                      int64_t leaf_base, int64_t leaf_cstride, int node_base, int grp, const StepDev* d_steps,
+                      SegDev* segs, StepDev* steps)
 {
-    for (int v = 0; v < ds->numnodes; v++) {
-        NodeDev& d = out[v];
-        d = NodeDev{};
-        if (ds->children[2 * v] < 0) continue;
-        d.n = (int)ds->nunique[v];
-        d.li = ds->d_lr + ds->lr_off[v];
-        d.ri = ds->d_lr + ds->lr_off[v] + ds->nunique[v];
-        const int c0 = ds->children[2 * v], c1 = ds->children[2 * v + 1];
-        d.self = node_base + v;
+    size_t at = 0;
+    for (size_t g = 0; g < ds->segs.size(); g++) {
+        const Segment& sg = ds->segs[g];
+        SegDev d{};
+        d.steps = d_steps + at;
+        d.idx = ds->d_idx + sg.idx_off;
+        d.rows = rows;
+        d.exps = exps;
+        d.n = (int)sg.n;
+        d.nsteps = (int)sg.steps.size();
+        d.nb = sg.nb;
+        d.nmat = sg.nmat;
         d.grp = grp;
-        for (int side = 0; side < 2; side++) {
-            const int c = side ? c1 : c0;
-            const float* f;
-            const int* ex;
-            long long cs;
-            if (ds->children[2 * c] < 0) {
-                f = leafmsg + (size_t)(leaf_base + ds->leaf_off[c]) * 16;
-                ex = nullptr;
-                cs = leaf_cstride;
-            } else {
-                f = arena_f + (size_t)(row_base + ds->row_off[c]) * 16;
-                ex = arena_e + row_base + ds->row_off[c];
-                cs = cstride;
-            }
-            if (side) { d.rf = f; d.re = ex; d.rcs = cs; }
-            else { d.lf = f; d.le = ex; d.lcs = cs; }
-        }
-        if (v != 0) {
-            d.of = arena_f + (size_t)(row_base + ds->row_off[v]) * 16;
-            d.oe = arena_e + row_base + ds->row_off[v];
-            d.ocs = cstride;
+        if (sg.root != 0) {
+            d.out = (unsigned)(row_base + sg.row_off);
+            d.ocs = (unsigned)cstride;
         } else {
             d.mix = ds->d_mix;
             d.mixlam = ds->d_mixlam;
         }
+        segs[g] = d;
+        for (const PlanStep& st : sg.steps) {
+            StepDev& o = steps[at++];
+            o = StepDev{};
+            o.self = node_base + st.self;
+            o.flags = st.flags;
+            if (st.child < 0) continue;
+            const int below = ds->seg_of[st.child];
+            if (below < 0) {
+                o.row = (unsigned)(leaf_base + ds->leaf_off[st.child]);
+                o.cs = (unsigned)leaf_cstride;
+                o.flags |= kStepLeaf;
+            } else {
+                o.row = (unsigned)(row_base + ds->segs[below].row_off);
+                o.cs = (unsigned)cstride;
+            }
+        }
     }
 }
 
-// Allocate the partial-row arena for C categories (as many per pass as fit)
-// and fill the node descriptors.
+// Allocate the message arena for C categories (as many per pass as fit) and
+// fill the segment descriptors.
 int allocate_arena(messi_dataset* ds, int C, std::string* err)
 {
     size_t freeb = 0, totalb = 0;
@@ -408,32 +617,42 @@ int allocate_arena(messi_dataset* ds, int C, std::string* err)
     size_t budget = freeb / 2;
     const int64_t leaf_rows = std::max<int64_t>(ds->leaf_rows, 1);
     int chunk = C;
-    while (chunk > 1 && (size_t)chunk * (ds->arena_rows + leaf_rows) * row_bytes > budget) chunk = (chunk + 1) / 2;
+    const int64_t all_rows = ds->arena_rows + leaf_rows;
+    while (chunk > 1 && ((size_t)chunk * all_rows * row_bytes > budget || chunk * all_rows > (int64_t)UINT32_MAX))
+        chunk = (chunk + 1) / 2;
+    if (all_rows > (int64_t)UINT32_MAX) {
+        *err = "message arena: more than 2^32 rows";
+        return MESSI_ENOMEM;
+    }
     if (ds->chunk != chunk) {
         if (ds->d_arena_f) cudaFree(ds->d_arena_f);
         if (ds->d_arena_e) cudaFree(ds->d_arena_e);
-        if (ds->d_leafmsg) cudaFree(ds->d_leafmsg);
         ds->d_arena_f = nullptr;
         ds->d_arena_e = nullptr;
         ds->d_leafmsg = nullptr;
         ds->chunk = 0;
-        cudaError_t e = cudaMalloc((void**)&ds->d_arena_f, (size_t)chunk * ds->arena_rows * 16 * sizeof(float));
+        // segment rows, then the leaf messages (which have no exponents)
+        cudaError_t e = cudaMalloc((void**)&ds->d_arena_f, (size_t)chunk * all_rows * 16 * sizeof(float));
         if (e == cudaSuccess) e = cudaMalloc((void**)&ds->d_arena_e, (size_t)chunk * ds->arena_rows * sizeof(int));
-        if (e == cudaSuccess) e = cudaMalloc((void**)&ds->d_leafmsg, (size_t)chunk * leaf_rows * 16 * sizeof(float));
         if (e != cudaSuccess) {
             *err = std::string("message arena: ") + cudaGetErrorString(e);
             return MESSI_ENOMEM;
         }
+        ds->d_leafmsg = ds->d_arena_f + (size_t)chunk * ds->arena_rows * 16;
         ds->chunk = chunk;
     }
     ds->arena_gen++;
-    ds->nodes_host.assign(ds->numnodes, NodeDev{});
-    fill_node_descriptors(ds, ds->d_arena_f, ds->d_arena_e, 0, ds->arena_rows, ds->d_leafmsg, 0, leaf_rows, 0, 0,
-                          ds->nodes_host.data());
-    const int nn = ds->numnodes;
-    cudaError_t e = cudaMemcpy(ds->d_nodes, ds->nodes_host.data(), sizeof(NodeDev) * nn, cudaMemcpyHostToDevice);
+    ds->segs_host.assign(ds->segs.size(), SegDev{});
+    ds->steps_host.assign((size_t)ds->nsteps, StepDev{});
+    fill_descriptors(ds, ds->d_arena_f, ds->d_arena_e, 0, ds->arena_rows, (int64_t)ds->chunk * ds->arena_rows,
+                     leaf_rows, 0, 0, ds->d_steps, ds->segs_host.data(), ds->steps_host.data());
+    cudaError_t e = cudaMemcpy(ds->d_segs, ds->segs_host.data(), sizeof(SegDev) * ds->segs.size(),
+                               cudaMemcpyHostToDevice);
+    if (e == cudaSuccess)
+        e = cudaMemcpy(ds->d_steps, ds->steps_host.data(), sizeof(StepDev) * (size_t)ds->nsteps,
+                       cudaMemcpyHostToDevice);
     if (e != cudaSuccess) {
-        *err = std::string("node descriptors: ") + cudaGetErrorString(e);
+        *err = std::string("segment descriptors: ") + cudaGetErrorString(e);
         return MESSI_ECUDA;
     }
     return MESSI_OK;

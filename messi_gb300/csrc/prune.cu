@@ -15,18 +15,19 @@
 //     felsenstein.cu:170-190); the root needs no mat-vec, only pi . x;
 //   * leaf_msg_kernel: the messages of the leaves (P_leaf x indicator rows)
 //     per category pass;
-//   * prune_msg_kernel: one launch per tree level and category pass; a warp
-//     owns 32 unique pairs of one node, gathers the two children's message
-//     rows with cp.async (two categories in flight) and does the mat-vec on
-//     the tensor cores (3xTF32 mma.sync, operands split into hi/lo in
-//     registers).  Rows are rescaled by an exact power of two (exponent kept
-//     as an int), which computes the same likelihood as the reference's
-//     divide-by-max (felsenstein.cu:193-198);
-//   * the root variant folds sumfinal and the category log-sum-exp into the
-//     same pass (FP64 log-likelihood reduction);
-//   * prune_tc_kernel: the interior update as tcgen05.mma (A in tensor
-//     memory, P in shared memory, accumulators in tensor memory), the same
-//     bits as prune_msg_kernel; chosen only on request (launch shape 3).
+//   * prune_path_kernel: one launch per level of tree segments and category
+//     pass; a warp owns 32 unique pairs and walks them through a segment's
+//     nodes with the running message in registers, gathering one child row
+//     per node and doing the mat-vec on the tensor cores (3xTF32 mma.sync,
+//     operands split into hi/lo).  Messages are rescaled by an exact power of
+//     two (exponent kept as an int), which computes the same likelihood as
+//     the reference's divide-by-max (felsenstein.cu:193-198); the root folds
+//     sumfinal and the category log-sum-exp into the same pass (FP64
+//     log-likelihood reduction);
+//   * prune_tc_kernel: the interior update of single-node segments as
+//     tcgen05.mma (A in tensor memory, P in shared memory, accumulators in
+//     tensor memory), the same bits as prune_path_kernel; chosen only on
+//     request (launch shape 3).
 // unpaired_site_kernel + unpaired_mix_kernel restate
 // computeunpairedlikelihoodscat (src/FARCE.jl:742-773) in FP64 with the CPU
 // rescaling rule.
@@ -45,6 +46,22 @@ namespace messi {
 // CTA per node and category staged U for every matrix and divided per entry:
 // 26 ms for the 1.28 M matrices of a 256-alignment batch.)
 constexpr int kP16Nodes = 32;
+
+// x as TF32 hi + lo: hi = x rounded to TF32 (half a TF32 ulp added to the
+// magnitude bits, then truncated: round to nearest, ties away), lo = x - hi,
+// exact in FP32.
+__device__ __forceinline__ float tf32_hi(float x)
+{
+    return __uint_as_float((__float_as_uint(x) + 0x1000u) & 0xffffe000u);
+}
+
+// Float offset of entry (a, d) in a stored matrix: the B fragments of the
+// pruning kernel, whose lane 4g + t loads P[4(g/2) + 2nt + g%2][4t..4t+3] for
+// N tile nt as one of 32 consecutive 16-byte words; the lo part 256 floats on.
+__host__ __device__ constexpr int p16_at(int a, int d)
+{
+    return ((a >> 1) & 1) * 128 + ((((a >> 2) << 1) | (a & 1)) * 4 + (d >> 2)) * 4 + (d & 3);
+}
 
 __global__ void build_P16_kernel(const double* __restrict__ eig, const double* __restrict__ bl,
                                  const int* __restrict__ nodegrp, int numnodes, int C, float* __restrict__ P)
@@ -82,7 +99,10 @@ __global__ void build_P16_kernel(const double* __restrict__ eig, const double* _
             acc *= R[t];
             out = (acc <= 0.0) ? 0.f : (float)acc;  // absmat clamp (1e-50 rounds to 0 in FP32)
         }
-        P[((size_t)c * numnodes + v) * 256 + t] = out;
+        float* p = P + ((size_t)c * numnodes + v) * kP16Floats + p16_at(a, d);
+        const float hi = tf32_hi(out);
+        p[0] = hi;
+        p[256] = out - hi;
     }
 }
 
@@ -125,8 +145,6 @@ int launch_build_P4(messi_ctx* ctx, const double* d_eig4, const double* d_bl, co
     return MESSI_OK;
 }
 
-__device__ __forceinline__ float4 ldg4(const float* p) { return __ldg(reinterpret_cast<const float4*>(p)); }
-
 __device__ __forceinline__ double lse_d(double a, double b)
 {
     if (b == -INFINITY) return a;
@@ -158,7 +176,7 @@ __global__ void __launch_bounds__(256) leaf_msg_kernel(const float* __restrict__
     const int a = threadIdx.x & 15, cc = blockIdx.y;
     if (r >= R) return;
     (void)C;
-    const float* p = P + ((size_t)(c0 + cc) * numnodes + __ldg(rownode + r)) * 256 + a * 16;
+    const float* p = P + ((size_t)(c0 + cc) * numnodes + __ldg(rownode + r)) * kP16Floats;
     const float4* x4 = reinterpret_cast<const float4*>(rows + r * 16);
     float x[16];
 #pragma unroll
@@ -175,7 +193,7 @@ __global__ void __launch_bounds__(256) leaf_msg_kernel(const float* __restrict__
     double s = 0.0;
 #pragma unroll
     for (int d = 0; d < 16; d++)
-        if (x[d] != 0.f) s += (double)__ldg(p + d) * (double)x[d];
+        if (x[d] != 0.f) s += (double)(__ldg(p + p16_at(a, d)) + __ldg(p + p16_at(a, d) + 256)) * (double)x[d];
     out[((size_t)cc * R + r) * 16 + a] = (float)s;
 }
 
@@ -190,12 +208,12 @@ int launch_leaf_messages(messi_ctx* ctx, const float* d_rows, const int* d_rowno
 }
 
 // ---------------------------------------------------------------------------
-// Tensor-core node update (3xTF32 mma.sync).  A warp owns 32 unique pairs of
-// one node.  For each category it forms x = m_left * m_right for its pairs
-// and, below the root, the product [32 pairs x 16] x [16 x 16]^T with P of
-// the node's own branch, as m16n8k8 TF32 MMAs with both operands split
-// hi + lo (hi*hi + hi*lo + lo*hi: FP32-level accuracy; all operands are
-// non-negative, so there is no cancellation).
+// Tensor-core node update (3xTF32 mma.sync): for 32 pairs of one node and one
+// category x = m_left * m_right and, below the root, the product
+// [32 pairs x 16] x [16 x 16]^T with P of the node's own branch, as m16n8k8
+// TF32 MMAs with both operands split hi + lo (hi*hi + hi*lo + lo*hi:
+// FP32-level accuracy; all operands are non-negative, so there is no
+// cancellation).
 // Rounding.  The tensor core rounds each MMA's FP32 result toward zero
 // (measured on GB300: 99.9% of outputs equal the truncation of the exact
 // sum, mean error -0.44 ulp), so a chain of MMAs loses about half an ulp per
@@ -207,11 +225,8 @@ int launch_leaf_messages(messi_ctx* ctx, const float* d_rows, const int* d_rowno
 // rounded to nearest: a tie, which rounds up or down on the last mantissa
 // bit, so the truncation bias of the two halves is returned on average.
 // The contraction index d is permuted so that lane (g, t) owns
-// d = 4t..4t+3: its A fragment for pair row r is one 16-byte load of each
-// child's row, and its B fragment one 16-byte load of P[8nt + g][4t..4t+3].
-// Lane (g, t) ends with states {2t, 2t+1, 8+2t, 9+2t} of pairs g, g+8,
-// g+16, g+24; lane t keeps the scalar bookkeeping (exponent, mixture) of pair
-// g + 8t.
+// d = 4t..4t+3: its A fragment for pair row r is one 16-byte piece of each
+// message, its B fragment 16 bytes of a row of P (p16_at).
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ float comp4(const float4& v, int k)
 {
@@ -220,69 +235,70 @@ __device__ __forceinline__ float comp4(const float4& v, int k)
 
 __device__ __forceinline__ void mma_tf32(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1)
 {
-    asm volatile(
+    asm(
         "mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
         "{%0,%1,%2,%3};\n"
         : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
         : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
-// A operand split: hi = x rounded to TF32 (adding half a TF32 ulp to the
-// magnitude bits and truncating is round-to-nearest, ties away, the same as
-// cvt.rna for the finite values here) and lo = x - hi (exact in FP32), fed
-// without conversion: the tensor core reads the top 19 bits of lo, an error
-// below 2^-21 |x| of either sign (lo is centred on zero).
+// The first MMA of a chain: the accumulator starts from zero (no registers to clear).
+__device__ __forceinline__ void mma_tf32_zero(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1)
+{
+    asm(
+        "mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
+        "{%10,%10,%10,%10};\n"
+        : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(0.f));
+}
+
+// A operand split: hi, and lo fed without conversion (the tensor core reads
+// the top 19 bits of lo, an error below 2^-21 |x| of either sign, as lo is
+// centred on zero).
 __device__ __forceinline__ void split_a(float x, uint32_t& hi, uint32_t& lo)
 {
-    hi = (__float_as_uint(x) + 0x1000u) & 0xffffe000u;
+    hi = __float_as_uint(tf32_hi(x));
     lo = __float_as_uint(x - __uint_as_float(hi));
 }
 
-// B operand (four entries of P) split the same way, in registers: one FP32
-// load per fragment instead of a hi and a lo load.
-__device__ __forceinline__ void split_b(const float4& p, float4& hi, float4& lo)
-{
-    uint32_t h[4], l[4];
-    split_a(p.x, h[0], l[0]);
-    split_a(p.y, h[1], l[1]);
-    split_a(p.z, h[2], l[2]);
-    split_a(p.w, h[3], l[3]);
-    hi = make_float4(__uint_as_float(h[0]), __uint_as_float(h[1]), __uint_as_float(h[2]), __uint_as_float(h[3]));
-    lo = make_float4(__uint_as_float(l[0]), __uint_as_float(l[1]), __uint_as_float(l[2]), __uint_as_float(l[3]));
-}
-
 // v + half an ulp of v, rounded to nearest (ties to even): v or v + ulp,
-// each for half of the mantissas.  v >= 0.
+// each for half of the mantissas.  v >= 0.  The exponent bits alone are the
+// power of two 2^e of v, so half an ulp is 2^e * 2^-24 (exact) and one FMA adds it.
 __device__ __forceinline__ float add_half_ulp(float v)
 {
-    const int e = (int)(__float_as_uint(v) & 0x7f800000u) - (24 << 23);
-    return v + __int_as_float(max(e, 0));
+    return fmaf(__uint_as_float(__float_as_uint(v) & 0x7f800000u), 5.9604644775390625e-8f, v);
 }
 
-// D0[mt][nt] += X x P^T over states k-step 0 (d = 4t, 4t+1), D1 over k-step 1
+// D0[mt][nt] = X x P^T over states k-step 0 (d = 4t, 4t+1), D1 over k-step 1
 // (d = 4t+2, 4t+3), each as lo*hi + hi*lo + hi*hi, for rows g + 8k (k = 0..3).
 __device__ __forceinline__ void msg_mma(const float4 (&X)[4], const float4 (&Bh)[2], const float4 (&Bl)[2],
                                         float (&D0)[2][2][4], float (&D1)[2][2][4])
 {
+    // The three products of an accumulator depend on one another: the four
+    // accumulators of a row half take turns, so that a product does not wait
+    // for the one before it.
 #pragma unroll
     for (int mt = 0; mt < 2; mt++) {
+        uint32_t ah[2][4], al[2][4];
 #pragma unroll
         for (int ks = 0; ks < 2; ks++) {
             const float av[4] = {comp4(X[2 * mt], 2 * ks), comp4(X[2 * mt + 1], 2 * ks), comp4(X[2 * mt], 2 * ks + 1),
                                  comp4(X[2 * mt + 1], 2 * ks + 1)};
-            uint32_t ah[4], al[4];
 #pragma unroll
-            for (int i = 0; i < 4; i++) split_a(av[i], ah[i], al[i]);
-#pragma unroll
-            for (int nt = 0; nt < 2; nt++) {
-                const uint32_t bh0 = __float_as_uint(comp4(Bh[nt], 2 * ks)), bh1 = __float_as_uint(comp4(Bh[nt], 2 * ks + 1));
-                const uint32_t bl0 = __float_as_uint(comp4(Bl[nt], 2 * ks)), bl1 = __float_as_uint(comp4(Bl[nt], 2 * ks + 1));
-                float (&D)[4] = ks ? D1[mt][nt] : D0[mt][nt];
-                mma_tf32(D, al, bh0, bh1);
-                mma_tf32(D, ah, bl0, bl1);
-                mma_tf32(D, ah, bh0, bh1);
-            }
+            for (int i = 0; i < 4; i++) split_a(av[i], ah[ks][i], al[ks][i]);
         }
+#pragma unroll
+        for (int term = 0; term < 3; term++)
+#pragma unroll
+            for (int ks = 0; ks < 2; ks++)
+#pragma unroll
+                for (int nt = 0; nt < 2; nt++) {
+                    float (&D)[4] = ks ? D1[mt][nt] : D0[mt][nt];
+                    const float4& B = (term == 1) ? Bl[nt] : Bh[nt];
+                    const uint32_t b0 = __float_as_uint(comp4(B, 2 * ks)), b1 = __float_as_uint(comp4(B, 2 * ks + 1));
+                    if (term == 0) mma_tf32_zero(D, al[ks], b0, b1);
+                    else mma_tf32(D, ah[ks], b0, b1);
+                }
     }
 }
 
@@ -320,188 +336,301 @@ __device__ __forceinline__ void pow2_scale(float m, int& ex, float& sc)
     }
 }
 
-// Pipeline shapes: STAGES categories in flight per warp (cp.async), MINB CTAs
-// of kTile = 128 threads per SM.  The default, 2 stages x 4 CTAs (16 warps,
-// 136 KB of stages per SM), leaves ~90 KB of the SM's L1 to cache the
-// gathered child rows, which parent pairs share heavily.
-
-// Per-warp staging of one category: 8 float4 per lane (child rows) + 2 exponents.
-struct WarpStage {
-    float4 x[8][32];
-    int e[2][32];
+// ---------------------------------------------------------------------------
+// Segment programs.  A warp owns 32 unique pairs (NP = 1, or 64: NP = 2) of a
+// segment's top node and, category by category, runs the segment's program on
+// them: the running message M stays in registers from node to node, so of a
+// node's two child rows only the one that comes from a table below is read
+// and nothing is written but the segment's last message.  (One launch per tree
+// level, every node's rows written and gathered again, moved 212 bytes per
+// update and was bound by the L1 data pipe, 71% of its wavefronts.)
+// Each step gathers one row per pair: the four lanes (g, t) of a pair read
+// 16 bytes each, straight to registers, and the rows of the next step are
+// asked for as soon as this step's are consumed, so they arrive under the
+// mat-vec (without that, 24 warps per SM instead of 20: 15% slower).  The
+// columns of P are assigned to the MMA's N index so that lane (g, t) ends with
+// states 4t..4t+3 of its pairs, which is the A layout of the next product:
+// column g of tile nt is state 4(g/2) + 2nt + g%2.
+// Measured (GB300, 64 x 1,000 columns, span 500, 36 categories): 2.96e8
+// distinct updates in 7.5 ms before; 3.6e8 (some recomputed) in 5.72 ms now,
+// DRAM traffic 35 GB -> ~7 GB.  What bounds it: about 300 instructions per 32
+// updates at 55% of the issue slots (HMMA busy 29%, L1 35%), i.e. the latency
+// of a step's dependent chain with the 16-20 warps the registers allow.
+// The CTA's warps are pg pair groups x cs category splits: with few pairs the
+// warps of one pair group take every cs-th category each (a level of 50
+// tiles of 128 pairs with all 36 categories in turn took 45 us).
+// ROOT: 0 = interior segment, 1 = the tree's root with the category mixture
+// kept in registers (cs = 1), 2 = the root with the categories' values
+// collected in shared memory and mixed afterwards in category order by one
+// warp, so that the sum has the same bits.
+// ---------------------------------------------------------------------------
+struct Mixture {
+    double m = -INFINITY;
+    float s = 0.f;
+    __device__ __forceinline__ void add(double tt)
+    {
+        if (tt > m) {
+            s = s * __expf((float)(m - tt)) + 1.f;
+            m = tt;
+        } else if (tt != -INFINITY) {
+            s += __expf((float)(tt - m));
+        }
+    }
+    __device__ __forceinline__ double value() const { return (m == -INFINITY) ? -INFINITY : m + log((double)s); }
 };
 
-template <bool ROOT, int STAGES, int MINB>
-__global__ void __launch_bounds__(kTile, MINB) prune_msg_kernel(
-    const NodeDev* __restrict__ nodes, const int2* __restrict__ tiles, const float* __restrict__ P, int numnodes,
+// Lane t's own one of four values (pair g + 8t).
+__device__ __forceinline__ int own4(const int4& v, int t) { return t == 0 ? v.x : (t == 1 ? v.y : (t == 2 ? v.z : v.w)); }
+
+// Reduces v[k] over the four lanes t of a pair; lane t keeps pair k = t: two
+// exchanges of halves instead of a butterfly per pair (three shuffles, not eight).
+template <typename Op>
+__device__ __forceinline__ float quad_reduce(const float (&v)[4], int t, Op op)
+{
+    const bool o1 = t & 1, o2 = t & 2;
+    const float a = op(o1 ? v[1] : v[0], __shfl_xor_sync(0xffffffffu, o1 ? v[0] : v[1], 1));
+    const float b = op(o1 ? v[3] : v[2], __shfl_xor_sync(0xffffffffu, o1 ? v[2] : v[3], 1));
+    return op(o2 ? b : a, __shfl_xor_sync(0xffffffffu, o2 ? a : b, 2));
+}
+
+__device__ __forceinline__ float4 mul4(const float4& a, const float4& b)
+{
+    return make_float4(__fmul_rn(a.x, b.x), __fmul_rn(a.y, b.y), __fmul_rn(a.z, b.z), __fmul_rn(a.w, b.w));
+}
+__device__ __forceinline__ float max4(const float4& v) { return fmaxf(fmaxf(v.x, v.y), fmaxf(v.z, v.w)); }
+
+template <int ROOT, int NP, int MAXT, int MINB>
+__global__ void __launch_bounds__(MAXT, MINB) prune_path_kernel(
+    const SegDev* __restrict__ segs, const int2* __restrict__ tiles, const float* __restrict__ P, int numnodes,
     int c0, int nc, int C, const float* __restrict__ pi16, const double* __restrict__ logw,
-    const int* __restrict__ lam, int per_lambda)
+    const int* __restrict__ lam, int per_lambda, int cs, int max_steps, int max_nb, int max_depth)
 {
     extern __shared__ float4 smem_raw[];
     const int2 tile = tiles[blockIdx.x];
-    const NodeDev& nd = nodes[tile.x];
-    const int n = nd.n;
+    const SegDev& sg = segs[tile.x];
+    const int n = sg.n, ns = sg.nsteps, nb = sg.nb;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int g = lane >> 2, t = lane & 3;
-    const int base = tile.y + warp * 32;  // first pair of this warp
-    if (base >= n) return;                // whole warp idle (warp-uniform)
-    WarpStage* stage = reinterpret_cast<WarpStage*>(smem_raw) + (size_t)warp * STAGES;
-    // child rows of pairs g + 8k (clamped to a valid row past the end)
-    int li[4], ri[4];
+    const int pgs = (int)(blockDim.x >> 5) / cs, pg = warp % pgs, split = warp / pgs;
+    const int base = tile.y + 32 * NP * pg;  // first pair of this warp
+    const bool active = base < n;
+    // shared memory: program, gather indices per pair group, set-aside messages per warp, collected values
+    int4* steps = reinterpret_cast<int4*>(smem_raw);
+    int4* sidx = steps + max_steps + pg * max_nb * 8 * NP;
+    float4* stack = smem_raw + max_steps + pgs * max_nb * 8 * NP + warp * max_depth * 128 * NP + lane;
+    double* collected = reinterpret_cast<double*>(smem_raw + max_steps + pgs * max_nb * 8 * NP +
+                                                  (int)(blockDim.x >> 5) * max_depth * 128 * NP);
+    for (int i = threadIdx.x; i < ns; i += blockDim.x) steps[i] = __ldg(reinterpret_cast<const int4*>(sg.steps) + i);
+    if (active) {
 #pragma unroll
-    for (int k = 0; k < 4; k++) {
-        const int u = base + g + 8 * k;
-        const int uc = (u < n) ? u : (n - 1);
-        li[k] = __ldg(nd.li + uc);
-        ri[k] = __ldg(nd.ri + uc);
-    }
-    const int myu = base + g + 8 * t;  // pair whose scalars this lane keeps
-    const bool myvalid = myu < n;
-    const int myl = li[0] * (t == 0) + li[1] * (t == 1) + li[2] * (t == 2) + li[3] * (t == 3);
-    const int myr = ri[0] * (t == 0) + ri[1] * (t == 1) + ri[2] * (t == 2) + ri[3] * (t == 3);
-    const float* lf = nd.lf;
-    const float* rf = nd.rf;
-    const int* le = nd.le;
-    const int* re = nd.re;
-    const long long lcs = nd.lcs, rcs = nd.rcs;
-    // issue the copies of category cc into its stage (each lane copies what it later reads)
-    auto issue = [&](int cc) {
-        WarpStage& st = stage[cc % STAGES];
-#pragma unroll
-        for (int k = 0; k < 4; k++) {
-            cp_async16(&st.x[k][lane], lf + ((size_t)cc * lcs + li[k]) * 16 + 4 * t);
-            cp_async16(&st.x[4 + k][lane], rf + ((size_t)cc * rcs + ri[k]) * 16 + 4 * t);
+        for (int h = 0; h < NP; h++) {  // (past the last pair the last tile again)
+            const int4* src = reinterpret_cast<const int4*>(sg.idx) + (size_t)min((base >> 5) + h, (n - 1) >> 5) * nb * 8;
+            for (int i = split * 32 + lane; i < nb * 8; i += 32 * cs) sidx[h * max_nb * 8 + i] = __ldg(src + i);
         }
-        if (le) cp_async4(&st.e[0][lane], le + (size_t)cc * lcs + myl);
-        if (re) cp_async4(&st.e[1][lane], re + (size_t)cc * rcs + myr);
-    };
-#pragma unroll
-    for (int s0 = 0; s0 < STAGES - 1; s0++) {
-        if (s0 < nc) issue(s0);
-        cp_async_commit();
     }
-    double mm = -INFINITY;
-    float ss = 0.f;
-    double lm[kMaxLambda];
-    float ls[kMaxLambda];
-    if (ROOT) {
+    __syncthreads();
+    const int myu = base + g + 8 * t;  // pair whose scalars this lane keeps (and myu + 32)
+    Mixture mix[NP];
+    if (active && split < nc) {
+        float4 M[NP][4], R[NP][4];
+        int e[NP], er[NP];
+        const float4* rows = reinterpret_cast<const float4*>(sg.rows) + t;
+        const int* exps = sg.exps;
+        // The rows of step st's table for category cc: states 4t..4t+3 of pairs g + 8k.
+        auto gather = [&](const int4& st, int cc) {
+            const unsigned row = (unsigned)st.x + (unsigned)cc * (unsigned)st.y;
+            const float4* f = rows + (size_t)row * 4;
+            const int slot = (st.w >> kStepSlotShift) * 8 + g;
 #pragma unroll
-        for (int q = 0; q < kMaxLambda; q++) { lm[q] = -INFINITY; ls[q] = 0.f; }
-    }
-    for (int cc = 0; cc < nc; cc++) {
-        if (cc + STAGES - 1 < nc) issue(cc + STAGES - 1);
-        cp_async_commit();
-        cp_async_wait<STAGES - 1>();
-        const WarpStage& st = stage[cc % STAGES];
-        // x = m_left * m_right: states 4t..4t+3 of pairs g + 8k
-        float4 X[4];
-#pragma unroll
-        for (int k = 0; k < 4; k++) {
-            const float4 a = st.x[k][lane], b = st.x[4 + k][lane];
-            X[k] = make_float4(a.x * b.x, a.y * b.y, a.z * b.z, a.w * b.w);
-        }
-        const int e = (le ? st.e[0][lane] : 0) + (re ? st.e[1][lane] : 0);
-        if (ROOT) {
-            const float4 pc = __ldg(reinterpret_cast<const float4*>(pi16 + ((size_t)nd.grp * C + c0 + cc) * 16) + t);
-            float dots[4];
-#pragma unroll
-            for (int k = 0; k < 4; k++) {
-                float dk = pc.x * X[k].x + pc.y * X[k].y + pc.z * X[k].z + pc.w * X[k].w;
-                dk += __shfl_xor_sync(0xffffffffu, dk, 1);
-                dk += __shfl_xor_sync(0xffffffffu, dk, 2);
-                dots[k] = dk;
+            for (int h = 0; h < NP; h++) {
+                const int4 id = sidx[h * max_nb * 8 + slot];
+                R[h][0] = __ldg(f + (size_t)(unsigned)id.x * 4);
+                R[h][1] = __ldg(f + (size_t)(unsigned)id.y * 4);
+                R[h][2] = __ldg(f + (size_t)(unsigned)id.z * 4);
+                R[h][3] = __ldg(f + (size_t)(unsigned)id.w * 4);
+                er[h] = (st.w & kStepLeaf) ? 0 : __ldg(exps + row + (unsigned)own4(id, t));
             }
-            const float dot = dots[0] * (t == 0) + dots[1] * (t == 1) + dots[2] * (t == 2) + dots[3] * (t == 3);
-            const double ll = (dot > 0.f) ? (double)logf(dot) + (double)e * 0.69314718055994530942 : -INFINITY;
-            if (nd.catll && myvalid) nd.catll[(size_t)(c0 + cc) * n + myu] = ll;
-            const double tt = __ldg(logw + (size_t)nd.grp * C + c0 + cc) + ll;
-            if (tt > mm) {
-                ss = ss * __expf((float)(mm - tt)) + 1.f;
-                mm = tt;
-            } else if (tt != -INFINITY) {
-                ss += __expf((float)(tt - mm));
-            }
-            if (per_lambda) {
-                const int kq = __ldg(lam + c0 + cc);
+        };
+        int4 st = steps[0];
+        gather(st, split);
+        for (int cc = split; cc < nc; cc += cs) {
+            const float4* Pc = reinterpret_cast<const float4*>(P + (size_t)(c0 + cc) * numnodes * kP16Floats) + lane;
 #pragma unroll
-                for (int q = 0; q < kMaxLambda; q++)
-                    if (q == kq) {
-                        if (tt > lm[q]) {
-                            ls[q] = ls[q] * __expf((float)(lm[q] - tt)) + 1.f;
-                            lm[q] = tt;
-                        } else if (tt != -INFINITY) {
-                            ls[q] += __expf((float)(tt - lm[q]));
-                        }
+            for (int h = 0; h < NP; h++) e[h] = 0;
+            float4* top = stack;
+            for (int s = 0; s < ns; s++) {
+                const int fl = st.w;
+                const float4* pv = Pc + (size_t)(unsigned)st.z * (kP16Floats / 4);
+                // the next step (the program's first for the next category)
+                const bool last = s + 1 == ns;
+                st = steps[last ? 0 : s + 1];
+                if (fl & kStepInit) {
+#pragma unroll
+                    for (int h = 0; h < NP; h++) {
+#pragma unroll
+                        for (int k = 0; k < 4; k++) M[h][k] = R[h][k];
+                        e[h] += er[h];
                     }
-            }
-        } else {
-            // m_v = P_v x (the node's own branch), then an exact power-of-two rescale
-            const float* pv = P + ((size_t)(c0 + cc) * numnodes + nd.self) * 256;
-            float4 Bh[2], Bl[2];
+                    gather(st, cc);
+                    continue;
+                }
+                float4 Bh[2], Bl[2];
+                if (!ROOT || !(fl & kStepRoot)) {
+                    Bh[0] = __ldg(pv);
+                    Bh[1] = __ldg(pv + 32);
+                    Bl[0] = __ldg(pv + 64);
+                    Bl[1] = __ldg(pv + 96);
+                }
+                // x = product of the two messages: states 4t..4t+3 of pairs g + 8k
+                if (fl & kStepPop) {
+                    top -= 128 * NP;
 #pragma unroll
-            for (int nt = 0; nt < 2; nt++) split_b(ldg4(pv + (8 * nt + g) * 16 + 4 * t), Bh[nt], Bl[nt]);
-            float D0[2][2][4], D1[2][2][4];
+                    for (int h = 0; h < NP; h++)
 #pragma unroll
-            for (int mt = 0; mt < 2; mt++)
+                        for (int k = 0; k < 4; k++) M[h][k] = mul4(M[h][k], top[128 * h + 32 * k]);
+                } else {
 #pragma unroll
-                for (int nt = 0; nt < 2; nt++)
+                    for (int h = 0; h < NP; h++) {
 #pragma unroll
-                    for (int i = 0; i < 4; i++) { D0[mt][nt][i] = 0.f; D1[mt][nt][i] = 0.f; }
-            msg_mma(X, Bh, Bl, D0, D1);
-            // V[k][j]: pair g + 8k, states {2t, 2t+1, 8+2t, 9+2t}; the two
-            // k-step halves added, then their truncation returned on average
-            float V[4][4];
+                        for (int k = 0; k < 4; k++) M[h][k] = mul4(M[h][k], R[h][k]);
+                        e[h] += er[h];
+                    }
+                }
+                // the next gathered rows arrive under this step's mat-vec
+                if ((st.w & kStepGather) && (!last || cc + cs < nc)) gather(st, last ? cc + cs : cc);
+                if (ROOT && (fl & kStepRoot)) {
+                    const float4 pc = __ldg(reinterpret_cast<const float4*>(pi16 + ((size_t)sg.grp * C + c0 + cc) * 16) + t);
 #pragma unroll
-            for (int k = 0; k < 4; k++) {
-                const int mt = k >> 1, h = k & 1;
-                V[k][0] = add_half_ulp(D0[mt][0][2 * h] + D1[mt][0][2 * h]);
-                V[k][1] = add_half_ulp(D0[mt][0][2 * h + 1] + D1[mt][0][2 * h + 1]);
-                V[k][2] = add_half_ulp(D0[mt][1][2 * h] + D1[mt][1][2 * h]);
-                V[k][3] = add_half_ulp(D0[mt][1][2 * h + 1] + D1[mt][1][2 * h + 1]);
-            }
-            int exk[4];
+                    for (int h = 0; h < NP; h++) {
+                        float d[4];
 #pragma unroll
-            for (int k = 0; k < 4; k++) {
-                float m = fmaxf(fmaxf(V[k][0], V[k][1]), fmaxf(V[k][2], V[k][3]));
-                m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 1));
-                m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 2));
-                int ex;
-                float sc;
-                pow2_scale(m, ex, sc);
-                exk[k] = ex;
-                const int u = base + g + 8 * k;
-                if (u < n) {
-                    float* o = nd.of + ((size_t)cc * nd.ocs + u) * 16;
-                    *reinterpret_cast<float2*>(o + 2 * t) = make_float2(V[k][0] * sc, V[k][1] * sc);
-                    *reinterpret_cast<float2*>(o + 8 + 2 * t) = make_float2(V[k][2] * sc, V[k][3] * sc);
+                        for (int k = 0; k < 4; k++)
+                            d[k] = pc.x * M[h][k].x + pc.y * M[h][k].y + pc.z * M[h][k].z + pc.w * M[h][k].w;
+                        const float dot = quad_reduce(d, t, [](float a, float b) { return a + b; });
+                        const double ll = (dot > 0.f) ? (double)logf(dot) + (double)e[h] * 0.69314718055994530942 : -INFINITY;
+                        if (sg.catll && myu + 32 * h < n) sg.catll[(size_t)(c0 + cc) * n + myu + 32 * h] = ll;
+                        const double tt = __ldg(logw + (size_t)sg.grp * C + c0 + cc) + ll;
+                        if (ROOT == 1) mix[h].add(tt);
+                        else collected[((pg * NP + h) * nc + cc) * 32 + lane] = tt;
+                    }
+                    continue;
+                }
+                // m_v = P_v x (the node's own branch)
+#pragma unroll
+                for (int h = 0; h < NP; h++) {
+                    float D0[2][2][4], D1[2][2][4];
+                    msg_mma(M[h], Bh, Bl, D0, D1);
+                    // pair g + 8k, states 4t..4t+3; the two k-step halves
+                    // added, then their truncation returned on average
+                    float mx[4];
+#pragma unroll
+                    for (int k = 0; k < 4; k++) {
+                        const int mt = k >> 1, o = 2 * (k & 1);
+                        M[h][k].x = add_half_ulp(D0[mt][0][o] + D1[mt][0][o]);
+                        M[h][k].y = add_half_ulp(D0[mt][0][o + 1] + D1[mt][0][o + 1]);
+                        M[h][k].z = add_half_ulp(D0[mt][1][o] + D1[mt][1][o]);
+                        M[h][k].w = add_half_ulp(D0[mt][1][o + 1] + D1[mt][1][o + 1]);
+                        mx[k] = max4(M[h][k]);
+                    }
+                    // Exact power-of-two rescale by the pair's largest state m to
+                    // [0.5, 1): 2^(126 - E), E the exponent field of m (E = 0, a
+                    // zero or denormal m, scales by 2^126, which is exact too).
+                    const unsigned mb = __float_as_uint(quad_reduce(mx, t, [](float a, float b) { return fmaxf(a, b); }));
+                    e[h] += (int)(mb >> 23) - 126;
+                    const float sc = __uint_as_float((253u << 23) - (mb & 0x7f800000u));
+#pragma unroll
+                    for (int k = 0; k < 4; k++) {
+                        const float sk = __shfl_sync(0xffffffffu, sc, (lane & 28) + k);
+                        M[h][k] = mul4(M[h][k], make_float4(sk, sk, sk, sk));
+                    }
+                }
+                if (fl & kStepPush) {
+#pragma unroll
+                    for (int h = 0; h < NP; h++)
+#pragma unroll
+                        for (int k = 0; k < 4; k++) top[128 * h + 32 * k] = M[h][k];
+                    top += 128 * NP;
                 }
             }
-            if (myvalid) {
-                const int ex = exk[0] * (t == 0) + exk[1] * (t == 1) + exk[2] * (t == 2) + exk[3] * (t == 3);
-                nd.oe[(size_t)cc * nd.ocs + myu] = e + ex;
-            }
-        }
-    }
-    cp_async_wait<0>();
-    if (ROOT && myvalid) {
-        const double res = (mm == -INFINITY) ? -INFINITY : mm + log((double)ss);
-        nd.mix[myu] = (c0 == 0) ? res : lse_d(nd.mix[myu], res);
-        if (per_lambda) {
+            if (!ROOT) {
 #pragma unroll
-            for (int q = 0; q < kMaxLambda; q++) {
-                const double rq = (lm[q] == -INFINITY) ? -INFINITY : lm[q] + log((double)ls[q]);
-                double* dst = nd.mixlam + (size_t)q * n + myu;
-                *dst = (c0 == 0) ? rq : lse_d(*dst, rq);
+                for (int h = 0; h < NP; h++) {
+                    const int u0 = base + 32 * h + g;
+                    const unsigned ob = sg.out + (unsigned)cc * sg.ocs;
+                    float4* o = reinterpret_cast<float4*>(sg.rows) + ((size_t)ob + u0) * 4 + t;
+#pragma unroll
+                    for (int k = 0; k < 4; k++)
+                        if (u0 + 8 * k < n) o[32 * k] = M[h][k];
+                    if (myu + 32 * h < n) sg.exps[(size_t)ob + myu + 32 * h] = e[h];
+                }
             }
         }
     }
+    if (ROOT == 2) {
+        __syncthreads();
+        if (split != 0 || !active) return;
+#pragma unroll
+        for (int h = 0; h < NP; h++)
+            for (int cc = 0; cc < nc; cc++) mix[h].add(collected[((pg * NP + h) * nc + cc) * 32 + lane]);
+    }
+    if (ROOT && active) {
+#pragma unroll
+        for (int h = 0; h < NP; h++) {
+            const int u = myu + 32 * h;
+            if (u >= n) continue;
+            const double res = mix[h].value();
+            sg.mix[u] = (c0 == 0) ? res : lse_d(sg.mix[u], res);
+            if (ROOT == 2 && per_lambda) {
+                for (int q = 0; q < kMaxLambda; q++) {
+                    Mixture ml;
+                    for (int cc = 0; cc < nc; cc++)
+                        if (__ldg(lam + c0 + cc) == q) ml.add(collected[((pg * NP + h) * nc + cc) * 32 + lane]);
+                    const double rq = ml.value();
+                    double* dst = sg.mixlam + (size_t)q * n + u;
+                    *dst = (c0 == 0) ? rq : lse_d(*dst, rq);
+                }
+            }
+        }
+    }
+}
+
+// Gather indices of a segment from the per-node child lists: position p of a
+// 32-pair tile holds pair g + 8k at p = 4g + k (the last pair repeated past
+// the end).  One thread per position follows the lists from the top node down.
+__global__ void __launch_bounds__(256) segment_idx_kernel(const IdxSeg* __restrict__ segs, const IdxOp* __restrict__ ops,
+                                                          int seg0, const int* __restrict__ lr, int* __restrict__ idx)
+{
+    const IdxSeg sg = segs[seg0 + blockIdx.y];
+    const long long pos = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const long long tile = pos >> 5;
+    if (tile * 32 >= sg.n) return;
+    const int p = (int)(pos & 31);
+    const int u = min((int)tile * 32 + (p >> 2) + 8 * (p & 3), sg.n - 1);
+    int row[kSegMaxNodes];
+    row[0] = u;
+    int* out = idx + sg.out + tile * sg.nb * 32 + p;
+    for (int o = sg.op0; o < sg.op1; o++) {
+        const IdxOp op = ops[o];
+        const int r = __ldg(lr + op.list + row[op.src]);
+        if (op.dst >= 0) row[op.dst] = r;
+        else out[(size_t)(~op.dst) * 32] = r;
+    }
+}
+
+int launch_segment_indices(const IdxSeg* d_segs, const IdxOp* d_ops, int nseg, int64_t maxn, const int* d_lr, int* d_idx)
+{
+    if (maxn <= 0) return MESSI_OK;
+    const unsigned gx = (unsigned)(((maxn + 31) / 32 * 32 + 255) / 256);
+    for (int s = 0; s < nseg; s += 65535)
+        segment_idx_kernel<<<dim3(gx, std::min(nseg - s, 65535)), 256>>>(d_segs, d_ops, s, d_lr, d_idx);
+    return cudaPeekAtLastError() == cudaSuccess ? MESSI_OK : MESSI_ECUDA;
 }
 
 // ---------------------------------------------------------------------------
 // tcgen05 form of the interior node update (launch shape 3, chosen only on
 // request: MESSI_PRUNE_SHAPE=3).  The CTA's 128 unique pairs of one node are
 // the M = 128 rows of one tcgen05.mma (kind::tf32, N = 16 states, K = 8):
-//   * the child rows are gathered with cp.async as in prune_msg_kernel, into
+//   * the child rows are gathered with cp.async into
 //     a stage of whole rows with XOR-ordered quads (Stage), so that both the
 //     gathers and thread p's reads of pair p's rows are free of bank
 //     conflicts;
@@ -515,10 +644,10 @@ __global__ void __launch_bounds__(kTile, MINB) prune_msg_kernel(
 //     256 bytes apart (LBO);
 //   * one thread issues, per K half, lo*hi, hi*lo, hi*hi into that half's
 //     own accumulator (TMEM columns 32..47 and 48..63), the same split and
-//     order as prune_msg_kernel (K half 0 = states {0,1,4,5,8,9,12,13}), and
+//     order as prune_path_kernel (K half 0 = states {0,1,4,5,8,9,12,13}), and
 //     commits them to an mbarrier;
 //   * thread p reads its pair's 2 x 16 accumulators back (tcgen05.ld), adds
-//     the halves and half an ulp as prune_msg_kernel does, rescales by a power
+//     the halves and half an ulp as prune_path_kernel does, rescales by a power
 //     of two and stores the row -- one category late: the MMAs of category c
 //     run while the CTA waits for and multiplies the rows of category c + 1,
 //     and P is loaded one category ahead.
@@ -646,14 +775,16 @@ __device__ __forceinline__ bool mbar_wait(unsigned addr, unsigned parity)
 }
 }  // namespace tc
 
-__global__ void __launch_bounds__(kTile, 6) prune_tc_kernel(const NodeDev* __restrict__ nodes,
+__global__ void __launch_bounds__(kTile, 6) prune_tc_kernel(const SegDev* __restrict__ segs,
                                                            const int2* __restrict__ tiles,
                                                            const float* __restrict__ P, int numnodes, int c0, int nc)
 {
     extern __shared__ float4 smem_raw[];
     tc::Smem& S = *reinterpret_cast<tc::Smem*>(smem_raw);
     const int2 tile = tiles[blockIdx.x];
-    const NodeDev& nd = nodes[tile.x];
+    const SegDev& nd = segs[tile.x];  // one node: its program is the two gathered children
+    const StepDev sl = nd.steps[0], sr = nd.steps[1];
+    const int self = sr.self;
     const int n = nd.n;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int g = lane >> 2, t = lane & 3;
@@ -678,21 +809,15 @@ __global__ void __launch_bounds__(kTile, 6) prune_tc_kernel(const NodeDev* __res
 
     // gathers: lane (g, t) copies state quad t of pairs g + 8k of its warp
     const int wbase = 32 * warp;
-    int li[4], ri[4];
-#pragma unroll
-    for (int k = 0; k < 4; k++) {
-        const int u = tile.y + wbase + g + 8 * k;
-        const int uc = (u < n) ? u : (n - 1);
-        li[k] = __ldg(nd.li + uc);
-        ri[k] = __ldg(nd.ri + uc);
-    }
-    const int myl = li[0] * (t == 0) + li[1] * (t == 1) + li[2] * (t == 2) + li[3] * (t == 3);
-    const int myr = ri[0] * (t == 0) + ri[1] * (t == 1) + ri[2] * (t == 2) + ri[3] * (t == 3);
-    const float* lf = nd.lf;
-    const float* rf = nd.rf;
-    const int* le = nd.le;
-    const int* re = nd.re;
-    const long long lcs = nd.lcs, rcs = nd.rcs;
+    const int4* src = reinterpret_cast<const int4*>(nd.idx) + (size_t)min((tile.y >> 5) + warp, (n - 1) >> 5) * 16 + g;
+    const int4 l4 = __ldg(src), r4 = __ldg(src + 8);
+    const int li[4] = {l4.x, l4.y, l4.z, l4.w}, ri[4] = {r4.x, r4.y, r4.z, r4.w};
+    const int myl = own4(l4, t), myr = own4(r4, t);
+    const float* lf = nd.rows + (size_t)sl.row * 16;
+    const float* rf = nd.rows + (size_t)sr.row * 16;
+    const int* le = (sl.flags & kStepLeaf) ? nullptr : nd.exps + sl.row;
+    const int* re = (sr.flags & kStepLeaf) ? nullptr : nd.exps + sr.row;
+    const long long lcs = sl.cs, rcs = sr.cs;
     auto issue = [&](int cc) {
         tc::Stage& st = S.st[cc % tc::kStages];
 #pragma unroll
@@ -717,8 +842,9 @@ __global__ void __launch_bounds__(kTile, 6) prune_tc_kernel(const NodeDev* __res
     const int bo = 2 * tid;
     const int pi_ = tc::brow(bo), pd = tc::bstate(bo);
     auto pload = [&](int cc) {
-        return __ldg(reinterpret_cast<const float2*>(P + ((size_t)(c0 + cc) * numnodes + nd.self) * 256 + pi_ * 16 +
-                                                     pd));
+        const float* p = P + ((size_t)(c0 + cc) * numnodes + self) * kP16Floats + p16_at(pi_, pd);
+        const float2 h = __ldg(reinterpret_cast<const float2*>(p)), l = __ldg(reinterpret_cast<const float2*>(p + 256));
+        return make_float2(h.x + l.x, h.y + l.y);
     };
     // category cf's accumulators back from TMEM (its MMAs ran while the next
     // category's rows were read), rescaled and stored with exponent ef
@@ -747,7 +873,7 @@ __global__ void __launch_bounds__(kTile, 6) prune_tc_kernel(const NodeDev* __res
         pow2_scale(m, ex, sc);
         if (myvalid) {
             // the row as two 32-byte stores: whole sectors
-            float* o = nd.of + ((size_t)cf * nd.ocs + myu) * 16;
+            float* o = nd.rows + ((size_t)nd.out + (size_t)cf * nd.ocs + myu) * 16;
 #pragma unroll
             for (int h = 0; h < 2; h++)
                 asm volatile("st.global.v8.f32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};\n" ::"l"(o + 8 * h),
@@ -755,7 +881,7 @@ __global__ void __launch_bounds__(kTile, 6) prune_tc_kernel(const NodeDev* __res
                              "f"(V[8 * h + 3] * sc), "f"(V[8 * h + 4] * sc), "f"(V[8 * h + 5] * sc),
                              "f"(V[8 * h + 6] * sc), "f"(V[8 * h + 7] * sc)
                              : "memory");
-            nd.oe[(size_t)cf * nd.ocs + myu] = ef + ex;
+            nd.exps[(size_t)nd.out + (size_t)cf * nd.ocs + myu] = ef + ex;
         }
     };
     float2 ppn = (nc > 0) ? pload(0) : make_float2(0.f, 0.f);
@@ -828,78 +954,83 @@ __global__ void __launch_bounds__(kTile, 6) prune_tc_kernel(const NodeDev* __res
     }
 }
 
-static int launch_prune_tc(messi_ctx* ctx, const NodeDev* d_nodes, const int2* d_tiles, int nt, const float* d_P,
+static int launch_prune_tc(messi_ctx* ctx, const SegDev* d_segs, const int2* d_tiles, int nt, const float* d_P,
                            int numnodes, int c0, int nc)
 {
-    prune_tc_kernel<<<nt, kTile, sizeof(tc::Smem), ctx->stream>>>(d_nodes, d_tiles, d_P, numnodes, c0, nc);
+    prune_tc_kernel<<<nt, kTile, sizeof(tc::Smem), ctx->stream>>>(d_segs, d_tiles, d_P, numnodes, c0, nc);
     LAUNCH_CHECK(ctx, "prune_tc_kernel");
     return MESSI_OK;
 }
 
-template <int STAGES, int MINB>
-static int launch_prune_shape(messi_ctx* ctx, const NodeDev* d_nodes, const int2* d_tiles, int nt, bool root,
-                              const float* d_P, int numnodes, int c0, int nc, int C, const float* d_pi16,
-                              const double* d_logw, const int* d_lam, bool per_lambda)
-{
-    static thread_local int smem_set_device = -1;
-    const size_t smem = (size_t)(kTile / 32) * STAGES * sizeof(WarpStage);
-    if (smem_set_device != ctx->device) {
-        cudaFuncSetAttribute(prune_msg_kernel<false, STAGES, MINB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)smem);
-        cudaFuncSetAttribute(prune_msg_kernel<true, STAGES, MINB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)smem);
-        smem_set_device = ctx->device;
-    }
-    if (root) {
-        prune_msg_kernel<true, STAGES, MINB><<<nt, kTile, smem, ctx->stream>>>(
-            d_nodes, d_tiles, d_P, numnodes, c0, nc, C, d_pi16, d_logw, d_lam, per_lambda ? 1 : 0);
-        LAUNCH_CHECK(ctx, "prune_msg_kernel<root>");
-    } else {
-        prune_msg_kernel<false, STAGES, MINB><<<nt, kTile, smem, ctx->stream>>>(
-            d_nodes, d_tiles, d_P, numnodes, c0, nc, C, d_pi16, d_logw, d_lam, per_lambda ? 1 : 0);
-        LAUNCH_CHECK(ctx, "prune_msg_kernel");
-    }
-    return MESSI_OK;
-}
-
-int launch_prune_tiles(messi_ctx* ctx, const NodeDev* d_nodes, const int2* d_tiles, int nt, bool root,
+// pgs: pair groups of 32 * NP pairs per CTA (the level's tiles hold 32 * lv.pg pairs)
+template <int ROOT, int NP, int MAXT, int MINB>
+static int launch_path(messi_ctx* ctx, const SegDev* d_segs, const int2* d_tiles, const SegLevel& lv, int cs,
                        const float* d_P, int numnodes, int c0, int nc, int C, const float* d_pi16,
                        const double* d_logw, const int* d_lam, bool per_lambda)
 {
-    if (nt <= 0) return MESSI_OK;
-    // shapes: 0 = 2 stages x 4 CTAs/SM, 1 = 3 stages x 3 CTAs, 2 = 2 stages x 3 CTAs (the autotuner's
-    // candidates); 3 = interior levels in the tcgen05 form, the roots as shape 0 (on request only)
-    if (ctx->prune_shape == 3 && !root) return launch_prune_tc(ctx, d_nodes, d_tiles, nt, d_P, numnodes, c0, nc);
-    switch (ctx->prune_shape) {
-        case 1: return launch_prune_shape<3, 3>(ctx, d_nodes, d_tiles, nt, root, d_P, numnodes, c0, nc, C, d_pi16,
-                                                d_logw, d_lam, per_lambda);
-        case 2: return launch_prune_shape<2, 3>(ctx, d_nodes, d_tiles, nt, root, d_P, numnodes, c0, nc, C, d_pi16,
-                                                d_logw, d_lam, per_lambda);
-        default: return launch_prune_shape<2, 4>(ctx, d_nodes, d_tiles, nt, root, d_P, numnodes, c0, nc, C, d_pi16,
-                                                 d_logw, d_lam, per_lambda);
+    const int pgs = lv.pg / NP, warps = pgs * cs;
+    const size_t smem = sizeof(float4) * ((size_t)lv.max_steps + (size_t)lv.pg * lv.max_nb * 8 +
+                                          (size_t)warps * NP * lv.max_depth * 128) +
+                        (ROOT == 2 ? sizeof(double) * 32 * (size_t)lv.pg * nc : 0);
+    static thread_local std::pair<int, size_t> granted{-1, 0};
+    if (granted.first != ctx->device || granted.second < smem) {
+        cudaError_t e = cudaFuncSetAttribute(prune_path_kernel<ROOT, NP, MAXT, MINB>,
+                                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) return cuda_fail(ctx, e, "prune_path_kernel attributes");
+        granted = {ctx->device, smem};
     }
+    prune_path_kernel<ROOT, NP, MAXT, MINB><<<lv.tile_cnt, 32 * warps, smem, ctx->stream>>>(
+        d_segs, d_tiles + lv.tile_off, d_P, numnodes, c0, nc, C, d_pi16, d_logw, d_lam, per_lambda ? 1 : 0, cs,
+        lv.max_steps, lv.max_nb, lv.max_depth);
+    LAUNCH_CHECK(ctx, ROOT ? "prune_path_kernel<root>" : "prune_path_kernel");
+    return MESSI_OK;
+}
+
+constexpr int kMaxSplits = 12;  // category splits of a pair group: CTAs of up to 384 threads
+
+int launch_prune_level(messi_ctx* ctx, const SegDev* d_segs, const int2* d_tiles, const SegLevel& lv, bool root,
+                       const float* d_P, int numnodes, int c0, int nc, int C, const float* d_pi16,
+                       const double* d_logw, const int* d_lam, bool per_lambda)
+{
+    if (lv.tile_cnt <= 0) return MESSI_OK;
+    if (ctx->prune_shape == 3 && !root && lv.max_nb == 2 && lv.pg == 4)
+        return launch_prune_tc(ctx, d_segs, d_tiles + lv.tile_off, lv.tile_cnt, d_P, numnodes, c0, nc);
+#define MESSI_PATH(ROOT, NP, MAXT, MINB, CS)                                                                         \
+    launch_path<ROOT, NP, MAXT, MINB>(ctx, d_segs, d_tiles, lv, CS, d_P, numnodes, c0, nc, C, d_pi16, d_logw, d_lam, \
+                                      per_lambda)
+    if (lv.pg == 4 && !per_lambda) {
+        switch (ctx->prune_shape) {
+            case 1: return root ? MESSI_PATH(1, 1, 128, 4, 1) : MESSI_PATH(0, 1, 128, 4, 1);
+            case 2: return root ? MESSI_PATH(1, 2, 64, 6, 1) : MESSI_PATH(0, 2, 64, 6, 1);
+            default: return root ? MESSI_PATH(1, 1, 128, 5, 1) : MESSI_PATH(0, 1, 128, 5, 1);
+        }
+    }
+    // few pairs (or per-lambda mixtures): the warps of a pair group share the
+    // categories until the GPU's 16 warps per SM are filled
+    const int sms = ctx->num_sms > 0 ? ctx->num_sms : 152;
+    int cs = (lv.pg == 1) ? (int)std::min<int64_t>(kMaxSplits, (16 * (int64_t)sms + lv.warps - 1) / std::max<int64_t>(lv.warps, 1)) : 1;
+    cs = std::max(1, std::min(cs, nc));
+    if (!root) return MESSI_PATH(0, 1, 32 * kMaxSplits, 1, cs);
+    return MESSI_PATH(2, 1, 32 * kMaxSplits, 1, cs);
+#undef MESSI_PATH
 }
 
 int run_pairs(messi_ctx* ctx, messi_dataset* ds, const float* d_P, const float* d_pi16, const double* d_logw,
               const int* d_lam, int C, int nlam, bool per_lambda)
 {
     (void)nlam;
-    const int chunk = ds->chunk;
+    const int chunk = std::min(ds->chunk, kCollectCategories);
     for (int c0 = 0; c0 < C; c0 += chunk) {
         const int nc = std::min(chunk, C - c0);
         int rc = launch_leaf_messages(ctx, ds->d_leaf, ds->d_leafnode, ds->leaf_rows, d_P, ds->numnodes, c0, nc, C,
                                       ds->d_leafmsg);
         if (rc) return rc;
-        for (int lv = 1; lv <= ds->H; lv++) {
-            const int nt = ds->tile_cnt[lv];
-            if (nt == 0) continue;
-            if (ctx->profiling) {
-                double units = 0.0;
-                for (int v : ds->level_nodes[lv]) units += (double)ds->nunique[v] * nc;
-                prof_begin(ctx, 0, units);
-            }
-            rc = launch_prune_tiles(ctx, ds->d_nodes, ds->d_tiles + ds->tile_off[lv], nt, lv == ds->H, d_P,
-                                    ds->numnodes, c0, nc, C, d_pi16, d_logw, d_lam, per_lambda);
+        for (int lv = 1; lv <= ds->SH; lv++) {
+            const SegLevel& sl = ds->seg_levels[lv];
+            if (sl.tile_cnt == 0) continue;
+            prof_begin(ctx, 0, sl.units * nc);
+            rc = launch_prune_level(ctx, ds->d_segs, ds->d_tiles, sl, lv == ds->SH, d_P, ds->numnodes, c0, nc, C,
+                                    d_pi16, d_logw, d_lam, per_lambda);
             if (rc) return rc;
             prof_end(ctx);
         }
