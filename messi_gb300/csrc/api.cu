@@ -697,7 +697,7 @@ int messi_siterate_conditionals(messi_ctx* ctx, messi_dataset* ds, const messi_m
     if ((rc = prepare_arena(ctx, ds, md.cat.C))) return rc;
     const int L = ds->L, C = md.cat.C, ns = md.cat.nsite;
     void *pc, *pv;
-    if ((rc = ensure(ctx, kSlotCatLL, (size_t)C * std::max<int64_t>(ds->nroot, 1) * sizeof(double), &pc))) return rc;
+    if ((rc = ensure(ctx, kSlotCatLL, (size_t)(C + 2 * ns) * std::max<int64_t>(ds->nroot, 1) * sizeof(double), &pc))) return rc;
     if ((rc = ensure(ctx, kSlotCond, ((size_t)L * L + (size_t)L * (ns + 1)) * sizeof(double), &pv))) return rc;
     double* d_catll = (double*)pc;
     double* d_pair = (double*)pv;
@@ -723,7 +723,7 @@ int messi_siterate_conditionals(messi_ctx* ctx, messi_dataset* ds, const messi_m
     if ((rc = h2d(ctx, d_pair, pairprobs, (size_t)L * L * sizeof(double)))) return rc;
     if ((rc = h2d(ctx, d_single, singleprobs, (size_t)L * sizeof(double)))) return rc;
     if ((rc = launch_siterate_conditionals(ctx, ds, d_catll, md.logw, ns, md.cat.nlam, d_single, d_pair, d_ull,
-                                           md.logw_site, d_out)))
+                                           md.logw_site, d_catll + (size_t)C * ds->nroot, d_out)))
         return rc;
     if ((rc = d2h(ctx, conditionals, d_out, (size_t)L * ns * sizeof(double)))) return rc;
     return finish(ctx);

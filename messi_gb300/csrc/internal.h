@@ -407,10 +407,11 @@ int launch_unpaired(messi_ctx* ctx, messi_dataset* ds, const double* d_P4, int p
                     const double* d_logw_site, int nsite, double* d_u, double* d_scratch);
 // Site-rate conditionals (prune.cu): catll [C][nroot] per-category root
 // log-likelihoods, ull [nsite][L] per-site unpaired log-likelihoods, single
-// [L] and pair [L x L] (column-major) posteriors; out [nsite x L] column-major.
+// [L] and pair [L x L] (column-major) posteriors; out [nsite x L] column-major;
+// d_pairll: 2 * nsite * nroot doubles of scratch.
 int launch_siterate_conditionals(messi_ctx* ctx, messi_dataset* ds, const double* d_catll, const double* d_logw,
                                  int nsite, int nlam, const double* d_single, const double* d_pair,
-                                 const double* d_ull, const double* d_logw_site, double* d_out);
+                                 const double* d_ull, const double* d_logw_site, double* d_pairll, double* d_out);
 // Fixed-structure sums (prune.cu, structure_sum_kernel); d_partner[c] is the
 // 0-based partner of column c (or -1), logwF the factorised lambda weight.
 int launch_structure_sum(messi_ctx* ctx, int L, double* d_u, const int* d_colu, const int* d_partner,

@@ -1213,13 +1213,6 @@ int launch_bandprep_from_mix(messi_ctx* ctx, messi_dataset* ds, const Band& t, c
 }
 
 // ---------------------------------------------------------------------------
-// Fixed-structure likelihood: sum of the unpaired columns and of the pairs
-// (one block, FP64, fixed reduction order).  On return u holds the unpaired
-// log-likelihood of unpaired columns and 0 on paired ones (the reference's
-// computeunpairedlikelihoods(..., paired), src/FARCE.jl:1222-1250), pairll
-// the pair log-likelihood at the first column of each pair and 0 elsewhere.
-// ---------------------------------------------------------------------------
-// ---------------------------------------------------------------------------
 // Site-rate conditionals (felsensteinposteriorsiterateconditionalscuda,
 // src/FelsensteinCUDA.jl:518-717): for column x and site-rate category s,
 //   LSE( log w_s + log single[x] + u_s[x],
@@ -1227,72 +1220,126 @@ int launch_bandprep_from_mix(messi_ctx* ctx, messi_dataset* ds, const Band& t, c
 //            log pair[x,y] + log w_c + ll_c(x, y),
 //        over band partners y < x, categories with s2 = s:
 //            log pair[y,x] + log w_c + ll_c(y, x) )
-// One thread per (column, category); categories in the order s1, s2, lambda.
+// Categories in the order s1, s2, lambda.  Two kernels:
+//   * siterate_pairs_kernel, a thread per (unique root pair, site-rate
+//     category, side): the log-sum-exp over the ns * nl categories that have
+//     the rate s at the pair's first (side 0) or second column (side 1), so
+//     that a column adds one term per partner, not ns * nl;
+//   * siterate_cols_kernel, a warp per (column, category): its partners over
+//     the lanes, each lane a running log-sum-exp, merged at the end.
+// FP64 throughout; bound by the FP64 pipe (one exp per pair and category).  A
+// term more than 45 nats below its maximum is below 2^-64 of the sum and its
+// exp is not formed.  (One thread per (column, category) walking every partner
+// and category with a log1p(exp) each took 16.6 ms at 64 x 600, span 300.)
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ double lse_acc(double a, double b)
+constexpr double kNegligible = -45.0;
+
+__global__ void __launch_bounds__(256) siterate_pairs_kernel(const double* __restrict__ catll, long long nroot,
+                                                             const double* __restrict__ logw, int ns, int nl,
+                                                             double* __restrict__ out)
 {
-    if (b == -INFINITY) return a;
-    if (a == -INFINITY) return b;
-    return (a < b) ? b + log1p(exp(a - b)) : a + log1p(exp(b - a));
+    const long long b = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const int s = blockIdx.y % ns, side = blockIdx.y / ns;
+    if (b >= nroot) return;
+    double m = -INFINITY;
+    for (int o = 0; o < ns; o++)
+        for (int l = 0; l < nl; l++) {
+            const int c = (side ? o * ns + s : s * ns + o) * nl + l;
+            m = fmax(m, logw[c] + catll[(size_t)c * nroot + b]);
+        }
+    double acc = 0.0;
+    if (m != -INFINITY)
+        for (int o = 0; o < ns; o++)
+            for (int l = 0; l < nl; l++) {
+                const int c = (side ? o * ns + s : s * ns + o) * nl + l;
+                const double d = logw[c] + catll[(size_t)c * nroot + b] - m;
+                if (d >= kNegligible) acc += exp(d);
+            }
+    out[(size_t)blockIdx.y * nroot + b] = (m == -INFINITY) ? -INFINITY : m + log(acc);
 }
 
-__global__ void siterate_cond_kernel(const int* __restrict__ bandidx, int L, int W, const double* __restrict__ catll,
-                                     int nroot, const double* __restrict__ logw, int ns, int nl,
-                                     const double* __restrict__ single, const double* __restrict__ pair,
-                                     const double* __restrict__ ull, const double* __restrict__ logw_site,
-                                     double* __restrict__ out)
+// Running log-sum-exp in FP64.
+struct LogSum {
+    double m = -INFINITY, s = 0.0;
+    __device__ __forceinline__ void add(double v, double w = 1.0)  // w e^v
+    {
+        if (v == -INFINITY) return;
+        if (v > m) {
+            s = (m - v >= kNegligible) ? s * exp(m - v) + w : w;
+            m = v;
+        } else if (v - m >= kNegligible) {
+            s += w * exp(v - m);
+        }
+    }
+    __device__ __forceinline__ double value() const { return (m == -INFINITY) ? -INFINITY : m + log(s); }
+};
+
+__global__ void __launch_bounds__(128) siterate_cols_kernel(const int* __restrict__ bandidx, int L, int W,
+                                                            const double* __restrict__ pairll, long long nroot, int ns,
+                                                            const double* __restrict__ single,
+                                                            const double* __restrict__ pair,
+                                                            const double* __restrict__ ull,
+                                                            const double* __restrict__ logw_site,
+                                                            double* __restrict__ out)
 {
-    const int x = blockIdx.x * blockDim.x + threadIdx.x;
+    const int x = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
     const int s = blockIdx.y;
-    if (x >= L) return;
-    double acc = -INFINITY;
-    const double us = ull[(size_t)s * L + x];
-    if (us != -INFINITY) acc = lse_acc(acc, logw_site[s] + log(single[x]) + us);
-    for (int k = 1; k <= W && x + k < L; k++) {
+    if (x >= L) return;  // warp-uniform
+    const double* first = pairll + (size_t)s * nroot;
+    const double* second = pairll + (size_t)(ns + s) * nroot;
+    LogSum acc;
+    if (lane == 0) {
+        const double us = ull[(size_t)s * L + x];
+        if (us != -INFINITY) acc.add(logw_site[s] + log(single[x]) + us);
+    }
+    for (int k = 1 + lane; k <= W && x + k < L; k += 32) {
         const int b = bandidx[(size_t)x * (W + 1) + k];
         if (b < 0) continue;
         const double pp = pair[(size_t)x + (size_t)(x + k) * L];
-        if (!(pp > 0.0)) continue;
-        const double lp = log(pp);
-        for (int s2 = 0; s2 < ns; s2++)
-            for (int l = 0; l < nl; l++) {
-                const int c = (s * ns + s2) * nl + l;
-                acc = lse_acc(acc, lp + logw[c] + catll[(size_t)c * nroot + b]);
-            }
+        if (pp > 0.0) acc.add(log(pp) + first[b]);
     }
-    for (int k = 1; k <= W && k <= x; k++) {
-        const int y = x - k;
-        const int b = bandidx[(size_t)y * (W + 1) + k];
+    for (int k = 1 + lane; k <= W && k <= x; k += 32) {
+        const int b = bandidx[(size_t)(x - k) * (W + 1) + k];
         if (b < 0) continue;
-        const double pp = pair[(size_t)y + (size_t)x * L];
-        if (!(pp > 0.0)) continue;
-        const double lp = log(pp);
-        for (int s1 = 0; s1 < ns; s1++)
-            for (int l = 0; l < nl; l++) {
-                const int c = (s1 * ns + s) * nl + l;
-                acc = lse_acc(acc, lp + logw[c] + catll[(size_t)c * nroot + b]);
-            }
+        const double pp = pair[(size_t)(x - k) + (size_t)x * L];
+        if (pp > 0.0) acc.add(log(pp) + second[b]);
     }
-    out[(size_t)s + (size_t)x * ns] = acc;
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) {
+        const double m2 = __shfl_down_sync(0xffffffffu, acc.m, off), s2 = __shfl_down_sync(0xffffffffu, acc.s, off);
+        acc.add(m2, s2);
+    }
+    if (lane == 0) out[(size_t)s + (size_t)x * ns] = acc.value();
 }
 
+// d_pairll: 2 * nsite * nroot doubles of scratch
 int launch_siterate_conditionals(messi_ctx* ctx, messi_dataset* ds, const double* d_catll, const double* d_logw,
                                  int nsite, int nlam, const double* d_single, const double* d_pair,
-                                 const double* d_ull, const double* d_logw_site, double* d_out)
+                                 const double* d_ull, const double* d_logw_site, double* d_pairll, double* d_out)
 {
-    const int bs = 64;
-    siterate_cond_kernel<<<dim3((ds->L + bs - 1) / bs, nsite), bs, 0, ctx->stream>>>(
-        ds->d_bandidx, ds->L, ds->W, d_catll, (int)ds->nroot, d_logw, nsite, nlam, d_single, d_pair, d_ull,
-        d_logw_site, d_out);
-    LAUNCH_CHECK(ctx, "siterate_cond_kernel");
+    if (ds->nroot > 0) {
+        siterate_pairs_kernel<<<dim3((unsigned)((ds->nroot + 255) / 256), 2 * nsite), 256, 0, ctx->stream>>>(
+            d_catll, ds->nroot, d_logw, nsite, nlam, d_pairll);
+        LAUNCH_CHECK(ctx, "siterate_pairs_kernel");
+    }
+    siterate_cols_kernel<<<dim3((ds->L + 3) / 4, nsite), 128, 0, ctx->stream>>>(
+        ds->d_bandidx, ds->L, ds->W, d_pairll, ds->nroot, nsite, d_single, d_pair, d_ull, d_logw_site, d_out);
+    LAUNCH_CHECK(ctx, "siterate_cols_kernel");
     return MESSI_OK;
 }
 
+// ---------------------------------------------------------------------------
+// Fixed-structure likelihood: sum of the unpaired columns and of the pairs
+// (one block, FP64, fixed reduction order).  On return u holds the unpaired
+// log-likelihood of unpaired columns and 0 on paired ones (the reference's
+// computeunpairedlikelihoods(..., paired), src/FARCE.jl:1222-1250), pairll
+// the pair log-likelihood at the first column of each pair and 0 elsewhere.
 // colu[c]: unique root pair of the pair opened at column c (>= 0), -2 on the
 // closing column of a pair, -1 on an unpaired column; partner[c] the other
 // column of the pair opened at c.  The factorised lambda categories add
 // logwF + u[c] + u[partner] to each pair, so the unpaired values of paired
 // columns are read before they are cleared.
+// ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(1024) structure_sum_kernel(double* __restrict__ u, const int* __restrict__ colu,
                                                              const int* __restrict__ partner, int L,
                                                              const double* __restrict__ mix, double logwF,
