@@ -892,7 +892,7 @@ int decode_device(messi_ctx* ctx, int L, const double* d_single, const double* d
     void *work, *ints;
     const size_t LL = (size_t)L * L;
     if ((rc = ensure(ctx, kSlotDecodeF, ((size_t)L + 3 * LL) * sizeof(float), &work))) return rc;
-    if ((rc = ensure(ctx, kSlotDecodeI, (LL + 3 * (size_t)L + 16 + kSyncWords) * sizeof(int), &ints))) return rc;
+    if ((rc = ensure(ctx, kSlotDecodeI, (LL + 3 * (size_t)L + 16 + decode_sync_words(L)) * sizeof(int), &ints))) return rc;
     int* scol = (int*)ints;
     int* stack = scol + LL;
     int* d_paired = stack + 2 * ((size_t)L + 1);

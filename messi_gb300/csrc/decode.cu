@@ -11,10 +11,9 @@
 //                   alpha*pair(i,j) + e(i+1,j-1),                          s = -2
 //                   max_k alpha*pair(i,k) + e(i+1,k-1) + e(k+1,j) )        s = k+1
 // with ties to the first alternative and the smallest k.  One persistent
-// cooperative launch walks the spans (grid barrier between spans); a cell's
-// split maximum is reduced by a group of lanes with a (value, k) arg-max.  e
-// is kept twice (row-major and column-major) so both operand streams of the
-// split are unit-stride; s is written column-major, the layout the Julia
+// cooperative launch walks the diagonals of 16 x 16 tiles (a grid barrier
+// between them).  e is kept row-major (the split's second factor) and
+// column-major (the output); s is written column-major, the layout the Julia
 // caller reads.  The traceback runs on the device in one thread.
 //
 // Structure sampling replaces samplestructure / samplestructurehelper
@@ -27,6 +26,7 @@
 // of a span, so the weights are the reference's up to a common factor.
 // Random numbers: SplitMix64 (Steele, Lea and Flood, OOPSLA 2014) over
 // (seed, structure, draw).
+#include <algorithm>
 #include <climits>
 #include <cmath>
 
@@ -59,177 +59,280 @@ __global__ void to_double_kernel(const float* __restrict__ in, double* __restric
     if (i < n) out[i] = (double)in[i];
 }
 
+// ---------------------------------------------------------------------------
+// Posterior decoding over tiles of 16 x 16 cells.
 // pair: L x L as uploaded from the Julia matrix (column-major); it is read as
 // pair[i*L + k], the reference kernel's indexing (the matrix is symmetric).
 //
-// Cell (i, j = i+d): the best split over k = i+1 .. j-1 of
-// alpha*pair(i,k) + e(i+1,k-1) + e(k+1,j), e2 = alpha*pair(i,j) + e(i+1,j-1)
-// and e1 = single(i) + e(i+1,j).  Split point k reads spans k-i-2 and j-k-1.
-// Diagonals go two per grid barrier, (dA, dB) = (2p-1, 2p): decode_split_t
-// takes the split points k = i+KLO .. j-KHI, whose spans are <= 2p-4 and so
-// complete before the wait on the barrier that completes 2p-2 (dA: KLO = 2,
-// KHI = 1; dB: KLO = 3, KHI = 2), as a lane-group (value, k) arg-max;
-// decode_finish_t adds the outer split points in ascending k, e2 and e1 and
-// writes the cell.  The maximum is exact and ties go to the smallest k (the
-// reference's loop order) however the points are split, so the bits are the
-// reference kernel's.
-struct DecodePart {
-    float bv;
-    int bk;
+// With a(i,k) = alpha*pair(i,k) + e(i+1,k-1), the value of "i pairs k and
+// encloses i+1 .. k-1" (which replaces pair(i,k) in memory once known),
+//     e(i,j) = max( single(i) + e(i+1,j), a(i,j), max_{i<k<j} a(i,k) + e(k+1,j) ):
+// a product of triangular matrices with max for the sum.  The maximum is exact
+// and ties go to the smallest k (the reference's loop order) in whatever order
+// the split points are taken, so the bits are the reference kernel's.
+//
+// CTA b owns the rows of the tiles (I, *), I = b, b + grid, ..., and computes
+// them in the order of the tile diagonals D = J - I.  Tile (I, J) needs row
+// block I + 1 up to diagonal D - 1, which needed row block I + 2 up to D - 2,
+// and so on: a CTA publishes its row block's finished diagonals in a flag
+// (release) and waits for its neighbour's alone (acquire, bounded), not for a
+// grid barrier.  Row index r = k + 1 of the second factor:
+//   * r in a block R strictly between I and J: both factors lie in finished
+//     tiles.  Sixteen groups of 64 threads take every sixteenth R; a thread
+//     keeps four cells of the tile and reads e(r, j) from L2 once for all four,
+//     a(i, .) from shared memory.  R = I + 1 and I + 2 may still be in the
+//     making when the CTA starts the tile, so they come after the wait and the
+//     rest before it;
+//   * r in I or J: the factors lie in the tile itself (and in the two diagonal
+//     tiles).  A thread per cell; the cells become final along the 31
+//     anti-diagonals from the lower left corner, and in every step each cell
+//     that is not yet final takes the two values that the last step's cells
+//     gave it (without branches: with the split index carried along and the
+//     stores inside, a step took 530 cycles).
+// Bound by the chain of L/16 waits and 31 steps each; a wavefront with one
+// grid barrier per two diagonals of cells took 3.61 ms at L = 1,000, this takes
+// 0.60 ms.
+// ---------------------------------------------------------------------------
+constexpr int kDT = 16;          // cells per tile side
+constexpr int kDThreads = 1024;  // 16 groups of 64 threads
+constexpr int kDGroups = kDThreads / 64;
+constexpr float kDecodeInit = -1e10f;  // the reference's initial maximum (with index 0)
+
+struct DecodeSmem {
+    float ad[kDT][kDT + 1];      // a of the row block's diagonal tile
+    float ed[kDT][kDT + 1];      // e of the column block's diagonal tile
+    float et[kDT + 1][kDT + 2];  // e of the tile: column J*16 - 1 at 0, row I*16 + 16 at 16
+    float at[kDT][kDT + 2];      // a of the tile: column J*16 - 1 at 0
+    float bv[kDGroups][kDT * kDT];
+    int bk[kDGroups][kDT * kDT];
 };
 
-template <int KLO, int KHI>
-__device__ __forceinline__ DecodePart decode_split_t(const float* __restrict__ pair, const float* erow,
-                                                     const float* ecol, int L, float alpha, int i, int d,
-                                                     bool valid, int lane, int G)
+// Waits (whole CTA) until flag >= want; false once any CTA has given up
+// waiting (sync[2], the host's error flag).
+__device__ bool flag_wait(const unsigned int* flag, unsigned int want, unsigned int* sync)
 {
-    DecodePart p{-1e10f, 0};  // the reference's initial maximum and index
-    const int j = i + d;
-    if (valid) {
-        const float* prow = pair + (size_t)i * L;
-        const float* er = erow + (size_t)(i + 1) * L;  // e(i+1, k-1)
-        const float* ec = ecol + (size_t)j * L;        // e(k+1, j)
-        const int kend = j - KHI;
-        int k = i + KLO + lane;
-        // four splits per step, loads issued together, compared in ascending k
-        for (; k + 3 * G <= kend; k += 4 * G) {
-            float v[4];
-#pragma unroll
-            for (int q = 0; q < 4; q++) {
-                const int kq = k + q * G;
-                v[q] = __fmaf_rn(alpha, __ldg(prow + kq), __ldcg(er + kq - 1)) + __ldcg(ec + kq + 1);
+    __shared__ int s_ok;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        unsigned int spins = 0;
+        bool ok = true;
+        while (ld_acquire_u32(flag) < want) {
+            if (++spins > kSpinLimit || ((spins & 1023u) == 0u && ld_acquire_u32(&sync[2]) != 0u)) {
+                atomicExch(&sync[2], 1u);
+                ok = false;
+                break;
             }
+            if (spins > 64u) __nanosleep(32);
+        }
+        s_ok = ok;
+    }
+    __syncthreads();
+    return s_ok != 0;
+}
+
+__device__ __forceinline__ void flag_set(unsigned int* flag, unsigned int v)
+{
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(flag), "r"(v) : "memory");
+    }
+}
+
+__device__ __forceinline__ void cells_barrier() { asm volatile("bar.sync 1, 256;" ::: "memory"); }
+
+// The diagonal tile of row block I: cell (a, b) by thread 16a + b, span by span.
+__device__ void decode_diag_tile(DecodeSmem& S, const float* __restrict__ single, float* A, int L, float alpha, int I,
+                                 float* erow, float* ecol, int* scol)
+{
+    const int a = threadIdx.x >> 4, b = threadIdx.x & 15;
+    const int i = I * kDT + a, j = I * kDT + b;
+    const bool valid = j < L && b >= a;  // j < L implies i < L
+    const float p = (valid && b > a) ? A[(size_t)i * L + j] : 0.f;
+    const float si = (i < L) ? __ldg(single + i) : 0.f;
+    S.et[a][b] = 0.f;
+    S.ad[a][b] = -INFINITY;
+    for (int d = 1; d < kDT; d++) {
+        cells_barrier();
+        if (!valid || b - a != d) continue;
+        float bv = kDecodeInit;
+        int bk = 0;
+        for (int c = a + 1; c < b; c++) {
+            const float v = S.ad[a][c] + S.et[c + 1][b];
+            if (v > bv) {
+                bv = v;
+                bk = I * kDT + c;
+            }
+        }
+        const float e2 = __fmaf_rn(alpha, p, S.et[a + 1][b - 1]);
+        float mv = si + S.et[a + 1][b];
+        int sv = -1;
+        if (e2 > mv) {
+            mv = e2;
+            sv = -2;
+        }
+        if (bv > mv) {
+            mv = bv;
+            sv = bk + 1;
+        }
+        S.et[a][b] = mv;
+        S.ad[a][b] = e2;
+        erow[(size_t)i * L + j] = mv;
+        ecol[(size_t)j * L + i] = mv;
+        scol[(size_t)j * L + i] = sv;
+    }
+    cells_barrier();
+    if (valid) A[(size_t)i * L + j] = S.ad[a][b];  // -inf on the diagonal: a column never pairs itself
+}
+
+// ROWS: the CTA has one row block whose a(i, r - 1) stay in shared memory at
+// arow[a * astride + r] (astride a multiple of 4); otherwise they are read from A.
+template <bool ROWS>
+__global__ void __launch_bounds__(kDThreads) decode_tile_kernel(const float* __restrict__ single, float* A, int L,
+                                                                float alpha, float* erow, float* ecol, int* scol,
+                                                                int astride, unsigned int* sync, unsigned int* flags)
+{
+    __shared__ DecodeSmem S;
+    extern __shared__ float4 decode_rows[];
+    float* arow = reinterpret_cast<float*>(decode_rows);
+    const int NB = (L + kDT - 1) / kDT, tid = threadIdx.x;
+    for (int I = blockIdx.x; I < NB; I += gridDim.x) {
+        if (tid < 256) {
+            decode_diag_tile(S, single, A, L, alpha, I, erow, ecol, scol);
+            if (ROWS && I * kDT + (tid & 15) < L) arow[(tid >> 4) * astride + I * kDT + (tid & 15) + 1] = S.ad[tid >> 4][tid & 15];
+        }
+        flag_set(flags + I, 1u);  // D + 1 finished diagonals
+    }
+    // phase 1: this thread's cells are (a0 + 4m, b)
+    const int grp = tid >> 6, b1 = tid & 15, a0 = (tid >> 4) & 3;
+    for (int D = 1; D < NB; D++) {
+        for (int I = blockIdx.x; I + D < NB; I += gridDim.x) {
+            const int J = I + D;
+            const int j1 = min(J * kDT + b1, L - 1);
+            float bv[4];
+            int bk[4];
 #pragma unroll
-            for (int q = 0; q < 4; q++)
-                if (v[q] > p.bv) {
-                    p.bv = v[q];
-                    p.bk = k + q * G;
+            for (int m = 0; m < 4; m++) {
+                bv[m] = kDecodeInit;
+                bk[m] = 0;
+            }
+            // rows r0 .. r0 + 4n - 1 of block R, four at a time
+            auto block = [&](int r0, int n) {
+                float ev[kDT];
+#pragma unroll
+                for (int x = 0; x < kDT; x++) ev[x] = (x < 4 * n) ? __ldcg(erow + (size_t)(r0 + x) * L + j1) : 0.f;
+#pragma unroll
+                for (int m = 0; m < 4; m++)
+#pragma unroll
+                    for (int q = 0; q < 4; q++) {
+                        if (q >= n) break;
+                        const int a = a0 + 4 * m, r = r0 + 4 * q;
+                        float4 av;
+                        if (ROWS) {
+                            av = *reinterpret_cast<const float4*>(arow + a * astride + r);
+                        } else {
+                            const float* g = A + (size_t)(I * kDT + a) * L + r - 1;
+                            av = make_float4(g[0], g[1], g[2], g[3]);
+                        }
+                        const float v[4] = {av.x + ev[4 * q], av.y + ev[4 * q + 1], av.z + ev[4 * q + 2], av.w + ev[4 * q + 3]};
+                        const float best = fmaxf(fmaxf(v[0], v[1]), fmaxf(v[2], v[3]));
+                        if (best >= bv[m])
+                            amax_merge(bv[m], bk[m], best,
+                                       r - 1 + (v[0] == best ? 0 : (v[1] == best ? 1 : (v[2] == best ? 2 : 3))));
+                    }
+            };
+            for (int R = I + 3 + grp; R < J; R += kDGroups) block(R * kDT, 4);
+            if (!flag_wait(flags + I + 1, (unsigned)D, sync)) return;
+            // cell (a, b) of this thread in the tile, and what it needs from the neighbouring tiles
+            const int a = tid >> 4, b = tid & 15, i = I * kDT + a, j = J * kDT + b;
+            const int jc = min(j, L - 1);
+            float p = 0.f, si = 0.f, ved = 0.f, vrow = 0.f, vcol = 0.f, acol = 0.f, vcorner = 0.f;
+            if (tid < 256) {  // every load first: one round trip together with the last blocks'
+                p = A[(size_t)i * L + jc];
+                si = __ldg(single + i);
+                ved = __ldcg(erow + (size_t)min(J * kDT + a, L - 1) * L + jc);
+                if (a == 0) vrow = __ldcg(erow + (size_t)((I + 1) * kDT) * L + jc);
+                if (b == 0) {
+                    vcol = __ldcg(erow + (size_t)i * L + J * kDT - 1);
+                    acol = A[(size_t)i * L + J * kDT - 1];
+                    if (a == 0) vcorner = __ldcg(erow + (size_t)((I + 1) * kDT) * L + J * kDT - 1);
                 }
-        }
-        for (; k <= kend; k += G) {
-            const float v = __fmaf_rn(alpha, __ldg(prow + k), __ldcg(er + k - 1)) + __ldcg(ec + k + 1);
-            if (v > p.bv) {
-                p.bv = v;
-                p.bk = k;
             }
-        }
-    }
-    if (__any_sync(0xffffffffu, valid))
-        for (int off = G >> 1; off > 0; off >>= 1) {
-            const float v2 = __shfl_xor_sync(0xffffffffu, p.bv, off);
-            const int k2 = __shfl_xor_sync(0xffffffffu, p.bk, off);
-            amax_merge(p.bv, p.bk, v2, k2);
-        }
-    return p;
-}
-
-template <int KLO, int KHI>
-__device__ __forceinline__ void decode_finish_t(const float* __restrict__ single, const float* __restrict__ pair,
-                                                float* erow, float* ecol, int* scol, int L, float alpha, int i,
-                                                int d, bool valid, DecodePart p)
-{
-    if (!valid) return;
-    const int j = i + d;
-    const float* prow = pair + (size_t)i * L;
-    const float* er = erow + (size_t)(i + 1) * L;
-    const float* ec = ecol + (size_t)j * L;
-    // the outer split points, ascending k (ties to the smaller k)
-    for (int k = i + 1; k <= min(i + KLO - 1, j - 1); k++)
-        amax_merge(p.bv, p.bk, __fmaf_rn(alpha, __ldg(prow + k), __ldcg(er + k - 1)) + __ldcg(ec + k + 1), k);
-    for (int k = max(i + KLO, j - KHI + 1); k <= j - 1; k++)
-        amax_merge(p.bv, p.bk, __fmaf_rn(alpha, __ldg(prow + k), __ldcg(er + k - 1)) + __ldcg(ec + k + 1), k);
-    const float e2 = __fmaf_rn(alpha, __ldg(prow + j), __ldcg(er + j - 1));
-    const float e1 = __ldg(single + i) + __ldcg(er + j);
-    float mv = e1;
-    int sv = -1;
-    if (e2 > mv) {
-        mv = e2;
-        sv = -2;
-    }
-    if (p.bv > mv) {
-        mv = p.bv;
-        sv = p.bk + 1;
-    }
-    erow[(size_t)i * L + j] = mv;
-    ecol[(size_t)j * L + i] = mv;
-    scol[(size_t)j * L + i] = sv;
-}
-
-// The cells of one diagonal with rows [r0, end), by all warps of the CTA:
-// split parts of the first two rows of every lane group before the wait,
-// their finishing parts (lanes 0 and 1 of a group side by side) and any
-// further rows whole after it.
-struct DecodeRows {
-    DecodePart c[2];
-};
-
-template <int KLO, int KHI>
-__device__ __forceinline__ DecodeRows decode_rows_split(const float* __restrict__ pair, const float* erow,
-                                                        const float* ecol, int L, float alpha, int d, int r0,
-                                                        int end)
-{
-    DecodeRows p;
-    const int G = group_width(d - 1), gpb = blockDim.x / G;
-    const int lane = threadIdx.x & (G - 1), g = threadIdx.x / G;
+            // the two blocks next to the diagonal, four rows each by eight groups
+            if (grp >= 4 && grp < 12) {
+                const int R = I + 1 + ((grp - 4) >> 2);
+                if (R < J) block(R * kDT + 4 * (grp & 3), 1);
+            }
+            if (tid < 256) {
+                S.ed[a][b] = ved;
+                if (!ROWS) S.ad[a][b] = A[(size_t)i * L + I * kDT + b];
+                if (a == 0) S.et[kDT][b + 1] = vrow;
+                if (b == 0) {
+                    S.et[a][0] = vcol;
+                    S.at[a][0] = acol;
+                    if (a == 0) S.et[kDT][0] = vcorner;
+                }
+            }
 #pragma unroll
-    for (int it = 0; it < 2; it++) {
-        const int i = r0 + g + it * gpb;
-        p.c[it] = decode_split_t<KLO, KHI>(pair, erow, ecol, L, alpha, i, d, i < end, lane, G);
-    }
-    return p;
-}
-
-template <int KLO, int KHI>
-__device__ __forceinline__ void decode_rows_finish(const float* __restrict__ single, const float* __restrict__ pair,
-                                                   float* erow, float* ecol, int* scol, int L, float alpha, int d,
-                                                   int r0, int end, const DecodeRows& p)
-{
-    const int G = group_width(d - 1), gpb = blockDim.x / G;
-    const int lane = threadIdx.x & (G - 1), g = threadIdx.x / G;
-    if (G >= 2) {
-        const int it = lane & 1;
-        const int i = r0 + g + it * gpb;
-        decode_finish_t<KLO, KHI>(single, pair, erow, ecol, scol, L, alpha, i, d, lane < 2 && i < end,
-                                  it ? p.c[1] : p.c[0]);
-    } else {
-#pragma unroll
-        for (int it = 0; it < 2; it++) {
-            const int i = r0 + g + it * gpb;
-            decode_finish_t<KLO, KHI>(single, pair, erow, ecol, scol, L, alpha, i, d, i < end, p.c[it]);
+            for (int m = 0; m < 4; m++) {
+                S.bv[grp][(a0 + 4 * m) * kDT + b1] = bv[m];
+                S.bk[grp][(a0 + 4 * m) * kDT + b1] = bk[m];
+            }
+            __syncthreads();
+            float v1 = kDecodeInit, v = 0.f, e1 = 0.f, e2 = 0.f;
+            int k1 = 0;
+            if (tid < 256) {
+                if (D >= 2)
+#pragma unroll 4
+                    for (int q = 0; q < kDGroups; q++) amax_merge(v1, k1, S.bv[q][tid], S.bk[q][tid]);
+                // k = J*16 - 1, the column before the tile
+                amax_merge(v1, k1, S.at[a][0] + S.ed[0][b], J * kDT - 1);
+                v = v1;
+                const int mine = 15 - a + b;  // the step in which this cell becomes final
+                for (int t = 0; t < 2 * kDT - 1; t++) {
+                    // the values alone: which split point gave them is looked up afterwards
+                    const int ar = kDT + b - t;  // cell (ar, b) became final in step t - 1
+                    const int bc = t - kDT + a;  // and so did (a, bc)
+                    const float x = (ar >= a + 2 && ar < kDT) ? S.ad[a][ar - 1] + S.et[ar][b + 1] : -INFINITY;
+                    const float y = (bc >= 0 && bc < b) ? S.at[a][bc + 1] + S.ed[bc + 1][b] : -INFINITY;
+                    v = fmaxf(v, fmaxf(x, y));
+                    if (mine == t) {
+                        e2 = __fmaf_rn(alpha, p, S.et[a + 1][b]);
+                        e1 = si + S.et[a + 1][b + 1];
+                        float mv = e1;
+                        if (e2 > mv) mv = e2;
+                        if (v > mv) mv = v;
+                        S.et[a][b + 1] = mv;
+                        S.at[a][b + 1] = e2;
+                    }
+                    cells_barrier();
+                }
+                if (j < L) {
+                    erow[(size_t)i * L + j] = S.et[a][b + 1];
+                    A[(size_t)i * L + j] = e2;
+                    if (ROWS) arow[a * astride + j + 1] = e2;
+                }
+            }
+            flag_set(flags + I, (unsigned)D + 1u);
+            // what no other tile reads, while the others' values arrive: the
+            // column-major copy and the traceback codes
+            if (tid < 256 && j < L) {
+                int sv = -1;
+                float mv = e1;
+                if (e2 > mv) {
+                    mv = e2;
+                    sv = -2;
+                }
+                if (v > mv) {
+                    for (int c = a + 1; c < kDT - 1; c++) amax_merge(v1, k1, S.ad[a][c] + S.et[c + 1][b + 1], I * kDT + c);
+                    for (int c = 0; c < b; c++) amax_merge(v1, k1, S.at[a][c + 1] + S.ed[c + 1][b], J * kDT + c);
+                    sv = k1 + 1;
+                }
+                ecol[(size_t)j * L + i] = S.et[a][b + 1];
+                scol[(size_t)j * L + i] = sv;
+            }
+            // (the next tile writes the shared arrays after its wait, which begins with a CTA barrier)
         }
-    }
-    for (int base = r0 + 2 * gpb; base < end; base += gpb) {
-        const int i = base + g;
-        const DecodePart c = decode_split_t<KLO, KHI>(pair, erow, ecol, L, alpha, i, d, i < end, lane, G);
-        decode_finish_t<KLO, KHI>(single, pair, erow, ecol, scol, L, alpha, i, d, i < end && lane == 0, c);
-    }
-}
-
-// All diagonals, two per grid barrier.  CTA b owns rows [b*R, (b+1)*R) of
-// every diagonal (R = ceil(L / CTAs)); for the pair (dA, dB) it computes dA
-// for its rows plus row (b+1)*R (which the next CTA also computes, to the
-// same bits) and then, after a CTA barrier, dB, whose e1 reads dA at row
-// i+1, its own.
-__global__ void __launch_bounds__(kWaveMaxThreads) decode_wave_kernel(const float* __restrict__ single,
-                                                          const float* __restrict__ pair, int L, float alpha,
-                                                          float* __restrict__ erow, float* __restrict__ ecol,
-                                                          int* __restrict__ scol, unsigned int* sync)
-{
-    unsigned int gen = 0;
-    grid_arrive(sync);  // spans 0 and -1 are the zero-filled tables
-    const int rows = (L + gridDim.x - 1) / gridDim.x;
-    const int r0 = blockIdx.x * rows;
-    for (int dA = 1; dA < L; dA += 2) {
-        const int dB = dA + 1;
-        const int endA = min(r0 + rows + 1, L - dA);
-        const int endB = (dB < L) ? min(r0 + rows, L - dB) : r0;
-        const DecodeRows pa = decode_rows_split<2, 1>(pair, erow, ecol, L, alpha, dA, r0, endA);
-        const DecodeRows pb = decode_rows_split<3, 2>(pair, erow, ecol, L, alpha, dB, r0, endB);
-        if (!grid_wait(sync, gen)) return;
-        decode_rows_finish<2, 1>(single, pair, erow, ecol, scol, L, alpha, dA, r0, endA, pa);
-        __syncthreads();  // diagonal dA of this CTA's rows before dB reads it
-        decode_rows_finish<3, 2>(single, pair, erow, ecol, scol, L, alpha, dB, r0, endB, pb);
-        grid_arrive(sync);
     }
 }
 
@@ -452,6 +555,8 @@ __global__ void __launch_bounds__(128) sample_structures_kernel(Band t, Rules R,
 // ---------------------------------------------------------------------------
 // host side
 // ---------------------------------------------------------------------------
+size_t decode_sync_words(int L) { return (size_t)kSyncWords + (L + kDT - 1) / kDT; }
+
 int run_posterior_decoding(messi_ctx* ctx, int L, const double* d_single, const double* d_pair, double alpha,
                            float* d_work, int* d_scol, unsigned int* d_sync, int* d_paired, int* d_stack,
                            double* d_eout)
@@ -469,17 +574,31 @@ int run_posterior_decoding(messi_ctx* ctx, int L, const double* d_single, const 
     LAUNCH_CHECK(ctx, "to_float_kernel");
     cudaError_t e = cudaMemsetAsync(erow, 0, sizeof(float) * 2 * LL, ctx->stream);
     if (e == cudaSuccess) e = cudaMemsetAsync(d_scol, 0, sizeof(int) * LL, ctx->stream);
-    if (e == cudaSuccess) e = cudaMemsetAsync(d_sync, 0, kSyncWords * sizeof(unsigned int), ctx->stream);
+    if (e == cudaSuccess) e = cudaMemsetAsync(d_sync, 0, decode_sync_words(L) * sizeof(unsigned int), ctx->stream);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "decoding tables reset");
     if (L > 1) {
         const float a = (float)alpha;
         int Lv = L;
-        void* args[] = {(void*)&f_single, (void*)&f_pair, &Lv, (void*)&a, &erow, &ecol, &d_scol, &d_sync};
-        // paired shape: a CTA's two diagonals of a pair (2 x rows + 1 cells)
-        // in one pass of its warps where the CTA can grow to hold them
-        const int rc = launch_wave(ctx, (const void*)decode_wave_kernel, args, d_sync, L, 0.5 * (double)L * L,
-                                   "decode_wave_kernel", 2);
-        if (rc) return rc;
+        const int NB = (L + kDT - 1) / kDT;
+        // one CTA per row block where the GPU holds that many; its rows of a
+        // then stay in shared memory if they fit
+        int sms = ctx->num_sms;
+        if (sms <= 0) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device);
+        int grid = std::min(NB, std::max(1, sms));
+        if (ctx->wave_ctas > 0) grid = std::min(grid, ctx->wave_ctas);
+        int astride = NB * kDT + 4;
+        unsigned int* d_flags = d_sync + kSyncWords;
+        const size_t bytes = (size_t)kDT * astride * sizeof(float);
+        const bool rows = grid == NB && bytes <= (size_t)160 * 1024;
+        const void* kernel = rows ? (const void*)decode_tile_kernel<true> : (const void*)decode_tile_kernel<false>;
+        if (rows) {
+            e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+            if (e != cudaSuccess) return cuda_fail(ctx, e, "decode_tile_kernel attributes");
+        }
+        void* args[] = {(void*)&f_single, (void*)&f_pair, &Lv, (void*)&a, &erow, &ecol, &d_scol, &astride, &d_sync, &d_flags};
+        e = cudaLaunchCooperativeKernel(kernel, dim3(grid), dim3(kDThreads), args, rows ? bytes : 0, ctx->stream);
+        ctx->launches++;
+        if (e != cudaSuccess) return cuda_fail(ctx, e, "decode_tile_kernel");
     }
     if (d_paired) {
         decode_traceback_kernel<<<1, 32, 0, ctx->stream>>>(d_scol, L, d_paired, d_stack);

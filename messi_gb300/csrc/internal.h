@@ -466,8 +466,9 @@ int launch_finish_Z(messi_ctx* ctx, const Band& t);
 // KH99 rule log-probabilities times B.
 Rules make_rules(double B);
 // Posterior decoding (decode.cu).  d_work: (L + 3 L^2) floats; d_scol: L^2
-// ints (the column-major s output); d_sync: 4 uints; d_paired (nullable):
+// ints (the column-major s output); d_sync: decode_sync_words(L) uints; d_paired (nullable):
 // [L]; d_stack: 2 (L + 1) ints; d_eout (nullable): L^2 doubles.
+size_t decode_sync_words(int L);
 int run_posterior_decoding(messi_ctx* ctx, int L, const double* d_single, const double* d_pair, double alpha,
                            float* d_work, int* d_scol, unsigned int* d_sync, int* d_paired, int* d_stack,
                            double* d_eout);
