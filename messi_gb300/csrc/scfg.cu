@@ -960,7 +960,7 @@ __device__ __forceinline__ void partial_issue(const Band& t, int i, int d, bool 
     }
 }
 
-template <int NLO, int NHI>
+template <int NLO, int NHI, bool LONG>
 __device__ __forceinline__ CellPartial partial_complete(const Band& t, int i, int d, bool valid, int lane, int G,
                                                         const PartialPre& pp)
 {
@@ -978,14 +978,23 @@ __device__ __forceinline__ CellPartial partial_complete(const Band& t, int i, in
         lse_add8(c.m, c.s, x1);
         const float* lrow = t.Lrow + (size_t)i * t.RS;
         const float* scol = t.Scol + (size_t)(i + d) * t.RS + (d - 1);
-        for (int k = NLO + lane + 16 * G; k < kend; k += 8 * G) {
-            float x[8];
+        int k = NLO + lane + 16 * G;
+        if (LONG && G == 32) {
+            // further points sixteen at a time: 32 loads per round trip
+            for (; k + 15 * 32 < kend; k += 16 * 32) split_full16<32>(c.m, c.s, lrow, scol, k);
+            const int rem = (kend - k + 31) / 32;  // points left (<= 0: none)
+            if (rem > 8) split_tail32<true>(c.m, c.s, lrow, scol, k, rem);
+            else if (rem > 0) split_tail32<false>(c.m, c.s, lrow, scol, k, rem);
+        } else {
+            for (; k < kend; k += 8 * G) {
+                float x[8];
 #pragma unroll
-            for (int q = 0; q < 8; q++) {
-                const int kq = k + q * G;
-                x[q] = (kq < kend) ? __ldcg(lrow + kq) + __ldcg(scol - kq) : -INFINITY;
+                for (int q = 0; q < 8; q++) {
+                    const int kq = k + q * G;
+                    x[q] = (kq < kend) ? __ldcg(lrow + kq) + __ldcg(scol - kq) : -INFINITY;
+                }
+                lse_add8(c.m, c.s, x);
             }
-            lse_add8(c.m, c.s, x);
         }
     }
     // the shuffles only where some lane group of the warp has a cell (the
@@ -1194,15 +1203,25 @@ __global__ void __launch_bounds__(kWaveMaxThreads) inside_wave_kernel(Band t, Ru
 // next pair's partial sums read (<= 2p-2), so a warp issues the loads of its
 // next cell's partial sum as soon as its current cell is finished, before
 // the arrival, and adds them after it.
+// LONG (bands in which a lane has more than the sixteen prefetched points):
+// the rows of a diagonal pair are dealt evenly over the CTAs pair by pair
+// (ceil((L - 2p + 1) / CTAs) each) -- everything a pair reads of earlier pairs
+// goes through global memory, so the owner of a row may change -- so that long
+// spans, which have few rows, do not leave the CTAs of the high rows idle
+// while those of the low rows sum them all, and a lane's further points are
+// loaded sixteen at a time (L = 2,001, every span: 7.29 -> 5.18 ms).
+// Bands up to kShortBand keep the fixed rows: they gain nothing from either
+// and lose registers to both (span 500 over 1,000 columns: 0.74 -> 0.92 ms).
+constexpr int kShortBand = 16 * 32;
+
+template <bool LONG>
 __global__ void __launch_bounds__(kWaveMaxThreads) inside_wave_pipe_kernel(Band t, Rules R, double B)
 {
     __shared__ float s_lv[kWaveMaxThreads / 64], s_sv[kWaveMaxThreads / 64];
     unsigned int gen = 0;
     const int L = t.L, Wb = t.Wb;
-    const int rows = (L + gridDim.x - 1) / gridDim.x;
-    const int r0 = blockIdx.x * rows;
     const int half = (int)(blockDim.x >> 6);
-    if (half < rows + 1) {  // not launched so; leave with the launch marked failed
+    if (half < (L + (int)gridDim.x - 1) / (int)gridDim.x + 1) {  // not launched so; leave with the launch marked failed
         if (blockIdx.x == 0 && threadIdx.x == 0) atomicExch(&t.sync[2], 1u);
         return;
     }
@@ -1210,29 +1229,33 @@ __global__ void __launch_bounds__(kWaveMaxThreads) inside_wave_pipe_kernel(Band 
     grid_arrive(t.sync);
     const bool odd = (int)(threadIdx.x >> 5) < half;
     const int tid = (int)threadIdx.x - (odd ? 0 : 32 * half);
-    // this warp's diagonal of pair p is 2p-1 (odd) or 2p; its cell's row r0 + g
-    auto row_end = [&](int d) {
-        return (d > Wb) ? r0 : (odd ? min(r0 + rows + 1, L - d) : min(r0 + rows, L - d));
-    };
+    // this warp's diagonal of pair p is 2p-1 (odd) or 2p; its cell's row is the
+    // tid / G-th from the CTA's first one, r0 = b * rows, of that pair
+    const int grid = (int)gridDim.x;
+    auto row_end = [&](int dg, int r, int rw) { return (dg > Wb) ? r : min(r + rw + (odd ? 1 : 0), L - dg); };
     int d = odd ? 1 : 2;
+    int rows = (L - (LONG ? 1 : 0) + grid - 1) / grid, r0 = blockIdx.x * rows;
     int G = group_width(d), lane = tid & (G - 1), i = r0 + tid / G;
-    bool valid = i < row_end(d);
+    bool valid = i < row_end(d, r0, rows);
     CellPartial c;
     {
         PartialPre pp;
         if (odd) {
             partial_issue<2, 2>(t, i, d, valid, lane, G, pp);
-            c = partial_complete<2, 2>(t, i, d, valid, lane, G, pp);
+            c = partial_complete<2, 2, LONG>(t, i, d, valid, lane, G, pp);
         } else {
             partial_issue<3, 3>(t, i, d, valid, lane, G, pp);
-            c = partial_complete<3, 3>(t, i, d, valid, lane, G, pp);
+            c = partial_complete<3, 3, LONG>(t, i, d, valid, lane, G, pp);
         }
     }
     for (int eA = 1; eA <= Wb; eA += 2) {
         if (!grid_wait(t.sync, gen)) return;
         const int dn = d + 2;
-        const int Gn = group_width(dn), lanen = tid & (Gn - 1), in = r0 + tid / Gn;
-        const bool validn = in < row_end(dn);
+        if (LONG)  // ceil((L - eA - 2) / grid) rows for the next pair
+            while (rows > 1 && (rows - 1) * grid >= L - eA - 2) rows--;
+        const int r0n = LONG ? (int)blockIdx.x * rows : r0;
+        const int Gn = group_width(dn), lanen = tid & (Gn - 1), in = r0n + tid / Gn;
+        const bool validn = in < row_end(dn, r0n, rows);
         PartialPre pn;
         int ib = -1;
         Outer<3, 3> ob;
@@ -1257,12 +1280,13 @@ __global__ void __launch_bounds__(kWaveMaxThreads) inside_wave_pipe_kernel(Band 
         // loads in flight for the fence to wait for; the CTA barrier also
         // orders these reads before the next pair's writes
         grid_arrive(t.sync, blockDim.x - 1);
-        c = odd ? partial_complete<2, 2>(t, in, dn, validn, lanen, Gn, pn)
-                : partial_complete<3, 3>(t, in, dn, validn, lanen, Gn, pn);
+        c = odd ? partial_complete<2, 2, LONG>(t, in, dn, validn, lanen, Gn, pn)
+                : partial_complete<3, 3, LONG>(t, in, dn, validn, lanen, Gn, pn);
         d = dn;
         G = Gn;
         lane = lanen;
         i = in;
+        r0 = r0n;
         valid = validn;
     }
 }
@@ -1728,7 +1752,9 @@ int run_inside(messi_ctx* ctx, const Band& t, double B)
     void* args[] = {&tt, &R, &Bv};
     prof_begin(ctx, 1, (double)t.L * (t.Wb + 1) - 0.5 * t.Wb * (t.Wb + 1.0));
     int rc = launch_wave(ctx, (const void*)inside_wave_kernel, args, t.sync, t.L, (double)t.L * (t.Wb + 1),
-                         "inside_wave_kernel", 2, (const void*)inside_wave_pipe_kernel);
+                         "inside_wave_kernel", 2,
+                         t.Wb > kShortBand ? (const void*)inside_wave_pipe_kernel<true>
+                                           : (const void*)inside_wave_pipe_kernel<false>);
     if (rc) return rc;
     prof_end(ctx);
     if (t.L - 1 > t.Wb) {
