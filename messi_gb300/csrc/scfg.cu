@@ -1410,6 +1410,7 @@ __device__ __forceinline__ SumPartial outside_sum_t(const Band& t, int i, int d,
     const int L = t.L, Wb = t.Wb, RS = t.RS;
     const int j = i + d;
     SumPartial c{-INFINITY, 0.f};
+    if (!__any_sync(0xffffffffu, valid)) return c;  // no cell in this warp (warp-uniform)
     if (valid) {
         int n;
         const float *o1, *o2, *in;
@@ -1472,9 +1473,7 @@ __device__ __forceinline__ SumPartial outside_sum_t(const Band& t, int i, int d,
         }
         lse_add(c.m, c.s, extra);
     }
-    // the shuffles only where some lane group of the warp has a cell (the
-    // callers pass every lane of the warp; an empty slot's result is unused)
-    if (__any_sync(0xffffffffu, valid)) group_reduce_rt(c.m, c.s, G);
+    group_reduce_rt(c.m, c.s, G);
     return c;
 }
 
@@ -1581,6 +1580,153 @@ __device__ __forceinline__ void out_sums_finish(const Band& t, int d, int start,
     }
 }
 
+// The finishing parts of a diagonal pair with a thread per near sum and per F
+// value instead of one per cell: warps 0 and 2 of the CTA take the two sums of
+// every row of diagonals e and e-1, warps 1 and 3 their F values.  Every
+// operand of both diagonals is loaded before the first one is finished; what
+// e-1 needs of e (the first near parent of each sum, the CTA's own cells)
+// comes through shared memory.  The same operations on the same values as
+// outside_finish_t.
+constexpr int kFinishWarps = 4;
+constexpr int kFinishRows = 16;  // rows of a diagonal that two lanes each of one warp hold
+__device__ __forceinline__ void finish_barrier() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
+
+template <int Q>
+struct NearSum {
+    float a[Q], b[Q], v[Q];
+};
+
+template <int Q>
+__device__ __forceinline__ NearSum<Q> near_load(const Band& t, int i, int d, int side, bool valid, bool defer)
+{
+    const int L = t.L, Wb = t.Wb, RS = t.RS, j = i + d;
+    int n = 0;
+    const float *o1 = t.OSrow, *o2 = t.OFrow, *in = t.Srow;
+    if (valid && side == 0) {
+        n = (j + 1 <= L - 1) ? min(i + Wb, L - 1) - j : 0;
+        o1 = t.OSrow + (size_t)i * RS + d + 1;
+        o2 = t.OFrow + (size_t)i * RS + d + 1;
+        in = t.Srow + (size_t)min(j + 1, L - 1) * RS;
+    } else if (valid) {
+        n = (i >= 1) ? i - max(0, j - Wb) : 0;
+        o1 = t.OScol + (size_t)j * RS + d + 1;
+        o2 = t.OFcol + (size_t)j * RS + d + 1;
+        in = t.Lcol + (size_t)max(i - 1, 0) * RS;
+    }
+    NearSum<Q> s;
+#pragma unroll
+    for (int q = 0; q < Q; q++) {
+        const bool on = q < n, now = on && !(defer && q == 0);  // defer: parent 0 comes from near_patch
+        s.v[q] = ldg_if(in + q, on, 0.f);
+        s.a[q] = ldcg_if(o1 + q, now, -INFINITY);
+        s.b[q] = ldcg_if(o2 + q, now, -INFINITY);
+    }
+    return s;
+}
+
+template <int Q>
+__device__ __forceinline__ float near_finish(const NearSum<Q>& s, float2 c, const Rules& R)
+{
+    float x[8];
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+        const bool on = q < Q;
+        const int qq = on ? q : 0;
+        x[2 * q] = on ? R.r[0] + s.a[qq] + s.v[qq] : -INFINITY;
+        x[2 * q + 1] = on ? R.r[4] + s.b[qq] + s.v[qq] : -INFINITY;
+    }
+    lse_add8(c.x, c.y, x);
+    return lse_val(c.x, c.y);
+}
+
+struct FOperands {
+    float pp, a, b, c;
+};
+
+__device__ __forceinline__ FOperands f_load(const Band& t, int i, int d, bool valid)
+{
+    const int j = i + d;
+    const bool enc = valid && i >= 1 && j <= t.L - 2 && d + 2 <= t.Wb;
+    const size_t pr = enc ? (size_t)(i - 1) * t.RS + d + 2 : 0;
+    return FOperands{ldg_if(t.pb + pr, enc, -INFINITY), ldcg_if(t.OSrow + pr, enc, -INFINITY),
+                     ldcg_if(t.OFrow + pr, enc, -INFINITY), ldcg_if(t.OLrow + pr, enc, -INFINITY)};
+}
+
+__device__ __forceinline__ float f_finish(const FOperands& f, const Rules& R)
+{
+    if (f.pp == -INFINITY) return -INFINITY;
+    float m = -INFINITY, s = 0.f;
+    lse_add4(m, s, R.r[2] + f.pp + f.a, R.r[3] + f.pp + f.b, R.r[6] + f.pp + f.c, -INFINITY);
+    return lse_val(m, s);
+}
+
+// Writes the finished value of a sum (side 0: OL, side 1: OS); returns it.
+__device__ __forceinline__ float sum_write(const Band& t, int i, int d, int side, float v)
+{
+    const int j = i + d;
+    if (side == 0) {
+        t.OLrow[(size_t)i * t.RS + d] = v;
+        return v;
+    }
+    if (i == 0 && j == t.L - 1) v = 0.f;
+    t.OSrow[(size_t)i * t.RS + d] = v;
+    t.OScol[(size_t)j * t.RS + d] = v;
+    if (j == t.L - 1) t.Osuf[i] = v;
+    return v;
+}
+
+__device__ __forceinline__ void f_write(const Band& t, int i, int d, float v)
+{
+    t.OFrow[(size_t)i * t.RS + d] = v;
+    t.OFcol[(size_t)(i + d) * t.RS + d] = v;
+}
+
+// Rows [sA, sA + nA) of diagonal eA and [r0, r0 + nB) of eB = eA - 1 (nB = 0:
+// none), at most kFinishRows each, by warps 0 .. 3; the others do not come
+// here.  oS, oF: [nA] of shared memory.  Ends with a barrier of the four warps.
+__device__ void out_pair_finish(const Band& t, int eA, int sA, int nA, int r0, int nB, const float2* slotA,
+                                const float2* slotB, float* oS, float* oF, const Rules& R)
+{
+    const int part = (int)threadIdx.x >> 5, x = (int)threadIdx.x & 31;
+    const int row = (part & 1) ? x : x >> 1, side = x & 1, eB = eA - 1;
+    if (part == 0) {
+        const bool valid = row < nA;
+        const NearSum<2> s = near_load<2>(t, sA + row, eA, side, valid, false);
+        if (valid) {
+            const float v = sum_write(t, sA + row, eA, side, near_finish<2>(s, slotA[x], R));
+            if (side == 1) oS[row] = v;
+        }
+        finish_barrier();
+    } else if (part == 1) {
+        const FOperands f = f_load(t, sA + row, eA, row < nA);
+        if (row < nA) {
+            const float v = f_finish(f, R);
+            f_write(t, sA + row, eA, v);
+            oF[row] = v;
+        }
+        finish_barrier();
+    } else if (part == 2) {
+        const bool valid = row < nB;
+        NearSum<3> s = near_load<3>(t, r0 + row, eB, side, valid, true);
+        finish_barrier();  // diagonal e of the CTA's rows in oS / oF
+        if (valid) {
+            // parent 0 is (i, j+1) for side 0 and (i-1, j) for side 1, on diagonal e
+            const int i = r0 + row, p = i - side - sA;
+            const bool on = side == 0 ? i + eB + 1 <= t.L - 1 : i >= 1;
+            if (on) {
+                s.a[0] = oS[p];
+                s.b[0] = oF[p];
+            }
+            sum_write(t, i, eB, side, near_finish<3>(s, slotB[x], R));
+        }
+    } else {
+        const FOperands f = f_load(t, r0 + row, eB, row < nB);
+        finish_barrier();
+        if (row < nB) f_write(t, r0 + row, eB, f_finish(f, R));
+    }
+    finish_barrier();
+}
+
 // Suffix-column terms of the outside S sums of the last column's band cells:
 // cell (i, L-1) has the parents (ip, L-1) beyond the band, ip = max(0, i-1-Wb)
 // .. L-2-Wb, each adding r1 + OS(ip, L-1) + L(ip, i-1).  They read only the
@@ -1611,34 +1757,81 @@ __global__ void outside_lastcol_kernel(Band t, Rules R)
 }
 
 // All band diagonals of the outside pass, descending spans, two per grid
-// barrier.  CTA b owns rows [b*R, (b+1)*R) of every diagonal (R = ceil(L /
-// CTAs)).  For the pair (e, e-1) it computes diagonal e for its rows plus row
-// b*R - 1 (which the previous CTA also computes, to the same bits) and then,
-// after a CTA barrier, diagonal e-1, whose cells read diagonal e only at rows
-// i and i-1.  The sums of both diagonals read spans >= e+3 and are computed
-// between the CTA's arrival at the barrier that completes e+1 and its wait
-// there; the finishing parts follow the wait.
+// barrier.  For the pair (e, e-1) CTA b owns rows [b*R, (b+1)*R), R = ceil(rows
+// of e-1 / CTAs): it computes diagonal e for its rows plus row b*R - 1 (which
+// the previous CTA also computes, to the same bits) and then diagonal e-1,
+// whose cells read diagonal e only at rows i and i-1.  The sums of a pair read
+// spans >= e+3, which the wait for the pair before (e+2, e+1) has made complete
+// for every row: where four warps hold a pair's finishing parts
+// (out_pair_finish) they finish the pair before and arrive for the CTA while
+// the other warps are already at this pair's sums, so a pair costs the longer
+// of the two, not their sum; otherwise (many rows per CTA) a thread per cell
+// finishes diagonal after diagonal and the sums follow the arrival.
+// Span 500 over 1,000 columns: 1.86 ms with rows owned for the whole pass and a
+// thread per cell finishing each diagonal in turn, 1.52 with out_pair_finish
+// alone, 1.41 now.
 __global__ void __launch_bounds__(kWaveMaxThreads) outside_wave_kernel(Band t, Rules R)
 {
     __shared__ float2 slotA[2 * kWaveMaxThreads], slotB[2 * kWaveMaxThreads];
+    // paired form: the sums of the pair being finished and of the next one
+    __shared__ float2 pairA[2][2 * kFinishRows], pairB[2][2 * kFinishRows];
+    __shared__ float oS[kFinishRows], oF[kFinishRows];
     unsigned int gen = 0;
-    const int L = t.L, Wb = t.Wb;
-    const int rows = (L + gridDim.x - 1) / gridDim.x;
-    const int r0 = blockIdx.x * rows;
+    const int L = t.L, Wb = t.Wb, grid = (int)gridDim.x;
+    int rows = (L - max(Wb - 1, 0) + grid - 1) / grid;
     grid_arrive(t.sync);  // the suffix column was written by the previous launch
-    for (int eA = Wb; eA >= 0; eA -= 2) {
-        const int eB = eA - 1;
-        const int sA = max(r0 - 1, 0), nA = min(r0 + rows, L - eA) - sA;
-        const int nB = (eB >= 0) ? min(r0 + rows, L - eB) - r0 : 0;
-        out_sums_partial<2>(t, eA, sA, nA, 0, slotA, R);
-        if (eB >= 0) out_sums_partial<3>(t, eB, r0, nB, 2 * max(nA, 0), slotB, R);
-        if (!grid_wait(t.sync, gen)) return;
-        out_sums_finish<2>(t, eA, sA, nA, slotA, R);
-        if (eB >= 0) {
-            __syncthreads();  // diagonal e of rows r0-1 .. before diagonal e-1 reads it
-            out_sums_finish<3>(t, eB, r0, nB, slotB, R);
+    struct Pair {
+        int e, sA, nA, r0, nB;
+        bool paired;  // one warp holds a diagonal's rows and every sum has a group (the same in every CTA)
+    };
+    auto pair_at = [&](int e) {  // e descending: the rows grow
+        Pair p;
+        p.e = e;
+        while (rows * grid < L - max(e - 1, 0)) rows++;
+        p.r0 = blockIdx.x * rows;
+        p.sA = max(p.r0 - 1, 0);
+        p.nA = max(min(p.r0 + rows, L - e) - p.sA, 0);
+        p.nB = (e >= 1) ? max(min(p.r0 + rows, L - e + 1) - p.r0, 0) : 0;
+        p.paired = rows + 1 <= kFinishRows && rows + 1 <= (int)blockDim.x / group_width(2 * (Wb - max(e - 1, 0)) + 2) &&
+                   blockDim.x > 32 * kFinishWarps;
+        return p;
+    };
+    auto sums = [&](const Pair& p, int buf) {
+        // tasks start behind the finishing warps, which take what is left over
+        const int first = kFinishWarps * (32 / group_width(2 * (Wb - p.e) + 2));
+        out_sums_partial<2>(t, p.e, p.sA, p.nA, first, p.paired ? pairA[buf] : slotA, R);
+        if (p.e >= 1) {
+            const int firstB = kFinishWarps * (32 / group_width(2 * (Wb - p.e + 1) + 2));
+            out_sums_partial<3>(t, p.e - 1, p.r0, p.nB, firstB + 2 * p.nA, p.paired ? pairB[buf] : slotB,
+                                R);
         }
-        grid_arrive(t.sync);  // begins with a CTA barrier: the slots are free again
+    };
+    Pair p = pair_at(Wb);
+    int buf = 0;
+    sums(p, buf);
+    for (;;) {
+        if (!grid_wait(t.sync, gen)) return;  // ends with a CTA barrier: the slots of p are complete
+        const int next = p.e - 2;
+        if (p.paired) {
+            if (threadIdx.x < 32 * kFinishWarps) {
+                out_pair_finish(t, p.e, p.sA, p.nA, p.r0, p.nB, pairA[buf], pairB[buf], oS, oF, R);
+                if (threadIdx.x == 0) {
+                    __threadfence();
+                    atomicAdd(&t.sync[0], 1u);
+                }
+            }
+        } else {
+            out_sums_finish<2>(t, p.e, p.sA, p.nA, slotA, R);
+            if (p.e >= 1) {
+                __syncthreads();  // diagonal e of this CTA's rows before e-1 reads it
+                out_sums_finish<3>(t, p.e - 1, p.r0, p.nB, slotB, R);
+            }
+            grid_arrive(t.sync);
+        }
+        if (next < 0) break;
+        p = pair_at(next);
+        buf ^= 1;
+        sums(p, buf);
     }
 }
 
