@@ -19,6 +19,12 @@
 // CTAs, a 256-wide K chunk staged per barrier, and the fused epilogues
 // remove the elementwise launches between the GEMMs.
 //
+// Networks whose activations of 16 rows fit half an SM's shared memory (widths
+// up to about 380) run in two kernels instead: mlp_rows_kernel takes 16 rows of
+// the batch through forward, loss and the backward data path, mlp_wgrad_kernel
+// forms all weight and bias gradients.  The GEMM per layer remains for wider
+// networks.
+//
 // Head per sample: [K logits | K*D means | K*D log-sd]; the loss is the
 // negative log-likelihood of a target vector under the mixture.
 #include <cuda_bf16.h>
@@ -47,6 +53,13 @@ struct messi_mlp {
     float* target = nullptr;
     float* loss = nullptr;             // [cap]
     float* stage = nullptr;            // host-pinned staging
+    // two-kernel form (fused): weights as BF16 with K padded to 32 and zero
+    // filled, W1 W2 W3 W2^T W3^T; the batch's operands of the weight gradients,
+    // feature-major; per-CTA column sums for the bias gradients
+    bool fused = false;
+    __nv_bfloat16* w16 = nullptr;
+    __nv_bfloat16 *xT = nullptr, *a1T = nullptr, *a2T = nullptr, *dyT = nullptr, *d2T = nullptr, *d1T = nullptr;
+    float* colsum = nullptr;
 };
 
 namespace messi {
@@ -337,6 +350,439 @@ __global__ void sumsq_kernel(const float* __restrict__ g, int n, float* __restri
     if (threadIdx.x == 0) atomicAdd(out, red[0]);
 }
 
+// ---------------------------------------------------------------------------
+// Two-kernel form.  The network is tiny (44 -> 256 -> 256 -> 92), so a launch
+// per GEMM was latency: 16-25 us each for a few dozen CTAs, 13 launches per
+// gradient.  Here a CTA keeps 16 rows in shared memory through every layer and
+// streams the weights (200 KB) from L2 as MMA fragments, 16 bytes per lane:
+// every contraction index is stored permuted within its 32 (kpos) so that a
+// lane's 16 bytes are its fragments of two m16n8k16 MMAs, the same products in
+// the same order as the GEMM per layer.  The weight gradients contract over
+// the batch: the row kernel leaves its operands feature-major, so their
+// fragments are 16-byte loads too.  One draw (batch 1): three GEMM launches 49 us ->
+// 16 us; gradients at batch 256: 210 us of kernels -> 40 us.
+// ---------------------------------------------------------------------------
+constexpr int kRows = 16;         // batch rows per CTA: one MMA tile
+constexpr size_t kRowsMaxSmem = 110 * 1024;
+constexpr int kRowThreads = 512;  // 16 warps
+
+__host__ __device__ inline int pad32(int k) { return (k + 31) & ~31; }
+
+// Place of contraction index k within its 32: lane t of an MMA quad holds
+// indices 2t, 2t+1, 2t+8, 2t+9 of both halves at places 8t .. 8t+7; kat is the
+// inverse.
+__host__ __device__ constexpr int kpos(int k)
+{
+    return (k & ~31) | (((k & 7) >> 1) << 3) | (((k >> 4) & 1) << 2) | (((k >> 3) & 1) << 1) | (k & 1);
+}
+__host__ __device__ constexpr int kat(int p)
+{
+    return (p & ~31) | (((p >> 2) & 1) << 4) | (((p >> 1) & 1) << 3) | (((p >> 3) & 3) << 1) | (p & 1);
+}
+constexpr bool kpos_ok()
+{
+    for (int k = 0; k < 64; k++)
+        if (kat(kpos(k)) != k || (kpos(k) ^ k) >= 32) return false;
+    return true;
+}
+static_assert(kpos_ok(), "kat inverts kpos within each 32");
+
+// Element offsets of the padded BF16 weights.
+struct PackedW {
+    size_t w1, w2, w3, w2t, w3t, total;
+};
+__host__ __device__ inline PackedW packed_layout(int in, int H, int out)
+{
+    PackedW p;
+    p.w1 = 0;
+    p.w2 = p.w1 + (size_t)H * pad32(in);
+    p.w3 = p.w2 + (size_t)H * pad32(H);
+    p.w2t = p.w3 + (size_t)out * pad32(H);
+    p.w3t = p.w2t + (size_t)H * pad32(H);
+    p.total = p.w3t + (size_t)H * pad32(out);
+    return p;
+}
+
+__global__ void pack_weights_kernel(const float* __restrict__ p32, __nv_bfloat16* __restrict__ w, int in, int H, int out)
+{
+    const PackedW L = packed_layout(in, H, out);
+    const size_t o1 = 0, o2 = (size_t)H * in + H, o3 = o2 + (size_t)H * H + H;  // W1, W2, W3 in p32
+    for (size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x; e < L.total; e += (size_t)gridDim.x * blockDim.x) {
+        float v = 0.f;
+        if (e < L.w2) {
+            const int K = pad32(in), n = (int)(e / K), k = kat((int)(e % K));
+            if (k < in) v = p32[o1 + (size_t)n * in + k];
+        } else if (e < L.w3) {
+            const int K = pad32(H), n = (int)((e - L.w2) / K), k = kat((int)((e - L.w2) % K));
+            if (k < H) v = p32[o2 + (size_t)n * H + k];
+        } else if (e < L.w2t) {
+            const int K = pad32(H), n = (int)((e - L.w3) / K), k = kat((int)((e - L.w3) % K));
+            if (k < H) v = p32[o3 + (size_t)n * H + k];
+        } else if (e < L.w3t) {
+            const int K = pad32(H), n = (int)((e - L.w2t) / K), k = kat((int)((e - L.w2t) % K));
+            if (k < H) v = p32[o2 + (size_t)k * H + n];
+        } else {
+            const int K = pad32(out), n = (int)((e - L.w3t) / K), k = kat((int)((e - L.w3t) % K));
+            if (k < out) v = p32[o3 + (size_t)k * H + n];
+        }
+        w[e] = __float2bfloat16(v);
+    }
+}
+
+// epi(n0, acc): acc = X W^T for the CTA's 16 rows and columns n0 .. n0 + 15, in
+// the accumulator layout of two N tiles; X in shared memory (row stride ld, a
+// multiple of 8 whose eighth is odd: conflict-free 16-byte reads), W in global
+// memory (row stride K = pad32), both with kpos order along k.  A warp takes
+// 16 columns at a time and loads 256 wide steps of both tiles at once.
+template <typename Epi>
+__device__ __forceinline__ void rows_layer(const __nv_bfloat16* X, int ld, int K, const __nv_bfloat16* __restrict__ W,
+                                           int N, Epi epi)
+{
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    const int g = lane >> 2, t = lane & 3;
+    for (int n0 = 16 * warp; n0 < N; n0 += 16 * nw) {
+        float acc[2][4] = {};
+        const uint4* w0 = reinterpret_cast<const uint4*>(W + (size_t)min(n0 + g, N - 1) * K) + t;
+        const uint4* w1 = reinterpret_cast<const uint4*>(W + (size_t)min(n0 + 8 + g, N - 1) * K) + t;
+        for (int kb = 0; kb < K; kb += 256) {
+            uint4 b[8][2];
+#pragma unroll
+            for (int u = 0; u < 8; u++) {
+                const bool on = kb + 32 * u < K;
+                b[u][0] = on ? __ldg(w0 + (kb >> 3) + 4 * u) : make_uint4(0, 0, 0, 0);
+                b[u][1] = on ? __ldg(w1 + (kb >> 3) + 4 * u) : make_uint4(0, 0, 0, 0);
+            }
+#pragma unroll
+            for (int u = 0; u < 8; u++) {
+                if (kb + 32 * u >= K) break;
+                const uint4 lo = *reinterpret_cast<const uint4*>(X + g * ld + kb + 32 * u + 8 * t);
+                const uint4 hi = *reinterpret_cast<const uint4*>(X + (8 + g) * ld + kb + 32 * u + 8 * t);
+                const uint32_t f0[4] = {lo.x, hi.x, lo.y, hi.y}, f1[4] = {lo.z, hi.z, lo.w, hi.w};
+#pragma unroll
+                for (int j = 0; j < 2; j++) {
+                    mma_bf16(acc[j], f0, b[u][j].x, b[u][j].y);
+                    mma_bf16(acc[j], f1, b[u][j].z, b[u][j].w);
+                }
+            }
+        }
+        epi(n0, acc);
+    }
+}
+
+// Shared memory of a row CTA, in bytes; grad: with what the backward pass keeps.
+struct RowsLayout {
+    int ldx, ldh, ldo;  // row strides (elements)
+    size_t x, a1, a2, z1, z2, y, dyf, dy, d2, comp, total;
+};
+__host__ __device__ inline RowsLayout rows_layout(int in, int H, int out, int D, bool grad)
+{
+    RowsLayout r;
+    r.ldx = pad32(in) + 8;
+    r.ldh = pad32(H) + 8;
+    r.ldo = pad32(out) + 8;
+    size_t o = 0;
+    auto take = [&](size_t bytes) {
+        const size_t at = o;
+        o += (bytes + 15) & ~size_t(15);
+        return at;
+    };
+    r.x = take(sizeof(__nv_bfloat16) * kRows * r.ldx);
+    r.a1 = take(sizeof(__nv_bfloat16) * kRows * r.ldh);
+    r.a2 = take(sizeof(__nv_bfloat16) * kRows * r.ldh);
+    r.z1 = r.z2 = r.y = r.dyf = r.dy = r.d2 = r.comp = 0;
+    if (grad) {
+        r.z1 = take(sizeof(float) * kRows * H);
+        r.z2 = take(sizeof(float) * kRows * H);
+        r.y = take(sizeof(float) * kRows * out);
+        r.dyf = take(sizeof(float) * kRows * out);
+        r.dy = take(sizeof(__nv_bfloat16) * kRows * r.ldo);
+        r.d2 = take(sizeof(__nv_bfloat16) * kRows * r.ldh);
+        r.comp = take(sizeof(float) * kRows * (17 + D));
+    }
+    r.total = o;
+    return r;
+}
+
+struct RowsArgs {
+    int B, BP, in, H, out, K, D;
+    const float *x, *target;          // [B][in], [B][D] (host-pinned)
+    const float* p32;                 // biases
+    const __nv_bfloat16* w;
+    float* y;                         // [B][out] (host-pinned; forward only)
+    float* loss;                      // [B] (host-pinned)
+    __nv_bfloat16 *xT, *a1T, *a2T, *dyT, *d2T, *d1T;  // [feature][BP]
+    float* colsum;                    // [CTAs][out + 2 H]: sums of dy, d2, d1 over the CTA's rows
+};
+
+// Sum over the CTA's 16 rows of one column pair of a layer's epilogue: v[q]
+// of lane (g, t) as in the accumulators; every lane ends with columns 2t, 2t+1.
+__device__ __forceinline__ float2 rows_colsum(const float (&v)[4])
+{
+    float2 s = make_float2(v[0] + v[2], v[1] + v[3]);
+#pragma unroll
+    for (int off = 4; off < 32; off <<= 1) {
+        s.x += __shfl_xor_sync(0xffffffffu, s.x, off);
+        s.y += __shfl_xor_sync(0xffffffffu, s.y, off);
+    }
+    return s;
+}
+
+// [16 rows][n] of shared memory (kpos order along n) to the CTA's half of a
+// 32-row group of [n][BP] in global memory (kpos order along the rows), 8
+// bytes of a feature per thread.
+__device__ __forceinline__ void rows_transpose(const __nv_bfloat16* S, int ld, int n, __nv_bfloat16* __restrict__ T,
+                                               int BP, int row0)
+{
+    const int base = row0 & ~31, half = (row0 >> 4) & 1;
+    for (int e = threadIdx.x; e < n * 4; e += blockDim.x) {
+        const int f = e >> 2, t = e & 3, c = kpos(f);
+        __align__(8) __nv_bfloat16 v[4];
+#pragma unroll
+        for (int q = 0; q < 4; q++) v[q] = S[(2 * t + (q & 1) + 8 * (q >> 1)) * ld + c];
+        *reinterpret_cast<uint2*>(T + (size_t)f * BP + base + 8 * t + 4 * half) = *reinterpret_cast<const uint2*>(v);
+    }
+}
+
+template <bool GRAD>
+__global__ void __launch_bounds__(kRowThreads) mlp_rows_kernel(const RowsArgs A)
+{
+    extern __shared__ uint4 rows_smem[];
+    char* base = reinterpret_cast<char*>(rows_smem);
+    const RowsLayout R = rows_layout(A.in, A.H, A.out, A.D, GRAD);
+    const PackedW L = packed_layout(A.in, A.H, A.out);
+    __nv_bfloat16* xs = reinterpret_cast<__nv_bfloat16*>(base + R.x);
+    __nv_bfloat16* a1 = reinterpret_cast<__nv_bfloat16*>(base + R.a1);
+    __nv_bfloat16* a2 = reinterpret_cast<__nv_bfloat16*>(base + R.a2);
+    float* z1 = reinterpret_cast<float*>(base + R.z1);
+    float* z2 = reinterpret_cast<float*>(base + R.z2);
+    float* ys = reinterpret_cast<float*>(base + R.y);
+    float* dyf = reinterpret_cast<float*>(base + R.dyf);
+    __nv_bfloat16* dys = reinterpret_cast<__nv_bfloat16*>(base + R.dy);
+    __nv_bfloat16* d2s = reinterpret_cast<__nv_bfloat16*>(base + R.d2);
+    float* comp = reinterpret_cast<float*>(base + R.comp);
+    const int tid = threadIdx.x, lane = tid & 31, g = lane >> 2, t = lane & 3;
+    const int row0 = blockIdx.x * kRows, H = A.H, out = A.out;
+    const float* b1 = A.p32 + (size_t)H * A.in;
+    const float* b2 = b1 + H + (size_t)H * H;
+    const float* b3 = b2 + H + (size_t)out * H;
+    // inputs rounded to BF16, zero beyond the batch and the input size; the
+    // padding of the activations is zero too (it meets zero weights)
+    for (int e = tid; e < kRows * R.ldx; e += kRowThreads) {
+        const int r = e / R.ldx, k = e % R.ldx;
+        if (k >= pad32(A.in)) continue;
+        xs[r * R.ldx + kpos(k)] =
+            __float2bfloat16((row0 + r < A.B && k < A.in) ? A.x[(size_t)(row0 + r) * A.in + k] : 0.f);
+    }
+    float* tgt = comp + kRows * 17;  // [32][D]
+    if (GRAD)
+        for (int e = tid; e < kRows * A.D; e += kRowThreads)
+            tgt[e] = (row0 + e / A.D < A.B) ? A.target[(size_t)row0 * A.D + e] : 0.f;
+    const int padH = pad32(H) - H;
+    for (int e = tid; e < kRows * padH; e += kRowThreads) {
+        const int r = e / padH, k = kpos(H + e % padH);
+        a1[r * R.ldh + k] = a2[r * R.ldh + k] = __float2bfloat16(0.f);
+        if (GRAD) d2s[r * R.ldh + k] = __float2bfloat16(0.f);
+    }
+    __syncthreads();
+    auto hidden = [&](const float* b, __nv_bfloat16* a, float* z) {
+        return [=](int n0, float (&acc)[2][4]) {
+#pragma unroll
+            for (int j = 0; j < 2; j++)
+#pragma unroll
+                for (int q = 0; q < 4; q++) {
+                    const int n = n0 + 8 * j + 2 * t + (q & 1), r = 8 * (q >> 1) + g;
+                    if (n >= H) continue;
+                    const float zz = acc[j][q] + __ldg(b + n);
+                    if (GRAD) z[r * H + n] = zz;
+                    a[r * R.ldh + kpos(n)] = __float2bfloat16(silu(zz));
+                }
+        };
+    };
+    rows_layer(xs, R.ldx, pad32(A.in), A.w + L.w1, H, hidden(b1, a1, z1));
+    __syncthreads();
+    rows_layer(a1, R.ldh, pad32(H), A.w + L.w2, H, hidden(b2, a2, z2));
+    __syncthreads();
+    rows_layer(a2, R.ldh, pad32(H), A.w + L.w3, out, [&](int n0, float (&acc)[2][4]) {
+#pragma unroll
+        for (int j = 0; j < 2; j++)
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                const int n = n0 + 8 * j + 2 * t + (q & 1), r = 8 * (q >> 1) + g;
+                if (n >= out) continue;
+                const float v = acc[j][q] + __ldg(b3 + n);
+                if (GRAD) ys[r * out + n] = v;
+                else if (row0 + r < A.B) A.y[(size_t)(row0 + r) * out + n] = v;
+            }
+    });
+    if (!GRAD) return;
+    __syncthreads();
+    // mixture negative log-likelihood (mixture_nll_kernel's formulas) and its
+    // gradient: a lane per component, then the lanes over the outputs
+    const int K = A.K, D = A.D, KD = K * D;
+    {
+        const int r = tid >> 5, k = tid & 31;  // a warp per row
+        const float* ym = ys + r * out;
+        const bool on = row0 + r < A.B;
+        if (on && k < K) {
+            float mx = -INFINITY;
+            for (int q = 0; q < K; q++) mx = fmaxf(mx, ym[q]);
+            float se = 0.f;
+            for (int q = 0; q < K; q++) se += __expf(ym[q] - mx);
+            const float lw = ym[k] - (mx + __logf(se));
+            float sl = -0.91893853320467274f * D;  // -D/2 log(2 pi)
+            const float* x = tgt + r * D;
+            for (int d = 0; d < D; d++) {
+                const float ls = fminf(fmaxf(ym[K + KD + k * D + d], -7.f), 5.f);
+                const float rr = (x[d] - ym[K + k * D + d]) * __expf(-ls);
+                sl += -0.5f * rr * rr - ls;
+            }
+            comp[r * 17 + k] = lw;
+            comp[r * 17 + 8 + k] = lw + sl;
+        }
+        __syncwarp();
+        float ll = 0.f;
+        if (on) {
+            float best = -INFINITY, tot = 0.f;
+            for (int q = 0; q < K; q++) best = fmaxf(best, comp[r * 17 + 8 + q]);
+            for (int q = 0; q < K; q++) tot += __expf(comp[r * 17 + 8 + q] - best);
+            ll = best + __logf(tot);
+            if (k == 0) A.loss[row0 + r] = -ll;
+        }
+        const float inv = 1.f / (float)A.B;
+        for (int o = k; o < pad32(out); o += 32) {
+            float v = 0.f;
+            if (on && o < out) {
+                const int q = (o < K) ? o : ((o - K) % KD) / D;
+                const float rk = __expf(comp[r * 17 + 8 + q] - ll);  // responsibility
+                if (o < K) {
+                    v = (__expf(comp[r * 17 + q]) - rk) * inv;  // d(-ll)/d logit
+                } else {
+                    const int d = (o - K) % D;
+                    const float raw = ym[K + KD + q * D + d];
+                    const float ls = fminf(fmaxf(raw, -7.f), 5.f);
+                    const float iv = __expf(-2.f * ls);
+                    const float diff = tgt[r * D + d] - ym[K + q * D + d];
+                    if (o < K + KD) v = -rk * diff * iv * inv;
+                    else if (raw > -7.f && raw < 5.f) v = (-rk * (diff * diff * iv - 1.f)) * inv;
+                }
+            }
+            dys[r * R.ldo + kpos(o)] = __float2bfloat16(v);
+            if (o < out) dyf[r * out + o] = v;
+        }
+    }
+    __syncthreads();
+    float* sums = A.colsum + (size_t)blockIdx.x * (out + 2 * H);
+    for (int o = tid; o < out; o += kRowThreads) {
+        float v = 0.f;
+        for (int r = 0; r < kRows; r++) v += dyf[r * out + o];
+        sums[o] = v;
+    }
+    rows_transpose(xs, R.ldx, A.in, A.xT, A.BP, row0);
+    rows_transpose(a1, R.ldh, H, A.a1T, A.BP, row0);
+    rows_transpose(a2, R.ldh, H, A.a2T, A.BP, row0);
+    rows_transpose(dys, R.ldo, out, A.dyT, A.BP, row0);
+    // backward data path: d = (d_next W) * silu'(z), rounded to BF16 for the
+    // next product, its FP32 column sums for the bias gradient
+    auto back = [&](__nv_bfloat16* d, const float* z, float* cs) {
+        return [=](int n0, float (&acc)[2][4]) {
+#pragma unroll
+            for (int j = 0; j < 2; j++) {
+                const int n = n0 + 8 * j + 2 * t;
+                float v[4];
+#pragma unroll
+                for (int q = 0; q < 4; q++) {
+                    const int r = 8 * (q >> 1) + g, nn = n + (q & 1);
+                    v[q] = (nn < H) ? acc[j][q] * dsilu(z[r * H + nn]) : 0.f;
+                    if (nn < H) d[r * R.ldh + kpos(nn)] = __float2bfloat16(v[q]);
+                }
+                const float2 cv = rows_colsum(v);
+                if (g == 0) {
+                    if (n < H) cs[n] = cv.x;
+                    if (n + 1 < H) cs[n + 1] = cv.y;
+                }
+            }
+        };
+    };
+    rows_layer(dys, R.ldo, pad32(out), A.w + L.w3t, H, back(d2s, z2, sums + out));
+    __syncthreads();  // d2 complete; a2 has been copied out and its place is free for d1
+    rows_transpose(d2s, R.ldh, H, A.d2T, A.BP, row0);
+    rows_layer(d2s, R.ldh, pad32(H), A.w + L.w2t, H, back(a2, z1, sums + out + H));
+    __syncthreads();
+    rows_transpose(a2, R.ldh, H, A.d1T, A.BP, row0);
+}
+
+// Weight gradients dW[m][n] = sum_b U[m][b] V[n][b] for the three layers, one
+// 32 x 32 tile per CTA (four warps of 16 x 16), both operands feature-major;
+// the last CTAs add the bias column sums of the row CTAs in order.
+struct WgradArgs {
+    int BP, in, H, out, nrows;  // nrows: row CTAs
+    const __nv_bfloat16 *xT, *a1T, *a2T, *dyT, *d2T, *d1T;
+    const float* colsum;
+    float* grad;
+};
+
+__global__ void __launch_bounds__(128) mlp_wgrad_kernel(const WgradArgs A)
+{
+    const int tO = (A.out + 31) / 32, tH = (A.H + 31) / 32, tI = (A.in + 31) / 32;
+    const size_t o1 = 0, ob1 = (size_t)A.H * A.in, o2 = ob1 + A.H, ob2 = o2 + (size_t)A.H * A.H, o3 = ob2 + A.H,
+                 ob3 = o3 + (size_t)A.out * A.H;
+    int job = blockIdx.x;
+    const __nv_bfloat16 *U, *V;
+    int M, N, tn;
+    float* C;
+    if (job < tH * tH) {
+        U = A.d2T, V = A.a1T, M = A.H, N = A.H, tn = tH, C = A.grad + o2;
+    } else if ((job -= tH * tH) < tO * tH) {
+        U = A.dyT, V = A.a2T, M = A.out, N = A.H, tn = tH, C = A.grad + o3;
+    } else if ((job -= tO * tH) < tH * tI) {
+        U = A.d1T, V = A.xT, M = A.H, N = A.in, tn = tI, C = A.grad + o1;
+    } else {
+        const int f = (job - tH * tI) * 128 + threadIdx.x, F = A.out + 2 * A.H;
+        if (f >= F) return;
+        float v = 0.f;
+        for (int c = 0; c < A.nrows; c++) v += A.colsum[(size_t)c * F + f];
+        A.grad[f < A.out ? ob3 + f : (f < A.out + A.H ? ob2 + f - A.out : ob1 + f - A.out - A.H)] = v;
+        return;
+    }
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
+    const int m0 = (job / tn) * 32 + 16 * (warp >> 1), n0 = (job % tn) * 32 + 16 * (warp & 1);
+    const uint4* u0 = reinterpret_cast<const uint4*>(U + (size_t)min(m0 + g, M - 1) * A.BP) + t;
+    const uint4* u1 = reinterpret_cast<const uint4*>(U + (size_t)min(m0 + 8 + g, M - 1) * A.BP) + t;
+    const uint4* v0 = reinterpret_cast<const uint4*>(V + (size_t)min(n0 + g, N - 1) * A.BP) + t;
+    const uint4* v1 = reinterpret_cast<const uint4*>(V + (size_t)min(n0 + 8 + g, N - 1) * A.BP) + t;
+    float acc[2][4] = {};
+    for (int kb = 0; kb < A.BP; kb += 128) {
+        uint4 a[4][2], b[4][2];
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            const bool on = kb + 32 * u < A.BP;
+            const int at = (kb >> 3) + 4 * u;
+            const uint4 zero = make_uint4(0, 0, 0, 0);
+            a[u][0] = on ? __ldg(u0 + at) : zero;
+            a[u][1] = on ? __ldg(u1 + at) : zero;
+            b[u][0] = on ? __ldg(v0 + at) : zero;
+            b[u][1] = on ? __ldg(v1 + at) : zero;
+        }
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            const uint32_t f0[4] = {a[u][0].x, a[u][1].x, a[u][0].y, a[u][1].y};
+            const uint32_t f1[4] = {a[u][0].z, a[u][1].z, a[u][0].w, a[u][1].w};
+#pragma unroll
+            for (int j = 0; j < 2; j++) {
+                mma_bf16(acc[j], f0, b[u][j].x, b[u][j].y);
+                mma_bf16(acc[j], f1, b[u][j].z, b[u][j].w);
+            }
+        }
+    }
+#pragma unroll
+    for (int j = 0; j < 2; j++)
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            const int m = m0 + g + 8 * (q >> 1), n = n0 + 8 * j + 2 * t + (q & 1);
+            if (m < M && n < N) C[(size_t)m * N + n] = acc[j][q];
+        }
+}
+
 }  // namespace
 
 static int mlp_offsets(const messi_mlp* m, size_t off[6])
@@ -353,44 +799,122 @@ static int mlp_offsets(const messi_mlp* m, size_t off[6])
 static int mlp_reserve(messi_ctx* ctx, messi_mlp* m, int batch)
 {
     if (batch <= m->cap) return MESSI_OK;
-    cudaFree(m->x);
-    cudaFree(m->a1);
-    cudaFree(m->a2);
-    cudaFree(m->z1);
-    cudaFree(m->z2);
-    cudaFree(m->y);
-    cudaFree(m->dy);
-    cudaFree(m->d2);
-    cudaFree(m->d1);
-    cudaFree(m->target);
-    cudaFree(m->loss);
+    void** act[] = {(void**)&m->x,  (void**)&m->a1, (void**)&m->a2, (void**)&m->z1,  (void**)&m->z2,  (void**)&m->y,
+                    (void**)&m->dy, (void**)&m->d2, (void**)&m->d1, (void**)&m->target, (void**)&m->loss,
+                    (void**)&m->xT, (void**)&m->a1T, (void**)&m->a2T, (void**)&m->dyT, (void**)&m->d2T,
+                    (void**)&m->d1T, (void**)&m->colsum};
+    for (void** p : act) {
+        cudaFree(*p);
+        *p = nullptr;
+    }
     cudaFreeHost(m->stage);
+    m->stage = nullptr;
+    m->cap = 0;
     const size_t B = (size_t)batch;
     cudaError_t e = cudaSuccess;
     auto al = [&](void** p, size_t bytes) {
         if (e == cudaSuccess) e = cudaMalloc(p, bytes);
     };
-    al((void**)&m->x, B * m->in * 2);
-    al((void**)&m->a1, B * m->H * 2);
-    al((void**)&m->a2, B * m->H * 2);
-    al((void**)&m->z1, B * m->H * 4);
-    al((void**)&m->z2, B * m->H * 4);
-    al((void**)&m->y, B * m->out * 4);
-    al((void**)&m->dy, B * m->out * 4);
-    al((void**)&m->d2, B * m->H * 4);
-    al((void**)&m->d1, B * m->H * 4);
-    al((void**)&m->target, B * m->D * 4);
-    al((void**)&m->loss, B * 4 + 64);
-    if (e == cudaSuccess) e = cudaMallocHost((void**)&m->stage, B * (m->in + m->out + m->D + 2) * 4 + 64);
-    if (e != cudaSuccess) {
-        m->cap = 0;
-        return cuda_fail(ctx, e, "mlp activations");
+    if (m->fused) {
+        const size_t BP = (size_t)pad32(batch);
+        al((void**)&m->xT, BP * m->in * 2);
+        al((void**)&m->a1T, BP * m->H * 2);
+        al((void**)&m->a2T, BP * m->H * 2);
+        al((void**)&m->dyT, BP * m->out * 2);
+        al((void**)&m->d2T, BP * m->H * 2);
+        al((void**)&m->d1T, BP * m->H * 2);
+        al((void**)&m->colsum, BP / kRows * (m->out + 2 * m->H) * 4);
+    } else {
+        al((void**)&m->x, B * m->in * 2);
+        al((void**)&m->a1, B * m->H * 2);
+        al((void**)&m->a2, B * m->H * 2);
+        al((void**)&m->z1, B * m->H * 4);
+        al((void**)&m->z2, B * m->H * 4);
+        al((void**)&m->y, B * m->out * 4);
+        al((void**)&m->dy, B * m->out * 4);
+        al((void**)&m->d2, B * m->H * 4);
+        al((void**)&m->d1, B * m->H * 4);
+        al((void**)&m->target, B * m->D * 4);
+        al((void**)&m->loss, B * 4 + 64);
     }
+    if (e == cudaSuccess) e = cudaMallocHost((void**)&m->stage, B * (m->in + m->out + m->D + 2) * 4 + 64);
+    if (e != cudaSuccess) return cuda_fail(ctx, e, "mlp activations");
     m->cap = batch;
     return MESSI_OK;
 }
 
 static inline unsigned blocks(long long n) { return (unsigned)((n + 255) / 256); }
+
+// ---- two-kernel form, host side ----
+// Repacks the BF16 weights from the FP32 master copy (queued on the stream).
+static int fused_pack(messi_ctx* ctx, messi_mlp* m)
+{
+    if (!m->fused) return MESSI_OK;
+    pack_weights_kernel<<<152, 256, 0, ctx->stream>>>(m->p32, m->w16, m->in, m->H, m->out);
+    LAUNCH_CHECK(ctx, "pack_weights_kernel");
+    return MESSI_OK;
+}
+
+// Host staging (pinned, read and written by the kernels): x, target, y, loss.
+static float* stage_target(messi_mlp* m) { return m->stage + (size_t)m->cap * m->in; }
+static float* stage_y(messi_mlp* m) { return stage_target(m) + (size_t)m->cap * m->D; }
+static float* stage_loss(messi_mlp* m) { return stage_y(m) + (size_t)m->cap * m->out; }
+
+static RowsArgs rows_args(messi_mlp* m, int batch)
+{
+    RowsArgs a{};
+    a.B = batch;
+    a.BP = pad32(batch);
+    a.in = m->in;
+    a.H = m->H;
+    a.out = m->out;
+    a.K = m->K;
+    a.D = m->D;
+    a.x = m->stage;
+    a.target = stage_target(m);
+    a.p32 = m->p32;
+    a.w = m->w16;
+    a.y = stage_y(m);
+    a.loss = stage_loss(m);
+    a.xT = m->xT;
+    a.a1T = m->a1T;
+    a.a2T = m->a2T;
+    a.dyT = m->dyT;
+    a.d2T = m->d2T;
+    a.d1T = m->d1T;
+    a.colsum = m->colsum;
+    return a;
+}
+
+static int fused_rows(messi_ctx* ctx, messi_mlp* m, int batch, bool grad)
+{
+    const size_t smem = rows_layout(m->in, m->H, m->out, m->D, grad).total;
+    const void* kernel = grad ? (const void*)mlp_rows_kernel<true> : (const void*)mlp_rows_kernel<false>;
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return cuda_fail(ctx, e, "mlp_rows_kernel attributes");
+    // the gradients' operands are whole groups of 32 rows
+    const int grid = grad ? pad32(batch) / kRows : (batch + kRows - 1) / kRows;
+    if (grad) mlp_rows_kernel<true><<<grid, kRowThreads, smem, ctx->stream>>>(rows_args(m, batch));
+    else mlp_rows_kernel<false><<<grid, kRowThreads, smem, ctx->stream>>>(rows_args(m, batch));
+    LAUNCH_CHECK(ctx, "mlp_rows_kernel");
+    return MESSI_OK;
+}
+
+// loss in the staging buffer, gradients in m->grad
+static int fused_gradients(messi_ctx* ctx, messi_mlp* m, int batch, const float* x, const float* target)
+{
+    std::memcpy(m->stage, x, sizeof(float) * batch * m->in);
+    std::memcpy(stage_target(m), target, sizeof(float) * batch * m->D);
+    int rc;
+    if ((rc = fused_rows(ctx, m, batch, true))) return rc;
+    WgradArgs w{pad32(batch), m->in, m->H, m->out, pad32(batch) / kRows, m->xT, m->a1T, m->a2T, m->dyT, m->d2T,
+                m->d1T, m->colsum, m->grad};
+    const int tO = (m->out + 31) / 32, tH = (m->H + 31) / 32, tI = (m->in + 31) / 32;
+    const int jobs = tH * tH + tO * tH + tH * tI + (m->out + 2 * m->H + 127) / 128;
+    mlp_wgrad_kernel<<<jobs, 128, 0, ctx->stream>>>(w);
+    LAUNCH_CHECK(ctx, "mlp_wgrad_kernel");
+    return MESSI_OK;
+}
 
 // forward pass on the batch already in m->x (BF16)
 static int mlp_forward_dev(messi_ctx* ctx, messi_mlp* m, int Bn)
@@ -520,11 +1044,22 @@ int messi_mlp_create(messi_ctx* ctx, int32_t in_dim, int32_t width, int32_t ncom
         messi_mlp_destroy(m);
         return cuda_fail(ctx, e, "mlp parameters");
     }
+    // two-kernel form where 16 rows of activations fit half an SM's shared memory
+    m->fused = rows_layout(in_dim, width, m->out, dim, true).total <= kRowsMaxSmem;
+    if (m->fused) {
+        const size_t n = packed_layout(in_dim, width, m->out).total;
+        e = cudaMalloc((void**)&m->w16, sizeof(__nv_bfloat16) * n);
+        if (e != cudaSuccess) {
+            messi_mlp_destroy(m);
+            return cuda_fail(ctx, e, "mlp packed weights");
+        }
+    }
     to_bf16_kernel<<<blocks(m->nparam), 256, 0, ctx->stream>>>(m->p32, m->p16, m->nparam);
+    const int prc = fused_pack(ctx, m);
     e = cudaStreamSynchronize(ctx->stream);
-    if (e != cudaSuccess) {
+    if (prc || e != cudaSuccess) {
         messi_mlp_destroy(m);
-        return cuda_fail(ctx, e, "mlp init");
+        return prc ? prc : cuda_fail(ctx, e, "mlp init");
     }
     *out = m;
     return MESSI_OK;
@@ -534,7 +1069,8 @@ int messi_mlp_destroy(messi_mlp* m)
 {
     if (!m) return MESSI_EINVAL;
     void* ptrs[] = {m->p32, m->p16, m->grad, m->m1, m->m2, m->x, m->a1, m->a2, m->z1,
-                    m->z2,  m->y,   m->dy,   m->d2, m->d1, m->target, m->loss};
+                    m->z2,  m->y,   m->dy,   m->d2, m->d1, m->target, m->loss,
+                    m->w16, m->xT,  m->a1T,  m->a2T, m->dyT, m->d2T, m->d1T, m->colsum};
     for (void* p : ptrs)
         if (p) cudaFree(p);
     if (m->stage) cudaFreeHost(m->stage);
@@ -564,8 +1100,9 @@ int messi_mlp_set_params(messi_ctx* ctx, messi_mlp* m, const float* host)
     cudaError_t e = cudaMemcpy(m->p32, host, sizeof(float) * m->nparam, cudaMemcpyHostToDevice);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "mlp set params");
     to_bf16_kernel<<<blocks(m->nparam), 256, 0, ctx->stream>>>(m->p32, m->p16, m->nparam);
+    const int rc = fused_pack(ctx, m);
     e = cudaStreamSynchronize(ctx->stream);
-    return (e == cudaSuccess) ? MESSI_OK : cuda_fail(ctx, e, "mlp set params");
+    return rc ? rc : ((e == cudaSuccess) ? MESSI_OK : cuda_fail(ctx, e, "mlp set params"));
 }
 
 int messi_mlp_forward(messi_ctx* ctx, messi_mlp* m, int32_t batch, const float* x, float* y)
@@ -574,6 +1111,15 @@ int messi_mlp_forward(messi_ctx* ctx, messi_mlp* m, int32_t batch, const float* 
     ctx->launches = 0;
     cudaSetDevice(ctx->device);
     int rc;
+    if (m->fused) {
+        if ((rc = mlp_reserve(ctx, m, batch))) return rc;
+        std::memcpy(m->stage, x, sizeof(float) * batch * m->in);
+        if ((rc = fused_rows(ctx, m, batch, false))) return rc;
+        const cudaError_t fe = cudaStreamSynchronize(ctx->stream);
+        if (fe != cudaSuccess) return cuda_fail(ctx, fe, "mlp forward");
+        std::memcpy(y, stage_y(m), sizeof(float) * batch * m->out);
+        return MESSI_OK;
+    }
     if ((rc = upload_batch(ctx, m, batch, x, nullptr))) return rc;
     if ((rc = mlp_forward_dev(ctx, m, batch))) return rc;
     cudaError_t e = cudaMemcpyAsync(y, m->y, sizeof(float) * batch * m->out, cudaMemcpyDeviceToHost, ctx->stream);
@@ -588,15 +1134,22 @@ int messi_mlp_gradients(messi_ctx* ctx, messi_mlp* m, int32_t batch, const float
     ctx->launches = 0;
     cudaSetDevice(ctx->device);
     int rc;
-    if ((rc = upload_batch(ctx, m, batch, x, target))) return rc;
-    if ((rc = mlp_forward_dev(ctx, m, batch))) return rc;
-    if ((rc = mlp_backward_dev(ctx, m, batch))) return rc;
     std::vector<float> l(batch);
-    cudaError_t e = cudaMemcpyAsync(l.data(), m->loss, sizeof(float) * batch, cudaMemcpyDeviceToHost, ctx->stream);
+    cudaError_t e = cudaSuccess;
+    if (m->fused) {
+        if ((rc = mlp_reserve(ctx, m, batch))) return rc;
+        if ((rc = fused_gradients(ctx, m, batch, x, target))) return rc;
+    } else {
+        if ((rc = upload_batch(ctx, m, batch, x, target))) return rc;
+        if ((rc = mlp_forward_dev(ctx, m, batch))) return rc;
+        if ((rc = mlp_backward_dev(ctx, m, batch))) return rc;
+        e = cudaMemcpyAsync(l.data(), m->loss, sizeof(float) * batch, cudaMemcpyDeviceToHost, ctx->stream);
+    }
     if (e == cudaSuccess && grads)
         e = cudaMemcpyAsync(grads, m->grad, sizeof(float) * m->nparam, cudaMemcpyDeviceToHost, ctx->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "mlp gradients");
+    if (m->fused) std::memcpy(l.data(), stage_loss(m), sizeof(float) * batch);
     if (loss) {
         double s = 0.0;
         for (float v : l) s += v;
@@ -626,6 +1179,7 @@ int messi_mlp_train_step(messi_ctx* ctx, messi_mlp* m, int32_t batch, const floa
     adam_kernel<<<blocks(m->nparam), 256, 0, ctx->stream>>>(m->p32, m->grad, m->m1, m->m2, m->p16, m->nparam, lr, b1,
                                                             b2, c1, c2, 1e-8f, clip);
     LAUNCH_CHECK(ctx, "adam_kernel");
+    if ((rc = fused_pack(ctx, m))) return rc;
     e = cudaStreamSynchronize(ctx->stream);
     return (e == cudaSuccess) ? MESSI_OK : cuda_fail(ctx, e, "adam");
 }
