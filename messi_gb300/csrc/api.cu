@@ -629,7 +629,7 @@ int messi_dataset_destroy(messi_dataset* ds)
         tune_forget(ctx, ds);
     }
     void* bufs[] = {ds->d_bandidx, ds->d_idx, ds->d_leaf, ds->d_segs, ds->d_steps, ds->d_tiles, ds->d_masks, ds->d_tree,
-                    ds->d_post, ds->d_arena_f, ds->d_arena_e, ds->d_mix, ds->d_mixlam, ds->d_leafnode};
+                    ds->d_uops, ds->d_arena_f, ds->d_arena_e, ds->d_mix, ds->d_mixlam, ds->d_leafnode};
     for (void* b : bufs)
         if (b) cudaFree(b);
     delete ds;
@@ -717,9 +717,7 @@ int messi_siterate_conditionals(messi_ctx* ctx, messi_dataset* ds, const messi_m
     if ((rc = ensure(ctx, kSlotVec, (size_t)L * sizeof(double), &pu))) return rc;
     if ((rc = launch_unpaired(ctx, ds, md.P4, ds->numnodes, md.pi4, md.logw_site, ns, (double*)pu, nullptr)))
         return rc;
-    // per-site unpaired log-likelihoods: the last block of the unpaired scratch
-    const size_t n = (size_t)ds->numnodes * L;
-    const double* d_ull = (const double*)ctx->scratch[20].p + (size_t)ns * n * 5;
+    const double* d_ull = (const double*)ctx->scratch[kSlotUnpaired].p;  // per-site unpaired log-likelihoods
     if ((rc = h2d(ctx, d_pair, pairprobs, (size_t)L * L * sizeof(double)))) return rc;
     if ((rc = h2d(ctx, d_single, singleprobs, (size_t)L * sizeof(double)))) return rc;
     if ((rc = launch_siterate_conditionals(ctx, ds, d_catll, md.logw, ns, md.cat.nlam, d_single, d_pair, d_ull,

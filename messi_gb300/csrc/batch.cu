@@ -587,11 +587,11 @@ int messi_batch_likelihood(messi_ctx* ctx, messi_batch* b, const messi_model* mo
         return fail(ctx, MESSI_ENOMEM, "batch unpaired transition matrices");
     if (b->stage.p != old_stage || b->P16.p != old_P || b->P4.p != old_P4) b->gen++;
     {
-        // unpaired scratch: one buffer sized for the largest alignment, reused in stream order
+        // per-site unpaired values: one buffer sized for the largest alignment, reused in stream order
         size_t scratch = 0;
         for (int a = 0; a < n; a++)
-            scratch = std::max(scratch, (size_t)nsite * ((size_t)b->ds[a]->numnodes * b->ds[a]->L * 5 + b->ds[a]->L));
-        if ((rc = ensure(ctx, 20, scratch * sizeof(double), &ps))) return rc;
+            scratch = std::max(scratch, (size_t)nsite * b->ds[a]->L);
+        if ((rc = ensure(ctx, kSlotUnpaired, scratch * sizeof(double), &ps))) return rc;
     }
     if ((rc = prepare_batch_arena(ctx, b, C))) return rc;
     if ((rc = write_descriptors(ctx, b, grp))) return rc;

@@ -20,7 +20,8 @@ constexpr int kTile = 128;          // unique pairs per CTA in the pruning kerne
 // host-visible error flag (wave.cuh).
 constexpr int kSyncWords = 4;
 constexpr int kMaxLambda = 8;       // per-lambda conditionals kept in registers
-constexpr int kMaxStack = 512;      // tree height limit of the unpaired kernel
+constexpr int kMaxStack = 512;      // tree height limit
+constexpr int kSlotUnpaired = 20;   // scratch slot of the per-site unpaired log-likelihoods
 constexpr int kEigStride = 16 + 256 + 16;  // eigenvalues, U (row-major), sqrt(pi)
 constexpr int kEig4Stride = 4 + 16 + 4;
 
@@ -296,7 +297,8 @@ struct messi_dataset {
     int2* d_tiles = nullptr;
     uint8_t* d_masks = nullptr;        // [N][L]
     int* d_tree = nullptr;             // [numnodes][4]: child0, child1, seqindex, pad
-    int* d_post = nullptr;             // [numnodes] post-order
+    int4* d_uops = nullptr;            // [N - 1] unpaired program: children A, B, their sequences or -1
+    int unpaired_depth = 0;            // results its stack holds at most
     float* d_arena_f = nullptr;
     int* d_arena_e = nullptr;
     double* d_mix = nullptr;           // [nroot]
@@ -401,10 +403,10 @@ int run_pairs(messi_ctx* ctx, messi_dataset* ds, const float* d_P, const float* 
               const int* d_lam, int C, int nlam, bool per_lambda);
 // Unpaired column likelihoods of one tree whose transition matrices start at
 // d_P4 with node stride `pstride` (nodes of all site categories: [s][pstride][16]).
-// d_scratch: nsite * (numnodes * L * 5 + L) doubles, or nullptr for the
+// d_ll: nsite * L doubles for the per-site log-likelihoods, or nullptr for the
 // context's buffer (reused in stream order).
 int launch_unpaired(messi_ctx* ctx, messi_dataset* ds, const double* d_P4, int pstride, const double* d_pi4,
-                    const double* d_logw_site, int nsite, double* d_u, double* d_scratch);
+                    const double* d_logw_site, int nsite, double* d_u, double* d_ll);
 // Site-rate conditionals (prune.cu): catll [C][nroot] per-category root
 // log-likelihoods, ull [nsite][L] per-site unpaired log-likelihoods, single
 // [L] and pair [L x L] (column-major) posteriors; out [nsite x L] column-major;

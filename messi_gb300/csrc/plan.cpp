@@ -261,6 +261,43 @@ int build_plan(messi_dataset* ds, const messi_alignment* aln, int W, const uint8
             ds->level[v] = 1 + std::max(ds->level[ds->children[2 * v]], ds->level[ds->children[2 * v + 1]]);
     ds->H = ds->level[0];
 
+    // ---- program of the unpaired columns: internal nodes in post-order, the
+    // subtree whose evaluation stacks more first
+    std::vector<int4> uops;
+    {
+        std::vector<int> need(nn, 0);  // results stacked while the subtree is evaluated
+        for (int v : ds->postorder) {
+            const int a = ds->children[2 * v], b = ds->children[2 * v + 1];
+            if (a < 0) continue;
+            const bool ia = ds->children[2 * a] >= 0, ib = ds->children[2 * b] >= 0;
+            if (ia && ib) need[v] = std::max(std::max(need[a], need[b]), 1 + std::min(need[a], need[b]));
+            else need[v] = ia ? need[a] : (ib ? need[b] : 0);
+        }
+        std::vector<std::pair<int, char>> stack{{0, 0}};
+        while (!stack.empty()) {
+            const auto [v, expanded] = stack.back();
+            stack.pop_back();
+            int a = ds->children[2 * v], b = ds->children[2 * v + 1];
+            if (a < 0) continue;
+            const bool ia = ds->children[2 * a] >= 0, ib = ds->children[2 * b] >= 0;
+            // a: the child whose result comes last (the top), or the leaf when both are leaves
+            if (ia && ib) {
+                if (need[a] > need[b]) std::swap(a, b);
+            } else if (ib) {
+                std::swap(a, b);
+            }
+            if (expanded) {
+                uops.push_back(make_int4(a, b, ds->seqindex[a], ds->children[2 * b] < 0 ? ds->seqindex[b] : -1));
+                if (ds->children[2 * a] >= 0) uops.back().z = -1;
+            } else {
+                stack.push_back({v, 1});
+                stack.push_back({a, 0});
+                stack.push_back({b, 0});  // evaluated first
+            }
+        }
+        ds->unpaired_depth = need[0];
+    }
+
     // ---- column pattern ids per node (dense, first-occurrence order)
     std::vector<std::vector<int32_t>> pid(nn);
     std::vector<int32_t> npat(nn, 0);
@@ -522,7 +559,7 @@ int build_plan(messi_dataset* ds, const messi_alignment* aln, int W, const uint8
     UPLOAD(ds->d_leafnode, ds->leafnode_host.data(), ds->leafnode_host.size() * sizeof(int));
     UPLOAD(ds->d_masks, ds->masks.data(), ds->masks.size());
     UPLOAD(ds->d_tree, tree.data(), tree.size() * sizeof(int));
-    UPLOAD(ds->d_post, ds->postorder.data(), ds->postorder.size() * sizeof(int));
+    UPLOAD(ds->d_uops, uops.data(), uops.size() * sizeof(int4));
 #undef UPLOAD
     if ((e = cudaMalloc((void**)&ds->d_mix, sizeof(double) * std::max<int64_t>(ds->nroot, 1))) != cudaSuccess)
         goto cuda_error;

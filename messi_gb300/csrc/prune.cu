@@ -1039,68 +1039,100 @@ int run_pairs(messi_ctx* ctx, messi_dataset* ds, const float* d_P, const float* 
 }
 
 // ---------------------------------------------------------------------------
-// Unpaired columns: one thread per (column, site-rate category), nodes in
-// post-order, partials of every node kept in a [nsite][numnodes][L][4]
-// scratch table (FP64; the FP64 pipe is narrow on this part, so the work is
-// spread over many small blocks); then the mixture over site rates in the
-// reference's order.
+// Unpaired columns (FP64), a warp per eight columns and site-rate category,
+// lane 4 col + a for state a, then the mixture over site rates in the
+// reference's order.  The FP64 units issue a warp only every 64 cycles per SM
+// quarter, so the work is spread over four times the warps a thread per column
+// would give, a leaf's 0/1 vector costs additions only for its second to
+// fourth state, and the maximum is taken on the bits.  The nodes come as a
+// program (plan.cpp): the last result stays in registers, one that waits for
+// its sibling goes to a stack in shared memory, the deeper subtree first, so
+// that the stack holds at most log2(sequences) results.  64 sequences x 1,000
+// columns: 198 us with every node's partials in global memory and a thread per
+// column, 160 with the program alone, 62 now; 100 x 733: 310 -> 96 us.
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(32) unpaired_site_kernel(const uint8_t* __restrict__ masks,
-                                                           const int* __restrict__ tree, const int* __restrict__ post,
-                                                           int nn, int L, const double* __restrict__ P4, int pstride,
-                                                           const double* __restrict__ pi4, double* __restrict__ part,
-                                                           double* __restrict__ lmv, double* __restrict__ ll)
+__device__ __forceinline__ double shfl_d(double v, int src) { return __shfl_sync(0xffffffffu, v, src); }
+
+// staged: the tile's masks fit shared memory
+__global__ void __launch_bounds__(32) unpaired_site_kernel(const uint8_t* __restrict__ masks, int N,
+                                                           const int4* __restrict__ ops, int nops, int depth,
+                                                           int staged, int L, const double* __restrict__ P4,
+                                                           int pstride, const double* __restrict__ pi4,
+                                                           double* __restrict__ ll)
 {
-    const int x = blockIdx.x * blockDim.x + threadIdx.x;
+    extern __shared__ double unpaired_smem[];
+    double* stack = unpaired_smem + threadIdx.x;  // [depth][state, log scale][32]
+    uint8_t* sm = reinterpret_cast<uint8_t*>(unpaired_smem + (size_t)depth * 64);
+    const int col = threadIdx.x >> 2, a = threadIdx.x & 3, quad = threadIdx.x & 28;
+    const int x = blockIdx.x * 8 + col, xc = min(x, L - 1);
     const int s = blockIdx.y;
-    if (x >= L) return;
-    const double* Ps = P4 + (size_t)s * pstride * 16;
-    double* ps = part + (size_t)s * nn * L * 4;
-    double* ls = lmv + (size_t)s * nn * L;
-    for (int t = 0; t < nn; t++) {
-        const int v = post[t];
-        const int c0 = tree[4 * v], c1 = tree[4 * v + 1];
-        double* pv = ps + ((size_t)v * L + x) * 4;
-        if (c0 < 0) {
-            const int m = masks[(size_t)tree[4 * v + 2] * L + x];
-#pragma unroll
-            for (int a = 0; a < 4; a++) pv[a] = (double)((m >> a) & 1);
-            ls[(size_t)v * L + x] = 0.0;
-            continue;
-        }
-        const double* p0 = ps + ((size_t)c0 * L + x) * 4;
-        const double* p1 = ps + ((size_t)c1 * L + x) * 4;
-        const double* P0 = Ps + (size_t)c0 * 16;
-        const double* P1 = Ps + (size_t)c1 * 16;
-        double l[4], r[4], o[4], m = -INFINITY;
-#pragma unroll
-        for (int a = 0; a < 4; a++) { l[a] = p0[a]; r[a] = p1[a]; }
-#pragma unroll
-        for (int a = 0; a < 4; a++) {
-            double sl = 0.0, sr = 0.0;
-#pragma unroll
-            for (int d = 0; d < 4; d++) {
-                sl += __ldg(P0 + a * 4 + d) * l[d];
-                sr += __ldg(P1 + a * 4 + d) * r[d];
-            }
-            o[a] = sl * sr;
-            m = fmax(m, o[a]);
-        }
-        double lm = ls[(size_t)c0 * L + x] + ls[(size_t)c1 * L + x];
-        if (m < 1e-20) {  // src/FARCE.jl:2226-2238
-#pragma unroll
-            for (int a = 0; a < 4; a++) o[a] /= m;
-            lm += log(m);
-        }
-#pragma unroll
-        for (int a = 0; a < 4; a++) pv[a] = o[a];
-        ls[(size_t)v * L + x] = lm;
+    const double* Ps = P4 + (size_t)s * pstride * 16 + 4 * a;  // this lane's row of every matrix
+    if (staged) {
+        for (int k = threadIdx.x; k < 8 * N; k += 32)
+            sm[k] = masks[(size_t)(k >> 3) * L + min((int)blockIdx.x * 8 + (k & 7), L - 1)];
+        __syncwarp();
     }
-    const double* pr = ps + (size_t)x * 4;  // root = node 0
+    // sum over the leaf's states of P[a][.], ascending as the full product would add them
+    auto leaf = [&](int seq, const double2& p01, const double2& p23) {
+        const int m = staged ? sm[seq * 8 + col] : masks[(size_t)seq * L + xc];
+        const double p[4] = {p01.x, p01.y, p23.x, p23.y};
+        const int first = __ffs(m) - 1;
+        double v = p[3];
+#pragma unroll
+        for (int d = 0; d < 3; d++)
+            if (first == d) v = p[d];
+#pragma unroll
+        for (int d = 1; d < 4; d++)
+            if (__any_sync(0xffffffffu, d > first && (m >> d & 1)) && d > first && (m >> d & 1)) v += p[d];
+        return v;
+    };
+    auto inner = [&](double own, const double2& p01, const double2& p23) {
+        double v = 0.0;
+        v += p01.x * shfl_d(own, quad);
+        v += p01.y * shfl_d(own, quad + 1);
+        v += p23.x * shfl_d(own, quad + 2);
+        v += p23.y * shfl_d(own, quad + 3);
+        return v;
+    };
+    double top = 0.0, lm = 0.0;
+    for (int t = 0; t < nops; t++) {
+        const int4 op = __ldg(ops + t);  // children A, B; sequence of A, B (-1: A = the last result, B = the stack's)
+        const double2* PA = reinterpret_cast<const double2*>(Ps + (size_t)op.x * 16);
+        const double2* PB = reinterpret_cast<const double2*>(Ps + (size_t)op.y * 16);
+        const double2 a01 = __ldg(PA), a23 = __ldg(PA + 1), b01 = __ldg(PB), b23 = __ldg(PB + 1);
+        double l, r;
+        if (op.z >= 0) {
+            if (t > 0) {  // a new path: the last result waits for its sibling
+                stack[0] = top;
+                stack[32] = lm;
+                stack += 64;
+            }
+            l = leaf(op.z, a01, a23);
+            lm = 0.0;
+        } else {
+            l = inner(top, a01, a23);
+        }
+        if (op.w >= 0) {
+            r = leaf(op.w, b01, b23);
+        } else {
+            stack -= 64;
+            r = inner(stack[0], b01, b23);
+            lm += stack[32];
+        }
+        top = l * r;
+        // the largest state: non-negative doubles compare as their bits
+        long long m = __double_as_longlong(top);
+        m = max(m, __shfl_xor_sync(0xffffffffu, m, 1));
+        m = max(m, __shfl_xor_sync(0xffffffffu, m, 2));
+        if (__longlong_as_double(m) < 1e-20) {  // src/FARCE.jl:2226-2238
+            top /= __longlong_as_double(m);
+            lm += log(__longlong_as_double(m));
+        }
+    }
     double tot = 0.0;
 #pragma unroll
-    for (int a = 0; a < 4; a++) tot += pi4[a] * pr[a];
-    ll[(size_t)s * L + x] = log(tot) + ls[x];
+    for (int d = 0; d < 4; d++) tot += pi4[d] * shfl_d(top, quad + d);
+    if (x < L && a == 0) ll[(size_t)s * L + x] = log(tot) + lm;
 }
 
 __global__ void unpaired_mix_kernel(const double* __restrict__ ll, const double* __restrict__ logw_site, int nsite,
@@ -1117,24 +1149,21 @@ __global__ void unpaired_mix_kernel(const double* __restrict__ ll, const double*
 }
 
 int launch_unpaired(messi_ctx* ctx, messi_dataset* ds, const double* d_P4, int pstride, const double* d_pi4,
-                    const double* d_logw_site, int nsite, double* d_u, double* d_scratch)
+                    const double* d_logw_site, int nsite, double* d_u, double* d_ll)
 {
-    // d_scratch: nsite * (numnodes * L * 5 + L) doubles, or nullptr for the context's buffer
-    const size_t n = (size_t)ds->numnodes * ds->L;
-    if (!d_scratch) {
+    // d_ll: nsite * L doubles, or nullptr for the context's buffer
+    if (!d_ll) {
         void* scratch;
-        int rc = ensure(ctx, 20, ((size_t)nsite * (n * 5 + ds->L)) * sizeof(double), &scratch);
+        int rc = ensure(ctx, kSlotUnpaired, (size_t)nsite * ds->L * sizeof(double), &scratch);
         if (rc) return rc;
-        d_scratch = (double*)scratch;
+        d_ll = (double*)scratch;
     }
-    double* part = d_scratch;
-    double* lmv = part + (size_t)nsite * n * 4;
-    double* ll = lmv + (size_t)nsite * n;
-    const int bs = 32;
-    unpaired_site_kernel<<<dim3((ds->L + bs - 1) / bs, nsite), bs, 0, ctx->stream>>>(
-        ds->d_masks, ds->d_tree, ds->d_post, ds->numnodes, ds->L, d_P4, pstride, d_pi4, part, lmv, ll);
+    const size_t stack = (size_t)ds->unpaired_depth * 64 * sizeof(double), tile = (size_t)ds->N * 8;
+    const int staged = stack + tile <= 48 * 1024 ? 1 : 0;
+    unpaired_site_kernel<<<dim3((ds->L + 7) / 8, nsite), 32, stack + (staged ? tile : 0), ctx->stream>>>(
+        ds->d_masks, ds->N, ds->d_uops, ds->N - 1, ds->unpaired_depth, staged, ds->L, d_P4, pstride, d_pi4, d_ll);
     LAUNCH_CHECK(ctx, "unpaired_site_kernel");
-    unpaired_mix_kernel<<<(ds->L + 127) / 128, 128, 0, ctx->stream>>>(ll, d_logw_site, nsite, ds->L, d_u);
+    unpaired_mix_kernel<<<(ds->L + 127) / 128, 128, 0, ctx->stream>>>(d_ll, d_logw_site, nsite, ds->L, d_u);
     LAUNCH_CHECK(ctx, "unpaired_mix_kernel");
     return MESSI_OK;
 }
