@@ -629,7 +629,7 @@ int messi_dataset_destroy(messi_dataset* ds)
         tune_forget(ctx, ds);
     }
     void* bufs[] = {ds->d_bandidx, ds->d_idx, ds->d_leaf, ds->d_segs, ds->d_steps, ds->d_tiles, ds->d_masks, ds->d_tree,
-                    ds->d_uops, ds->d_arena_f, ds->d_arena_e, ds->d_mix, ds->d_mixlam, ds->d_leafnode};
+                    ds->d_uops, ds->d_arena_f, ds->d_arena_e, ds->d_mix, ds->d_mixlam};
     for (void* b : bufs)
         if (b) cudaFree(b);
     delete ds;

@@ -66,8 +66,7 @@ struct messi_batch {
     // and the leaf messages of the current category pass
     std::vector<int64_t> leaf_base;
     int64_t total_leaf_rows = 0;
-    float* d_leafrows = nullptr;
-    int* d_leafnode = nullptr;
+    int2* d_leafrows = nullptr;
     float* d_leafmsg = nullptr;
     int chunk = 0, arena_C = 0;
     BandBatch bands;
@@ -133,7 +132,7 @@ void destroy_batch(messi_batch* b)
     for (messi_dataset* d : b->ds)
         if (d) messi_dataset_destroy(d);
     void* bufs[] = {b->d_tiles, b->d_segs, b->d_steps, b->d_arena_f, b->d_arena_e, b->stage.p, b->P16.p, b->P4.p,
-                    b->d_leafrows, b->d_leafnode};
+                    b->d_leafrows};
     for (void* p : bufs)
         if (p) cudaFree(p);
     bandbatch_free(&b->bands);
@@ -243,8 +242,8 @@ int enqueue_batch(messi_ctx* ctx, messi_batch* b, const BatchStep& s)
     for (const messi_batch::Group& gr : b->groups) {
         for (int c0 = 0; c0 < C; c0 += chunk) {
             const int nc = std::min(chunk, C - c0);
-            if ((rc = launch_leaf_messages(ctx, b->d_leafrows + (size_t)gr.leaf0 * 16, b->d_leafnode + gr.leaf0,
-                                           gr.leaf_rows, s.P, b->total_nodes, c0, nc, C, b->d_leafmsg)))
+            if ((rc = launch_leaf_messages(ctx, b->d_leafrows + gr.leaf0, gr.leaf_rows, s.P, b->total_nodes, c0, nc,
+                                           b->d_leafmsg)))
                 return rc;
             for (int lv = 1; lv <= gr.H; lv++) {
                 for (int root = 0; root < 2; root++) {
@@ -436,18 +435,14 @@ int messi_batch_create(messi_ctx* ctx, int32_t n, const messi_alignment* alns, c
     {
         // leaf rows of all alignments and their global node ids
         const size_t R = (size_t)std::max<int64_t>(b->total_leaf_rows, 1);
-        std::vector<float> rows(R * 16, 0.f);
-        std::vector<int> rownode(R, 0);
-        for (int a = 0; a < n; a++) {
-            const messi_dataset* d = b->ds[a];
-            std::copy(d->leaf_host.begin(), d->leaf_host.begin() + (size_t)d->leaf_rows * 16,
-                      rows.begin() + (size_t)b->leaf_base[a] * 16);
-            for (int64_t r = 0; r < d->leaf_rows; r++) rownode[b->leaf_base[a] + r] = b->node_base[a] + d->leafnode_host[r];
-        }
-        if (e == cudaSuccess) e = cudaMalloc((void**)&b->d_leafrows, R * 16 * sizeof(float));
-        if (e == cudaSuccess) e = cudaMalloc((void**)&b->d_leafnode, R * sizeof(int));
-        if (e == cudaSuccess) e = cudaMemcpy(b->d_leafrows, rows.data(), R * 16 * sizeof(float), cudaMemcpyHostToDevice);
-        if (e == cudaSuccess) e = cudaMemcpy(b->d_leafnode, rownode.data(), R * sizeof(int), cudaMemcpyHostToDevice);
+        std::vector<int2> rows(R, make_int2(0, 1));
+        for (int a = 0; a < n; a++)
+            for (int64_t r = 0; r < b->ds[a]->leaf_rows; r++) {
+                const int2 row = b->ds[a]->leaf_host[r];
+                rows[b->leaf_base[a] + r] = make_int2(b->node_base[a] + row.x, row.y);
+            }
+        if (e == cudaSuccess) e = cudaMalloc((void**)&b->d_leafrows, R * sizeof(int2));
+        if (e == cudaSuccess) e = cudaMemcpy(b->d_leafrows, rows.data(), R * sizeof(int2), cudaMemcpyHostToDevice);
     }
     if (e != cudaSuccess) {
         destroy_batch(b);

@@ -291,7 +291,7 @@ struct messi_dataset {
     // device
     int* d_bandidx = nullptr;          // [L][W+1]
     int* d_idx = nullptr;              // gather indices of all segments
-    float* d_leaf = nullptr;           // concatenated leaf tables
+    int2* d_leaf = nullptr;            // [leaf_rows] (leaf node, 16-bit mask of the pair states)
     messi::SegDev* d_segs = nullptr;   // [segments]
     messi::StepDev* d_steps = nullptr; // [nsteps]
     int2* d_tiles = nullptr;
@@ -307,9 +307,7 @@ struct messi_dataset {
     std::vector<messi::StepDev> steps_host;
     std::vector<int64_t> leaf_off;     // per leaf offset (rows) into d_leaf
     int64_t leaf_rows = 0;             // rows of d_leaf (unique pairs summed over the leaves)
-    std::vector<float> leaf_host;      // [leaf_rows][16] host copy of d_leaf
-    std::vector<int> leafnode_host;    // [leaf_rows] leaf node of each row
-    int* d_leafnode = nullptr;         // device copy of leafnode_host
+    std::vector<int2> leaf_host;       // host copy of d_leaf
     float* d_leafmsg = nullptr;        // [chunk][leaf_rows][16] leaf messages of the current pass (end of d_arena_f)
 };
 
@@ -390,11 +388,11 @@ int launch_build_P16(messi_ctx* ctx, const double* d_eig, const double* d_bl, co
                      int C, float* d_P);
 int launch_build_P4(messi_ctx* ctx, const double* d_eig4, const double* d_bl, const int* d_nodegrp, int numnodes,
                     int nsite, double* d_P4);
-// Leaf messages of categories c0 .. c0+nc-1: out[cc][r] = P[c0+cc][rownode[r]]
-// x rows[r] for the R leaf rows (FP64 accumulation, stored FP32); d_P holds
-// C categories.
-int launch_leaf_messages(messi_ctx* ctx, const float* d_rows, const int* d_rownode, int64_t R, const float* d_P,
-                         int numnodes, int c0, int nc, int C, float* d_out);
+// Leaf messages of categories c0 .. c0+nc-1 of the R leaf rows (node, mask):
+// out[cc][r] = the sum of P[c0+cc][node]'s columns in the mask (FP64
+// accumulation, stored FP32).
+int launch_leaf_messages(messi_ctx* ctx, const int2* d_rows, int64_t R, const float* d_P, int numnodes, int c0, int nc,
+                         float* d_out);
 // The segments of one level (the root segments when root) over categories c0 .. c0+nc-1.
 int launch_prune_level(messi_ctx* ctx, const SegDev* d_segs, const int2* d_tiles, const SegLevel& lv, bool root,
                        const float* d_P, int numnodes, int c0, int nc, int C, const float* d_pi16,

@@ -442,23 +442,22 @@ int build_plan(messi_dataset* ds, const messi_alignment* aln, int W, const uint8
     for (const SegLevel& lv : ds->seg_levels) ds->executed += (int64_t)lv.units;
     ds->naive = ds->band_pairs * (int64_t)(N - 1);
 
-    // ---- leaf tables: row u = outer product of the two column masks
+    // ---- leaf rows: the 16 pair states allowed by the two column masks
     ds->leaf_off.assign(nn, -1);
     int64_t leaf_rows = 0;
     for (int v = 0; v < nn; v++)
         if (ds->children[2 * v] < 0) { ds->leaf_off[v] = leaf_rows; leaf_rows += ds->nunique[v]; }
     ds->leaf_rows = leaf_rows;
-    std::vector<float>& leaf = ds->leaf_host;
-    leaf.assign((size_t)std::max<int64_t>(leaf_rows, 1) * 16, 0.f);
-    ds->leafnode_host.assign((size_t)std::max<int64_t>(leaf_rows, 1), 0);
+    std::vector<int2>& leaf = ds->leaf_host;
+    leaf.assign((size_t)std::max<int64_t>(leaf_rows, 1), make_int2(0, 1));
     for (int v = 0; v < nn; v++) {
         if (ds->children[2 * v] >= 0) continue;
         const uint8_t* row = &ds->masks[(size_t)ds->seqindex[v] * L];
         for (int64_t u = 0; u < ds->nunique[v]; u++) {
-            uint8_t mx = row[rep[v][2 * u]], my = row[rep[v][2 * u + 1]];
-            float* o = &leaf[(size_t)(ds->leaf_off[v] + u) * 16];
-            for (int a = 0; a < 16; a++) o[a] = (float)(((mx >> (a / 4)) & 1) * ((my >> (a % 4)) & 1));
-            ds->leafnode_host[ds->leaf_off[v] + u] = v;
+            const uint8_t mx = row[rep[v][2 * u]], my = row[rep[v][2 * u + 1]];
+            int states = 0;
+            for (int a = 0; a < 16; a++) states |= (((mx >> (a / 4)) & 1) & ((my >> (a % 4)) & 1)) << a;
+            leaf[(size_t)(ds->leaf_off[v] + u)] = make_int2(v, states);
         }
     }
 
@@ -555,8 +554,7 @@ int build_plan(messi_dataset* ds, const messi_alignment* aln, int W, const uint8
         e = cudaGetLastError();
         goto cuda_error;
     }
-    UPLOAD(ds->d_leaf, leaf.data(), leaf.size() * sizeof(float));
-    UPLOAD(ds->d_leafnode, ds->leafnode_host.data(), ds->leafnode_host.size() * sizeof(int));
+    UPLOAD(ds->d_leaf, leaf.data(), leaf.size() * sizeof(int2));
     UPLOAD(ds->d_masks, ds->masks.data(), ds->masks.size());
     UPLOAD(ds->d_tree, tree.data(), tree.size() * sizeof(int));
     UPLOAD(ds->d_uops, uops.data(), uops.size() * sizeof(int4));

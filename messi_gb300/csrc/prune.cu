@@ -40,12 +40,14 @@ namespace messi {
 
 // P[c][v][a][d] in FP32 (row = parent state), from the FP64 eigensystem:
 // P = D^-1/2 U exp(W t) U^T D^1/2.  One CTA per category and run of
-// kP16Nodes nodes, a thread per entry: the CTA stages the category's U and
-// the ratios sqrt(pi_d) / sqrt(pi_a) once per model group and, per node,
-// W[a][k] = U[a][k] exp(w_k t), so an entry is 16 FP64 multiply-adds.  (One
-// CTA per node and category staged U for every matrix and divided per entry:
-// 26 ms for the 1.28 M matrices of a 256-alignment batch.)
-constexpr int kP16Nodes = 32;
+// kP16Nodes nodes, a thread per entry: the CTA forms the exponentials of all
+// its nodes at once, stages the category's U and the ratios sqrt(pi_d) /
+// sqrt(pi_a) once per model group and, per node, W[a][k] = U[a][k] exp(w_k t),
+// so an entry is 16 FP64 multiply-adds (36 categories of 127 nodes: 32 us of
+// the FP64 pipe).  With 32 nodes per CTA and a node's exponentials on its
+// critical path it took 73 us there and 69 us for 31 nodes (36 CTAs); now
+// 53 and 17 us.
+constexpr int kP16Nodes = 8;
 
 // x as TF32 hi + lo: hi = x rounded to TF32 (half a TF32 ulp added to the
 // magnitude bits, then truncated: round to nearest, ties away), lo = x - hi,
@@ -63,29 +65,33 @@ __host__ __device__ constexpr int p16_at(int a, int d)
     return ((a >> 1) & 1) * 128 + ((((a >> 2) << 1) | (a & 1)) * 4 + (d >> 2)) * 4 + (d & 3);
 }
 
-__global__ void build_P16_kernel(const double* __restrict__ eig, const double* __restrict__ bl,
-                                 const int* __restrict__ nodegrp, int numnodes, int C, float* __restrict__ P)
+__global__ void __launch_bounds__(256) build_P16_kernel(const double* __restrict__ eig, const double* __restrict__ bl,
+                                                       const int* __restrict__ nodegrp, int numnodes, int C,
+                                                       float* __restrict__ P)
 {
     const int c = blockIdx.x, t = threadIdx.x;
     const int a = t >> 4, d = t & 15;
     const int v0 = blockIdx.y * kP16Nodes, v1 = min(numnodes, v0 + kP16Nodes);
-    __shared__ double U[256], W[256], R[256], w[16], ex[16];
+    __shared__ double U[256], W[2][256], R[256], ex[kP16Nodes][16];
+    auto group = [&](int v) { return nodegrp ? nodegrp[v] : (v == 0 ? -1 : 0); };  // the same in every thread
+    if (t < 16 * kP16Nodes && v0 + a < v1) {
+        const int grp = group(v0 + a);
+        if (grp >= 0) ex[a][d] = exp(eig[((size_t)grp * C + c) * kEigStride + d] * bl[v0 + a]);
+    }
     int cur = -1;
     for (int v = v0; v < v1; v++) {
-        const int grp = nodegrp ? nodegrp[v] : (v == 0 ? -1 : 0);  // the same in every thread
+        const int grp = group(v), buf = v & 1;
         const double tl = bl[v];
-        __syncthreads();  // the previous node's reads of the staged arrays are done
         if (grp >= 0 && grp != cur) {
             const double* e = eig + ((size_t)grp * C + c) * kEigStride;
+            __syncthreads();  // the previous group's U is no longer read
             U[t] = e[16 + t];
             R[t] = e[16 + 256 + d] / e[16 + 256 + a];
-            if (t < 16) w[t] = e[t];
             cur = grp;
             __syncthreads();
         }
-        if (grp >= 0 && t < 16) ex[t] = exp(w[t] * tl);
-        __syncthreads();
-        if (grp >= 0) W[t] = U[t] * ex[d];  // W[a][k], k = d
+        // W[a][k], k = d; the other buffer may still be read for the node before
+        if (grp >= 0) W[buf][t] = U[t] * ex[v - v0][d];
         __syncthreads();
         float out;
         if (grp < 0) {
@@ -95,7 +101,7 @@ __global__ void build_P16_kernel(const double* __restrict__ eig, const double* _
         } else {
             double acc = 0.0;
 #pragma unroll
-            for (int k = 0; k < 16; k++) acc += W[a * 16 + k] * U[d * 16 + k];
+            for (int k = 0; k < 16; k++) acc += W[buf][a * 16 + k] * U[d * 16 + k];
             acc *= R[t];
             out = (acc <= 0.0) ? 0.f : (float)acc;  // absmat clamp (1e-50 rounds to 0 in FP32)
         }
@@ -165,44 +171,37 @@ __device__ __forceinline__ double lse_d_fast(double a, double b)
 }
 
 // ---------------------------------------------------------------------------
-// Leaf messages: out[cc][r][a] = sum_d P[c0+cc][node(r)][a][d] * rows[r][d]
-// (16 threads per row, FP64 accumulation, one FP32 rounding).
+// Leaf messages: out[cc][r][a] = sum_d P[c0+cc][node(r)][a][d] over the states
+// d of row r's mask (16 threads per row, FP64 accumulation, one FP32 rounding).
+// An observed base pair is one state and needs no FP64 at all; those units
+// issue a warp only every 64 cycles per SM quarter, and the 0/1 rows' full
+// products kept them busy for 86 us (1,600 rows of 36 categories), now 16.
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) leaf_msg_kernel(const float* __restrict__ rows, const int* __restrict__ rownode,
-                                                       long long R, const float* __restrict__ P, int numnodes, int c0,
-                                                       int C, float* __restrict__ out)
+__global__ void __launch_bounds__(256) leaf_msg_kernel(const int2* __restrict__ rows, long long R,
+                                                       const float* __restrict__ P, int numnodes, int c0,
+                                                       float* __restrict__ out)
 {
     const long long r = (long long)blockIdx.x * 16 + (threadIdx.x >> 4);
     const int a = threadIdx.x & 15, cc = blockIdx.y;
     if (r >= R) return;
-    (void)C;
-    const float* p = P + ((size_t)(c0 + cc) * numnodes + __ldg(rownode + r)) * kP16Floats;
-    const float4* x4 = reinterpret_cast<const float4*>(rows + r * 16);
-    float x[16];
-#pragma unroll
-    for (int q = 0; q < 4; q++) {
-        const float4 v = __ldg(x4 + q);
-        x[4 * q] = v.x;
-        x[4 * q + 1] = v.y;
-        x[4 * q + 2] = v.z;
-        x[4 * q + 3] = v.w;
+    const int2 row = __ldg(rows + r);  // leaf node, mask of its states
+    const float* p = P + ((size_t)(c0 + cc) * numnodes + row.x) * kP16Floats;
+    auto entry = [&](int d) { return __ldg(p + p16_at(a, d)) + __ldg(p + p16_at(a, d) + 256); };
+    const int first = __ffs(row.y) - 1;
+    float v = entry(first);
+    if (row.y & (row.y - 1)) {  // ambiguous: ascending, as the full product adds them
+        double s = (double)v;
+        for (int m = row.y & (row.y - 1); m; m &= m - 1) s += (double)entry(__ffs(m) - 1);
+        v = (float)s;
     }
-    // an observed base pair is one nonzero state: its zero terms are skipped
-    // (adding +0.0 would leave the sum as it is), the same branch for the 16
-    // threads of the row
-    double s = 0.0;
-#pragma unroll
-    for (int d = 0; d < 16; d++)
-        if (x[d] != 0.f) s += (double)(__ldg(p + p16_at(a, d)) + __ldg(p + p16_at(a, d) + 256)) * (double)x[d];
-    out[((size_t)cc * R + r) * 16 + a] = (float)s;
+    out[((size_t)cc * R + r) * 16 + a] = v;
 }
 
-int launch_leaf_messages(messi_ctx* ctx, const float* d_rows, const int* d_rownode, int64_t R, const float* d_P,
-                         int numnodes, int c0, int nc, int C, float* d_out)
+int launch_leaf_messages(messi_ctx* ctx, const int2* d_rows, int64_t R, const float* d_P, int numnodes, int c0, int nc,
+                         float* d_out)
 {
     if (R <= 0 || nc <= 0) return MESSI_OK;
-    leaf_msg_kernel<<<dim3((unsigned)((R + 15) / 16), nc), 256, 0, ctx->stream>>>(d_rows, d_rownode, R, d_P,
-                                                                                  numnodes, c0, C, d_out);
+    leaf_msg_kernel<<<dim3((unsigned)((R + 15) / 16), nc), 256, 0, ctx->stream>>>(d_rows, R, d_P, numnodes, c0, d_out);
     LAUNCH_CHECK(ctx, "leaf_msg_kernel");
     return MESSI_OK;
 }
@@ -1022,8 +1021,7 @@ int run_pairs(messi_ctx* ctx, messi_dataset* ds, const float* d_P, const float* 
     const int chunk = std::min(ds->chunk, kCollectCategories);
     for (int c0 = 0; c0 < C; c0 += chunk) {
         const int nc = std::min(chunk, C - c0);
-        int rc = launch_leaf_messages(ctx, ds->d_leaf, ds->d_leafnode, ds->leaf_rows, d_P, ds->numnodes, c0, nc, C,
-                                      ds->d_leafmsg);
+        int rc = launch_leaf_messages(ctx, ds->d_leaf, ds->leaf_rows, d_P, ds->numnodes, c0, nc, ds->d_leafmsg);
         if (rc) return rc;
         for (int lv = 1; lv <= ds->SH; lv++) {
             const SegLevel& sl = ds->seg_levels[lv];
