@@ -344,17 +344,21 @@ __device__ __forceinline__ void pow2_scale(float m, int& ex, float& sc)
 // level, every node's rows written and gathered again, moved 212 bytes per
 // update and was bound by the L1 data pipe, 71% of its wavefronts.)
 // Each step gathers one row per pair: the four lanes (g, t) of a pair read
-// 16 bytes each, straight to registers, and the rows of the next step are
-// asked for as soon as this step's are consumed, so they arrive under the
-// mat-vec (without that, 24 warps per SM instead of 20: 15% slower).  The
-// columns of P are assigned to the MMA's N index so that lane (g, t) ends with
+// 16 bytes each, straight to registers.  The gathers are a stream of their
+// own: a row is asked for as soon as the one before it is consumed, so that it
+// arrives under the mat-vec (without that, 24 warps per SM instead of 20: 15%
+// slower), and so is the next matrix, as soon as the MMAs have read this
+// one's, both across the end of a category (matrices asked for where they are
+// used: lower levels 15-20% slower).  The columns of P are assigned to the MMA's N index so that lane (g, t) ends with
 // states 4t..4t+3 of its pairs, which is the A layout of the next product:
 // column g of tile nt is state 4(g/2) + 2nt + g%2.
 // Measured (GB300, 64 x 1,000 columns, span 500, 36 categories): 2.96e8
-// distinct updates in 7.5 ms before; 3.6e8 (some recomputed) in 5.72 ms now,
-// DRAM traffic 35 GB -> ~7 GB.  What bounds it: about 300 instructions per 32
-// updates at 55% of the issue slots (HMMA busy 29%, L1 35%), i.e. the latency
-// of a step's dependent chain with the 16-20 warps the registers allow.
+// distinct updates in 7.5 ms before; 3.6e8 (some recomputed) in 5.2 ms now,
+// DRAM traffic 35 GB -> ~7 GB.  What bounds it: about 245 instructions per 32
+// updates at half of the issue slots, the tensor pipe 41% busy (24 MMAs of 8.5
+// cycles a step), with the 20 warps per SM the registers allow: 16 took 13%
+// more per warp and step, a third of the MMAs 20% less, constant rows or
+// matrices 3% less each.
 // The CTA's warps are pg pair groups x cs category splits: with few pairs the
 // warps of one pair group take every cs-th category each (a level of 50
 // tiles of 128 pairs with all 36 categories in turn took 45 us).
@@ -380,6 +384,16 @@ struct Mixture {
 
 // Lane t's own one of four values (pair g + 8t).
 __device__ __forceinline__ int own4(const int4& v, int t) { return t == 0 ? v.x : (t == 1 ? v.y : (t == 2 ? v.z : v.w)); }
+
+// A read-only integer load where `pred`, else 0, as one predicated instruction.
+__device__ __forceinline__ int ldg_int_if(const int* p, bool pred)
+{
+    int v;
+    asm("{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %2, 0;\n\tmov.b32 %0, 0;\n\t@q ld.global.nc.b32 %0, [%1];\n\t}"
+        : "=r"(v)
+        : "l"(__cvta_generic_to_global(p)), "r"((int)pred));
+    return v;
+}
 
 // Reduces v[k] over the four lanes t of a pair; lane t keeps pair k = t: two
 // exchanges of halves instead of a butterfly per pair (three shuffles, not eight).
@@ -413,18 +427,42 @@ __global__ void __launch_bounds__(MAXT, MINB) prune_path_kernel(
     const int pgs = (int)(blockDim.x >> 5) / cs, pg = warp % pgs, split = warp / pgs;
     const int base = tile.y + 32 * NP * pg;  // first pair of this warp
     const bool active = base < n;
-    // shared memory: program, gather indices per pair group, set-aside messages per warp, collected values
-    int4* steps = reinterpret_cast<int4*>(smem_raw);
-    int4* sidx = steps + max_steps + pg * max_nb * 8 * NP;
-    float4* stack = smem_raw + max_steps + pgs * max_nb * 8 * NP + warp * max_depth * 128 * NP + lane;
-    double* collected = reinterpret_cast<double*>(smem_raw + max_steps + pgs * max_nb * 8 * NP +
-                                                  (int)(blockDim.x >> 5) * max_depth * 128 * NP);
-    for (int i = threadIdx.x; i < ns; i += blockDim.x) steps[i] = __ldg(reinterpret_cast<const int4*>(sg.steps) + i);
+    // shared memory: gathers (slot nb repeats slot 0: the stream's last look
+    // ahead), mat-vec steps, gather indices per pair group, set-aside messages
+    // per warp, collected values
+    int4* gathers = reinterpret_cast<int4*>(smem_raw);
+    int2* ops = reinterpret_cast<int2*>(gathers + max_nb + 1);
+    float4* rest = smem_raw + (max_nb + 1) + (max_steps + 1) / 2;
+    int4* sidx = reinterpret_cast<int4*>(rest) + pg * (max_nb + 1) * 8 * NP;
+    rest += pgs * (max_nb + 1) * 8 * NP;
+    float4* stack = rest + warp * max_depth * 128 * NP + lane;
+    double* collected = reinterpret_cast<double*>(rest + (int)(blockDim.x >> 5) * max_depth * 128 * NP);
+    const int nmul = ROOT ? ns - 1 : ns;  // the root's step has no mat-vec
+    for (int i = threadIdx.x; i < ns; i += blockDim.x) {
+        const int4* steps = reinterpret_cast<const int4*>(sg.steps);
+        const int4 st = __ldg(steps + i);
+        // the next mat-vec's matrix; after the last, the next category's first
+        unsigned ahead;
+        if (i + 1 < nmul) {
+            int4 nx = __ldg(steps + i + 1);
+            if (nx.w & kStepInit) nx = __ldg(steps + i + 2);
+            ahead = (unsigned)nx.z;
+        } else {
+            ahead = (unsigned)__ldg(steps + 1).z + (unsigned)(cs * numnodes);
+        }
+        ops[i] = make_int2((int)ahead, st.w);
+        if (st.w & kStepGather) {
+            const int slot = st.w >> kStepSlotShift;
+            gathers[slot] = make_int4(st.x, st.y, st.w & kStepLeaf, -1);
+            if (slot == 0) gathers[nb] = make_int4(st.x + cs * st.y, st.y, st.w & kStepLeaf, st.x + (nc - 1) * st.y);
+        }
+    }
     if (active) {
 #pragma unroll
         for (int h = 0; h < NP; h++) {  // (past the last pair the last tile again)
             const int4* src = reinterpret_cast<const int4*>(sg.idx) + (size_t)min((base >> 5) + h, (n - 1) >> 5) * nb * 8;
-            for (int i = split * 32 + lane; i < nb * 8; i += 32 * cs) sidx[h * max_nb * 8 + i] = __ldg(src + i);
+            int4* dst = sidx + h * (max_nb + 1) * 8;
+            for (int i = split * 32 + lane; i < (nb + 1) * 8; i += 32 * cs) dst[i] = __ldg(src + (i < nb * 8 ? i : i - nb * 8));
         }
     }
     __syncthreads();
@@ -435,90 +473,87 @@ __global__ void __launch_bounds__(MAXT, MINB) prune_path_kernel(
         int e[NP], er[NP];
         const float4* rows = reinterpret_cast<const float4*>(sg.rows) + t;
         const int* exps = sg.exps;
-        // The rows of step st's table for category cc: states 4t..4t+3 of pairs g + 8k.
-        auto gather = [&](const int4& st, int cc) {
-            const unsigned row = (unsigned)st.x + (unsigned)cc * (unsigned)st.y;
+        const int4* gp;
+        const int* si;
+        int cc;
+        // The next gather of the stream: states 4t..4t+3 of pairs g + 8k, and
+        // the exponent of the lane's own pair.
+        auto next = [&]() {
+            const int4 gd = *gp++;
+            const unsigned row = min((unsigned)gd.x + (unsigned)cc * (unsigned)gd.y, (unsigned)gd.w);
             const float4* f = rows + (size_t)row * 4;
-            const int slot = (st.w >> kStepSlotShift) * 8 + g;
 #pragma unroll
             for (int h = 0; h < NP; h++) {
-                const int4 id = sidx[h * max_nb * 8 + slot];
+                const int* sh = si + h * (max_nb + 1) * 32;
+                const int4 id = *reinterpret_cast<const int4*>(sh + 4 * g);
                 R[h][0] = __ldg(f + (size_t)(unsigned)id.x * 4);
                 R[h][1] = __ldg(f + (size_t)(unsigned)id.y * 4);
                 R[h][2] = __ldg(f + (size_t)(unsigned)id.z * 4);
                 R[h][3] = __ldg(f + (size_t)(unsigned)id.w * 4);
-                er[h] = (st.w & kStepLeaf) ? 0 : __ldg(exps + row + (unsigned)own4(id, t));
+                er[h] = ldg_int_if(exps + row + (unsigned)sh[lane], gd.z == 0);
             }
+            si += 32;
         };
-        int4 st = steps[0];
-        gather(st, split);
-        for (int cc = split; cc < nc; cc += cs) {
-            const float4* Pc = reinterpret_cast<const float4*>(P + (size_t)(c0 + cc) * numnodes * kP16Floats) + lane;
+        auto pop = [&](float4*& top) {
+            top -= 128 * NP;
+#pragma unroll
+            for (int h = 0; h < NP; h++)
+#pragma unroll
+                for (int k = 0; k < 4; k++) M[h][k] = mul4(M[h][k], top[128 * h + 32 * k]);
+        };
+        auto product = [&]() {  // x = M * R, then the next rows are asked for
+#pragma unroll
+            for (int h = 0; h < NP; h++) {
+#pragma unroll
+                for (int k = 0; k < 4; k++) M[h][k] = mul4(M[h][k], R[h][k]);
+                e[h] += er[h];
+            }
+            next();
+        };
+        float4 Bh[2], Bl[2];
+        const float4* Pc = reinterpret_cast<const float4*>(P + (size_t)(c0 + split) * numnodes * kP16Floats) + lane;
+        auto matrix = [&](unsigned node) {
+            const float4* pv = Pc + (size_t)node * (kP16Floats / 4);
+            Bh[0] = __ldg(pv);
+            Bh[1] = __ldg(pv + 32);
+            Bl[0] = __ldg(pv + 64);
+            Bl[1] = __ldg(pv + 96);
+        };
+        cc = split;
+        gp = gathers;
+        si = reinterpret_cast<const int*>(sidx);
+        next();
+        matrix((unsigned)__ldg(&sg.steps[1].self));
+        for (; cc < nc; cc += cs, Pc += (size_t)cs * numnodes * (kP16Floats / 4)) {
+            const unsigned last = (unsigned)((nc - cc) * numnodes - 1);
+            gp = gathers + 1;
+            si = reinterpret_cast<const int*>(sidx) + 32;
 #pragma unroll
             for (int h = 0; h < NP; h++) e[h] = 0;
             float4* top = stack;
-            for (int s = 0; s < ns; s++) {
-                const int fl = st.w;
-                const float4* pv = Pc + (size_t)(unsigned)st.z * (kP16Floats / 4);
-                // the next step (the program's first for the next category)
-                const bool last = s + 1 == ns;
-                st = steps[last ? 0 : s + 1];
-                if (fl & kStepInit) {
+            for (int s = 0; s < nmul; s++) {
+                const int2 op = ops[s];
+                if (op.y & (kStepInit | kStepPop)) {
+                    if (op.y & kStepInit) {
 #pragma unroll
-                    for (int h = 0; h < NP; h++) {
+                        for (int h = 0; h < NP; h++) {
 #pragma unroll
-                        for (int k = 0; k < 4; k++) M[h][k] = R[h][k];
-                        e[h] += er[h];
+                            for (int k = 0; k < 4; k++) M[h][k] = R[h][k];
+                            e[h] += er[h];
+                        }
+                        next();
+                        continue;
                     }
-                    gather(st, cc);
-                    continue;
-                }
-                float4 Bh[2], Bl[2];
-                if (!ROOT || !(fl & kStepRoot)) {
-                    Bh[0] = __ldg(pv);
-                    Bh[1] = __ldg(pv + 32);
-                    Bl[0] = __ldg(pv + 64);
-                    Bl[1] = __ldg(pv + 96);
-                }
-                // x = product of the two messages: states 4t..4t+3 of pairs g + 8k
-                if (fl & kStepPop) {
-                    top -= 128 * NP;
-#pragma unroll
-                    for (int h = 0; h < NP; h++)
-#pragma unroll
-                        for (int k = 0; k < 4; k++) M[h][k] = mul4(M[h][k], top[128 * h + 32 * k]);
+                    pop(top);
                 } else {
-#pragma unroll
-                    for (int h = 0; h < NP; h++) {
-#pragma unroll
-                        for (int k = 0; k < 4; k++) M[h][k] = mul4(M[h][k], R[h][k]);
-                        e[h] += er[h];
-                    }
-                }
-                // the next gathered rows arrive under this step's mat-vec
-                if ((st.w & kStepGather) && (!last || cc + cs < nc)) gather(st, last ? cc + cs : cc);
-                if (ROOT && (fl & kStepRoot)) {
-                    const float4 pc = __ldg(reinterpret_cast<const float4*>(pi16 + ((size_t)sg.grp * C + c0 + cc) * 16) + t);
-#pragma unroll
-                    for (int h = 0; h < NP; h++) {
-                        float d[4];
-#pragma unroll
-                        for (int k = 0; k < 4; k++)
-                            d[k] = pc.x * M[h][k].x + pc.y * M[h][k].y + pc.z * M[h][k].z + pc.w * M[h][k].w;
-                        const float dot = quad_reduce(d, t, [](float a, float b) { return a + b; });
-                        const double ll = (dot > 0.f) ? (double)logf(dot) + (double)e[h] * 0.69314718055994530942 : -INFINITY;
-                        if (sg.catll && myu + 32 * h < n) sg.catll[(size_t)(c0 + cc) * n + myu + 32 * h] = ll;
-                        const double tt = __ldg(logw + (size_t)sg.grp * C + c0 + cc) + ll;
-                        if (ROOT == 1) mix[h].add(tt);
-                        else collected[((pg * NP + h) * nc + cc) * 32 + lane] = tt;
-                    }
-                    continue;
+                    product();
                 }
                 // m_v = P_v x (the node's own branch)
 #pragma unroll
                 for (int h = 0; h < NP; h++) {
                     float D0[2][2][4], D1[2][2][4];
                     msg_mma(M[h], Bh, Bl, D0, D1);
+                    if (h == NP - 1) matrix(min((unsigned)op.x, last));
                     // pair g + 8k, states 4t..4t+3; the two k-step halves
                     // added, then their truncation returned on average
                     float mx[4];
@@ -543,7 +578,7 @@ __global__ void __launch_bounds__(MAXT, MINB) prune_path_kernel(
                         M[h][k] = mul4(M[h][k], make_float4(sk, sk, sk, sk));
                     }
                 }
-                if (fl & kStepPush) {
+                if (op.y & kStepPush) {
 #pragma unroll
                     for (int h = 0; h < NP; h++)
 #pragma unroll
@@ -551,7 +586,24 @@ __global__ void __launch_bounds__(MAXT, MINB) prune_path_kernel(
                     top += 128 * NP;
                 }
             }
-            if (!ROOT) {
+            if (ROOT) {
+                if (ops[nmul].y & kStepPop) pop(top);
+                else product();
+                const float4 pc = __ldg(reinterpret_cast<const float4*>(pi16 + ((size_t)sg.grp * C + c0 + cc) * 16) + t);
+#pragma unroll
+                for (int h = 0; h < NP; h++) {
+                    float d[4];
+#pragma unroll
+                    for (int k = 0; k < 4; k++)
+                        d[k] = pc.x * M[h][k].x + pc.y * M[h][k].y + pc.z * M[h][k].z + pc.w * M[h][k].w;
+                    const float dot = quad_reduce(d, t, [](float a, float b) { return a + b; });
+                    const double ll = (dot > 0.f) ? (double)logf(dot) + (double)e[h] * 0.69314718055994530942 : -INFINITY;
+                    if (sg.catll && myu + 32 * h < n) sg.catll[(size_t)(c0 + cc) * n + myu + 32 * h] = ll;
+                    const double tt = __ldg(logw + (size_t)sg.grp * C + c0 + cc) + ll;
+                    if (ROOT == 1) mix[h].add(tt);
+                    else collected[((pg * NP + h) * nc + cc) * 32 + lane] = tt;
+                }
+            } else {
 #pragma unroll
                 for (int h = 0; h < NP; h++) {
                     const int u0 = base + 32 * h + g;
@@ -968,7 +1020,7 @@ static int launch_path(messi_ctx* ctx, const SegDev* d_segs, const int2* d_tiles
                        const double* d_logw, const int* d_lam, bool per_lambda)
 {
     const int pgs = lv.pg / NP, warps = pgs * cs;
-    const size_t smem = sizeof(float4) * ((size_t)lv.max_steps + (size_t)lv.pg * lv.max_nb * 8 +
+    const size_t smem = sizeof(float4) * ((size_t)(lv.max_nb + 1) * (1 + 8 * lv.pg) + (lv.max_steps + 1) / 2 +
                                           (size_t)warps * NP * lv.max_depth * 128) +
                         (ROOT == 2 ? sizeof(double) * 32 * (size_t)lv.pg * nc : 0);
     static thread_local std::pair<int, size_t> granted{-1, 0};
