@@ -15,8 +15,8 @@
 //     with one eigensystem set per distinct model (models that differ only
 //     in their branch lengths share it);
 //   * the inside passes of all alignments run in one persistent wavefront
-//     (inside_wave_batch_kernel): diagonal d of every alignment whose band
-//     reaches it is one step, so the number of grid barriers is the largest
+//     (inside_pair_kernel): a pair of diagonals of every alignment whose band
+//     reaches it is one step, so the number of steps is half the largest
 //     band width in the batch instead of the sum over alignments;
 //   * the device work of a step is captured as a CUDA graph on the second
 //     call with the same layout and replayed from then on (per-call values

@@ -149,6 +149,7 @@ struct Band {
 struct BandBatch {
     int n = 0;
     long long total_cols = 0;
+    size_t polled = 0;             // floats of the tables that the inside kernel waits on, from the first band's Lrow
     std::vector<Band> host;
     std::vector<int> order, slot;  // slot[alignment] = band index
     Band* d_bands = nullptr;
@@ -499,6 +500,6 @@ int queue_status_readback(messi_ctx* ctx, const Band& t);
 // barrier words, picks the CTA size and grid; share > 0 for kernels that own
 // rows of diagonal pairs (warps per row and pair).
 int launch_wave(messi_ctx* ctx, const void* kernel, void** args, unsigned int* sync, int L, double band_cells,
-                const char* what, int share = 0, const void* halves_kernel = nullptr);
+                const char* what, int share = 0);
 
 }  // namespace messi

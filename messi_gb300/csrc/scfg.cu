@@ -27,18 +27,20 @@
 //
 // Schedule.  One persistent cooperative launch walks the band diagonals (a
 // wavefront): all cells of a span are independent, so each diagonal is spread
-// over the whole grid and grid barriers separate diagonals (the inside pass
-// takes two diagonals per barrier: a CTA owns a block of rows and the second
-// diagonal of a pair reads the first only at the CTA's own rows).  The
-// barrier spins with a bounded iteration count; on timeout it raises an
-// error flag, every CTA leaves, Z becomes NaN and the host returns
-// MESSI_ETIMEOUT.  A cell's split sum is reduced by a group of G lanes (G
-// grows with the number of split points) with shuffle log-sum-exp; its
-// middle split points, which do not read the diagonals just finished, are
-// summed while a barrier is in progress.  The suffix recurrences run in one
+// over the whole grid, two diagonals at a time (a CTA owns a block of rows and
+// the second diagonal of a pair reads the first only at the CTA's own rows).
+// The CTAs of the inside pass wait for one another's cells, those of the
+// outside pass at a grid barrier between pairs; both waits have a bounded
+// iteration count: on timeout an error flag is raised, every CTA leaves, Z
+// becomes NaN and the host returns MESSI_ETIMEOUT.  A cell's split sum is
+// reduced by a group of G lanes (G grows with the number of split points) with
+// shuffle log-sum-exp; its middle split points, which do not read the diagonals
+// just finished, are summed one pair ahead.  The suffix recurrences run in one
 // CTA in blocks of 32 cells: the terms that reach outside the block are
 // summed by 32 warps in parallel, the in-block triangle by one warp.
 #include <algorithm>
+#include <array>
+#include <climits>
 #include <cmath>
 
 #include "internal.h"
@@ -772,10 +774,10 @@ __device__ __forceinline__ void inside_init_cell(const Band& t, int i, const Rul
     const float Lv = (ui == -INFINITY) ? -INFINITY : (float)(B * ui + (double)R.r[5] - t.b[i]);
     const size_t o = (size_t)i * t.RS;
     t.Srow[o] = S;
-    t.Scol[o] = S;
-    t.Lrow[o] = Lv;
+    st_cell(t.Scol + o, S);
+    st_cell(t.Lrow + o, Lv);
     t.Lcol[o] = Lv;
-    t.Frow[o] = -INFINITY;
+    st_cell(t.Frow + o, -INFINITY);
     if (i == t.L - 1) t.Ssuf[i] = S;
 }
 
@@ -790,10 +792,6 @@ __device__ __forceinline__ void inside_init_cell(const Band& t, int i, const Rul
 // 3: the partial sums of a diagonal pair (2p-1, 2p) then read spans <= 2p-4
 // only, which the paired wavefront has before its wait, and every kernel
 // splits a cell the same way, so all of them give the same bits.
-struct CellPartial {
-    float m, s, pbv;
-};
-
 // Sixteen split points of a lane that are all in range (two blocks of eight,
 // summed in order): no predicates, and with the group width a constant the
 // 32 loads take immediate offsets from two base addresses.  Long spans spend
@@ -850,58 +848,27 @@ __device__ __forceinline__ void split_tail32(float& m, float& s, const float* lr
     }
 }
 
-template <int NLO, int NHI, bool WIDE>
-__device__ __forceinline__ CellPartial cell_partial_t(const Band& t, int i, int d, bool valid, int lane, int G)
+// Split points k = e .. d-e-1 of cell (i, i+d), its L row and S column given
+// (scol at span d-1), reduced over the group; lane 0 of the group has the sum.
+__device__ __forceinline__ void cell_partial(const float* lrow, const float* scol, int d, int e, bool valid, int lane,
+                                             int G, float& m, float& s)
 {
-    const int RS = t.RS;
-    CellPartial c{-INFINITY, 0.f, -INFINITY};
-    // lanes 0 and 1: either may finish the cell (rows_finish)
-    if (valid && lane < 2 && d >= 2) c.pbv = t.pb[(size_t)i * RS + d];
-    const int kend = d - NHI;
-    if (valid && kend > NLO) {
-        const float* lrow = t.Lrow + (size_t)i * RS;
-        const float* scol = t.Scol + (size_t)(i + d) * RS + (d - 1);
-        // blocks of eight split points per lane, summed in order.  WIDE: while
-        // a lane has more than eight points left, two blocks' 32 loads are
-        // issued together (one L2 round trip for sixteen points: long spans
-        // have up to 47 points per lane); the narrow form keeps 16 loads in
-        // flight for kernels without the registers.  Points past the end are
-        // -inf, which lse_add8 skips exactly, so both forms give the same bits.
-        int k = NLO + lane;
+    m = -INFINITY;
+    s = 0.f;
+    const int kend = d - e;
+    if (valid && kend > e) {
+        // blocks of eight split points per lane, summed in order; while a lane
+        // has more than eight points left, two blocks' 32 loads are issued
+        // together (one L2 round trip for sixteen points: long spans have up
+        // to 63 points per lane).  Points past the end are -inf, which
+        // lse_add8 skips exactly.
+        int k = e + lane;
         if (G == 32) {  // warp-uniform: one cell per warp, constant strides
-            int rem;
-            if (WIDE) {
-                for (; k + 15 * 32 < kend; k += 16 * 32) split_full16<32>(c.m, c.s, lrow, scol, k);
-                rem = (kend - k + 31) / 32;  // points left (<= 0: none)
-                if (rem > 8) {
-                    split_tail32<true>(c.m, c.s, lrow, scol, k, rem);
-                    rem = 0;
-                }
-            } else {
-                rem = (kend - k + 31) / 32;
-            }
-            for (; rem > 0; rem -= 8, k += 8 * 32) split_tail32<false>(c.m, c.s, lrow, scol, k, rem);
+            for (; k + 15 * 32 < kend; k += 16 * 32) split_full16<32>(m, s, lrow, scol, k);
+            const int rem = (kend - k + 31) / 32;  // points left (<= 0: none)
+            if (rem > 8) split_tail32<true>(m, s, lrow, scol, k, rem);
+            else if (rem > 0) split_tail32<false>(m, s, lrow, scol, k, rem);
         } else {
-            if (WIDE) {
-                for (; k + 8 * G < kend; k += 16 * G) {
-                    float a[16], b[16];
-#pragma unroll
-                    for (int q = 0; q < 16; q++) {
-                        const int kq = k + q * G;
-                        const bool on = kq < kend;
-                        a[q] = ldcg_if(lrow + kq, on, -INFINITY);
-                        b[q] = ldcg_if(scol - kq, on, -INFINITY);
-                    }
-                    float x0[8], x1[8];
-#pragma unroll
-                    for (int q = 0; q < 8; q++) {
-                        x0[q] = a[q] + b[q];
-                        x1[q] = a[8 + q] + b[8 + q];
-                    }
-                    lse_add8(c.m, c.s, x0);
-                    lse_add8(c.m, c.s, x1);
-                }
-            }
             for (; k < kend; k += 8 * G) {
                 float x[8];
 #pragma unroll
@@ -910,398 +877,105 @@ __device__ __forceinline__ CellPartial cell_partial_t(const Band& t, int i, int 
                     const bool on = kq < kend;
                     x[q] = ldcg_if(lrow + kq, on, -INFINITY) + ldcg_if(scol - kq, on, -INFINITY);
                 }
-                lse_add8(c.m, c.s, x);
+                lse_add8(m, s, x);
             }
         }
     }
-    // the shuffles only where some lane group of the warp has a cell (the
-    // callers pass every lane of the warp; an empty slot's result is unused)
-    if (__any_sync(0xffffffffu, valid)) group_reduce_rt(c.m, c.s, G);
-    return c;
+    // the shuffles only where some lane group of the warp has a cell
+    if (__any_sync(0xffffffffu, valid)) group_reduce_rt(m, s, G);
 }
 
-// cell_partial_t in two steps, for a wavefront that issues a cell's loads
-// one phase before it needs them: partial_issue loads the pair score and the
-// operands of the first two blocks (sixteen split points per lane) without
-// using them, so that the loads stay in flight; partial_complete adds them
-// and any further blocks in the same order and reduces over the group, so the
-// result has the bits of cell_partial_t.
-struct PartialPre {
-    float a[16], b[16];
-    float pbv;
-};
-
-template <int NLO, int NHI>
-__device__ __forceinline__ void partial_issue(const Band& t, int i, int d, bool valid, int lane, int G,
-                                              PartialPre& pp)
-{
-    const int RS = t.RS;
-    pp.pbv = (valid && lane == 0 && d >= 2) ? t.pb[(size_t)i * RS + d] : -INFINITY;
-    const int kend = d - NHI;
-    const float* lrow = t.Lrow + (size_t)i * RS;
-    const float* scol = t.Scol + (size_t)(i + d) * RS + (d - 1);
-    if (G == 32) {  // constant strides from two base addresses
-        const float* pa = lrow + NLO + lane;
-        const float* pb = scol - NLO - lane;
-#pragma unroll
-        for (int q = 0; q < 16; q++) {
-            const bool on = valid && NLO + lane + q * 32 < kend;
-            pp.a[q] = ldcg_if(pa + q * 32, on, -INFINITY);
-            pp.b[q] = ldcg_if(pb - q * 32, on, -INFINITY);
-        }
-    } else {
-#pragma unroll
-        for (int q = 0; q < 16; q++) {
-            const int kq = NLO + lane + q * G;
-            const bool on = valid && kq < kend;
-            pp.a[q] = ldcg_if(lrow + kq, on, -INFINITY);
-            pp.b[q] = ldcg_if(scol - kq, on, -INFINITY);
-        }
-    }
-}
-
-template <int NLO, int NHI, bool LONG>
-__device__ __forceinline__ CellPartial partial_complete(const Band& t, int i, int d, bool valid, int lane, int G,
-                                                        const PartialPre& pp)
-{
-    CellPartial c{-INFINITY, 0.f, pp.pbv};
-    const int kend = d - NHI;
-    if (valid && kend > NLO) {
-        // a block that cell_partial_t would not reach is all -inf: lse_add8 leaves (m, s) as they are
-        float x0[8], x1[8];
-#pragma unroll
-        for (int q = 0; q < 8; q++) {
-            x0[q] = pp.a[q] + pp.b[q];
-            x1[q] = pp.a[8 + q] + pp.b[8 + q];
-        }
-        lse_add8(c.m, c.s, x0);
-        lse_add8(c.m, c.s, x1);
-        const float* lrow = t.Lrow + (size_t)i * t.RS;
-        const float* scol = t.Scol + (size_t)(i + d) * t.RS + (d - 1);
-        int k = NLO + lane + 16 * G;
-        if (LONG && G == 32) {
-            // further points sixteen at a time: 32 loads per round trip
-            for (; k + 15 * 32 < kend; k += 16 * 32) split_full16<32>(c.m, c.s, lrow, scol, k);
-            const int rem = (kend - k + 31) / 32;  // points left (<= 0: none)
-            if (rem > 8) split_tail32<true>(c.m, c.s, lrow, scol, k, rem);
-            else if (rem > 0) split_tail32<false>(c.m, c.s, lrow, scol, k, rem);
-        } else {
-            for (; k < kend; k += 8 * G) {
-                float x[8];
-#pragma unroll
-                for (int q = 0; q < 8; q++) {
-                    const int kq = k + q * G;
-                    x[q] = (kq < kend) ? __ldcg(lrow + kq) + __ldcg(scol - kq) : -INFINITY;
-                }
-                lse_add8(c.m, c.s, x);
-            }
-        }
-    }
-    // the shuffles only where some lane group of the warp has a cell (the
-    // callers pass every lane of the warp; an empty slot's result is unused)
-    if (__any_sync(0xffffffffu, valid)) group_reduce_rt(c.m, c.s, G);
-    return c;
-}
-
-// Operands of a cell's outer split points, k < NLO and k >= hb = max(NLO,
-// d-NHI) in ascending k: L(i, i+k) and S(i+k+1, j), both -inf where the
-// split point is absent (an absent term is then -inf, which lse_add skips
-// exactly), and the enclosed F(i+1, j-1).
-template <int NLO, int NHI>
+// Operands of a cell's outer split points, k < N and k >= hb = max(N, d-N) in
+// ascending k: L(i, i+k) and S(i+k+1, j), both -inf where the split point is
+// absent (an absent term is then -inf, which lse_add8 skips exactly), and the
+// enclosed F(i+1, j-1).  With N = 3 (even spans) L(i, i+d-1) and S(i+1, j), the
+// two operands on diagonal d-1, are left to outer_patch.
+template <int N>
 struct Outer {
-    float l[NLO + NHI], s[NLO + NHI], fin;
+    float l[2 * N], s[2 * N], fin;
+    __device__ __forceinline__ bool complete() const
+    {
+        bool ok = !unwritten(fin);
+#pragma unroll
+        for (int q = 0; q < 2 * N; q++) ok = ok && !unwritten(l[q]) && !unwritten(s[q]);
+        return ok;
+    }
 };
 
-// defer: leave L(i, i+d-1) and S(i+1, j), the two operands on diagonal d-1,
-// to outer_patch.
-template <int NLO, int NHI>
-__device__ __forceinline__ Outer<NLO, NHI> outer_load(const Band& t, int i, int d, bool defer)
+template <int N>
+__device__ __forceinline__ void outer_load(const Band& t, int i, int d, Outer<N>& o)
 {
-    Outer<NLO, NHI> o;
-    const int RS = t.RS;
-    const float* lrow = t.Lrow + (size_t)i * RS;
-    const float* scol = t.Scol + (size_t)(i + d) * RS + (d - 1);
-    const int hb = max(NLO, d - NHI);
+    const float* lrow = t.Lrow + (size_t)i * t.RS;
+    const float* scol = t.Scol + (size_t)(i + d) * t.RS + (d - 1);
+    const int hb = max(N, d - N);
 #pragma unroll
-    for (int q = 0; q < NLO + NHI; q++) {
-        const int k = (q < NLO) ? q : hb + (q - NLO);
-        const bool present = k < d;
-        o.l[q] = !present ? -INFINITY : ((defer && k == d - 1) ? 0.f : __ldcg(lrow + k));
-        o.s[q] = !present ? -INFINITY : ((defer && k == 0) ? 0.f : __ldcg(scol - k));
+    for (int q = 0; q < 2 * N; q++) {
+        const int k = (q < N) ? q : hb + (q - N);
+        o.l[q] = o.s[q] = -INFINITY;
+        if (k < d && !(N == 3 && k == d - 1)) o.l[q] = ld_cell(lrow + k);
+        if (k < d && !(N == 3 && q == 0)) o.s[q] = ld_cell(scol - k);
     }
-    o.fin = (d >= 2) ? __ldcg(t.Frow + (size_t)(i + 1) * RS + (d - 2)) : -INFINITY;
-    return o;
+    o.fin = -INFINITY;
+    if (d >= 2) o.fin = ld_cell(t.Frow + (size_t)(i + 1) * t.RS + (d - 2));
 }
 
-template <int NLO, int NHI>
-__device__ __forceinline__ void outer_patch(Outer<NLO, NHI>& o, int d, float l_last, float s_first)
+// The same once every operand is there, for the whole warp; false if that took too long.
+template <int N>
+__device__ __forceinline__ bool outer_wait(const Band& t, int i, int d, bool mine, Outer<N>& o, unsigned int* sync)
 {
-    const int hb = max(NLO, d - NHI);
-#pragma unroll
-    for (int q = 0; q < NLO + NHI; q++) {
-        const int k = (q < NLO) ? q : hb + (q - NLO);
-        if (k < d && k == d - 1) o.l[q] = l_last;
-        if (k < d && k == 0) o.s[q] = s_first;
+    unsigned int spins = 0;
+    for (;;) {
+        if (mine) outer_load<N>(t, i, d, o);
+        mine = mine && !o.complete();
+        if (!__any_sync(0xffffffffu, mine)) return true;
+        if (!keep_waiting(spins, sync)) return false;
     }
 }
 
-// Adds the outer split points to the partial sum and writes cell (i, i+d);
-// lv/sv, when given, also receive its L and S.
-template <int NLO, int NHI>
-__device__ __forceinline__ void cell_write_t(const Band& t, int i, int d, CellPartial c, const Outer<NLO, NHI>& o,
-                                             const Rules& R, float* lv = nullptr, float* sv = nullptr)
+__device__ __forceinline__ void outer_patch(Outer<3>& o, int d, float l_last, float s_first)
+{
+    const int hb = max(3, d - 3);
+#pragma unroll
+    for (int q = 0; q < 6; q++)
+        if (((q < 3) ? q : hb + (q - 3)) == d - 1) o.l[q] = l_last;
+    o.s[0] = s_first;
+}
+
+// Adds the outer split points to the partial sum (m, s) and writes cell
+// (i, i+d); returns its L and S.  pbv: the pair's score.
+template <int N>
+__device__ __forceinline__ float2 cell_write(const Band& t, int i, int d, float m, float s, float pbv,
+                                             const Outer<N>& o, const Rules& R)
 {
     const int RS = t.RS;
     const int j = i + d;
     // the outer split points as one block (one max, independent exponentials:
-    // this is the serial part of a cell after the barrier)
+    // this is the serial part of a cell after the wait)
     float x[8];
 #pragma unroll
-    for (int q = 0; q < 8; q++) x[q] = (q < NLO + NHI) ? o.l[q % (NLO + NHI)] + o.s[q % (NLO + NHI)] : -INFINITY;
-    lse_add8(c.m, c.s, x);
-    const float tmp = lse_val(c.m, c.s);
-    const float v = c.pbv + o.fin;
+    for (int q = 0; q < 8; q++) x[q] = (q < 2 * N) ? o.l[q % (2 * N)] + o.s[q % (2 * N)] : -INFINITY;
+    lse_add8(m, s, x);
+    const float tmp = lse_val(m, s);
+    const float v = pbv + o.fin;
     const float S = lse2f(R.r[0] + tmp, R.r[2] + v);
     const float F = lse2f(R.r[4] + tmp, R.r[3] + v);
     const float Lv = R.r[6] + v;
-    t.Lrow[(size_t)i * RS + d] = Lv;
+    st_cell(t.Lrow + (size_t)i * RS + d, Lv);
+    st_cell(t.Scol + (size_t)j * RS + d, S);
+    st_cell(t.Frow + (size_t)i * RS + d, F);
     t.Lcol[(size_t)j * RS + d] = Lv;
     t.Srow[(size_t)i * RS + d] = S;
-    t.Scol[(size_t)j * RS + d] = S;
-    t.Frow[(size_t)i * RS + d] = F;
     if (j == t.L - 1) t.Ssuf[i] = S;
-    if (lv) {
-        *lv = Lv;
-        *sv = S;
-    }
+    return make_float2(Lv, S);
 }
 
-template <int NLO, int NHI>
-__device__ __forceinline__ void cell_finish_t(const Band& t, int i, int d, bool valid, int lane, CellPartial c,
-                                              const Rules& R)
-{
-    if (!(valid && lane == 0)) return;
-    cell_write_t<NLO, NHI>(t, i, d, c, outer_load<NLO, NHI>(t, i, d, false), R);
-}
-
-template <bool WIDE>
-__device__ __forceinline__ CellPartial inside_cell_partial(const Band& t, int i, int d, bool valid, int lane, int G)
-{
-    return (d & 1) ? cell_partial_t<2, 2, WIDE>(t, i, d, valid, lane, G) : cell_partial_t<3, 3, WIDE>(t, i, d, valid, lane, G);
-}
-
-__device__ __forceinline__ void inside_cell_finish(const Band& t, int i, int d, bool valid, int lane, CellPartial c,
-                                                   const Rules& R)
-{
-    if (d & 1) cell_finish_t<2, 2>(t, i, d, valid, lane, c, R);
-    else cell_finish_t<3, 3>(t, i, d, valid, lane, c, R);
-}
-
-template <bool WIDE>
-__device__ __forceinline__ void inside_cell(const Band& t, int i, int d, bool valid, int lane, int G, const Rules& R)
-{
-    inside_cell_finish(t, i, d, valid, lane, inside_cell_partial<WIDE>(t, i, d, valid, lane, G), R);
-}
-
-// The cells of one diagonal that a CTA owns (rows [r0, end)), computed by the
-// CTA's warps [w0, w0 + nw) in two phases: partial sums of the first two rows
-// of every group, then (after the caller's wait) their finishing parts and any
-// further rows whole.  Which warp computes a cell does not change its bits.
-struct RowsPart {
-    CellPartial c[2];
-};
-
-struct WarpSet {
-    int w0, nw;
-    __device__ __forceinline__ bool mine() const
-    {
-        const int w = threadIdx.x >> 5;
-        return w >= w0 && w < w0 + nw;
-    }
-};
-
-template <bool WIDE>
-__device__ __forceinline__ RowsPart rows_partial(const Band& t, int d, int r0, int end, WarpSet ws)
-{
-    RowsPart p;
-    p.c[0] = p.c[1] = CellPartial{-INFINITY, 0.f, -INFINITY};
-    if (!ws.mine()) return p;  // warp-uniform: the group shuffles stay within the warp
-    const int G = group_width(d), gpb = ws.nw * (32 / G);
-    const int lane = threadIdx.x & (G - 1), g = (threadIdx.x - 32 * ws.w0) / G;
-#pragma unroll
-    for (int it = 0; it < 2; it++) {
-        const int i = r0 + g + it * gpb;
-        p.c[it] = inside_cell_partial<WIDE>(t, i, d, i < end, lane, G);
-    }
-    return p;
-}
-
-template <bool WIDE>
-__device__ __forceinline__ void rows_finish(const Band& t, int d, int r0, int end, const RowsPart& p, const Rules& R,
-                                            WarpSet ws)
-{
-    if (!ws.mine()) return;
-    const int G = group_width(d), gpb = ws.nw * (32 / G);
-    const int lane = threadIdx.x & (G - 1), g = (threadIdx.x - 32 * ws.w0) / G;
-    if (G >= 2) {
-        // every lane of a group holds both reduced partial sums: lanes 0 and 1
-        // finish the group's two cells side by side
-        const int it = lane & 1;
-        const int i = r0 + g + it * gpb;
-        inside_cell_finish(t, i, d, lane < 2 && i < end, 0, it ? p.c[1] : p.c[0], R);
-    } else {
-#pragma unroll
-        for (int it = 0; it < 2; it++) {
-            const int i = r0 + g + it * gpb;
-            inside_cell_finish(t, i, d, i < end, lane, p.c[it], R);
-        }
-    }
-    for (int base = r0 + 2 * gpb; base < end; base += gpb) {
-        const int i = base + g;
-        inside_cell<WIDE>(t, i, d, i < end, lane, G, R);
-    }
-}
-
-// All band diagonals of the inside pass, two per grid barrier.  CTA b owns
-// rows [b*R, (b+1)*R) of every diagonal (R = ceil(L / CTAs)).  For the pair
-// (2p-1, 2p) it computes diagonal 2p-1 for its rows plus row (b+1)*R (which
-// the next CTA also computes, to the same bits) and then, after a CTA
-// barrier, diagonal 2p, whose cells read diagonal 2p-1 only at rows i and
-// i+1, its own.  The partial sums of both diagonals read spans <= 2p-4 and
-// are computed between the CTA's arrival at the barrier that completes
-// diagonal 2p-2 and its wait there; every warp computes both diagonals'
-// cells, one after the other.
-__global__ void __launch_bounds__(kWaveMaxThreads) inside_wave_kernel(Band t, Rules R, double B)
-{
-    unsigned int gen = 0;
-    const int L = t.L;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < L; i += gridDim.x * blockDim.x) inside_init_cell(t, i, R, B);
-    grid_arrive(t.sync);
-    const int rows = (L + gridDim.x - 1) / gridDim.x;
-    const int r0 = blockIdx.x * rows;
-    const WarpSet all{0, (int)(blockDim.x >> 5)};
-    for (int eA = 1; eA <= t.Wb; eA += 2) {
-        const int eB = eA + 1;
-        const int endA = min(r0 + rows + 1, L - eA);
-        const int endB = (eB <= t.Wb) ? min(r0 + rows, L - eB) : r0;
-        const RowsPart pa = rows_partial<true>(t, eA, r0, endA, all);
-        const RowsPart pb = rows_partial<true>(t, eB, r0, endB, all);
-        if (!grid_wait(t.sync, gen)) return;
-        // further rows (short spans only) in the narrow form: the wide one
-        // would spill beside the partial sums held across the wait
-        rows_finish<false>(t, eA, r0, endA, pa, R, all);
-        __syncthreads();  // diagonal 2p-1 of this CTA's rows before diagonal 2p reads it
-        rows_finish<false>(t, eB, r0, endB, pb, R, all);
-        grid_arrive(t.sync);
-    }
-}
-
-// inside_wave_kernel when the CTA's rows fit one per warp in each half of
-// the CTA (the host launches it only then): the odd diagonals' cells go to
-// the first half, the even ones' to the second, one cell per lane group.
-// The wait that completes diagonal 2p-2 also completes every span that the
-// next pair's partial sums read (<= 2p-2), so a warp issues the loads of its
-// next cell's partial sum as soon as its current cell is finished, before
-// the arrival, and adds them after it.
-// LONG (bands in which a lane has more than the sixteen prefetched points):
-// the rows of a diagonal pair are dealt evenly over the CTAs pair by pair
-// (ceil((L - 2p + 1) / CTAs) each) -- everything a pair reads of earlier pairs
-// goes through global memory, so the owner of a row may change -- so that long
-// spans, which have few rows, do not leave the CTAs of the high rows idle
-// while those of the low rows sum them all, and a lane's further points are
-// loaded sixteen at a time (L = 2,001, every span: 7.29 -> 5.18 ms).
-// Bands up to kShortBand keep the fixed rows: they gain nothing from either
-// and lose registers to both (span 500 over 1,000 columns: 0.74 -> 0.92 ms).
-constexpr int kShortBand = 16 * 32;
-
-template <bool LONG>
-__global__ void __launch_bounds__(kWaveMaxThreads) inside_wave_pipe_kernel(Band t, Rules R, double B)
-{
-    __shared__ float s_lv[kWaveMaxThreads / 64], s_sv[kWaveMaxThreads / 64];
-    unsigned int gen = 0;
-    const int L = t.L, Wb = t.Wb;
-    const int half = (int)(blockDim.x >> 6);
-    if (half < (L + (int)gridDim.x - 1) / (int)gridDim.x + 1) {  // not launched so; leave with the launch marked failed
-        if (blockIdx.x == 0 && threadIdx.x == 0) atomicExch(&t.sync[2], 1u);
-        return;
-    }
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < L; i += gridDim.x * blockDim.x) inside_init_cell(t, i, R, B);
-    grid_arrive(t.sync);
-    const bool odd = (int)(threadIdx.x >> 5) < half;
-    const int tid = (int)threadIdx.x - (odd ? 0 : 32 * half);
-    // this warp's diagonal of pair p is 2p-1 (odd) or 2p; its cell's row is the
-    // tid / G-th from the CTA's first one, r0 = b * rows, of that pair
-    const int grid = (int)gridDim.x;
-    auto row_end = [&](int dg, int r, int rw) { return (dg > Wb) ? r : min(r + rw + (odd ? 1 : 0), L - dg); };
-    int d = odd ? 1 : 2;
-    int rows = (L - (LONG ? 1 : 0) + grid - 1) / grid, r0 = blockIdx.x * rows;
-    int G = group_width(d), lane = tid & (G - 1), i = r0 + tid / G;
-    bool valid = i < row_end(d, r0, rows);
-    CellPartial c;
-    {
-        PartialPre pp;
-        if (odd) {
-            partial_issue<2, 2>(t, i, d, valid, lane, G, pp);
-            c = partial_complete<2, 2, LONG>(t, i, d, valid, lane, G, pp);
-        } else {
-            partial_issue<3, 3>(t, i, d, valid, lane, G, pp);
-            c = partial_complete<3, 3, LONG>(t, i, d, valid, lane, G, pp);
-        }
-    }
-    for (int eA = 1; eA <= Wb; eA += 2) {
-        if (!grid_wait(t.sync, gen)) return;
-        const int dn = d + 2;
-        if (LONG)  // ceil((L - eA - 2) / grid) rows for the next pair
-            while (rows > 1 && (rows - 1) * grid >= L - eA - 2) rows--;
-        const int r0n = LONG ? (int)blockIdx.x * rows : r0;
-        const int Gn = group_width(dn), lanen = tid & (Gn - 1), in = r0n + tid / Gn;
-        const bool validn = in < row_end(dn, r0n, rows);
-        PartialPre pn;
-        int ib = -1;
-        Outer<3, 3> ob;
-        if (odd) {
-            if (valid && lane == 0)
-                cell_write_t<2, 2>(t, i, d, c, outer_load<2, 2>(t, i, d, false), R, s_lv + (i - r0), s_sv + (i - r0));
-        } else if (valid && lane == 0) {
-            ob = outer_load<3, 3>(t, i, d, true);
-            ib = i;
-        }
-        __syncthreads();  // diagonal 2p-1 of this CTA's rows in s_lv / s_sv
-        if (ib >= 0) {
-            outer_patch<3, 3>(ob, d, s_lv[ib - r0], s_sv[ib + 1 - r0]);
-            cell_write_t<3, 3>(t, ib, d, c, ob, R);
-        }
-        // the next cell's loads go out after the current cells' (issued
-        // earlier they queue ahead of the finishing loads, which are on the
-        // critical path) and stay in flight across the arrival
-        if (odd) partial_issue<2, 2>(t, in, dn, validn, lanen, Gn, pn);
-        else partial_issue<3, 3>(t, in, dn, validn, lanen, Gn, pn);
-        // the last warp never has a cell (its group index is >= rows), so no
-        // loads in flight for the fence to wait for; the CTA barrier also
-        // orders these reads before the next pair's writes
-        grid_arrive(t.sync, blockDim.x - 1);
-        c = odd ? partial_complete<2, 2, LONG>(t, in, dn, validn, lanen, Gn, pn)
-                : partial_complete<3, 3, LONG>(t, in, dn, validn, lanen, Gn, pn);
-        d = dn;
-        G = Gn;
-        lane = lanen;
-        i = in;
-        r0 = r0n;
-        valid = validn;
-    }
-}
-
-// Batched inside over n alignments in one persistent launch: diagonal d of
-// every alignment whose band reaches it is one step of the wavefront.  Bands
-// are sorted by band width, descending, so the alignments active at span d
-// are a prefix [0, nact) and the cells of diagonal d, flattened in band order,
-// start at cumL[b] - d*b for band b (cumL: exclusive prefix of the lengths).
+// Band of the batch with span d or more: bands are sorted by width, descending.
 __device__ __forceinline__ int batch_active(const int* __restrict__ wbs, int n, int d)
 {
     int lo = 0, hi = n;  // first band with Wb < d
     while (lo < hi) {
         const int mid = (lo + hi) >> 1;
-        if (wbs[mid] >= d) lo = mid + 1;
+        if (__ldg(wbs + mid) >= d) lo = mid + 1;
         else hi = mid;
     }
     return lo;
@@ -1312,50 +986,292 @@ __device__ __forceinline__ int batch_band(const long long* __restrict__ cumL, in
     int lo = 0, hi = nact - 1;  // last band b with cumL[b] - d*b <= item
     while (lo < hi) {
         const int mid = (lo + hi + 1) >> 1;
-        if (cumL[mid] - (long long)d * mid <= item) lo = mid;
+        if (__ldg(cumL + mid) - (long long)d * mid <= item) lo = mid;
         else hi = mid - 1;
     }
     return lo;
 }
 
-__global__ void __launch_bounds__(kWaveMaxThreads) inside_wave_batch_kernel(const Band* __restrict__ bands,
-                                                                const long long* __restrict__ cumL,
-                                                                const int* __restrict__ wbs, int n, Rules R,
-                                                                double B, unsigned int* sync)
+constexpr int kInsideThreads = 512;       // 128 registers a thread
+constexpr int kInsideManyThreads = 768;   // 80
+constexpr int kInsideManyRows = 16;       // cells of a diagonal per CTA from which on there are so many threads
+constexpr int kInsideFinish = 64;  // threads that finish each diagonal of a pair
+constexpr int kInsideCells = 512;  // cells of a diagonal that a CTA takes at a time
+
+// The bands of an inside launch: one (t) or a batch of n, whose cells of
+// diagonal d, flattened in band order, start at cumL[b] - d*b for band b.
+template <bool BATCH>
+struct InsideBands {
+    Band t;
+    const Band* bands;
+    const long long* cumL;
+    const int* wbs;
+    int n;
+    __device__ __forceinline__ const Band& at(int b) const { return BATCH ? bands[b] : t; }
+};
+
+// The cells of diagonal d (the pair's odd one) that this CTA owns: [f0, f0 +
+// nb) of the flattened list; of the odd diagonal also the one after them
+// (na = nb + 1, unless the list ends there).
+struct PairRows {
+    long long f0;
+    int nact, na, nb;
+};
+
+template <bool BATCH>
+__device__ __forceinline__ PairRows pair_rows(const InsideBands<BATCH>& ib, int d)
 {
-    unsigned int gen = 0;
-    {
-        const long long total = cumL[n];
-        for (long long it = blockIdx.x * (long long)blockDim.x + threadIdx.x; it < total;
-             it += (long long)gridDim.x * blockDim.x) {
-            const int b = batch_band(cumL, n, 0, it);
-            inside_init_cell(bands[b], (int)(it - cumL[b]), R, B);
-        }
+    PairRows p;
+    p.nact = BATCH ? batch_active(ib.wbs, ib.n, d) : 1;
+    const long long ncell = BATCH ? __ldg(ib.cumL + p.nact) - (long long)d * p.nact : ib.t.L - d;
+    const int rows = (int)(((unsigned)ncell + gridDim.x - 1) / gridDim.x);
+    p.f0 = (long long)blockIdx.x * rows;
+    const long long left = ncell - p.f0;
+    p.nb = (int)max(0ll, min((long long)rows, left));
+    p.na = (int)max(0ll, min((long long)rows + 1, left));
+    return p;
+}
+
+template <bool BATCH>
+__device__ __forceinline__ int2 pair_cell(const InsideBands<BATCH>& ib, const PairRows& p, int d, int r)
+{
+    if (!BATCH) return make_int2(0, (int)p.f0 + r);
+    const int b = batch_band(ib.cumL, p.nact, d, p.f0 + r);
+    return make_int2(b, (int)(p.f0 + r - (__ldg(ib.cumL + b) - (long long)d * b)));
+}
+
+// All band diagonals of the inside pass (of one alignment, or of a batch: one
+// diagonal of every alignment at a time), in pairs (d = 2p-1, d+1).  The cells
+// of a pair are dealt evenly over the CTAs, pair by pair.  A CTA finishes
+// diagonal d for its cells and the next CTA's first one (which that CTA also
+// computes, to the same bits) and then diagonal d+1, whose cells read diagonal
+// d only at rows i and i+1, its own.
+// Four warps finish the cells, a thread per cell and two warps per diagonal:
+// they add the outer split points and write the cells.  The other warps
+// meanwhile form the partial sums of the next pair, which read spans <= d-1, and
+// leave them in shared memory: the sums are off the critical path, and a
+// finishing lane does not idle the rest of its warp.
+// The CTAs wait for one another's cells, not at a barrier: the tables are
+// filled with kUnwritten before the launch and a cell is its own flag (a grid
+// barrier's release alone took 2,100 cycles of a pair's 4,900: every store has
+// to be acknowledged before the arrival).  The finishing threads look at their
+// operands until all are there.  Those are spans d-1 and d-2, and what the other
+// warps read for the pair p+1 was written before them by the same chain of
+// CTAs, so a partial sum hardly ever meets an unwritten cell; it would be NaN,
+// and is then formed again once its cells are there.
+// Bound by the chain write -> look from L2 -> cells of d -> cells of d+1, about
+// 1.7 us a pair, and on long bands by the latency of the partial sums' loads.
+// Against one grid barrier per pair with every warp summing and then finishing
+// its own cell: span 500 of 1,000 columns 0.74 -> 0.51 ms, every span of 120
+// 154 -> 93 us and of 2,001 5.18 -> 3.78 ms, span 800 of 9,000 4.82 -> 4.70 ms;
+// 24 alignments of 80-600 columns, with a barrier per diagonal before, 3.23 ->
+// 1.23 ms.
+template <bool BATCH, int MAXT>
+__global__ void __launch_bounds__(MAXT) inside_pair_kernel(InsideBands<BATCH> ib, Rules R, double B,
+                                                                      unsigned int* sync)
+{
+    __shared__ float2 part[2][2][kInsideCells + 1];  // [pair parity][diagonal][cell]: partial (max, sum)
+    __shared__ float score[2][2][kInsideCells + 1];  // and the pair's score
+    __shared__ float2 last[kInsideCells + 1];        // L and S of diagonal d
+    __shared__ int2 cells[2][BATCH ? kInsideCells + 1 : 1];
+    __shared__ PairRows rows[2];
+    const int tid = threadIdx.x, nwork = (int)blockDim.x - 2 * kInsideFinish;
+    const bool fin = tid < 2 * kInsideFinish;
+    const int maxW = BATCH ? (ib.n > 0 ? ib.wbs[0] : 0) : ib.t.Wb;
+    bool bad = false;      // a wait of this thread took too long
+    bool own_nan = false;  // this warp has met a NaN that was no unwritten cell
+    for (long long it = blockIdx.x * (long long)blockDim.x + tid; it < (BATCH ? ib.cumL[ib.n] : ib.t.L);
+         it += (long long)gridDim.x * blockDim.x) {
+        const int b = BATCH ? batch_band(ib.cumL, ib.n, 0, it) : 0;
+        inside_init_cell(ib.at(b), (int)(BATCH ? it - ib.cumL[b] : it), R, B);
     }
-    grid_arrive(sync);
-    const int maxW = n > 0 ? wbs[0] : 0;
-    for (int d = 1; d <= maxW; d++) {
-        const int nact = batch_active(wbs, n, d);
-        const long long ncell = cumL[nact] - (long long)d * nact;
-        const int G = group_width(d);
-        const int gpb = blockDim.x / G;
-        const long long total = (long long)gridDim.x * gpb;
-        const int lane = threadIdx.x & (G - 1);
-        const long long gid0 = (long long)blockIdx.x * gpb + threadIdx.x / G;
-        // first cells: partial sums before the wait (as in inside_wave_kernel)
-        const bool v0 = gid0 < ncell;
-        const int b0 = v0 ? batch_band(cumL, nact, d, gid0) : 0;
-        const int i0 = v0 ? (int)(gid0 - (cumL[b0] - (long long)d * b0)) : 0;
-        const CellPartial c = inside_cell_partial<true>(bands[b0], i0, d, v0, lane, G);
-        if (!grid_wait(sync, gen)) return;
-        inside_cell_finish(bands[b0], i0, d, v0, lane, c, R);
-        for (long long base = total; base < ncell; base += total) {
-            const long long it = base + gid0;
-            const bool valid = it < ncell;
-            const int b = valid ? batch_band(cumL, nact, d, it) : 0;
-            inside_cell<true>(bands[b], valid ? (int)(it - (cumL[b] - (long long)d * b)) : 0, d, valid, lane, G, R);
+
+    // A partial sum came out NaN: again, until the cells are there.  After 64
+    // times (or once that has been the case) the cells are looked at one by one;
+    // a NaN of written cells is the scores' own.
+    auto again = [&](const float* lrow, const float* scol, int dd, int e, bool valid, int lane, int G, float& m,
+                     float& s) {
+        unsigned int spins = 0;
+        for (bool there = false; !there;) {
+            bad = __any_sync(0xffffffffu, !keep_waiting(spins, sync)) || bad;
+            if (bad) break;
+            if (own_nan || (spins & 63u) == 0u) {
+                bool missing = false;
+                if (valid)
+                    for (int k = e + lane; k < dd - e; k += G)
+                        missing = missing || unwritten(ld_cell(lrow + k)) || unwritten(ld_cell(scol - k));
+                there = !__any_sync(0xffffffffu, missing);
+                own_nan = own_nan || there;
+            }
+            asm volatile("" : "+l"(lrow), "+l"(scol)::"memory");  // not the cells read before
+            cell_partial(lrow, scol, dd, e, valid, lane, G, m, s);
+            if (!__any_sync(0xffffffffu, valid && s != s)) break;
         }
-        grid_arrive(sync);
+    };
+
+    // partial sums of cells [c0, c0 + kInsideCells) of the pair (d, d+1), by the other warps
+    auto partials = [&](const PairRows& p, int d, int c0, int buf) {
+        const int na = min(kInsideCells + 1, p.na - c0), nb = min(kInsideCells, p.nb - c0);
+        const int wt = tid - 2 * kInsideFinish;
+        if (BATCH) {
+            for (int r = wt; r < na; r += nwork) cells[buf][r] = pair_cell(ib, p, d, c0 + r);
+            asm volatile("bar.sync 2, %0;" ::"r"(nwork) : "memory");
+        }
+        if (c0 == 0) {
+            if (wt == 0) rows[buf] = p;
+            asm volatile("bar.arrive 3, %0;" ::"r"(nwork + 2 * kInsideFinish) : "memory");
+        }
+        const int G = group_width(d);  // of both diagonals: the limits are even, d is odd
+        const int gpb = nwork / G, lane = wt & (G - 1);
+        // Sum w of the pair: of cell r of diagonal dd, its L row and S column.
+        struct Item {
+            const float *lrow, *scol;
+            int r, dd;
+            float pbv;
+            bool valid;
+        };
+        auto item = [&](int w) {
+            Item q;
+            const int x = w >= na ? 1 : 0;
+            q.r = x ? w - na : w;
+            q.dd = d + x;
+            q.valid = w < na + nb;
+            const int2 c = BATCH ? cells[buf][q.valid ? q.r : 0] : make_int2(0, (int)p.f0 + c0 + q.r);
+            const Band& t = ib.at(c.x);
+            q.valid = q.valid && c.y + q.dd < t.L && q.dd <= t.Wb;
+            q.lrow = t.Lrow + (size_t)c.y * t.RS;
+            q.scol = t.Scol + (size_t)(c.y + q.dd) * t.RS + (q.dd - 1);
+            q.pbv = (q.valid && lane == 0 && q.dd >= 2) ? __ldg(t.pb + (size_t)c.y * t.RS + q.dd) : -INFINITY;
+            return q;
+        };
+        // A cell's sum is formed (m, s): kept, unless it is NaN for cells that
+        // were not there yet.
+        auto keep = [&](const Item& q, float m, float s) {
+            if (__any_sync(0xffffffffu, q.valid && s != s)) again(q.lrow, q.scol, q.dd, 2 + (q.dd - d), q.valid, lane, G, m, s);
+            if (q.valid && lane == 0) {
+                part[buf][q.dd - d][q.r] = make_float2(m, s);
+                score[buf][q.dd - d][q.r] = q.pbv;
+            }
+        };
+        if (G < 32 || MAXT > kInsideThreads) {
+            for (int base = 0; base < na + nb; base += gpb) {
+                const Item q = item(base + wt / G);
+                float m, s;
+                cell_partial(q.lrow, q.scol, q.dd, 2 + (q.dd - d), q.valid, lane, G, m, s);
+                keep(q, m, s);
+            }
+            return;
+        }
+        // A warp per cell: sixteen split points of a lane at a time, the loads
+        // of the next sixteen (of this cell or the warp's next one) in flight
+        // meanwhile (span 500 of 1,000 columns: 537 -> 511 us, the batch of 24
+        // 1.37 -> 1.23 ms).
+        auto load = [&](const Item& q, int k, float (&a)[16], float (&b)[16]) {
+            const int e = 2 + (q.dd - d), rem = q.valid ? (q.dd - e - k + 31) / 32 : 0;
+            const float* pa = q.lrow + k;
+            const float* pb = q.scol - k;
+#pragma unroll
+            for (int j = 0; j < 16; j++) {
+                a[j] = ldcg_if(pa + j * 32, j < rem, -INFINITY);
+                b[j] = ldcg_if(pb - j * 32, j < rem, -INFINITY);
+            }
+        };
+        int w = wt >> 5;
+        if (w >= na + nb) return;
+        Item q = item(w);
+        int k = 2 + (q.dd - d) + lane;
+        float a[16], b[16], m = -INFINITY, s = 0.f;
+        load(q, k, a, b);
+        for (bool next = true; next;) {
+            float x0[8], x1[8];
+#pragma unroll
+            for (int j = 0; j < 8; j++) {
+                x0[j] = a[j] + b[j];
+                x1[j] = a[8 + j] + b[8 + j];
+            }
+            const Item now = q;
+            const int left = now.valid ? now.dd - 2 - (now.dd - d) - (k - lane) : 0;  // split points from here on
+            const bool more = left > 512;                                               // of this cell, after these
+            next = more || w + gpb < na + nb;
+            if (more) {
+                k += 512;
+            } else if (next) {
+                q = item(w += gpb);
+                k = 2 + (q.dd - d) + lane;
+            }
+            if (next) load(q, k, a, b);
+            lse_add8(m, s, x0);
+            if (left > 256) lse_add8(m, s, x1);
+            if (!more) {
+                group_reduce_rt(m, s, 32);
+                keep(now, m, s);
+                m = -INFINITY;
+                s = 0.f;
+            }
+        }
+    };
+
+    // The cells [c0, c0 + kInsideCells) of diagonal dd = d + N - 2, by a thread
+    // each of 64; `ready`: what to do between the first cells' operands and the rest.
+    auto finish = [&](auto width, const PairRows& p, int d, int c0, int buf, auto ready) {
+        constexpr int N = decltype(width)::value;
+        const int x = N - 2, dd = d + x, n = x ? min(kInsideCells, p.nb - c0) : min(kInsideCells + 1, p.na - c0);
+        const int first = tid & (kInsideFinish - 1);
+        for (int r = first; r - (first & 31) < n || r == first; r += kInsideFinish) {
+            bool mine = r < n;
+            int2 c = make_int2(0, 0);
+            if (mine) c = (BATCH && c0 == 0) ? cells[buf][r] : pair_cell(ib, p, d, c0 + r);
+            const Band& t = ib.at(c.x);
+            mine = mine && c.y + dd < t.L && dd <= t.Wb;
+            Outer<N> o;
+            bad = !outer_wait<N>(t, c.y, dd, mine, o, sync) || bad;
+            if (r == first) ready();
+            if (!mine) continue;
+            if constexpr (N == 3) outer_patch(o, dd, last[r].x, last[r + 1].y);
+            const float2 ms = part[buf][x][r];
+            const float2 ls = cell_write<N>(t, c.y, dd, ms.x, ms.y, score[buf][x][r], o, R);
+            if constexpr (N == 2) last[r] = ls;
+        }
+    };
+    auto inside_barrier = [] { asm volatile("bar.sync 1, %0;" ::"n"(2 * kInsideFinish) : "memory"); };
+
+    int buf = 0;
+    if (!fin && maxW > 0) partials(pair_rows(ib, 1), 1, 0, 0);
+    for (int d = 1; d <= maxW; d += 2, buf ^= 1) {
+        PairRows p;
+        bool stop = false;
+        // every thread: the pair's partial sums are there, and its operands
+        auto together = [&] { stop = __syncthreads_or(bad) != 0; };
+        if (fin) {
+            asm volatile("bar.sync 3, %0;" ::"r"(nwork + 2 * kInsideFinish) : "memory");
+            p = rows[buf];
+            if (tid < kInsideFinish) {
+                finish(std::integral_constant<int, 2>{}, p, d, 0, buf, together);
+                inside_barrier();
+            } else {
+                finish(std::integral_constant<int, 3>{}, p, d, 0, buf, [&] {
+                    together();
+                    inside_barrier();  // diagonal d of this CTA's cells is in `last`
+                });
+            }
+        } else {
+            together();
+            p = rows[buf];
+            if (!stop && d + 2 <= maxW) partials(pair_rows(ib, d + 2), d + 2, 0, buf ^ 1);
+        }
+        // more cells than a CTA holds: the rest apart
+        for (int c0 = kInsideCells; c0 < p.nb; c0 += kInsideCells) {
+            __syncthreads();
+            if (!fin) partials(p, d, c0, buf);
+            __syncthreads();
+            if (tid < kInsideFinish) {
+                finish(std::integral_constant<int, 2>{}, p, d, c0, buf, [] {});
+                inside_barrier();
+            } else if (fin) {
+                finish(std::integral_constant<int, 3>{}, p, d, c0, buf, inside_barrier);
+            }
+        }
+        if (stop) return;
     }
 }
 
@@ -1872,16 +1788,13 @@ static int ctas_for_rows(int L, int warps) { return (warps > 1) ? (L + warps - 2
 // Launch a persistent wavefront kernel (cooperative: every CTA resident).
 // share > 0 (paired kernels): the CTA owns ceil(L / grid) rows of every
 // diagonal plus one, and a row wants `share` warps per diagonal pair (the
-// inside pass: one per diagonal, 2; the outside pass: one per parent sum of
-// each diagonal, 4).  The CTA grows (up to 1,024 threads, unless its size is
+// outside pass: one per parent sum of each diagonal, 4).  The CTA grows (up to 1,024 threads, unless its size is
 // set) to the smallest size at which warps / share of its warps hold those
-// rows one per warp with at most one CTA per SM (inside: the pipelined halves
-// kernel then runs; GB300, band of 500: 23-29% faster for 1,200-2,000
-// columns than 256- or 512-thread CTAs of the plain kernel); the grid then
-// grows (up to one CTA per SM) until the rows fit, or else fit one per warp
-// of the whole CTA.
+// rows one per warp with at most one CTA per SM; the grid then grows (up to
+// one CTA per SM) until the rows fit, or else fit one per warp of the whole
+// CTA.
 int launch_wave(messi_ctx* ctx, const void* kernel, void** args, unsigned int* sync, int L, double band_cells,
-                const char* what, int share, const void* halves_kernel)
+                const char* what, int share)
 {
     int threads = wave_threads(ctx, band_cells);
     cudaError_t e = cudaMemsetAsync(sync, 0, kSyncWords * sizeof(unsigned int), ctx->stream);
@@ -1900,9 +1813,6 @@ int launch_wave(messi_ctx* ctx, const void* kernel, void** args, unsigned int* s
         const int half = ctas_for_rows(L, warps / share);
         const int want = (half <= ctx->num_sms) ? half : ctas_for_rows(L, warps);
         grid = std::max(grid, std::min(want, ctx->num_sms));
-        // the halves shape (rows + 1 <= warps / 2 for ceil(L / grid) rows)
-        const int rows = (L + grid - 1) / grid;
-        if (halves_kernel && rows + 1 <= warps / 2) kernel = halves_kernel;
     }
     e = cudaLaunchCooperativeKernel(kernel, dim3(grid), dim3(threads), args, 0, ctx->stream);
     ctx->launches++;
@@ -1929,6 +1839,38 @@ int launch_barrier_selftest(messi_ctx* ctx, unsigned int* d_sync)
     return MESSI_OK;
 }
 
+// The inside kernel (cooperative: every CTA resident), one CTA per SM, after
+// the tables it waits on are filled with kUnwritten (each: first cell, cells).
+// 512 threads (1,024 leave 64 registers a thread and spill: span 500 of 1,000
+// columns 0.67 ms against 0.54); 256 where a CTA has at most two cells of a
+// diagonal and four warps form their sums (L = 120: 93 us against 102, L = 300:
+// 250 against 266, but L = 600, four cells: 370 against 277).  `many`, null for
+// a batch: with 16 cells and more per CTA twenty warps that form the sums are
+// worth more than twelve with their next loads in flight (span 800 of 3,000,
+// 4,500, 6,000 columns: 1.83, 2.52, 3.22 ms against 1.99, 2.87, 3.75; L = 2,001,
+// 13 cells: 3.98 against 3.78; the batch, which needs more registers, 1.34
+// against 1.23).
+static int launch_inside(messi_ctx* ctx, const void* kernel, const void* many, void** args, unsigned int* sync,
+                         long long columns, std::array<std::pair<float*, size_t>, 3> cells)
+{
+    cudaError_t e = cudaMemsetAsync(sync, 0, kSyncWords * sizeof(unsigned int), ctx->stream);
+    for (int k = 0; k < 3 && e == cudaSuccess; k++)
+        if (cells[k].second) e = cudaMemsetAsync(cells[k].first, 0xff, cells[k].second * sizeof(float), ctx->stream);
+    if (e != cudaSuccess) return cuda_fail(ctx, e, "inside table reset");
+    const int most = wave_grid(ctx, kernel, INT_MAX / 32, kInsideThreads);  // also sets ctx->num_sms
+    const int grid = (int)std::min<long long>(most, columns);
+    int threads = columns <= 2 * (long long)ctx->num_sms ? kInsideThreads / 2 : kInsideThreads;
+    if (ctx->wave_threads == 256 || ctx->wave_threads >= kInsideThreads)
+        threads = std::min(ctx->wave_threads, kInsideThreads);
+    if (many && threads == kInsideThreads && columns >= (long long)kInsideManyRows * grid) {
+        kernel = many;
+        threads = kInsideManyThreads;
+    }
+    e = cudaLaunchCooperativeKernel(kernel, dim3(grid), dim3(threads), args, 0, ctx->stream);
+    ctx->launches++;
+    return e == cudaSuccess ? MESSI_OK : cuda_fail(ctx, e, "inside_pair_kernel");
+}
+
 int queue_status_readback(messi_ctx* ctx, const Band& t)
 {
     if (!ctx->status_host) return MESSI_OK;
@@ -1940,14 +1882,15 @@ int queue_status_readback(messi_ctx* ctx, const Band& t)
 int run_inside(messi_ctx* ctx, const Band& t, double B)
 {
     Rules R = make_rules(B);
-    Band tt = t;
+    const size_t tab = (size_t)t.L * t.RS;
+    InsideBands<false> ib{t, nullptr, nullptr, nullptr, 1};
     double Bv = B;
-    void* args[] = {&tt, &R, &Bv};
+    unsigned int* sync = t.sync;
+    void* args[] = {&ib, &R, &Bv, &sync};
     prof_begin(ctx, 1, (double)t.L * (t.Wb + 1) - 0.5 * t.Wb * (t.Wb + 1.0));
-    int rc = launch_wave(ctx, (const void*)inside_wave_kernel, args, t.sync, t.L, (double)t.L * (t.Wb + 1),
-                         "inside_wave_kernel", 2,
-                         t.Wb > kShortBand ? (const void*)inside_wave_pipe_kernel<true>
-                                           : (const void*)inside_wave_pipe_kernel<false>);
+    int rc = launch_inside(ctx, (const void*)inside_pair_kernel<false, kInsideThreads>,
+                           (const void*)inside_pair_kernel<false, kInsideManyThreads>, args, sync, t.L,
+                           {{{t.Lrow, tab}, {t.Scol, tab}, {t.Frow, tab}}});
     if (rc) return rc;
     prof_end(ctx);
     if (t.L - 1 > t.Wb) {
@@ -1976,13 +1919,19 @@ int bandbatch_alloc(const std::vector<int>& L, const std::vector<int>& Wb, BandB
     for (int k = 0; k < n; k++) bb->slot[bb->order[k]] = k;
     // one allocation: per band 6 tables, Ssuf/Osuf, b/cb/u/Zd; then the batch arrays
     auto al = [](size_t x) { return (x + 255) & ~size_t(255); };
-    std::vector<size_t> off_tab(n), off_suf(n), off_dbl(n);
+    std::vector<size_t> off_polled(n), off_tab(n), off_suf(n), off_dbl(n);
     size_t bytes = 0;
+    for (int k = 0; k < n; k++) {  // the tables that the inside kernel waits on, for one fill
+        const int a = bb->order[k];
+        off_polled[k] = bytes;
+        bytes = al(bytes + 3 * (size_t)L[a] * (((size_t)Wb[a] + 1 + 31) / 32 * 32) * sizeof(float));
+    }
+    bb->polled = bytes / sizeof(float);
     for (int k = 0; k < n; k++) {
         const int a = bb->order[k];
         const size_t RS = ((size_t)Wb[a] + 1 + 31) / 32 * 32;
         off_tab[k] = bytes;
-        bytes = al(bytes + 6 * (size_t)L[a] * RS * sizeof(float));
+        bytes = al(bytes + 3 * (size_t)L[a] * RS * sizeof(float));
         off_suf[k] = bytes;
         bytes = al(bytes + (size_t)(L[a] + 1) * 2 * sizeof(float));
         off_dbl[k] = bytes;
@@ -2017,13 +1966,14 @@ int bandbatch_alloc(const std::vector<int>& L, const std::vector<int>& Wb, BandB
         t.Wb = Wb[a];
         t.RS = ((Wb[a] + 1 + 31) / 32) * 32;
         const size_t tab = (size_t)t.L * t.RS;
-        float* f = (float*)(base + off_tab[k]);
+        float* f = (float*)(base + off_polled[k]);
         t.Lrow = f;
-        t.Lcol = f + tab;
-        t.Srow = f + 2 * tab;
-        t.Scol = f + 3 * tab;
-        t.Frow = f + 4 * tab;
-        t.pb = f + 5 * tab;
+        t.Scol = f + tab;
+        t.Frow = f + 2 * tab;
+        f = (float*)(base + off_tab[k]);
+        t.Lcol = f;
+        t.Srow = f + tab;
+        t.pb = f + 2 * tab;
         t.Ssuf = (float*)(base + off_suf[k]);
         t.Osuf = t.Ssuf + (t.L + 1);
         t.b = (double*)(base + off_dbl[k]);
@@ -2076,22 +2026,15 @@ int run_inside_batch(messi_ctx* ctx, const BandBatch& bb, double B)
     int n = bb.n;
     double Bv = B;
     unsigned int* sync = bb.d_sync;
-    void* args[] = {&bands, &cum, &wbs, &n, &R, &Bv, &sync};
-    double cells = 0.0, band = 0.0;
-    for (const Band& t : bb.host) {
-        cells += (double)t.L * (t.Wb + 1) - 0.5 * t.Wb * (t.Wb + 1.0);
-        band += (double)t.L * (t.Wb + 1);
-    }
-    const int threads = wave_threads(ctx, band);
-    const int grid = wave_grid(ctx, (const void*)inside_wave_batch_kernel,
-                               (int)std::min<long long>(bb.total_cols, 1 << 30), threads);
+    InsideBands<true> ib{bb.host[0], bands, cum, wbs, n};
+    void* args[] = {&ib, &R, &Bv, &sync};
+    double cells = 0.0;
+    for (const Band& t : bb.host) cells += (double)t.L * (t.Wb + 1) - 0.5 * t.Wb * (t.Wb + 1.0);
     prof_begin(ctx, 1, cells);
-    cudaError_t e = cudaMemsetAsync(sync, 0, kSyncWords * sizeof(unsigned int), ctx->stream);
-    if (e != cudaSuccess) return cuda_fail(ctx, e, "barrier reset");
-    e = cudaLaunchCooperativeKernel((const void*)inside_wave_batch_kernel, dim3(grid), dim3(threads), args, 0,
-                                    ctx->stream);
-    ctx->launches++;
-    if (e != cudaSuccess) return cuda_fail(ctx, e, "inside_wave_batch_kernel");
+    int rc = launch_inside(ctx, (const void*)inside_pair_kernel<true, kInsideThreads>, nullptr, args, sync, bb.total_cols,
+                           {{{bb.host[0].Lrow, bb.polled}, {nullptr, 0}, {nullptr, 0}}});
+    if (rc) return rc;
+    cudaError_t e;
     prof_end(ctx);
     prof_begin(ctx, 2, 0.0);
     const int win = suffix_batch_window(bb);

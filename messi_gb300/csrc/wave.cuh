@@ -74,6 +74,40 @@ static __device__ bool grid_wait(unsigned int* sync, unsigned int& gen, unsigned
     return s_ok != 0;
 }
 
+// Dataflow waits: a table of FP32 cells filled with kUnwritten before the
+// launch, whose cells are their own flags.  The bits are a NaN that no
+// arithmetic gives (those are 0x7fffffff), so a cell is complete exactly when
+// it reads as anything else, and no fence or barrier need order its write with
+// another.  Reads and writes are relaxed at device scope (L2).
+constexpr unsigned int kUnwritten = 0xffffffffu;
+
+static __device__ __forceinline__ bool unwritten(float v) { return __float_as_uint(v) == kUnwritten; }
+
+static __device__ __forceinline__ float ld_cell(const float* p)
+{
+    float v;
+    asm volatile("ld.relaxed.gpu.global.f32 %0, [%1];" : "=f"(v) : "l"(p) : "memory");
+    return v;
+}
+
+static __device__ __forceinline__ void st_cell(float* p, float v)
+{
+    asm volatile("st.relaxed.gpu.global.f32 [%0], %1;" ::"l"(p), "f"(v) : "memory");
+}
+
+// One more failed look at cells that are not there yet: false (and the
+// launch marked failed) once the waiting has taken one to two seconds, or
+// some other CTA has given up.
+static __device__ __forceinline__ bool keep_waiting(unsigned int& spins, unsigned int* sync)
+{
+    if (++spins > kSpinLimit || ((spins & 1023u) == 0u && ld_acquire_u32(&sync[2]) != 0u)) {
+        atomicExch(&sync[2], 1u);
+        return false;
+    }
+    if (spins > 64u) __nanosleep(32);
+    return true;
+}
+
 static __device__ bool grid_sync(unsigned int* sync, unsigned int& gen, unsigned int spin_limit = kSpinLimit)
 {
     grid_arrive(sync);
