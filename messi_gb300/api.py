@@ -76,9 +76,9 @@ class Context:
         return n.value
 
     def selftest_bounded_wait(self):
-        """Status produced by a device wait that cannot complete (a grid
-        barrier one CTA never reaches): MESSI_ETIMEOUT when the bounded wait
-        gives up as designed.  The context stays usable."""
+        """Status produced by a device wait that cannot complete (for a cell
+        that nothing writes): MESSI_ETIMEOUT when the bounded wait gives up as
+        designed.  The context stays usable."""
         st = ctypes.c_int32()
         self.check(self.lib.messi_selftest_bounded_wait(self.handle, ctypes.byref(st)), "messi_selftest_bounded_wait")
         return st.value

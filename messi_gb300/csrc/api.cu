@@ -222,7 +222,7 @@ int finish(messi_ctx* ctx)
     e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_fail(ctx, e, "kernel execution");
     if (ctx->status_host && *ctx->status_host != 0u)
-        return fail(ctx, MESSI_ETIMEOUT, "wavefront grid barrier gave up waiting (bounded spin)");
+        return fail(ctx, MESSI_ETIMEOUT, "wavefront kernel gave up waiting (bounded spin)");
     return MESSI_OK;
 }
 
@@ -557,7 +557,7 @@ int messi_selftest_bounded_wait(messi_ctx* ctx, int32_t* status)
     void* p;
     if ((rc = ensure(ctx, kSlotVec, kSyncWords * sizeof(unsigned int), &p))) return rc;
     unsigned int flag = 0;
-    if ((rc = launch_barrier_selftest(ctx, (unsigned int*)p))) return rc;
+    if ((rc = launch_wait_selftest(ctx, (unsigned int*)p))) return rc;
     if ((rc = d2h(ctx, &flag, (unsigned int*)p + 2, sizeof(unsigned int)))) return rc;
     if ((rc = finish(ctx))) return rc;
     *status = flag ? MESSI_ETIMEOUT : MESSI_OK;

@@ -11,8 +11,8 @@
 //                   alpha*pair(i,j) + e(i+1,j-1),                          s = -2
 //                   max_k alpha*pair(i,k) + e(i+1,k-1) + e(k+1,j) )        s = k+1
 // with ties to the first alternative and the smallest k.  One persistent
-// cooperative launch walks the diagonals of 16 x 16 tiles (a grid barrier
-// between them).  e is kept row-major (the split's second factor) and
+// cooperative launch walks the diagonals of 16 x 16 tiles (a row block waits
+// for the next one's flag).  e is kept row-major (the split's second factor) and
 // column-major (the output); s is written column-major, the layout the Julia
 // caller reads.  The traceback runs on the device in one thread.
 //

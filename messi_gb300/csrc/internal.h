@@ -16,8 +16,8 @@
 namespace messi {
 
 constexpr int kTile = 128;          // unique pairs per CTA in the pruning kernels
-// Grid-barrier words of the wavefront kernels: [0] = arrivals, [2] =
-// host-visible error flag (wave.cuh).
+// Status words of the wavefront kernels: [2] = host-visible error flag of their
+// bounded waits (wave.cuh).
 constexpr int kSyncWords = 4;
 constexpr int kMaxLambda = 8;       // per-lambda conditionals kept in registers
 constexpr int kMaxStack = 512;      // tree height limit
@@ -141,7 +141,7 @@ struct Band {
     float* OSlast;  // suffix-column terms of the outside S sums of the last column's band cells
     double *b, *cb, *u, *Zd;
     int* maxspan;
-    unsigned int* sync;  // kSyncWords grid-barrier words of the wavefront kernels
+    unsigned int* sync;  // kSyncWords status words of the wavefront kernels
 };
 
 // Band tables of a batch of alignments for the batched inside pass.  Bands
@@ -254,7 +254,7 @@ struct messi_ctx {
     messi::DevBuf scratch[32];
     void* pinned = nullptr;
     size_t pinned_bytes = 0;
-    unsigned int* status_host = nullptr;  // pinned word: wavefront barrier status of the last call
+    unsigned int* status_host = nullptr;  // pinned word: wavefront wait status of the last call
     // device buffers are reallocated only when they grow; every reallocation
     // bumps the epoch, so a captured launch sequence knows its pointers are stale
     uint64_t alloc_epoch = 0;
@@ -431,9 +431,9 @@ struct SideLaunches {
     ~SideLaunches() { ctx->stream = main; }
 };
 
-// Bounded-wait self-test (scfg.cu): a two-CTA grid barrier that one CTA never
-// reaches; d_sync[2] becomes 1 when the other CTA's wait gives up.
-int launch_barrier_selftest(messi_ctx* ctx, unsigned int* d_sync);
+// Bounded-wait self-test (scfg.cu): a wait for a cell that nothing writes;
+// d_sync[2] becomes 1 when it gives up.
+int launch_wait_selftest(messi_ctx* ctx, unsigned int* d_sync);
 // Dense L x L pair matrix: vals (nullable) of the unique root pairs, mixed with
 // addw + u[x] + u[y] when addw is finite (the factorised lambda categories).
 int launch_scatter_dense(messi_ctx* ctx, messi_dataset* ds, const double* d_vals, const double* d_u, double addw,
@@ -478,9 +478,6 @@ int run_posterior_decoding(messi_ctx* ctx, int L, const double* d_single, const 
 // (nullable): [nstruct] log KH99 prior of each structure; d_status: 1 uint.
 int run_sample_structures(messi_ctx* ctx, const Band& t, double B, int nstruct, unsigned long long seed,
                           int* d_paired, int* d_stack, double* d_prior, unsigned int* d_status);
-// Grid and CTA size of a persistent wavefront kernel (cooperative launch).
-int wave_threads(const messi_ctx* ctx, double band_cells);
-int wave_grid(messi_ctx* ctx, const void* kernel, int L, int threads);
 int bandbatch_alloc(const std::vector<int>& L, const std::vector<int>& Wb, BandBatch* bb, std::string* err);
 void bandbatch_free(BandBatch* bb);
 int launch_baseline_batch(messi_ctx* ctx, const BandBatch& bb, double B);
@@ -494,12 +491,7 @@ void tune_begin(messi_ctx* ctx, const void* key, int C);
 void tune_mark(messi_ctx* ctx, int i);
 void tune_end(messi_ctx* ctx, const void* key, int C);
 void tune_forget(messi_ctx* ctx, const void* key);
-// Queue a copy of the wavefront barrier status into ctx->status_host.
+// Queue a copy of the wavefront wait status into ctx->status_host.
 int queue_status_readback(messi_ctx* ctx, const Band& t);
-// Cooperative launch of a persistent wavefront kernel (scfg.cu): resets the
-// barrier words, picks the CTA size and grid; share > 0 for kernels that own
-// rows of diagonal pairs (warps per row and pair).
-int launch_wave(messi_ctx* ctx, const void* kernel, void** args, unsigned int* sync, int L, double band_cells,
-                const char* what, int share = 0);
 
 }  // namespace messi

@@ -16,11 +16,11 @@
 //
 // Sharing.  All calls on a device use the same array and it keeps the last
 // call's contents; every cell a call reads is written by that call first (the
-// band tables are filled before use, the span counter and the wavefront
-// barrier are cleared).  Calls that overlap on the GPU (two streams, or two
+// band tables are filled before use, the span counter and the wavefront's
+// status are cleared).  Calls that overlap on the GPU (two streams, or two
 // host threads) race on the array, so callers serialise them.
 //
-// Errors.  If the wavefront's bounded barrier wait gives up, the call has
+// Errors.  If the wavefront's bounded wait gives up, the call has
 // already returned MESSI_OK (the kernels run after it returns) and the only
 // sign is *d_Z == NaN: callers check Z.  maxspan < 0 reads the inferred span
 // back to the host and synchronises the stream once; on a stream that is
@@ -46,7 +46,7 @@ struct NoAllocScratch {
     float suf[2 * (kNoAllocMaxL + 1)];      // Ssuf (+ unused outside half)
     double vec[2 * kNoAllocMaxL + 8];       // b, cb
     int maxspan[16];
-    unsigned int sync[kSyncWords];          // grid-barrier words of the wavefront kernel
+    unsigned int sync[kSyncWords];          // status words of the wavefront kernel
 };
 
 // Host code must not use this name as a device address: it is a host-side

@@ -29,8 +29,7 @@
 // wavefront): all cells of a span are independent, so each diagonal is spread
 // over the whole grid, two diagonals at a time (a CTA owns a block of rows and
 // the second diagonal of a pair reads the first only at the CTA's own rows).
-// The CTAs of the inside pass wait for one another's cells, those of the
-// outside pass at a grid barrier between pairs; both waits have a bounded
+// The CTAs wait for one another's cells; the waits have a bounded
 // iteration count: on timeout an error flag is raised, every CTA leaves, Z
 // becomes NaN and the host returns MESSI_ETIMEOUT.  A cell's split sum is
 // reduced by a group of G lanes (G grows with the number of split points) with
@@ -40,7 +39,6 @@
 // summed by 32 warps in parallel, the in-block triangle by one warp.
 #include <algorithm>
 #include <array>
-#include <climits>
 #include <cmath>
 
 #include "internal.h"
@@ -1277,18 +1275,46 @@ __global__ void __launch_bounds__(MAXT) inside_pair_kernel(InsideBands<BATCH> ib
 
 // Outside cell (i, j = i+d): the parent sums run over q of OS/OF(i, j+1+q) *
 // S(j+1, j+1+q) (side 0, "L") and of OS/OF(i-1-q, j) * L(i-1-q, i-1) (side
-// 1, "S"), spans d+1+q.  Each sum is computed apart, by its own lane group
-// (outside_sum_t: q >= Q and the suffix-column terms, reduced over the
-// group); the finishing part (outside_finish_t, one thread) adds q = 0 ..
-// Q-1 of both sums in ascending order, forms the F value from the enclosing
-// pair (i-1, j+1) (span d+2) and writes the cell.  Diagonals go two per
-// barrier, (e, e-1), with Q = 2 for e and Q = 3 for e-1: the sums then read
-// spans >= e+3 only, which are complete before the wait that completes e+2
-// and e+1.  A cell's bits depend only on its span (the group width), not on
-// which CTA, warp or thread computes it.
-struct SumPartial {
-    float m, s;
+// 1, "S"), spans d+1+q.  Each sum is computed apart: q >= Q and the
+// suffix-column terms by a lane group (outside_sum, reduced over the group),
+// then q = 0 .. Q-1 in ascending order by one thread (near_finish); the F value
+// comes from the enclosing pair (i-1, j+1) (span d+2).  Diagonals go in pairs
+// (e, e-1), with Q = 2 for e and Q = 3 for e-1: the sums then read spans >= e+3
+// only, which are complete when the finishing threads have the operands of the
+// pair before, (e+2, e+1).  A cell's bits depend only on its span (the group
+// width), not on which CTA, warp or thread computes it.
+
+// Parents q < n of one sum: OS and OF at o1[q], o2[q], the inside factor at
+// in[q]; extra: the suffix column's part.
+struct SumArgs {
+    const float *o1, *o2, *in;
+    int n;
+    float extra;
 };
+
+__device__ __forceinline__ SumArgs sum_args(const Band& t, int i, int d, int side, bool first, const Rules& R)
+{
+    const int L = t.L, Wb = t.Wb, RS = t.RS, j = i + d;
+    SumArgs a;
+    a.extra = -INFINITY;
+    if (side == 0) {
+        const bool has = j + 1 <= L - 1;
+        a.n = has ? min(i + Wb, L - 1) - j : 0;
+        a.o1 = t.OSrow + (size_t)i * RS + d + 1;
+        a.o2 = t.OFrow + (size_t)i * RS + d + 1;
+        a.in = t.Srow + (size_t)min(j + 1, L - 1) * RS;
+        if (first && has && L - 1 > i + Wb) a.extra = R.r[0] + __ldcg(t.Osuf + i) + t.Ssuf[j + 1];
+    } else {
+        const bool has = i >= 1;
+        a.n = has ? i - max(0, j - Wb) : 0;
+        a.o1 = t.OScol + (size_t)j * RS + d + 1;
+        a.o2 = t.OFcol + (size_t)j * RS + d + 1;
+        a.in = t.Lcol + (size_t)max(i - 1, 0) * RS;
+        // the last column's parents beyond the band, summed before the launch
+        if (first && has && j == L - 1) a.extra = t.OSlast[i];
+    }
+    return a;
+}
 
 // Eight points of one sum that are all in range (two blocks of four points,
 // eight terms each, summed in order): no range checks, and with the group
@@ -1319,42 +1345,20 @@ __device__ __forceinline__ void outside_full8(float& m, float& s, const float* o
     lse_add8(m, s, x1);
 }
 
-template <int Q>
-__device__ __forceinline__ SumPartial outside_sum_t(const Band& t, int i, int d, int side, bool valid, int lane,
-                                                    int G, const Rules& R)
+__device__ __forceinline__ float2 outside_sum(const SumArgs& g, int Q, bool valid, int lane, int G, const Rules& R)
 {
-    const int L = t.L, Wb = t.Wb, RS = t.RS;
-    const int j = i + d;
-    SumPartial c{-INFINITY, 0.f};
-    if (!__any_sync(0xffffffffu, valid)) return c;  // no cell in this warp (warp-uniform)
+    float m = -INFINITY, s = 0.f;
+    if (!__any_sync(0xffffffffu, valid)) return make_float2(m, s);  // no cell in this warp (warp-uniform)
     if (valid) {
-        int n;
-        const float *o1, *o2, *in;
-        float extra = -INFINITY;
-        if (side == 0) {
-            const bool has = j + 1 <= L - 1;
-            n = has ? min(i + Wb, L - 1) - j : 0;
-            o1 = t.OSrow + (size_t)i * RS + d + 1;
-            o2 = t.OFrow + (size_t)i * RS + d + 1;
-            in = t.Srow + (size_t)min(j + 1, L - 1) * RS;
-            if (lane == 0 && has && L - 1 > i + Wb) extra = R.r[0] + __ldcg(t.Osuf + i) + t.Ssuf[j + 1];
-        } else {
-            const bool has = i >= 1;
-            n = has ? i - max(0, j - Wb) : 0;
-            o1 = t.OScol + (size_t)j * RS + d + 1;
-            o2 = t.OFcol + (size_t)j * RS + d + 1;
-            in = t.Lcol + (size_t)max(i - 1, 0) * RS;
-            // the last column's parents beyond the band, summed before the launch
-            if (lane == 0 && has && j == L - 1) extra = t.OSlast[i];
-        }
+        const int n = g.n;
         int q = Q + lane;
         if (G == 32) {  // warp-uniform: one sum per warp, constant strides
-            for (; q + 7 * 32 < n; q += 8 * 32) outside_full8<32>(c.m, c.s, o1, o2, in, q, R);
+            for (; q + 7 * 32 < n; q += 8 * 32) outside_full8<32>(m, s, g.o1, g.o2, g.in, q, R);
             const int rem = (n - q + 31) / 32;  // points left (0..7)
             if (rem > 0) {
-                const float* p1 = o1 + q;
-                const float* p2 = o2 + q;
-                const float* p3 = in + q;
+                const float* p1 = g.o1 + q;
+                const float* p2 = g.o2 + q;
+                const float* p3 = g.in + q;
                 float x0[8], x1[8];
 #pragma unroll
                 for (int u = 0; u < 8; u++) {
@@ -1366,8 +1370,8 @@ __device__ __forceinline__ SumPartial outside_sum_t(const Band& t, int i, int d,
                     x[2 * (u & 3)] = R.r[0] + a + v;
                     x[2 * (u & 3) + 1] = R.r[4] + b + v;
                 }
-                lse_add8(c.m, c.s, x0);
-                lse_add8(c.m, c.s, x1);
+                lse_add8(m, s, x0);
+                lse_add8(m, s, x1);
             }
             q = n;
         }
@@ -1377,167 +1381,51 @@ __device__ __forceinline__ SumPartial outside_sum_t(const Band& t, int i, int d,
             for (int u = 0; u < 8; u++) {
                 const int qq = q + u * G;
                 const bool on = qq < n;
-                const float v = on ? in[qq] : 0.f;
-                const float a = on ? __ldcg(o1 + qq) : -INFINITY;
-                const float b = on ? __ldcg(o2 + qq) : -INFINITY;
+                const float v = ldg_if(g.in + qq, on, 0.f);
+                const float a = ldcg_if(g.o1 + qq, on, -INFINITY);
+                const float b = ldcg_if(g.o2 + qq, on, -INFINITY);
                 float* x = (u < 4) ? x0 : x1;
                 x[2 * (u & 3)] = R.r[0] + a + v;
                 x[2 * (u & 3) + 1] = R.r[4] + b + v;
             }
-            lse_add8(c.m, c.s, x0);
-            lse_add8(c.m, c.s, x1);
+            lse_add8(m, s, x0);
+            lse_add8(m, s, x1);
         }
-        lse_add(c.m, c.s, extra);
+        lse_add(m, s, g.extra);
     }
-    group_reduce_rt(c.m, c.s, G);
-    return c;
+    group_reduce_rt(m, s, G);
+    return make_float2(m, s);
 }
 
-template <int Q>
-__device__ __forceinline__ void outside_finish_t(const Band& t, int i, int d, SumPartial cl, SumPartial cs,
-                                                 const Rules& R)
-{
-    const int L = t.L, Wb = t.Wb, RS = t.RS;
-    const int j = i + d;
-    const bool hasL = j + 1 <= L - 1, hasS = i >= 1;
-    const int nL = hasL ? min(i + Wb, L - 1) - j : 0;
-    const int nS = hasS ? i - max(0, j - Wb) : 0;
-    // every operand first (one round trip), then the sums in ascending q
-    float sib[Q], osl[Q], ofl[Q], lft[Q], oss[Q], ofs[Q];
-    const size_t orow = (size_t)i * RS + d + 1, ocol = (size_t)j * RS + d + 1;
-    const size_t srow = (size_t)min(j + 1, L - 1) * RS, lc = (size_t)max(i - 1, 0) * RS;
-#pragma unroll
-    for (int q = 0; q < Q; q++) {
-        const bool onL = q < nL, onS = q < nS;
-        sib[q] = onL ? t.Srow[srow + q] : 0.f;
-        osl[q] = onL ? __ldcg(t.OSrow + orow + q) : -INFINITY;
-        ofl[q] = onL ? __ldcg(t.OFrow + orow + q) : -INFINITY;
-        lft[q] = onS ? t.Lcol[lc + q] : 0.f;
-        oss[q] = onS ? __ldcg(t.OScol + ocol + q) : -INFINITY;
-        ofs[q] = onS ? __ldcg(t.OFcol + ocol + q) : -INFINITY;
-    }
-    const bool enc = hasS && j <= L - 2 && d + 2 <= Wb;
-    const size_t pr = (size_t)max(i - 1, 0) * RS + d + 2;
-    const float pp = enc ? t.pb[pr] : -INFINITY;
-    const float fa = enc ? __ldcg(t.OSrow + pr) : -INFINITY;
-    const float fb = enc ? __ldcg(t.OFrow + pr) : -INFINITY;
-    const float fc = enc ? __ldcg(t.OLrow + pr) : -INFINITY;
-    float oF = -INFINITY;
-    if (pp != -INFINITY) {
-        float m = -INFINITY, s = 0.f;
-        lse_add4(m, s, R.r[2] + pp + fa, R.r[3] + pp + fb, R.r[6] + pp + fc, -INFINITY);
-        oF = lse_val(m, s);
-    }
-    // the near parents of each sum as one block (one max, independent exponentials)
-    float xl[8], xs[8];
-#pragma unroll
-    for (int q = 0; q < 4; q++) {
-        const bool on = q < Q;
-        const int qq = on ? q : 0;
-        xl[2 * q] = on ? R.r[0] + osl[qq] + sib[qq] : -INFINITY;
-        xl[2 * q + 1] = on ? R.r[4] + ofl[qq] + sib[qq] : -INFINITY;
-        xs[2 * q] = on ? R.r[0] + oss[qq] + lft[qq] : -INFINITY;
-        xs[2 * q + 1] = on ? R.r[4] + ofs[qq] + lft[qq] : -INFINITY;
-    }
-    lse_add8(cl.m, cl.s, xl);
-    lse_add8(cs.m, cs.s, xs);
-    const float oL = lse_val(cl.m, cl.s);
-    float oS = lse_val(cs.m, cs.s);
-    if (i == 0 && j == L - 1) oS = 0.f;
-    t.OSrow[(size_t)i * RS + d] = oS;
-    t.OScol[(size_t)j * RS + d] = oS;
-    t.OFrow[(size_t)i * RS + d] = oF;
-    t.OFcol[(size_t)j * RS + d] = oF;
-    t.OLrow[(size_t)i * RS + d] = oL;
-    if (j == L - 1) t.Osuf[i] = oS;
-}
-
-// The sums of one diagonal's rows [start, start + nrows) before the wait:
-// task tau = 2r + side (row r, one of its two sums) goes to lane group
-// (first + tau) mod (groups per CTA), two tasks per group, each group's
-// result to slot[tau].  The second diagonal of a pair starts on the groups
-// the first one leaves idle.
-template <int Q>
-__device__ __forceinline__ void out_sums_partial(const Band& t, int d, int start, int nrows, int first,
-                                                 float2* slot, const Rules& R)
-{
-    const int G = group_width(2 * (t.Wb - d) + 2), gpb = blockDim.x / G;
-    const int lane = threadIdx.x & (G - 1), g = (threadIdx.x / G + gpb - first % gpb) % gpb;
-    const int ntask = 2 * min(nrows, gpb);
-#pragma unroll
-    for (int it = 0; it < 2; it++) {
-        const int tau = g + it * gpb;
-        const bool valid = tau < ntask;
-        const SumPartial c = outside_sum_t<Q>(t, start + (tau >> 1), d, tau & 1, valid, lane, G, R);
-        if (valid && lane == 0) slot[tau] = make_float2(c.m, c.s);
-    }
-}
-
-// After the wait: one thread per row finishes the rows whose sums are in the
-// slots; rows beyond the groups of the CTA are computed whole, both sums by
-// one group and the cell finished by its lane 0.
-template <int Q>
-__device__ __forceinline__ void out_sums_finish(const Band& t, int d, int start, int nrows, const float2* slot,
-                                                const Rules& R)
-{
-    const int G = group_width(2 * (t.Wb - d) + 2), gpb = blockDim.x / G;
-    const int np = min(nrows, gpb);
-    for (int r = threadIdx.x; r < np; r += blockDim.x) {
-        const float2 a = slot[2 * r], b = slot[2 * r + 1];
-        outside_finish_t<Q>(t, start + r, d, SumPartial{a.x, a.y}, SumPartial{b.x, b.y}, R);
-    }
-    const int lane = threadIdx.x & (G - 1), g = threadIdx.x / G;
-    for (int base = np; base < nrows; base += gpb) {
-        const int r = base + g;
-        const bool valid = r < nrows;
-        const SumPartial cl = outside_sum_t<Q>(t, start + r, d, 0, valid, lane, G, R);
-        const SumPartial cs = outside_sum_t<Q>(t, start + r, d, 1, valid, lane, G, R);
-        if (valid && lane == 0) outside_finish_t<Q>(t, start + r, d, cl, cs, R);
-    }
-}
-
-// The finishing parts of a diagonal pair with a thread per near sum and per F
-// value instead of one per cell: warps 0 and 2 of the CTA take the two sums of
-// every row of diagonals e and e-1, warps 1 and 3 their F values.  Every
-// operand of both diagonals is loaded before the first one is finished; what
-// e-1 needs of e (the first near parent of each sum, the CTA's own cells)
-// comes through shared memory.  The same operations on the same values as
-// outside_finish_t.
-constexpr int kFinishWarps = 4;
-constexpr int kFinishRows = 16;  // rows of a diagonal that two lanes each of one warp hold
-__device__ __forceinline__ void finish_barrier() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
-
+// Parents 0 .. Q-1 of one sum.
 template <int Q>
 struct NearSum {
     float a[Q], b[Q], v[Q];
+    __device__ __forceinline__ bool complete() const
+    {
+        bool ok = true;
+#pragma unroll
+        for (int q = 0; q < Q; q++) ok = ok && !unwritten(a[q]) && !unwritten(b[q]);
+        return ok;
+    }
 };
 
+// Q = 3 (diagonal e-1): parent 0, on diagonal e, comes from shared memory.
 template <int Q>
-__device__ __forceinline__ NearSum<Q> near_load(const Band& t, int i, int d, int side, bool valid, bool defer)
+__device__ __forceinline__ void near_load(const SumArgs& g, NearSum<Q>& s)
 {
-    const int L = t.L, Wb = t.Wb, RS = t.RS, j = i + d;
-    int n = 0;
-    const float *o1 = t.OSrow, *o2 = t.OFrow, *in = t.Srow;
-    if (valid && side == 0) {
-        n = (j + 1 <= L - 1) ? min(i + Wb, L - 1) - j : 0;
-        o1 = t.OSrow + (size_t)i * RS + d + 1;
-        o2 = t.OFrow + (size_t)i * RS + d + 1;
-        in = t.Srow + (size_t)min(j + 1, L - 1) * RS;
-    } else if (valid) {
-        n = (i >= 1) ? i - max(0, j - Wb) : 0;
-        o1 = t.OScol + (size_t)j * RS + d + 1;
-        o2 = t.OFcol + (size_t)j * RS + d + 1;
-        in = t.Lcol + (size_t)max(i - 1, 0) * RS;
-    }
-    NearSum<Q> s;
 #pragma unroll
     for (int q = 0; q < Q; q++) {
-        const bool on = q < n, now = on && !(defer && q == 0);  // defer: parent 0 comes from near_patch
-        s.v[q] = ldg_if(in + q, on, 0.f);
-        s.a[q] = ldcg_if(o1 + q, now, -INFINITY);
-        s.b[q] = ldcg_if(o2 + q, now, -INFINITY);
+        s.v[q] = 0.f;
+        s.a[q] = s.b[q] = -INFINITY;
+        if (q < g.n) {
+            s.v[q] = __ldg(g.in + q);
+            if (Q == 2 || q > 0) {
+                s.a[q] = ld_cell(g.o1 + q);
+                s.b[q] = ld_cell(g.o2 + q);
+            }
+        }
     }
-    return s;
 }
 
 template <int Q>
@@ -1557,15 +1445,15 @@ __device__ __forceinline__ float near_finish(const NearSum<Q>& s, float2 c, cons
 
 struct FOperands {
     float pp, a, b, c;
+    __device__ __forceinline__ bool complete() const { return !unwritten(a) && !unwritten(b) && !unwritten(c); }
 };
 
-__device__ __forceinline__ FOperands f_load(const Band& t, int i, int d, bool valid)
+__device__ __forceinline__ void f_load(const Band& t, int i, int d, FOperands& f)
 {
-    const int j = i + d;
-    const bool enc = valid && i >= 1 && j <= t.L - 2 && d + 2 <= t.Wb;
-    const size_t pr = enc ? (size_t)(i - 1) * t.RS + d + 2 : 0;
-    return FOperands{ldg_if(t.pb + pr, enc, -INFINITY), ldcg_if(t.OSrow + pr, enc, -INFINITY),
-                     ldcg_if(t.OFrow + pr, enc, -INFINITY), ldcg_if(t.OLrow + pr, enc, -INFINITY)};
+    f = FOperands{-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+    if (i < 1 || i + d > t.L - 2 || d + 2 > t.Wb) return;
+    const size_t pr = (size_t)(i - 1) * t.RS + d + 2;
+    f = FOperands{__ldg(t.pb + pr), ld_cell(t.OSrow + pr), ld_cell(t.OFrow + pr), ld_cell(t.OLrow + pr)};
 }
 
 __device__ __forceinline__ float f_finish(const FOperands& f, const Rules& R)
@@ -1581,66 +1469,20 @@ __device__ __forceinline__ float sum_write(const Band& t, int i, int d, int side
 {
     const int j = i + d;
     if (side == 0) {
-        t.OLrow[(size_t)i * t.RS + d] = v;
+        st_cell(t.OLrow + (size_t)i * t.RS + d, v);
         return v;
     }
     if (i == 0 && j == t.L - 1) v = 0.f;
-    t.OSrow[(size_t)i * t.RS + d] = v;
-    t.OScol[(size_t)j * t.RS + d] = v;
+    st_cell(t.OSrow + (size_t)i * t.RS + d, v);
+    st_cell(t.OScol + (size_t)j * t.RS + d, v);
     if (j == t.L - 1) t.Osuf[i] = v;
     return v;
 }
 
 __device__ __forceinline__ void f_write(const Band& t, int i, int d, float v)
 {
-    t.OFrow[(size_t)i * t.RS + d] = v;
-    t.OFcol[(size_t)(i + d) * t.RS + d] = v;
-}
-
-// Rows [sA, sA + nA) of diagonal eA and [r0, r0 + nB) of eB = eA - 1 (nB = 0:
-// none), at most kFinishRows each, by warps 0 .. 3; the others do not come
-// here.  oS, oF: [nA] of shared memory.  Ends with a barrier of the four warps.
-__device__ void out_pair_finish(const Band& t, int eA, int sA, int nA, int r0, int nB, const float2* slotA,
-                                const float2* slotB, float* oS, float* oF, const Rules& R)
-{
-    const int part = (int)threadIdx.x >> 5, x = (int)threadIdx.x & 31;
-    const int row = (part & 1) ? x : x >> 1, side = x & 1, eB = eA - 1;
-    if (part == 0) {
-        const bool valid = row < nA;
-        const NearSum<2> s = near_load<2>(t, sA + row, eA, side, valid, false);
-        if (valid) {
-            const float v = sum_write(t, sA + row, eA, side, near_finish<2>(s, slotA[x], R));
-            if (side == 1) oS[row] = v;
-        }
-        finish_barrier();
-    } else if (part == 1) {
-        const FOperands f = f_load(t, sA + row, eA, row < nA);
-        if (row < nA) {
-            const float v = f_finish(f, R);
-            f_write(t, sA + row, eA, v);
-            oF[row] = v;
-        }
-        finish_barrier();
-    } else if (part == 2) {
-        const bool valid = row < nB;
-        NearSum<3> s = near_load<3>(t, r0 + row, eB, side, valid, true);
-        finish_barrier();  // diagonal e of the CTA's rows in oS / oF
-        if (valid) {
-            // parent 0 is (i, j+1) for side 0 and (i-1, j) for side 1, on diagonal e
-            const int i = r0 + row, p = i - side - sA;
-            const bool on = side == 0 ? i + eB + 1 <= t.L - 1 : i >= 1;
-            if (on) {
-                s.a[0] = oS[p];
-                s.b[0] = oF[p];
-            }
-            sum_write(t, i, eB, side, near_finish<3>(s, slotB[x], R));
-        }
-    } else {
-        const FOperands f = f_load(t, r0 + row, eB, row < nB);
-        finish_barrier();
-        if (row < nB) f_write(t, r0 + row, eB, f_finish(f, R));
-    }
-    finish_barrier();
+    st_cell(t.OFrow + (size_t)i * t.RS + d, v);
+    st_cell(t.OFcol + (size_t)(i + d) * t.RS + d, v);
 }
 
 // Suffix-column terms of the outside S sums of the last column's band cells:
@@ -1649,7 +1491,7 @@ __device__ void out_pair_finish(const Band& t, int eA, int sA, int nA, int r0, i
 // suffix column and the inside tables, so one launch before the wavefront
 // sums them for every row, a warp per row: inside the wavefront the cell of
 // diagonal d has d+1 of them, summed by the single lane group of a long
-// diagonal while every other CTA waited at the next barrier.
+// diagonal while every other CTA waited.
 __global__ void outside_lastcol_kernel(Band t, Rules R)
 {
     const int L = t.L, Wb = t.Wb, RS = t.RS;
@@ -1672,101 +1514,180 @@ __global__ void outside_lastcol_kernel(Band t, Rules R)
     if (lane == 0) t.OSlast[i] = lse_val(m, s);
 }
 
-// All band diagonals of the outside pass, descending spans, two per grid
-// barrier.  For the pair (e, e-1) CTA b owns rows [b*R, (b+1)*R), R = ceil(rows
-// of e-1 / CTAs): it computes diagonal e for its rows plus row b*R - 1 (which
-// the previous CTA also computes, to the same bits) and then diagonal e-1,
-// whose cells read diagonal e only at rows i and i-1.  The sums of a pair read
-// spans >= e+3, which the wait for the pair before (e+2, e+1) has made complete
-// for every row: where four warps hold a pair's finishing parts
-// (out_pair_finish) they finish the pair before and arrive for the CTA while
-// the other warps are already at this pair's sums, so a pair costs the longer
-// of the two, not their sum; otherwise (many rows per CTA) a thread per cell
-// finishes diagonal after diagonal and the sums follow the arrival.
-// Span 500 over 1,000 columns: 1.86 ms with rows owned for the whole pass and a
-// thread per cell finishing each diagonal in turn, 1.52 with out_pair_finish
-// alone, 1.41 now.
-__global__ void __launch_bounds__(kWaveMaxThreads) outside_wave_kernel(Band t, Rules R)
+constexpr int kOutsideFinish = 128;   // threads that finish a pair: two warps per diagonal
+constexpr int kOutsideRows = 256;     // rows of a diagonal that a CTA takes at a time
+
+// All band diagonals of the outside pass, descending spans, in pairs (e, e-1).
+// The rows of a pair are dealt evenly over the CTAs, pair by pair: a CTA owns
+// rows [r0, r0 + nb) of diagonal e-1 and finishes diagonal e for rows r0 - 1 ..
+// r0 + nb - 1 (row r0 - 1 is computed by the previous CTA too, to the same
+// bits): a cell of e-1 reads diagonal e only at rows i and i-1.
+// As in the inside pass, the CTAs wait for one another's cells (the five tables
+// are filled with kUnwritten before the launch) and four warps finish a pair
+// while the others form the sums of the next one.  Of the four, warps 0 and 2
+// take the two near sums of the rows of e and e-1, two lanes a row, warps 1 and
+// 3 their F values; what e-1 needs of e comes through shared memory.
+// Against one grid barrier per pair: span 500 over 1,000 columns 1.41 -> 1.07 ms,
+// 300 over 600 0.81 -> 0.44, every span of 300 611 -> 308 us, span 500 over
+// 3,000 columns 4.51 -> 2.29 ms.  Bound by the sums (24 loads and 16
+// exponentials of a lane per L2 round trip); with few rows by the chain write
+// -> look -> cells of e -> cells of e-1, as the inside pass.
+template <int MAXT>
+__global__ void __launch_bounds__(MAXT) outside_pair_kernel(Band t, Rules R, unsigned int* sync)
 {
-    __shared__ float2 slotA[2 * kWaveMaxThreads], slotB[2 * kWaveMaxThreads];
-    // paired form: the sums of the pair being finished and of the next one
-    __shared__ float2 pairA[2][2 * kFinishRows], pairB[2][2 * kFinishRows];
-    __shared__ float oS[kFinishRows], oF[kFinishRows];
-    unsigned int gen = 0;
+    __shared__ float2 part[2][2][2 * (kOutsideRows + 1)];  // [pair parity][diagonal][2 row + side]
+    __shared__ float oS[kOutsideRows + 1], oF[kOutsideRows + 1];
+    const int tid = threadIdx.x, nwork = (int)blockDim.x - kOutsideFinish;
+    const bool fin = tid < kOutsideFinish;
     const int L = t.L, Wb = t.Wb, grid = (int)gridDim.x;
-    int rows = (L - max(Wb - 1, 0) + grid - 1) / grid;
-    grid_arrive(t.sync);  // the suffix column was written by the previous launch
+    bool bad = false;      // a wait of this thread took too long
+    bool own_nan = false;  // this warp has met a NaN that was no unwritten cell
+    int rows = 1;
     struct Pair {
-        int e, sA, nA, r0, nB;
-        bool paired;  // one warp holds a diagonal's rows and every sum has a group (the same in every CTA)
+        int r0, na, nb;  // rows r0 - 1 .. of diagonal e (row -1 is none), r0 .. of diagonal e - 1
     };
     auto pair_at = [&](int e) {  // e descending: the rows grow
+        const int most = L - max(e - 1, 0);
+        rows = max(rows, (most + grid - 1) / grid);
         Pair p;
-        p.e = e;
-        while (rows * grid < L - max(e - 1, 0)) rows++;
         p.r0 = blockIdx.x * rows;
-        p.sA = max(p.r0 - 1, 0);
-        p.nA = max(min(p.r0 + rows, L - e) - p.sA, 0);
-        p.nB = (e >= 1) ? max(min(p.r0 + rows, L - e + 1) - p.r0, 0) : 0;
-        p.paired = rows + 1 <= kFinishRows && rows + 1 <= (int)blockDim.x / group_width(2 * (Wb - max(e - 1, 0)) + 2) &&
-                   blockDim.x > 32 * kFinishWarps;
+        const int nr = max(min(rows, most - p.r0), 0);
+        p.na = nr > 0 ? min(p.r0 + rows, L - e) - (p.r0 - 1) : 0;
+        p.nb = e >= 1 ? nr : 0;
         return p;
     };
-    auto sums = [&](const Pair& p, int buf) {
-        // tasks start behind the finishing warps, which take what is left over
-        const int first = kFinishWarps * (32 / group_width(2 * (Wb - p.e) + 2));
-        out_sums_partial<2>(t, p.e, p.sA, p.nA, first, p.paired ? pairA[buf] : slotA, R);
-        if (p.e >= 1) {
-            const int firstB = kFinishWarps * (32 / group_width(2 * (Wb - p.e + 1) + 2));
-            out_sums_partial<3>(t, p.e - 1, p.r0, p.nB, firstB + 2 * p.nA, p.paired ? pairB[buf] : slotB,
-                                R);
+
+    // the sums of rows [c0, c0 + kOutsideRows) of the pair (e, e-1), by the other warps
+    auto sums = [&](const Pair& p, int e, int c0, int buf) {
+        const int na = min(kOutsideRows + 1, p.na - c0), nb = max(min(kOutsideRows, p.nb - c0), 0);
+        const int wt = tid - kOutsideFinish;
+        const int G = group_width(2 * (Wb - e) + 2);  // of both: the limits are multiples of four
+        const int gpb = nwork / G, lane = wt & (G - 1);
+        for (int base = 0; base < 2 * (na + nb); base += gpb) {
+            const int w = base + wt / G;
+            const int x = w >= 2 * na ? 1 : 0, tau = x ? w - 2 * na : w, d = e - x;
+            const int i = p.r0 - 1 + x + c0 + (tau >> 1);
+            const bool valid = w < 2 * (na + nb) && i >= 0;
+            SumArgs g{nullptr, nullptr, nullptr, 0, -INFINITY};
+            if (valid) g = sum_args(t, i, d, tau & 1, lane == 0, R);
+            unsigned int spins = 0;
+            float2 c;
+            for (bool there = false;;) {
+                c = outside_sum(g, 2 + x, valid, lane, G, R);
+                if (there || !__any_sync(0xffffffffu, valid && c.y != c.y)) break;
+                // a NaN: again, as in the inside pass
+                bad = __any_sync(0xffffffffu, !keep_waiting(spins, sync)) || bad;
+                if (bad) break;
+                if (own_nan || (spins & 63u) == 0u) {
+                    bool missing = false;
+                    for (int q = 2 + x + lane; q < g.n; q += G)
+                        missing = missing || unwritten(ld_cell(g.o1 + q)) || unwritten(ld_cell(g.o2 + q));
+                    there = !__any_sync(0xffffffffu, missing);
+                    own_nan = own_nan || there;
+                }
+                asm volatile("" : "+l"(g.o1), "+l"(g.o2)::"memory");  // not the cells read before
+            }
+            if (valid && lane == 0) part[buf][x][tau] = c;
         }
     };
-    Pair p = pair_at(Wb);
-    int buf = 0;
-    sums(p, buf);
-    for (;;) {
-        if (!grid_wait(t.sync, gen)) return;  // ends with a CTA barrier: the slots of p are complete
-        const int next = p.e - 2;
-        if (p.paired) {
-            if (threadIdx.x < 32 * kFinishWarps) {
-                out_pair_finish(t, p.e, p.sA, p.nA, p.r0, p.nB, pairA[buf], pairB[buf], oS, oF, R);
-                if (threadIdx.x == 0) {
-                    __threadfence();
-                    atomicAdd(&t.sync[0], 1u);
+
+    auto fin_barrier = [] { asm volatile("bar.sync 1, %0;" ::"n"(kOutsideFinish) : "memory"); };
+    // until the warp's operands are there
+    auto await = [&](bool mine, auto load, auto complete) {
+        for (unsigned int spins = 0;;) {
+            if (mine) load();
+            mine = mine && !complete();
+            if (!__any_sync(0xffffffffu, mine)) return;
+            if (!keep_waiting(spins, sync)) {
+                bad = true;
+                return;
+            }
+        }
+    };
+    // The near sums (a lane per side) or F values of diagonal d = e - Q + 2 for
+    // its rows [c0, c0 + kOutsideRows); `ready`: what to do between the first
+    // rows' operands and the rest.
+    auto finish_sums = [&](auto parents, const Pair& p, int e, int c0, int buf, auto ready) {
+        constexpr int Q = decltype(parents)::value;
+        const int x = Q - 2, d = e - x, n = x ? min(kOutsideRows, p.nb - c0) : min(kOutsideRows + 1, p.na - c0);
+        const int side = tid & 1;
+        for (int base = 0; base < n || base == 0; base += 16) {
+            const int r = base + ((tid & 31) >> 1), i = p.r0 - 1 + x + c0 + r;
+            const bool mine = r < n && i >= 0;
+            SumArgs g{nullptr, nullptr, nullptr, 0, -INFINITY};
+            if (mine) g = sum_args(t, i, d, side, false, R);
+            NearSum<Q> s;
+            await(mine, [&] { near_load<Q>(g, s); }, [&] { return s.complete(); });
+            if (base == 0) ready();
+            if (!mine) continue;
+            if constexpr (Q == 3) {
+                if (g.n > 0) {  // parent 0: (i, j+1) for side 0 and (i-1, j) for side 1
+                    s.a[0] = oS[r + 1 - side];
+                    s.b[0] = oF[r + 1 - side];
                 }
             }
-        } else {
-            out_sums_finish<2>(t, p.e, p.sA, p.nA, slotA, R);
-            if (p.e >= 1) {
-                __syncthreads();  // diagonal e of this CTA's rows before e-1 reads it
-                out_sums_finish<3>(t, p.e - 1, p.r0, p.nB, slotB, R);
-            }
-            grid_arrive(t.sync);
+            const float v = sum_write(t, i, d, side, near_finish<Q>(s, part[buf][x][2 * r + side], R));
+            if (Q == 2 && side == 1) oS[r] = v;
         }
-        if (next < 0) break;
-        p = pair_at(next);
-        buf ^= 1;
-        sums(p, buf);
+    };
+    auto finish_f = [&](int x, const Pair& p, int e, int c0, auto ready) {
+        const int d = e - x, n = x ? min(kOutsideRows, p.nb - c0) : min(kOutsideRows + 1, p.na - c0);
+        for (int base = 0; base < n || base == 0; base += 32) {
+            const int r = base + (tid & 31), i = p.r0 - 1 + x + c0 + r;
+            const bool mine = r < n && i >= 0;
+            FOperands f;
+            await(mine, [&] { f_load(t, i, d, f); }, [&] { return f.complete(); });
+            if (base == 0) ready();
+            if (!mine) continue;
+            const float v = f_finish(f, R);
+            f_write(t, i, d, v);
+            if (x == 0) oF[r] = v;
+        }
+    };
+    // Diagonal e by warps 0 and 1, then (behind a barrier of the four) e-1 by 2 and 3.
+    auto finish = [&](const Pair& p, int e, int c0, int buf, auto ready) {
+        const int warp = tid >> 5;
+        const auto both = [&] {
+            ready();
+            fin_barrier();  // diagonal e of this CTA's rows is in oS / oF
+        };
+        if (warp == 0) finish_sums(std::integral_constant<int, 2>{}, p, e, c0, buf, ready);
+        else if (warp == 1) finish_f(0, p, e, c0, ready);
+        else if (warp == 2) finish_sums(std::integral_constant<int, 3>{}, p, e, c0, buf, both);
+        else finish_f(1, p, e, c0, both);
+        if (warp < 2) fin_barrier();
+    };
+
+    int buf = 0;
+    Pair p = pair_at(Wb);
+    if (!fin) sums(p, Wb, 0, 0);
+    for (int e = Wb; e >= 0; e -= 2, buf ^= 1) {
+        bool stop = false;
+        // every thread: the pair's sums are there, and its operands
+        auto together = [&] { stop = __syncthreads_or(bad) != 0; };
+        const Pair next = e >= 2 ? pair_at(e - 2) : Pair{0, 0, 0};
+        if (fin) {
+            finish(p, e, 0, buf, together);
+        } else {
+            together();
+            if (!stop && e >= 2) sums(next, e - 2, 0, buf ^ 1);
+        }
+        // more rows than a CTA holds: the rest apart
+        for (int c0 = kOutsideRows; c0 < max(p.na - 1, p.nb); c0 += kOutsideRows) {
+            __syncthreads();
+            if (!fin) sums(p, e, c0, buf);
+            __syncthreads();
+            if (fin) finish(p, e, c0, buf, [] {});
+        }
+        if (stop) return;
+        p = next;
     }
 }
 
-// CTA size of a persistent wavefront launch.  The split sums are bound by
-// the latency of their L2 loads: long bands need many warps per SM to keep
-// enough loads in flight, short ones pay more for the larger CTA barrier
-// than they gain (GB300: 256 threads best at L x W = 0.5e6, 1024 at 7e6).
-int wave_threads(const messi_ctx* ctx, double cells)
+// CTAs of a cooperative launch: one per SM at most (more would share the SM's
+// loads and lengthen every wait), fewer where the context caps them.
+static int wave_grid(messi_ctx* ctx)
 {
-    const int t = ctx->wave_threads;
-    if (t == 256 || t == 512 || t == 1024) return t;
-    return cells < 1.5e6 ? 256 : (cells < 4e6 ? 512 : kWaveMaxThreads);
-}
-
-int wave_grid(messi_ctx* ctx, const void* kernel, int L, int threads)
-{
-    int per_sm = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, 0) != cudaSuccess || per_sm < 1)
-        per_sm = 1;
     int sms = ctx->num_sms;
     if (sms <= 0) {
         int dev = 0;
@@ -1774,69 +1695,7 @@ int wave_grid(messi_ctx* ctx, const void* kernel, int L, int threads)
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
         ctx->num_sms = sms;
     }
-    // one CTA per SM at most keeps the barrier cheap; a context may cap it lower
-    const int useful = (int)std::min<long long>((long long)L * 32 / threads + 1, (long long)per_sm * sms);
-    int grid = std::max(1, std::min(useful, sms));
-    if (ctx->wave_ctas > 0) grid = std::min(grid, ctx->wave_ctas);
-    return grid;
-}
-
-// CTAs for which a CTA's ceil(L / CTAs) rows plus one fit one per warp in
-// `warps` warps.
-static int ctas_for_rows(int L, int warps) { return (warps > 1) ? (L + warps - 2) / (warps - 1) : L; }
-
-// Launch a persistent wavefront kernel (cooperative: every CTA resident).
-// share > 0 (paired kernels): the CTA owns ceil(L / grid) rows of every
-// diagonal plus one, and a row wants `share` warps per diagonal pair (the
-// outside pass: one per parent sum of each diagonal, 4).  The CTA grows (up to 1,024 threads, unless its size is
-// set) to the smallest size at which warps / share of its warps hold those
-// rows one per warp with at most one CTA per SM; the grid then grows (up to
-// one CTA per SM) until the rows fit, or else fit one per warp of the whole
-// CTA.
-int launch_wave(messi_ctx* ctx, const void* kernel, void** args, unsigned int* sync, int L, double band_cells,
-                const char* what, int share)
-{
-    int threads = wave_threads(ctx, band_cells);
-    cudaError_t e = cudaMemsetAsync(sync, 0, kSyncWords * sizeof(unsigned int), ctx->stream);
-    if (e != cudaSuccess) return cuda_fail(ctx, e, "barrier reset");
-    int grid = wave_grid(ctx, kernel, L, threads);  // also sets ctx->num_sms
-    if (share > 0 && ctx->wave_ctas <= 0) {
-        for (int t2 = threads; t2 <= (ctx->wave_threads ? threads : kWaveMaxThreads); t2 *= 2)
-            if (ctas_for_rows(L, t2 / 32 / share) <= ctx->num_sms) {
-                if (t2 != threads) {
-                    threads = t2;
-                    grid = wave_grid(ctx, kernel, L, threads);
-                }
-                break;
-            }
-        const int warps = threads / 32;
-        const int half = ctas_for_rows(L, warps / share);
-        const int want = (half <= ctx->num_sms) ? half : ctas_for_rows(L, warps);
-        grid = std::max(grid, std::min(want, ctx->num_sms));
-    }
-    e = cudaLaunchCooperativeKernel(kernel, dim3(grid), dim3(threads), args, 0, ctx->stream);
-    ctx->launches++;
-    if (e != cudaSuccess) return cuda_fail(ctx, e, what);
-    return MESSI_OK;
-}
-
-// Self-test of the bounded grid barrier: CTA 1 never arrives, so CTA 0's wait
-// gives up after `limit` polls, raises the error flag (sync[2]) and returns.
-// Nothing faults and nothing waits unboundedly; the context stays usable.
-__global__ void barrier_selftest_kernel(unsigned int* sync, unsigned int limit)
-{
-    if (blockIdx.x != 0) return;
-    unsigned int gen = 0;
-    grid_sync(sync, gen, limit);
-}
-
-int launch_barrier_selftest(messi_ctx* ctx, unsigned int* d_sync)
-{
-    cudaError_t e = cudaMemsetAsync(d_sync, 0, kSyncWords * sizeof(unsigned int), ctx->stream);
-    if (e != cudaSuccess) return cuda_fail(ctx, e, "barrier self-test reset");
-    barrier_selftest_kernel<<<2, 32, 0, ctx->stream>>>(d_sync, 1u << 12);
-    LAUNCH_CHECK(ctx, "barrier_selftest_kernel");
-    return MESSI_OK;
+    return ctx->wave_ctas > 0 ? std::min(sms, ctx->wave_ctas) : std::max(sms, 1);
 }
 
 // The inside kernel (cooperative: every CTA resident), one CTA per SM, after
@@ -1857,7 +1716,7 @@ static int launch_inside(messi_ctx* ctx, const void* kernel, const void* many, v
     for (int k = 0; k < 3 && e == cudaSuccess; k++)
         if (cells[k].second) e = cudaMemsetAsync(cells[k].first, 0xff, cells[k].second * sizeof(float), ctx->stream);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "inside table reset");
-    const int most = wave_grid(ctx, kernel, INT_MAX / 32, kInsideThreads);  // also sets ctx->num_sms
+    const int most = wave_grid(ctx);  // also sets ctx->num_sms
     const int grid = (int)std::min<long long>(most, columns);
     int threads = columns <= 2 * (long long)ctx->num_sms ? kInsideThreads / 2 : kInsideThreads;
     if (ctx->wave_threads == 256 || ctx->wave_threads >= kInsideThreads)
@@ -1871,12 +1730,56 @@ static int launch_inside(messi_ctx* ctx, const void* kernel, const void* many, v
     return e == cudaSuccess ? MESSI_OK : cuda_fail(ctx, e, "inside_pair_kernel");
 }
 
+// Self-test of the bounded wait: one thread waits for a cell (sync[3]) that
+// nothing writes, gives up after `limit` looks, raises the error flag (sync[2])
+// and returns.  Nothing faults and nothing waits unboundedly; the context stays
+// usable.
+__global__ void wait_selftest_kernel(unsigned int* sync, unsigned int limit)
+{
+    unsigned int spins = 0;
+    while (unwritten(ld_cell(reinterpret_cast<const float*>(sync + 3))))
+        if (!keep_waiting(spins, sync, limit)) return;
+}
+
+int launch_wait_selftest(messi_ctx* ctx, unsigned int* d_sync)
+{
+    cudaError_t e = cudaMemsetAsync(d_sync, 0, kSyncWords * sizeof(unsigned int), ctx->stream);
+    if (e == cudaSuccess) e = cudaMemsetAsync(d_sync + 3, 0xff, sizeof(unsigned int), ctx->stream);
+    if (e != cudaSuccess) return cuda_fail(ctx, e, "wait self-test reset");
+    wait_selftest_kernel<<<1, 1, 0, ctx->stream>>>(d_sync, 1u << 12);
+    LAUNCH_CHECK(ctx, "wait_selftest_kernel");
+    return MESSI_OK;
+}
+
 int queue_status_readback(messi_ctx* ctx, const Band& t)
 {
     if (!ctx->status_host) return MESSI_OK;
     cudaError_t e = cudaMemcpyAsync(ctx->status_host, t.sync + 2, sizeof(unsigned int), cudaMemcpyDeviceToHost,
                                     ctx->stream);
     return (e == cudaSuccess) ? MESSI_OK : cuda_fail(ctx, e, "status readback");
+}
+
+// The outside kernel (cooperative), one CTA per SM, after its tables are filled
+// with kUnwritten.  More rows per CTA want more warps for their sums, although
+// fewer registers a thread then spill: 512, 768, 1,024 threads took 308, 366, 433
+// us with 2 rows (every span of 300 columns), 522, 439, 492 with 4 (span 300 of
+// 600) and 1,217, 1,175, 1,065 with 7 (span 500 of 1,000).
+static int launch_outside(messi_ctx* ctx, const Band& t, void** args, unsigned int* sync)
+{
+    cudaError_t e = cudaMemsetAsync(sync, 0, kSyncWords * sizeof(unsigned int), ctx->stream);
+    const size_t tab = (size_t)t.L * t.RS * sizeof(float);
+    for (float* cells : {t.OSrow, t.OScol, t.OFrow, t.OFcol, t.OLrow})
+        if (e == cudaSuccess) e = cudaMemsetAsync(cells, 0xff, tab, ctx->stream);
+    if (e != cudaSuccess) return cuda_fail(ctx, e, "outside table reset");
+    const void* kernel = (const void*)outside_pair_kernel<1024>;
+    const int grid = std::min(wave_grid(ctx), t.L);
+    const int rows = (t.L + grid - 1) / grid;
+    int threads = ctx->wave_threads ? ctx->wave_threads : (rows <= 2 ? 512 : (rows <= 5 ? 768 : 1024));
+    if (threads <= 512) kernel = (const void*)outside_pair_kernel<512>;
+    else if (threads == 768) kernel = (const void*)outside_pair_kernel<768>;
+    e = cudaLaunchCooperativeKernel(kernel, dim3(grid), dim3(threads), args, 0, ctx->stream);
+    ctx->launches++;
+    return e == cudaSuccess ? MESSI_OK : cuda_fail(ctx, e, "outside_pair_kernel");
 }
 
 int run_inside(messi_ctx* ctx, const Band& t, double B)
@@ -2260,12 +2163,10 @@ int run_outside(messi_ctx* ctx, const Band& t, double B)
         }
     }
     Band tt = t;
-    void* args[] = {&tt, &R};
+    unsigned int* sync = t.sync;
+    void* args[] = {&tt, &R, &sync};
     prof_begin(ctx, 3, (double)t.L * (t.Wb + 1) - 0.5 * t.Wb * (t.Wb + 1.0));
-    // paired: the two sums of each cell of a CTA's diagonal pair (2 x (2 x
-    // rows + 1) sums) in one pass of its warps where the CTA can grow to hold them
-    int rc = launch_wave(ctx, (const void*)outside_wave_kernel, args, t.sync, t.L, (double)t.L * (t.Wb + 1),
-                         "outside_wave_kernel", 4);
+    int rc = launch_outside(ctx, tt, args, sync);
     if (rc) return rc;
     prof_end(ctx);
     return queue_status_readback(ctx, t);
