@@ -628,10 +628,12 @@ int messi_dataset_destroy(messi_dataset* ds)
         }
         tune_forget(ctx, ds);
     }
-    void* bufs[] = {ds->d_bandidx, ds->d_idx, ds->d_leaf, ds->d_segs, ds->d_steps, ds->d_tiles, ds->d_masks, ds->d_tree,
-                    ds->d_uops, ds->d_arena_f, ds->d_arena_e, ds->d_mix, ds->d_mixlam};
-    for (void* b : bufs)
-        if (b) cudaFree(b);
+    void* plan[] = {ds->d_bandidx, ds->d_idx, ds->d_leaf, ds->d_segs, ds->d_steps, ds->d_tiles,
+                    ds->d_masks, ds->d_tree, ds->d_uops, ds->d_mix, ds->d_mixlam};
+    for (void* b : plan)
+        if (b && !ds->lent_plan) cudaFree(b);
+    for (void* b : {(void*)ds->d_arena_f, (void*)ds->d_arena_e})
+        if (b && !ds->lent_arena) cudaFree(b);
     delete ds;
     return MESSI_OK;
 }
@@ -1006,6 +1008,16 @@ int messi_structure_likelihood(messi_ctx* ctx, messi_dataset* ds, const messi_mo
             pairs.push_back(make_int2(i, k - 1));
         }
     }
+    // the model and the unpaired columns first: the device has them to do while the host plans
+    ModelDev md;
+    if ((rc = upload_model(ctx, ds, model, !pairs.empty(), true, nullptr, &md, true))) return rc;
+    void* dv;
+    if ((rc = ensure(ctx, kSlotVec, (2 * (size_t)L + 8) * sizeof(double), &dv))) return rc;
+    double* d_u = (double*)dv;
+    double* d_pairll = d_u + L;
+    double* d_total = d_pairll + L;
+    if ((rc = launch_unpaired(ctx, ds, md.P4, ds->numnodes, md.pi4, md.logw_site, md.cat.nsite, d_u, nullptr)))
+        return rc;
     // plan of exactly the structure's pairs (subtree-pattern dedup as for the band)
     messi_dataset* sub = nullptr;
     std::vector<int32_t> pu;
@@ -1013,6 +1025,7 @@ int messi_structure_likelihood(messi_ctx* ctx, messi_dataset* ds, const messi_mo
         sub = new (std::nothrow) messi_dataset();
         if (!sub) return fail(ctx, MESSI_ENOMEM, "structure likelihood: host allocation");
         sub->ctx = ctx;
+        sub->lent = true;
         sub->fuse = ctx->prune_shape != 3;
         messi_alignment aln{ds->N, ds->L, ds->numnodes, ds->masks.data(), ds->children.data(), ds->seqindex.data()};
         std::string err;
@@ -1025,19 +1038,13 @@ int messi_structure_likelihood(messi_ctx* ctx, messi_dataset* ds, const messi_mo
         if (sub) messi_dataset_destroy(sub);
         return code;
     };
-    ModelDev md;
-    if ((rc = upload_model(ctx, ds, model, !pairs.empty(), true, nullptr, &md, true))) return done(rc);
     if (sub) {
         if ((rc = prepare_arena(ctx, sub, md.cat.C))) return done(rc);
         if ((rc = run_pairs(ctx, sub, md.P16, md.pi16, md.logw, md.lam, md.cat.C, md.cat.nlam, false)))
             return done(rc);
     }
-    void *dv, *di;
-    if ((rc = ensure(ctx, kSlotVec, (2 * (size_t)L + 8) * sizeof(double), &dv))) return done(rc);
+    void* di;
     if ((rc = ensure(ctx, kSlotDecodeI, (2 * (size_t)L + 8) * sizeof(int32_t), &di))) return done(rc);
-    double* d_u = (double*)dv;
-    double* d_pairll = d_u + L;
-    double* d_total = d_pairll + L;
     int32_t* d_col = (int32_t*)di;
     std::vector<int32_t> colu(2 * (size_t)L, -1);  // root pair ids, then 0-based partners
     for (int i = 0; i < L; i++) {
@@ -1045,8 +1052,6 @@ int messi_structure_likelihood(messi_ctx* ctx, messi_dataset* ds, const messi_mo
         else if (paired[i] > 0) colu[i] = -2;
         colu[(size_t)L + i] = paired[i] - 1;
     }
-    if ((rc = launch_unpaired(ctx, ds, md.P4, ds->numnodes, md.pi4, md.logw_site, md.cat.nsite, d_u, nullptr)))
-        return done(rc);
     if ((rc = h2d(ctx, d_col, colu.data(), 2 * (size_t)L * sizeof(int32_t)))) return done(rc);
     if ((rc = launch_structure_sum(ctx, L, d_u, d_col, d_col + L, sub ? sub->d_mix : nullptr, md.cat.logwF, d_total,
                                    d_pairll)))

@@ -22,6 +22,10 @@ constexpr int kSyncWords = 4;
 constexpr int kMaxLambda = 8;       // per-lambda conditionals kept in registers
 constexpr int kMaxStack = 512;      // tree height limit
 constexpr int kSlotUnpaired = 20;   // scratch slot of the per-site unpaired log-likelihoods
+constexpr int kSlotPlan = 26;       // of the plan of one structure's pairs
+constexpr int kSlotPlanRows = 27;   // of its message arena: rows, then exponents
+// Most of either that stays with the context; more is allocated for the call.
+constexpr size_t kKeptPlanBytes = size_t(256) << 20;
 constexpr int kEigStride = 16 + 256 + 16;  // eigenvalues, U (row-major), sqrt(pi)
 constexpr int kEig4Stride = 4 + 16 + 4;
 
@@ -290,6 +294,8 @@ struct messi_dataset {
     int arena_C = 0;                   // category count the arena was laid out for
     uint64_t arena_gen = 0;            // bumped whenever the arena and node descriptors are rewritten
     // device
+    bool lent = false;                 // a plan for one call: its buffers may lie in the context's scratch
+    bool lent_plan = false, lent_arena = false;  // they do (not freed with the dataset)
     int* d_bandidx = nullptr;          // [L][W+1]
     int* d_idx = nullptr;              // gather indices of all segments
     int2* d_leaf = nullptr;            // [leaf_rows] (leaf node, 16-bit mask of the pair states)
@@ -376,7 +382,8 @@ struct IdxSeg {
     long long out;   // ints into d_idx
     int op0, op1, n, nb;
 };
-int launch_segment_indices(const IdxSeg* d_segs, const IdxOp* d_ops, int nseg, int64_t maxn, const int* d_lr, int* d_idx);
+int launch_segment_indices(const IdxSeg* d_segs, const IdxOp* d_ops, int nseg, int64_t maxn, const int* d_lr, int* d_idx,
+                           cudaStream_t stream);
 
 // ---- pruning kernels (prune.cu) ----
 constexpr int kP16Floats = 512;  // floats of one 16 x 16 transition matrix (hi part, lo part)

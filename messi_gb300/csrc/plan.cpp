@@ -204,7 +204,7 @@ int build_plan(messi_dataset* ds, const messi_alignment* aln, int W, const uint8
     ds->children.assign(aln->children, aln->children + 2 * nn);
     ds->seqindex.assign(aln->seqindex, aln->seqindex + nn);
     ds->masks.assign(aln->masks, aln->masks + (size_t)N * L);
-    for (size_t i = 0; i < ds->masks.size(); i++)
+    for (size_t i = 0; i < ds->masks.size() && !pairs; i++)  // (a list's alignment is a dataset's, checked before)
         if (ds->masks[i] == 0 || ds->masks[i] > 15) {
             *err = "alignment: nucleotide masks must be in 1..15";
             return MESSI_EINVAL;
@@ -299,6 +299,18 @@ int build_plan(messi_dataset* ds, const messi_alignment* aln, int W, const uint8
     }
 
     // ---- column pattern ids per node (dense, first-occurrence order)
+    // (of the pairs' columns alone where a list of pairs is given)
+    std::vector<int32_t> cols;
+    if (pairs) {
+        std::vector<char> in(L, 0);
+        for (const int2& p : *pairs)
+            if (p.x >= 0 && p.x < p.y && p.y < L) in[p.x] = in[p.y] = 1;
+        for (int x = 0; x < L; x++)
+            if (in[x]) cols.push_back(x);
+    } else {
+        cols.resize(L);
+        for (int x = 0; x < L; x++) cols[x] = x;
+    }
     std::vector<std::vector<int32_t>> pid(nn);
     std::vector<int32_t> npat(nn, 0);
     KeyMap km;
@@ -309,16 +321,16 @@ int build_plan(messi_dataset* ds, const messi_alignment* aln, int W, const uint8
             for (int k = 0; k < 16; k++) first[k] = -1;
             const uint8_t* row = &ds->masks[(size_t)ds->seqindex[v] * L];
             int n = 0;
-            for (int x = 0; x < L; x++) {
+            for (int x : cols) {
                 if (first[row[x]] < 0) first[row[x]] = n++;
                 pid[v][x] = first[row[x]];
             }
             npat[v] = n;
         } else {
             int c0 = ds->children[2 * v], c1 = ds->children[2 * v + 1];
-            km.reset(std::min<size_t>((size_t)L, (size_t)npat[c0] * npat[c1]));
+            km.reset(std::min<size_t>(cols.size(), (size_t)npat[c0] * npat[c1]));
             int n = 0;
-            for (int x = 0; x < L; x++) {
+            for (int x : cols) {
                 bool ins;
                 int64_t key = (int64_t)pid[c0][x] * npat[c1] + pid[c1][x];
                 pid[v][x] = km.get_or_insert(key, n, &ins);
@@ -522,7 +534,7 @@ int build_plan(messi_dataset* ds, const messi_alignment* aln, int W, const uint8
     }
 
     // ---- upload static device data
-    cudaError_t e;
+    cudaError_t e = cudaSuccess;
     int* d_lr = nullptr;
     IdxOp* d_ops = nullptr;
     IdxSeg* d_isegs = nullptr;
@@ -539,61 +551,82 @@ int build_plan(messi_dataset* ds, const messi_alignment* aln, int W, const uint8
         tree[4 * v + 2] = ds->seqindex[v];
         tree[4 * v + 3] = 0;
     }
-#define UPLOAD(dst, src, bytes)                                                       \
-    do {                                                                              \
-        if ((e = cudaMalloc((void**)&(dst), (bytes))) != cudaSuccess) goto cuda_error; \
-        if ((e = cudaMemcpy((dst), (src), (bytes), cudaMemcpyHostToDevice)) != cudaSuccess) goto cuda_error; \
-    } while (0)
-    UPLOAD(ds->d_bandidx, bandidx.data(), bandidx.size() * sizeof(int32_t));
-    UPLOAD(d_lr, lr.data(), lr.size() * sizeof(int32_t));
-    UPLOAD(d_ops, idx_ops.data(), idx_ops.size() * sizeof(IdxOp));
-    UPLOAD(d_isegs, idx_segs.data(), idx_segs.size() * sizeof(IdxSeg));
-    if ((e = cudaMalloc((void**)&ds->d_idx, (size_t)std::max<int64_t>(idx_total, 1) * sizeof(int))) != cudaSuccess)
-        goto cuda_error;
-    if (launch_segment_indices(d_isegs, d_ops, (int)idx_segs.size(), max_seg_n, d_lr, ds->d_idx)) {
-        e = cudaGetLastError();
-        goto cuda_error;
+    // tiles per level
+    std::vector<int2> tiles;
+    for (int lv = 1; lv <= ds->SH; lv++) {
+        SegLevel& sl = ds->seg_levels[lv];
+        sl.tile_off = (int)tiles.size();
+        for (size_t g = 0; g < ds->segs.size(); g++)
+            if (ds->segs[g].level == lv)
+                for (int64_t b = 0; b < ds->segs[g].n; b += 32 * sl.pg) tiles.push_back(make_int2((int)g, (int)b));
+        sl.tile_cnt = (int)tiles.size() - sl.tile_off;
     }
-    UPLOAD(ds->d_leaf, leaf.data(), leaf.size() * sizeof(int2));
-    UPLOAD(ds->d_masks, ds->masks.data(), ds->masks.size());
-    UPLOAD(ds->d_tree, tree.data(), tree.size() * sizeof(int));
-    UPLOAD(ds->d_uops, uops.data(), uops.size() * sizeof(int4));
-#undef UPLOAD
-    if ((e = cudaMalloc((void**)&ds->d_mix, sizeof(double) * std::max<int64_t>(ds->nroot, 1))) != cudaSuccess)
-        goto cuda_error;
-    if ((e = cudaMalloc((void**)&ds->d_mixlam, sizeof(double) * kMaxLambda * std::max<int64_t>(ds->nroot, 1))) !=
-        cudaSuccess)
-        goto cuda_error;
-    {
-        // tiles per level
-        std::vector<int2> tiles;
-        for (int lv = 1; lv <= ds->SH; lv++) {
-            SegLevel& sl = ds->seg_levels[lv];
-            sl.tile_off = (int)tiles.size();
-            for (size_t g = 0; g < ds->segs.size(); g++)
-                if (ds->segs[g].level == lv)
-                    for (int64_t b = 0; b < ds->segs[g].n; b += 32 * sl.pg) tiles.push_back(make_int2((int)g, (int)b));
-            sl.tile_cnt = (int)tiles.size() - sl.tile_off;
+    if (tiles.empty()) tiles.push_back(make_int2(0, 0));
+
+    // device buffers: what is uploaded, then what is only laid out
+    struct Buffer {
+        void** p;
+        const void* src;
+        size_t bytes;
+        bool temporary;
+    };
+    const Buffer buffers[] = {
+        {(void**)&ds->d_bandidx, bandidx.data(), bandidx.size() * sizeof(int32_t), false},
+        {(void**)&d_lr, lr.data(), lr.size() * sizeof(int32_t), true},
+        {(void**)&d_ops, idx_ops.data(), idx_ops.size() * sizeof(IdxOp), true},
+        {(void**)&d_isegs, idx_segs.data(), idx_segs.size() * sizeof(IdxSeg), true},
+        {(void**)&ds->d_leaf, leaf.data(), leaf.size() * sizeof(int2), false},
+        {(void**)&ds->d_masks, ds->masks.data(), ds->masks.size(), false},
+        {(void**)&ds->d_tree, tree.data(), tree.size() * sizeof(int), false},
+        {(void**)&ds->d_uops, uops.data(), uops.size() * sizeof(int4), false},
+        {(void**)&ds->d_tiles, tiles.data(), tiles.size() * sizeof(int2), false},
+        {(void**)&ds->d_idx, nullptr, (size_t)std::max<int64_t>(idx_total, 1) * sizeof(int), false},
+        {(void**)&ds->d_mix, nullptr, sizeof(double) * std::max<int64_t>(ds->nroot, 1), false},
+        {(void**)&ds->d_mixlam, nullptr, sizeof(double) * kMaxLambda * std::max<int64_t>(ds->nroot, 1), false},
+        {(void**)&ds->d_segs, nullptr, sizeof(SegDev) * ds->segs.size(), false},
+        {(void**)&ds->d_steps, nullptr, sizeof(StepDev) * std::max(1, ds->nsteps), false},
+    };
+    auto room = [](size_t bytes) { return (bytes + 255) & ~size_t(255); };
+    size_t total = 0, uploaded = 0;
+    for (const Buffer& b : buffers) {
+        total += room(b.bytes);
+        if (b.src) uploaded += room(b.bytes);
+    }
+    if (ds->lent && total <= kKeptPlanBytes) {
+        // one copy into the context's scratch, in its stream's order (a dozen
+        // allocations and their frees took 0.2 ms of a structure's call)
+        void* slab = nullptr;
+        if (const int rc = ensure(ds->ctx, kSlotPlan, total, &slab)) {
+            *err = "dataset upload: " + ds->ctx->last_error;
+            return rc;
         }
-        if (tiles.empty()) tiles.push_back(make_int2(0, 0));
-        if ((e = cudaMalloc((void**)&ds->d_tiles, tiles.size() * sizeof(int2))) != cudaSuccess) goto cuda_error;
-        if ((e = cudaMemcpy(ds->d_tiles, tiles.data(), tiles.size() * sizeof(int2), cudaMemcpyHostToDevice)) !=
-            cudaSuccess)
-            goto cuda_error;
-        if ((e = cudaMalloc((void**)&ds->d_segs, sizeof(SegDev) * ds->segs.size())) != cudaSuccess) goto cuda_error;
-        if ((e = cudaMalloc((void**)&ds->d_steps, sizeof(StepDev) * std::max(1, ds->nsteps))) != cudaSuccess)
-            goto cuda_error;
+        ds->lent_plan = true;
+        std::vector<char> stage(uploaded);
+        size_t at = 0;
+        for (const Buffer& b : buffers) {
+            *b.p = (char*)slab + at;
+            if (b.src && b.bytes) std::memcpy(stage.data() + at, b.src, b.bytes);
+            at += room(b.bytes);
+        }
+        e = cudaMemcpyAsync(slab, stage.data(), uploaded, cudaMemcpyHostToDevice, ds->ctx->stream);
+        if (e == cudaSuccess && launch_segment_indices(d_isegs, d_ops, (int)idx_segs.size(), max_seg_n, d_lr, ds->d_idx,
+                                                       ds->ctx->stream))
+            e = cudaGetLastError();
+        if (e == cudaSuccess) return MESSI_OK;
+    } else {
+        for (const Buffer& b : buffers) {
+            if (e == cudaSuccess) e = cudaMalloc(b.p, b.bytes);
+            if (e == cudaSuccess && b.src) e = cudaMemcpy(*b.p, b.src, b.bytes, cudaMemcpyHostToDevice);
+        }
+        if (e == cudaSuccess &&
+            launch_segment_indices(d_isegs, d_ops, (int)idx_segs.size(), max_seg_n, d_lr, ds->d_idx, 0))
+            e = cudaGetLastError();
+        // the index kernel ran on the default stream: done before any context stream reads its output
+        if (e == cudaSuccess) e = cudaStreamSynchronize(0);
+        for (const Buffer& b : buffers)
+            if (b.temporary) cudaFree(*b.p);
+        if (e == cudaSuccess) return MESSI_OK;
     }
-    // the index kernel ran on the default stream: done before any context stream reads its output
-    if ((e = cudaStreamSynchronize(0)) != cudaSuccess) goto cuda_error;
-    cudaFree(d_lr);
-    cudaFree(d_ops);
-    cudaFree(d_isegs);
-    return MESSI_OK;
-cuda_error:
-    cudaFree(d_lr);
-    cudaFree(d_ops);
-    cudaFree(d_isegs);
     *err = std::string("dataset upload: ") + cudaGetErrorString(e);
     return (e == cudaErrorMemoryAllocation) ? MESSI_ENOMEM : MESSI_ECUDA;
 }
@@ -660,15 +693,28 @@ int allocate_arena(messi_dataset* ds, int C, std::string* err)
         return MESSI_ENOMEM;
     }
     if (ds->chunk != chunk) {
-        if (ds->d_arena_f) cudaFree(ds->d_arena_f);
-        if (ds->d_arena_e) cudaFree(ds->d_arena_e);
+        if (ds->d_arena_f && !ds->lent_arena) cudaFree(ds->d_arena_f);
+        if (ds->d_arena_e && !ds->lent_arena) cudaFree(ds->d_arena_e);
         ds->d_arena_f = nullptr;
         ds->d_arena_e = nullptr;
         ds->d_leafmsg = nullptr;
         ds->chunk = 0;
+        const size_t fbytes = (size_t)chunk * all_rows * 16 * sizeof(float), ebytes = (size_t)chunk * ds->arena_rows * sizeof(int);
+        ds->lent_arena = ds->lent && fbytes + ebytes <= kKeptPlanBytes;
         // segment rows, then the leaf messages (which have no exponents)
-        cudaError_t e = cudaMalloc((void**)&ds->d_arena_f, (size_t)chunk * all_rows * 16 * sizeof(float));
-        if (e == cudaSuccess) e = cudaMalloc((void**)&ds->d_arena_e, (size_t)chunk * ds->arena_rows * sizeof(int));
+        cudaError_t e = cudaSuccess;
+        if (ds->lent_arena) {
+            void* rows = nullptr;
+            if (const int rc = ensure(ds->ctx, kSlotPlanRows, fbytes + ebytes, &rows)) {
+                *err = "message arena: " + ds->ctx->last_error;
+                return rc;
+            }
+            ds->d_arena_f = (float*)rows;
+            ds->d_arena_e = (int*)((char*)rows + fbytes);
+        } else {
+            e = cudaMalloc((void**)&ds->d_arena_f, fbytes);
+            if (e == cudaSuccess) e = cudaMalloc((void**)&ds->d_arena_e, ebytes);
+        }
         if (e != cudaSuccess) {
             *err = std::string("message arena: ") + cudaGetErrorString(e);
             return MESSI_ENOMEM;
@@ -681,11 +727,13 @@ int allocate_arena(messi_dataset* ds, int C, std::string* err)
     ds->steps_host.assign((size_t)ds->nsteps, StepDev{});
     fill_descriptors(ds, ds->d_arena_f, ds->d_arena_e, 0, ds->arena_rows, (int64_t)ds->chunk * ds->arena_rows,
                      leaf_rows, 0, 0, ds->d_steps, ds->segs_host.data(), ds->steps_host.data());
-    cudaError_t e = cudaMemcpy(ds->d_segs, ds->segs_host.data(), sizeof(SegDev) * ds->segs.size(),
-                               cudaMemcpyHostToDevice);
-    if (e == cudaSuccess)
-        e = cudaMemcpy(ds->d_steps, ds->steps_host.data(), sizeof(StepDev) * (size_t)ds->nsteps,
-                       cudaMemcpyHostToDevice);
+    // (a lent plan's in the stream's order, behind the last user of its scratch)
+    auto upload = [&](void* dst, const void* src, size_t bytes) {
+        return ds->lent ? cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, ds->ctx->stream)
+                        : cudaMemcpy(dst, src, bytes, cudaMemcpyHostToDevice);
+    };
+    cudaError_t e = upload(ds->d_segs, ds->segs_host.data(), sizeof(SegDev) * ds->segs.size());
+    if (e == cudaSuccess) e = upload(ds->d_steps, ds->steps_host.data(), sizeof(StepDev) * (size_t)ds->nsteps);
     if (e != cudaSuccess) {
         *err = std::string("segment descriptors: ") + cudaGetErrorString(e);
         return MESSI_ECUDA;

@@ -668,12 +668,13 @@ __global__ void __launch_bounds__(256) segment_idx_kernel(const IdxSeg* __restri
     }
 }
 
-int launch_segment_indices(const IdxSeg* d_segs, const IdxOp* d_ops, int nseg, int64_t maxn, const int* d_lr, int* d_idx)
+int launch_segment_indices(const IdxSeg* d_segs, const IdxOp* d_ops, int nseg, int64_t maxn, const int* d_lr, int* d_idx,
+                           cudaStream_t stream)
 {
     if (maxn <= 0) return MESSI_OK;
     const unsigned gx = (unsigned)(((maxn + 31) / 32 * 32 + 255) / 256);
     for (int s = 0; s < nseg; s += 65535)
-        segment_idx_kernel<<<dim3(gx, std::min(nseg - s, 65535)), 256>>>(d_segs, d_ops, s, d_lr, d_idx);
+        segment_idx_kernel<<<dim3(gx, std::min(nseg - s, 65535)), 256, 0, stream>>>(d_segs, d_ops, s, d_lr, d_idx);
     return cudaPeekAtLastError() == cudaSuccess ? MESSI_OK : MESSI_ECUDA;
 }
 
