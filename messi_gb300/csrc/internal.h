@@ -24,7 +24,8 @@ constexpr int kMaxStack = 512;      // tree height limit
 constexpr int kSlotUnpaired = 20;   // scratch slot of the per-site unpaired log-likelihoods
 constexpr int kSlotPlan = 26;       // of the plan of one structure's pairs
 constexpr int kSlotPlanRows = 27;   // of its message arena: rows, then exponents
-// Most of either that stays with the context; more is allocated for the call.
+constexpr int kSlotCatMix = 28;     // of the root categories' values where several CTAs share a pair group
+// Most of a structure's plan or arena that stays with the context; more is allocated for the call.
 constexpr size_t kKeptPlanBytes = size_t(256) << 20;
 constexpr int kEigStride = 16 + 256 + 16;  // eigenvalues, U (row-major), sqrt(pi)
 constexpr int kEig4Stride = 4 + 16 + 4;

@@ -362,10 +362,14 @@ __device__ __forceinline__ void pow2_scale(float m, int& ex, float& sc)
 // The CTA's warps are pg pair groups x cs category splits: with few pairs the
 // warps of one pair group take every cs-th category each (a level of 50
 // tiles of 128 pairs with all 36 categories in turn took 45 us).
+// Where a pair group's twelve splits still leave the chip idle, gridDim.y CTAs
+// share its categories (the 150 pairs of a structure over 64 sequences, 5 pair
+// groups: root level 156 -> 35 us with three CTAs each, and 13 us for the mixtures).
 // ROOT: 0 = interior segment, 1 = the tree's root with the category mixture
 // kept in registers (cs = 1), 2 = the root with the categories' values
-// collected in shared memory and mixed afterwards in category order by one
-// warp, so that the sum has the same bits.
+// collected in shared memory (in `shared_values` where CTAs share a group) and
+// mixed afterwards in category order by one warp, so that the sum has the same
+// bits.
 // ---------------------------------------------------------------------------
 struct Mixture {
     double m = -INFINITY;
@@ -381,6 +385,32 @@ struct Mixture {
     }
     __device__ __forceinline__ double value() const { return (m == -INFINITY) ? -INFINITY : m + log((double)s); }
 };
+
+// Mixes the categories' values v[32 cc] of pair u in category order.
+__device__ __forceinline__ void mix_values(const SegDev& sg, const double* v, int u, int c0, int nc,
+                                           const int* __restrict__ lam, int per_lambda)
+{
+    Mixture mix;
+    for (int c1 = 0; c1 < nc; c1 += 12) {
+        double x[12];  // twelve loads in flight (one after another: 18 us for 36 categories)
+#pragma unroll
+        for (int k = 0; k < 12; k++) x[k] = v[(size_t)min(c1 + k, nc - 1) * 32];
+#pragma unroll
+        for (int k = 0; k < 12; k++)
+            if (c1 + k < nc) mix.add(x[k]);
+    }
+    const double res = mix.value();
+    sg.mix[u] = (c0 == 0) ? res : lse_d(sg.mix[u], res);
+    if (!per_lambda) return;
+    for (int q = 0; q < kMaxLambda; q++) {
+        Mixture ml;
+        for (int cc = 0; cc < nc; cc++)
+            if (__ldg(lam + c0 + cc) == q) ml.add(v[(size_t)cc * 32]);
+        const double rq = ml.value();
+        double* dst = sg.mixlam + (size_t)q * sg.n + u;
+        *dst = (c0 == 0) ? rq : lse_d(*dst, rq);
+    }
+}
 
 // Lane t's own one of four values (pair g + 8t).
 __device__ __forceinline__ int own4(const int4& v, int t) { return t == 0 ? v.x : (t == 1 ? v.y : (t == 2 ? v.z : v.w)); }
@@ -416,7 +446,8 @@ template <int ROOT, int NP, int MAXT, int MINB>
 __global__ void __launch_bounds__(MAXT, MINB) prune_path_kernel(
     const SegDev* __restrict__ segs, const int2* __restrict__ tiles, const float* __restrict__ P, int numnodes,
     int c0, int nc, int C, const float* __restrict__ pi16, const double* __restrict__ logw,
-    const int* __restrict__ lam, int per_lambda, int cs, int max_steps, int max_nb, int max_depth)
+    const int* __restrict__ lam, int per_lambda, int cs, int max_steps, int max_nb, int max_depth,
+    double* __restrict__ shared_values)
 {
     extern __shared__ float4 smem_raw[];
     const int2 tile = tiles[blockIdx.x];
@@ -424,7 +455,8 @@ __global__ void __launch_bounds__(MAXT, MINB) prune_path_kernel(
     const int n = sg.n, ns = sg.nsteps, nb = sg.nb;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int g = lane >> 2, t = lane & 3;
-    const int pgs = (int)(blockDim.x >> 5) / cs, pg = warp % pgs, split = warp / pgs;
+    const int pgs = (int)(blockDim.x >> 5) / cs, pg = warp % pgs;
+    const int split = warp / pgs + cs * (int)blockIdx.y, stride = cs * (int)gridDim.y;  // this warp's categories
     const int base = tile.y + 32 * NP * pg;  // first pair of this warp
     const bool active = base < n;
     // shared memory: gathers (slot nb repeats slot 0: the stream's last look
@@ -436,7 +468,9 @@ __global__ void __launch_bounds__(MAXT, MINB) prune_path_kernel(
     int4* sidx = reinterpret_cast<int4*>(rest) + pg * (max_nb + 1) * 8 * NP;
     rest += pgs * (max_nb + 1) * 8 * NP;
     float4* stack = rest + warp * max_depth * 128 * NP + lane;
-    double* collected = reinterpret_cast<double*>(rest + (int)(blockDim.x >> 5) * max_depth * 128 * NP);
+    double* collected = (ROOT == 2 && gridDim.y > 1)
+                            ? shared_values + (size_t)blockIdx.x * pgs * NP * nc * 32
+                            : reinterpret_cast<double*>(rest + (int)(blockDim.x >> 5) * max_depth * 128 * NP);
     const int nmul = ROOT ? ns - 1 : ns;  // the root's step has no mat-vec
     for (int i = threadIdx.x; i < ns; i += blockDim.x) {
         const int4* steps = reinterpret_cast<const int4*>(sg.steps);
@@ -448,13 +482,13 @@ __global__ void __launch_bounds__(MAXT, MINB) prune_path_kernel(
             if (nx.w & kStepInit) nx = __ldg(steps + i + 2);
             ahead = (unsigned)nx.z;
         } else {
-            ahead = (unsigned)__ldg(steps + 1).z + (unsigned)(cs * numnodes);
+            ahead = (unsigned)__ldg(steps + 1).z + (unsigned)(stride * numnodes);
         }
         ops[i] = make_int2((int)ahead, st.w);
         if (st.w & kStepGather) {
             const int slot = st.w >> kStepSlotShift;
             gathers[slot] = make_int4(st.x, st.y, st.w & kStepLeaf, -1);
-            if (slot == 0) gathers[nb] = make_int4(st.x + cs * st.y, st.y, st.w & kStepLeaf, st.x + (nc - 1) * st.y);
+            if (slot == 0) gathers[nb] = make_int4(st.x + stride * st.y, st.y, st.w & kStepLeaf, st.x + (nc - 1) * st.y);
         }
     }
     if (active) {
@@ -462,7 +496,7 @@ __global__ void __launch_bounds__(MAXT, MINB) prune_path_kernel(
         for (int h = 0; h < NP; h++) {  // (past the last pair the last tile again)
             const int4* src = reinterpret_cast<const int4*>(sg.idx) + (size_t)min((base >> 5) + h, (n - 1) >> 5) * nb * 8;
             int4* dst = sidx + h * (max_nb + 1) * 8;
-            for (int i = split * 32 + lane; i < (nb + 1) * 8; i += 32 * cs) dst[i] = __ldg(src + (i < nb * 8 ? i : i - nb * 8));
+            for (int i = warp / pgs * 32 + lane; i < (nb + 1) * 8; i += 32 * cs) dst[i] = __ldg(src + (i < nb * 8 ? i : i - nb * 8));
         }
     }
     __syncthreads();
@@ -473,9 +507,9 @@ __global__ void __launch_bounds__(MAXT, MINB) prune_path_kernel(
         int e[NP], er[NP];
         const float4* rows = reinterpret_cast<const float4*>(sg.rows) + t;
         const int* exps = sg.exps;
-        const int4* gp;
-        const int* si;
-        int cc;
+        const int4* gp = gathers;
+        const int* si = reinterpret_cast<const int*>(sidx);
+        int cc = split;
         // The next gather of the stream: states 4t..4t+3 of pairs g + 8k, and
         // the exponent of the lane's own pair.
         auto next = [&]() {
@@ -519,12 +553,9 @@ __global__ void __launch_bounds__(MAXT, MINB) prune_path_kernel(
             Bl[0] = __ldg(pv + 64);
             Bl[1] = __ldg(pv + 96);
         };
-        cc = split;
-        gp = gathers;
-        si = reinterpret_cast<const int*>(sidx);
         next();
         matrix((unsigned)__ldg(&sg.steps[1].self));
-        for (; cc < nc; cc += cs, Pc += (size_t)cs * numnodes * (kP16Floats / 4)) {
+        for (; cc < nc; cc += stride, Pc += (size_t)stride * numnodes * (kP16Floats / 4)) {
             const unsigned last = (unsigned)((nc - cc) * numnodes - 1);
             gp = gathers + 1;
             si = reinterpret_cast<const int*>(sidx) + 32;
@@ -618,31 +649,37 @@ __global__ void __launch_bounds__(MAXT, MINB) prune_path_kernel(
         }
     }
     if (ROOT == 2) {
+        if (gridDim.y > 1) return;  // mix_values_kernel follows
         __syncthreads();
         if (split != 0 || !active) return;
 #pragma unroll
         for (int h = 0; h < NP; h++)
-            for (int cc = 0; cc < nc; cc++) mix[h].add(collected[((pg * NP + h) * nc + cc) * 32 + lane]);
+            if (myu + 32 * h < n)
+                mix_values(sg, collected + (size_t)(pg * NP + h) * nc * 32 + lane, myu + 32 * h, c0, nc, lam, per_lambda);
     }
-    if (ROOT && active) {
+    if (ROOT == 1 && active) {
 #pragma unroll
         for (int h = 0; h < NP; h++) {
             const int u = myu + 32 * h;
             if (u >= n) continue;
             const double res = mix[h].value();
             sg.mix[u] = (c0 == 0) ? res : lse_d(sg.mix[u], res);
-            if (ROOT == 2 && per_lambda) {
-                for (int q = 0; q < kMaxLambda; q++) {
-                    Mixture ml;
-                    for (int cc = 0; cc < nc; cc++)
-                        if (__ldg(lam + c0 + cc) == q) ml.add(collected[((pg * NP + h) * nc + cc) * 32 + lane]);
-                    const double rq = ml.value();
-                    double* dst = sg.mixlam + (size_t)q * n + u;
-                    *dst = (c0 == 0) ? rq : lse_d(*dst, rq);
-                }
-            }
         }
     }
+}
+
+// The mixtures of the root's pairs whose categories several CTAs have shared: a
+// warp per tile of 32 pairs.
+__global__ void __launch_bounds__(128) mix_values_kernel(const SegDev* __restrict__ segs, const int2* __restrict__ tiles,
+                                                         int ntiles, const double* __restrict__ values, int c0, int nc,
+                                                         const int* __restrict__ lam, int per_lambda)
+{
+    const int w = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
+    if (w >= ntiles) return;
+    const int2 tile = tiles[w];
+    const SegDev& sg = segs[tile.x];
+    const int u = tile.y + (lane >> 2) + 8 * (lane & 3);
+    if (u < sg.n) mix_values(sg, values + (size_t)w * nc * 32 + lane, u, c0, nc, lam, per_lambda);
 }
 
 // Gather indices of a segment from the per-node child lists: position p of a
@@ -1018,12 +1055,13 @@ static int launch_prune_tc(messi_ctx* ctx, const SegDev* d_segs, const int2* d_t
 template <int ROOT, int NP, int MAXT, int MINB>
 static int launch_path(messi_ctx* ctx, const SegDev* d_segs, const int2* d_tiles, const SegLevel& lv, int cs,
                        const float* d_P, int numnodes, int c0, int nc, int C, const float* d_pi16,
-                       const double* d_logw, const int* d_lam, bool per_lambda)
+                       const double* d_logw, const int* d_lam, bool per_lambda, int ctas = 1,
+                       double* shared_values = nullptr)
 {
     const int pgs = lv.pg / NP, warps = pgs * cs;
     const size_t smem = sizeof(float4) * ((size_t)(lv.max_nb + 1) * (1 + 8 * lv.pg) + (lv.max_steps + 1) / 2 +
                                           (size_t)warps * NP * lv.max_depth * 128) +
-                        (ROOT == 2 ? sizeof(double) * 32 * (size_t)lv.pg * nc : 0);
+                        (ROOT == 2 && ctas == 1 ? sizeof(double) * 32 * (size_t)lv.pg * nc : 0);
     static thread_local std::pair<int, size_t> granted{-1, 0};
     if (granted.first != ctx->device || granted.second < smem) {
         cudaError_t e = cudaFuncSetAttribute(prune_path_kernel<ROOT, NP, MAXT, MINB>,
@@ -1031,9 +1069,9 @@ static int launch_path(messi_ctx* ctx, const SegDev* d_segs, const int2* d_tiles
         if (e != cudaSuccess) return cuda_fail(ctx, e, "prune_path_kernel attributes");
         granted = {ctx->device, smem};
     }
-    prune_path_kernel<ROOT, NP, MAXT, MINB><<<lv.tile_cnt, 32 * warps, smem, ctx->stream>>>(
+    prune_path_kernel<ROOT, NP, MAXT, MINB><<<dim3(lv.tile_cnt, ctas), 32 * warps, smem, ctx->stream>>>(
         d_segs, d_tiles + lv.tile_off, d_P, numnodes, c0, nc, C, d_pi16, d_logw, d_lam, per_lambda ? 1 : 0, cs,
-        lv.max_steps, lv.max_nb, lv.max_depth);
+        lv.max_steps, lv.max_nb, lv.max_depth, shared_values);
     LAUNCH_CHECK(ctx, ROOT ? "prune_path_kernel<root>" : "prune_path_kernel");
     return MESSI_OK;
 }
@@ -1060,10 +1098,25 @@ int launch_prune_level(messi_ctx* ctx, const SegDev* d_segs, const int2* d_tiles
     // few pairs (or per-lambda mixtures): the warps of a pair group share the
     // categories until the GPU's 16 warps per SM are filled
     const int sms = ctx->num_sms > 0 ? ctx->num_sms : 152;
-    int cs = (lv.pg == 1) ? (int)std::min<int64_t>(kMaxSplits, (16 * (int64_t)sms + lv.warps - 1) / std::max<int64_t>(lv.warps, 1)) : 1;
-    cs = std::max(1, std::min(cs, nc));
-    if (!root) return MESSI_PATH(0, 1, 32 * kMaxSplits, 1, cs);
-    return MESSI_PATH(2, 1, 32 * kMaxSplits, 1, cs);
+    const int64_t want = (lv.pg == 1) ? (16 * (int64_t)sms + lv.warps - 1) / std::max<int64_t>(lv.warps, 1) : 1;
+    const int splits = (int)std::max<int64_t>(1, std::min<int64_t>(want, nc));
+    const int ctas = (splits + kMaxSplits - 1) / kMaxSplits, cs = (splits + ctas - 1) / ctas;
+    if (!root)
+        return launch_path<0, 1, 32 * kMaxSplits, 1>(ctx, d_segs, d_tiles, lv, cs, d_P, numnodes, c0, nc, C, d_pi16, d_logw,
+                                                     d_lam, per_lambda, ctas);
+    void* values = nullptr;
+    if (ctas > 1) {
+        const int rc = ensure(ctx, kSlotCatMix, (size_t)lv.tile_cnt * nc * 32 * sizeof(double), &values);
+        if (rc) return rc;
+    }
+    const int rc = launch_path<2, 1, 32 * kMaxSplits, 1>(ctx, d_segs, d_tiles, lv, cs, d_P, numnodes, c0, nc, C, d_pi16,
+                                                         d_logw, d_lam, per_lambda, ctas, (double*)values);
+    if (rc || ctas == 1) return rc;
+    mix_values_kernel<<<(lv.tile_cnt + 3) / 4, 128, 0, ctx->stream>>>(d_segs, d_tiles + lv.tile_off, lv.tile_cnt,
+                                                                     (const double*)values, c0, nc, d_lam,
+                                                                     per_lambda ? 1 : 0);
+    LAUNCH_CHECK(ctx, "mix_values_kernel");
+    return MESSI_OK;
 #undef MESSI_PATH
 }
 
@@ -1420,27 +1473,35 @@ int launch_siterate_conditionals(messi_ctx* ctx, messi_dataset* ds, const double
 // logwF + u[c] + u[partner] to each pair, so the unpaired values of paired
 // columns are read before they are cleared.
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(1024) structure_sum_kernel(double* __restrict__ u, const int* __restrict__ colu,
+// A pair's value by a thread each, a warp per CTA: the FP64 units take 64 cycles
+// a warp instruction, and one CTA's 1,000 columns kept its SM busy for 21 us.
+__global__ void __launch_bounds__(32) structure_pairs_kernel(const double* __restrict__ u, const int* __restrict__ colu,
                                                              const int* __restrict__ partner, int L,
                                                              const double* __restrict__ mix, double logwF,
-                                                             double* __restrict__ total, double* __restrict__ pairll)
+                                                             double* __restrict__ pairll)
+{
+    const int c = blockIdx.x * 32 + threadIdx.x;
+    if (c >= L) return;
+    const int k = colu[c];
+    double pv = 0.0;
+    if (k >= 0) {
+        pv = mix[k];
+        if (logwF != -INFINITY) pv = lse_d(pv, logwF + u[c] + u[partner[c]]);
+    }
+    pairll[c] = pv;
+}
+
+__global__ void __launch_bounds__(1024) structure_sum_kernel(double* __restrict__ u, const int* __restrict__ colu, int L,
+                                                             double* __restrict__ total,
+                                                             const double* __restrict__ pairll)
 {
     __shared__ double part[1024];
     double acc = 0.0;
     for (int c = threadIdx.x; c < L; c += blockDim.x) {
-        const int k = colu[c];
-        double pv = 0.0;
-        if (k >= 0) {
-            pv = mix[k];
-            if (logwF != -INFINITY) pv = lse_d(pv, logwF + u[c] + u[partner[c]]);
-        }
-        if (k == -1) acc += u[c];
-        pairll[c] = pv;
-        acc += pv;
+        if (colu[c] == -1) acc += u[c];
+        else u[c] = 0.0;
+        acc += pairll[c];
     }
-    __syncthreads();
-    for (int c = threadIdx.x; c < L; c += blockDim.x)
-        if (colu[c] != -1) u[c] = 0.0;
     part[threadIdx.x] = acc;
     __syncthreads();
     for (int off = blockDim.x / 2; off > 0; off >>= 1) {
@@ -1453,7 +1514,9 @@ __global__ void __launch_bounds__(1024) structure_sum_kernel(double* __restrict_
 int launch_structure_sum(messi_ctx* ctx, int L, double* d_u, const int* d_colu, const int* d_partner,
                          const double* d_mix, double logwF, double* d_total, double* d_pairll)
 {
-    structure_sum_kernel<<<1, 1024, 0, ctx->stream>>>(d_u, d_colu, d_partner, L, d_mix, logwF, d_total, d_pairll);
+    structure_pairs_kernel<<<(L + 31) / 32, 32, 0, ctx->stream>>>(d_u, d_colu, d_partner, L, d_mix, logwF, d_pairll);
+    LAUNCH_CHECK(ctx, "structure_pairs_kernel");
+    structure_sum_kernel<<<1, 1024, 0, ctx->stream>>>(d_u, d_colu, L, d_total, d_pairll);
     LAUNCH_CHECK(ctx, "structure_sum_kernel");
     return MESSI_OK;
 }
