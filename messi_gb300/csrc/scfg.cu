@@ -1060,8 +1060,8 @@ __device__ __forceinline__ int2 pair_cell(const InsideBands<BATCH>& ib, const Pa
 // Bound by the chain write -> look from L2 -> cells of d -> cells of d+1, about
 // 1.7 us a pair, and on long bands by the latency of the partial sums' loads.
 // Against one grid barrier per pair with every warp summing and then finishing
-// its own cell: span 500 of 1,000 columns 0.74 -> 0.51 ms, every span of 120
-// 154 -> 93 us and of 2,001 5.18 -> 3.78 ms, span 800 of 9,000 4.82 -> 4.70 ms;
+// its own cell: span 500 of 1,000 columns 0.74 -> 0.49 ms, every span of 120
+// 154 -> 93 us and of 2,001 5.18 -> 3.39 ms, span 800 of 9,000 4.82 -> 4.70 ms;
 // 24 alignments of 80-600 columns, with a barrier per diagonal before, 3.23 ->
 // 1.23 ms.
 template <bool BATCH, int MAXT>
@@ -1165,13 +1165,24 @@ __global__ void __launch_bounds__(MAXT) inside_pair_kernel(InsideBands<BATCH> ib
         // meanwhile (span 500 of 1,000 columns: 537 -> 511 us, the batch of 24
         // 1.37 -> 1.23 ms).
         auto load = [&](const Item& q, int k, float (&a)[16], float (&b)[16]) {
-            const int e = 2 + (q.dd - d), rem = q.valid ? (q.dd - e - k + 31) / 32 : 0;
+            // (sixteen that all 32 lanes have go without predicates: span 500 of
+            // 1,000 columns 520 -> 489 us, L = 2,001 3.81 -> 3.39 ms)
+            const int left = q.valid ? q.dd - 2 - (q.dd - d) - (k - lane) : 0;  // split points from here on
             const float* pa = q.lrow + k;
             const float* pb = q.scol - k;
+            if (left >= 512) {
+#pragma unroll
+                for (int j = 0; j < 16; j++) {
+                    a[j] = __ldcg(pa + j * 32);
+                    b[j] = __ldcg(pb - j * 32);
+                }
+                return;
+            }
 #pragma unroll
             for (int j = 0; j < 16; j++) {
-                a[j] = ldcg_if(pa + j * 32, j < rem, -INFINITY);
-                b[j] = ldcg_if(pb - j * 32, j < rem, -INFINITY);
+                const bool on = j * 32 + lane < left;
+                a[j] = ldcg_if(pa + j * 32, on, -INFINITY);
+                b[j] = ldcg_if(pb - j * 32, on, -INFINITY);
             }
         };
         int w = wt >> 5;
@@ -1707,7 +1718,7 @@ static int wave_grid(messi_ctx* ctx)
 // a batch: with 16 cells and more per CTA twenty warps that form the sums are
 // worth more than twelve with their next loads in flight (span 800 of 3,000,
 // 4,500, 6,000 columns: 1.83, 2.52, 3.22 ms against 1.99, 2.87, 3.75; L = 2,001,
-// 13 cells: 3.98 against 3.78; the batch, which needs more registers, 1.34
+// 13 cells: 3.98 against 3.39; the batch, which needs more registers, 1.34
 // against 1.23).
 static int launch_inside(messi_ctx* ctx, const void* kernel, const void* many, void** args, unsigned int* sync,
                          long long columns, std::array<std::pair<float*, size_t>, 3> cells)
