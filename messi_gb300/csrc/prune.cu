@@ -43,11 +43,13 @@ namespace messi {
 // kP16Nodes nodes, a thread per entry: the CTA forms the exponentials of all
 // its nodes at once, stages the category's U and the ratios sqrt(pi_d) /
 // sqrt(pi_a) once per model group and, per node, W[a][k] = U[a][k] exp(w_k t),
-// so an entry is 16 FP64 multiply-adds (36 categories of 127 nodes: 32 us of
-// the FP64 pipe).  With 32 nodes per CTA and a node's exponentials on its
-// critical path it took 73 us there and 69 us for 31 nodes (36 CTAs); now
-// 53 and 17 us.
+// so an entry is 16 FP64 multiply-adds; U exp(W t) U^T is symmetric, so a thread
+// forms one of its 136 entries and scales it both ways.  Bound by the FP64 pipe.
+// 36 categories of 127 nodes, of 31 nodes: with 32 nodes per CTA and a node's
+// exponentials on its critical path 73 and 69 us (36 CTAs), with all 256 entries
+// 53 and 17 us, now 41 and 15; 1,584 nodes 577 -> 448 us.
 constexpr int kP16Nodes = 8;
+constexpr int kP16Entries = 136;  // i <= j
 
 // x as TF32 hi + lo: hi = x rounded to TF32 (half a TF32 ulp added to the
 // magnitude bits, then truncated: round to nearest, ties away), lo = x - hi,
@@ -78,6 +80,10 @@ __global__ void __launch_bounds__(256) build_P16_kernel(const double* __restrict
         const int grp = group(v0 + a);
         if (grp >= 0) ex[a][d] = exp(eig[((size_t)grp * C + c) * kEigStride + d] * bl[v0 + a]);
     }
+    // this thread's entry (i, j), i <= j, of a node: the t-th, row by row
+    int i = 0, j = t;
+    while (i < 16 && j >= 16 - i) j -= 16 - i++;
+    j += i;
     int cur = -1;
     for (int v = v0; v < v1; v++) {
         const int grp = group(v), buf = v & 1;
@@ -93,22 +99,28 @@ __global__ void __launch_bounds__(256) build_P16_kernel(const double* __restrict
         // W[a][k], k = d; the other buffer may still be read for the node before
         if (grp >= 0) W[buf][t] = U[t] * ex[v - v0][d];
         __syncthreads();
-        float out;
+        if (t >= kP16Entries) continue;
+        float up, low;  // (i, j) and (j, i)
         if (grp < 0) {
-            out = 0.f;  // a root has no branch (gettransitionmatriceslist, src/FARCE.jl:416)
+            up = low = 0.f;  // a root has no branch (gettransitionmatriceslist, src/FARCE.jl:416)
         } else if (tl == 0.0) {
-            out = (a == d) ? 1.f : 0.f;
+            up = low = (i == j) ? 1.f : 0.f;
         } else {
             double acc = 0.0;
 #pragma unroll
-            for (int k = 0; k < 16; k++) acc += W[buf][a * 16 + k] * U[d * 16 + k];
-            acc *= R[t];
-            out = (acc <= 0.0) ? 0.f : (float)acc;  // absmat clamp (1e-50 rounds to 0 in FP32)
+            for (int k = 0; k < 16; k++) acc += W[buf][i * 16 + k] * U[j * 16 + k];
+            auto entry = [&](double x) { return (x <= 0.0) ? 0.f : (float)x; };  // absmat clamp (1e-50 rounds to 0 in FP32)
+            up = entry(acc * R[i * 16 + j]);
+            low = entry(acc * R[j * 16 + i]);
         }
-        float* p = P + ((size_t)c * numnodes + v) * kP16Floats + p16_at(a, d);
-        const float hi = tf32_hi(out);
-        p[0] = hi;
-        p[256] = out - hi;
+        float* p = P + ((size_t)c * numnodes + v) * kP16Floats;
+        auto put = [&](int at, float x) {
+            const float hi = tf32_hi(x);
+            p[at] = hi;
+            p[at + 256] = x - hi;
+        };
+        put(p16_at(i, j), up);
+        if (i != j) put(p16_at(j, i), low);
     }
 }
 
