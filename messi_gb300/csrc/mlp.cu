@@ -20,7 +20,7 @@
 // remove the elementwise launches between the GEMMs.
 //
 // Networks whose activations of 16 rows fit half an SM's shared memory (widths
-// up to about 380) run in two kernels instead: mlp_rows_kernel takes 16 rows of
+// up to about 350) run in two kernels instead: mlp_rows_kernel takes 16 rows of
 // the batch through forward, loss and the backward data path, mlp_wgrad_kernel
 // forms all weight and bias gradients.  The GEMM per layer remains for wider
 // networks.

@@ -183,9 +183,16 @@ void level_add(SegLevel* lv, const Segment& sg)
     lv->units += (double)sg.n * (sg.nmat + (sg.root == 0 ? 1 : 0));
 }
 
-// Four pair groups per CTA where the level's pairs alone fill the GPU; below
-// that one pair group per CTA, whose warps share the categories (launch_prune_level).
-void level_shape(SegLevel* lv, bool fuse) { lv->pg = (lv->warps >= 4096 || !fuse) ? 4 : 1; }
+// Four pair groups per CTA, all categories in turn, where the level's pairs alone
+// give the GPU's 152 SMs twelve warps each; below that one pair group per CTA,
+// whose warps share the categories (launch_prune_level).  With the line at 4,096
+// warps a level of 3,803 took 171 us and takes 118, one of 3,344 (a batch) 341 ->
+// 251, the 1,872 of a root segment of 100 sequences 2,107 -> 1,517 (warps that
+// share the categories do not share their matrices in L1); below the line 1,807
+// take 475 us as they are and would take 505, 1,672 399 and 530.
+constexpr int64_t kGroupWarps = 12 * 152;
+
+void level_shape(SegLevel* lv, bool fuse) { lv->pg = (lv->warps >= kGroupWarps || !fuse) ? 4 : 1; }
 
 int build_plan(messi_dataset* ds, const messi_alignment* aln, int W, const uint8_t* pairmask, std::string* err,
                const std::vector<int2>* pairs, std::vector<int32_t>* pair_unique)
