@@ -40,11 +40,17 @@ WORKLOAD_TEXT = {"c2": "c2: 64 seqs x 1,000 nt, max pair span 500",
                  "c4": "c4: 30 seqs x 9,000 nt, max pair span 800",
                  "c4p": "c4p: 8 seqs x 9,000 nt, max pair span 800",
                  "c1": "c1: 16 seqs x 120 nt, all pairs"}
-BYTES_PER_UPDATE = 212  # algorithmic bytes of one node update (2 child rows + exps + indices in, 1 row out)
+# One node update as the kernel does it: a 16 x 16 mat-vec as three TF32
+# products of the split operands.
+FLOPS_PER_UPDATE = 3 * 512
+# TF32 rate of mma.sync on GB300: 8.5 cycles per m16n8k8 (2,048 flops) and SM
+# quarter, measured, at 152 SMs and 1.93 GHz; a tcgen05 GEMM reaches half of
+# the measured BF16 rate.
+MMA_SYNC_TF32_TFLOPS = 283.0
 # DRAM bytes (read + write) per node update of the pruning kernel from one ncu
-# capture of the c2-shaped profiling case, averaged over two interior-level
-# launches (profiles/prune_msg_kernel_c2p.md); scaled by updates per launch.
-TRAFFIC_BYTES_PER_UPDATE = 118.3
+# capture of all launches of one evaluation of the c2-shaped profiling case
+# (profiles/prune_path_kernel_c2p.md); scaled by updates per launch.
+TRAFFIC_BYTES_PER_UPDATE = 20.0
 
 
 def measured_peaks():
@@ -54,6 +60,14 @@ def measured_peaks():
         return float(d["hbm_gbs"]), "measured"
     except Exception:
         return 6800.0, "fallback"
+
+
+def measured_tf32():
+    try:
+        with open(os.path.join(ROOT, "MEASURED_PEAKS.json")) as f:
+            return 0.5 * float(json.load(f)["bf16_tflops"]), "measured"
+    except Exception:
+        return 950.0, "fallback"
 
 
 class Clocks:
@@ -422,15 +436,18 @@ def run_ours(args):
     s_ms, s_n, s_cells = ctx.profile_read(2)
     ctx.profile(False)
     peak, peak_kind = measured_peaks()
-    achieved = (p_units * BYTES_PER_UPDATE / 1e9) / (p_ms / 1e3) if p_ms > 0 else None
+    tf32_peak, tf32_kind = measured_tf32()
+    achieved = (p_units * FLOPS_PER_UPDATE / 1e12) / (p_ms / 1e3) if p_ms > 0 else None
     units_per_launch = p_units / p_n if p_n else None
     roofline = {
-        "bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
-        "frac": (achieved / peak) if achieved else None,
+        "bound": "tensor", "achieved": achieved, "peak": tf32_peak, "unit": "TFLOP/s",
+        "frac": (achieved / tf32_peak) if achieved else None,
+        "mma_sync_peak": MMA_SYNC_TF32_TFLOPS, "mma_sync_frac": (achieved / MMA_SYNC_TF32_TFLOPS) if achieved else None,
+        "hbm_frac": (TRAFFIC_BYTES_PER_UPDATE * p_units / 1e9) / (p_ms / 1e3) / peak if p_ms > 0 else None,
         "traffic": (TRAFFIC_BYTES_PER_UPDATE * units_per_launch) if (TRAFFIC_BYTES_PER_UPDATE and units_per_launch)
         else None,
-        "kernel": "prune_msg_kernel", "peak_source": f"{peak_kind} hbm_gbs",
-        "bytes_per_unit": BYTES_PER_UPDATE, "unit_name": "node update (pair x category x internal node)",
+        "kernel": "prune_path_kernel", "peak_source": f"half of the {tf32_kind} bf16_tflops; {peak_kind} hbm_gbs",
+        "flops_per_unit": FLOPS_PER_UPDATE, "unit_name": "node update (pair x category x internal node)",
         "units_per_launch": units_per_launch, "launches": p_n, "avg_launch_ms": p_ms / p_n if p_n else None,
         "kernel_ms_per_step": p_ms / nprof,
     }
@@ -668,7 +685,7 @@ def run_batch(args):
             "graph_replays_in_timed_steps": batch_replays, "launch_shapes": shapes,
             "max_rel_diff_vs_sequential": rel, "plan_seconds": t_plan, "synth_seconds": t_synth, "stats": st,
             "kernels": {"prune_ms": p_ms, "prune_updates": p_units, "inside_ms": i_ms, "inside_cells": i_cells,
-                        "prune_GBps_algorithmic": (p_units * BYTES_PER_UPDATE / 1e9) / (p_ms / 1e3) if p_ms else None},
+                        "prune_tf32_tflops": (p_units * FLOPS_PER_UPDATE / 1e12) / (p_ms / 1e3) if p_ms else None},
             "clocks": clk.summary()}
     print(json.dumps(line), flush=True)
 

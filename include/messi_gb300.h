@@ -89,8 +89,9 @@ int messi_ctx_graph_replays(messi_ctx* ctx, int64_t* replays);
 /* Launch shapes of the last likelihood evaluation (no counterpart in the
  * reference): the pruning shape (0 = 32 pairs per warp, 20 warps per
  * SM, 1 = 16 warps, 2 = 64 pairs per warp, 12 warps; 3 = the interior levels
- * in the tcgen05 form, chosen only by MESSI_PRUNE_SHAPE=3) and the wavefront CTA size (0 = chosen by band size),
- * and how many workloads have finished autotuning.  The first four
+ * in the tcgen05 form, chosen only by MESSI_PRUNE_SHAPE=3) and the wavefront
+ * CTA size (0 = chosen by the rows per CTA), and how many workloads have
+ * finished autotuning.  The first four
  * evaluations of a dataset (or batch) at a category count try candidate
  * shapes, timed with CUDA events, and later ones use the fastest
  * (MESSI_AUTOTUNE=0 at context creation turns this off; MESSI_PRUNE_SHAPE or
@@ -139,7 +140,8 @@ int messi_dataset_destroy(messi_dataset* ds);
  * values (the reference's Julia matrix). */
 int messi_subcolumnrefs(messi_ctx* ctx, messi_dataset* ds, int32_t* subcolumnrefs);
 /* Plan statistics: out[0] pairs in band, [1] unique root pairs, [2] node
- * updates per category executed (sum over internal nodes of unique pairs),
+ * updates per category executed (unique pairs summed over internal nodes, a
+ * node that is recomputed for its ancestor's pairs counted with those),
  * [3] naive node updates per category (pairs x internal nodes), [4] tree
  * levels, [5] partial-buffer rows per category, [6] categories per pass.
  * n = number of entries wanted (<= 7). */
