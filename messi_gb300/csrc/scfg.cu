@@ -38,7 +38,6 @@
 // CTA in blocks of 32 cells: the terms that reach outside the block are
 // summed by 32 warps in parallel, the in-block triangle by one warp.
 #include <algorithm>
-#include <array>
 #include <cmath>
 
 #include "internal.h"
@@ -1709,8 +1708,47 @@ static int wave_grid(messi_ctx* ctx)
     return ctx->wave_ctas > 0 ? std::min(sms, ctx->wave_ctas) : std::max(sms, 1);
 }
 
+// Tables to be filled with kUnwritten before a wavefront launch, and its status
+// words cleared, in one launch (a memset each: four or six launches, 6-10 us of
+// a small alignment's pass).
+struct WaitTables {
+    float* cells[5] = {};
+    size_t n[5] = {};  // multiples of 4
+};
+
+__global__ void __launch_bounds__(256) wait_tables_kernel(WaitTables w, unsigned int* sync)
+{
+    if (blockIdx.x == 0 && threadIdx.x < kSyncWords) sync[threadIdx.x] = 0u;
+    const uint4 v = make_uint4(kUnwritten, kUnwritten, kUnwritten, kUnwritten);
+    for (int k = 0; k < 5; k++) {
+        uint4* c = reinterpret_cast<uint4*>(w.cells[k]);
+        for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < w.n[k] / 4; i += (size_t)gridDim.x * blockDim.x)
+            c[i] = v;
+    }
+}
+
+static int launch_wait_tables(messi_ctx* ctx, const WaitTables& w, unsigned int* sync)
+{
+    size_t total = 0;
+    bool aligned = true;
+    for (int k = 0; k < 5; k++) {
+        total += w.n[k];
+        aligned = aligned && ((uintptr_t)w.cells[k] & 15) == 0 && w.n[k] % 4 == 0;
+    }
+    if (!aligned) {
+        cudaError_t e = cudaMemsetAsync(sync, 0, kSyncWords * sizeof(unsigned int), ctx->stream);
+        for (int k = 0; k < 5 && e == cudaSuccess; k++)
+            if (w.n[k]) e = cudaMemsetAsync(w.cells[k], 0xff, w.n[k] * sizeof(float), ctx->stream);
+        return e == cudaSuccess ? MESSI_OK : cuda_fail(ctx, e, "wavefront table reset");
+    }
+    const int grid = (int)std::max<size_t>(1, std::min<size_t>(total / 4 / 256, 152 * 8));
+    wait_tables_kernel<<<grid, 256, 0, ctx->stream>>>(w, sync);
+    LAUNCH_CHECK(ctx, "wait_tables_kernel");
+    return MESSI_OK;
+}
+
 // The inside kernel (cooperative: every CTA resident), one CTA per SM, after
-// the tables it waits on are filled with kUnwritten (each: first cell, cells).
+// the tables it waits on are filled with kUnwritten.
 // 512 threads (1,024 leave 64 registers a thread and spill: span 500 of 1,000
 // columns 0.67 ms against 0.54); 256 where a CTA has at most two cells of a
 // diagonal and four warps form their sums (L = 120: 93 us against 102, L = 300:
@@ -1721,12 +1759,9 @@ static int wave_grid(messi_ctx* ctx)
 // 13 cells: 3.98 against 3.39; the batch, which needs more registers, 1.34
 // against 1.23).
 static int launch_inside(messi_ctx* ctx, const void* kernel, const void* many, void** args, unsigned int* sync,
-                         long long columns, std::array<std::pair<float*, size_t>, 3> cells)
+                         long long columns, const WaitTables& tables)
 {
-    cudaError_t e = cudaMemsetAsync(sync, 0, kSyncWords * sizeof(unsigned int), ctx->stream);
-    for (int k = 0; k < 3 && e == cudaSuccess; k++)
-        if (cells[k].second) e = cudaMemsetAsync(cells[k].first, 0xff, cells[k].second * sizeof(float), ctx->stream);
-    if (e != cudaSuccess) return cuda_fail(ctx, e, "inside table reset");
+    if (const int rc = launch_wait_tables(ctx, tables, sync)) return rc;
     const int most = wave_grid(ctx);  // also sets ctx->num_sms
     const int grid = (int)std::min<long long>(most, columns);
     int threads = columns <= 2 * (long long)ctx->num_sms ? kInsideThreads / 2 : kInsideThreads;
@@ -1736,7 +1771,7 @@ static int launch_inside(messi_ctx* ctx, const void* kernel, const void* many, v
         kernel = many;
         threads = kInsideManyThreads;
     }
-    e = cudaLaunchCooperativeKernel(kernel, dim3(grid), dim3(threads), args, 0, ctx->stream);
+    const cudaError_t e = cudaLaunchCooperativeKernel(kernel, dim3(grid), dim3(threads), args, 0, ctx->stream);
     ctx->launches++;
     return e == cudaSuccess ? MESSI_OK : cuda_fail(ctx, e, "inside_pair_kernel");
 }
@@ -1777,18 +1812,16 @@ int queue_status_readback(messi_ctx* ctx, const Band& t)
 // 600) and 1,217, 1,175, 1,065 with 7 (span 500 of 1,000).
 static int launch_outside(messi_ctx* ctx, const Band& t, void** args, unsigned int* sync)
 {
-    cudaError_t e = cudaMemsetAsync(sync, 0, kSyncWords * sizeof(unsigned int), ctx->stream);
-    const size_t tab = (size_t)t.L * t.RS * sizeof(float);
-    for (float* cells : {t.OSrow, t.OScol, t.OFrow, t.OFcol, t.OLrow})
-        if (e == cudaSuccess) e = cudaMemsetAsync(cells, 0xff, tab, ctx->stream);
-    if (e != cudaSuccess) return cuda_fail(ctx, e, "outside table reset");
+    const size_t tab = (size_t)t.L * t.RS;
+    const WaitTables tables{{t.OSrow, t.OScol, t.OFrow, t.OFcol, t.OLrow}, {tab, tab, tab, tab, tab}};
+    if (const int rc = launch_wait_tables(ctx, tables, sync)) return rc;
     const void* kernel = (const void*)outside_pair_kernel<1024>;
     const int grid = std::min(wave_grid(ctx), t.L);
     const int rows = (t.L + grid - 1) / grid;
     int threads = ctx->wave_threads ? ctx->wave_threads : (rows <= 2 ? 512 : (rows <= 5 ? 768 : 1024));
     if (threads <= 512) kernel = (const void*)outside_pair_kernel<512>;
     else if (threads == 768) kernel = (const void*)outside_pair_kernel<768>;
-    e = cudaLaunchCooperativeKernel(kernel, dim3(grid), dim3(threads), args, 0, ctx->stream);
+    const cudaError_t e = cudaLaunchCooperativeKernel(kernel, dim3(grid), dim3(threads), args, 0, ctx->stream);
     ctx->launches++;
     return e == cudaSuccess ? MESSI_OK : cuda_fail(ctx, e, "outside_pair_kernel");
 }
@@ -1804,7 +1837,7 @@ int run_inside(messi_ctx* ctx, const Band& t, double B)
     prof_begin(ctx, 1, (double)t.L * (t.Wb + 1) - 0.5 * t.Wb * (t.Wb + 1.0));
     int rc = launch_inside(ctx, (const void*)inside_pair_kernel<false, kInsideThreads>,
                            (const void*)inside_pair_kernel<false, kInsideManyThreads>, args, sync, t.L,
-                           {{{t.Lrow, tab}, {t.Scol, tab}, {t.Frow, tab}}});
+                           WaitTables{{t.Lrow, t.Scol, t.Frow}, {tab, tab, tab}});
     if (rc) return rc;
     prof_end(ctx);
     if (t.L - 1 > t.Wb) {
@@ -1946,7 +1979,7 @@ int run_inside_batch(messi_ctx* ctx, const BandBatch& bb, double B)
     for (const Band& t : bb.host) cells += (double)t.L * (t.Wb + 1) - 0.5 * t.Wb * (t.Wb + 1.0);
     prof_begin(ctx, 1, cells);
     int rc = launch_inside(ctx, (const void*)inside_pair_kernel<true, kInsideThreads>, nullptr, args, sync, bb.total_cols,
-                           {{{bb.host[0].Lrow, bb.polled}, {nullptr, 0}, {nullptr, 0}}});
+                           WaitTables{{bb.host[0].Lrow}, {bb.polled}});
     if (rc) return rc;
     cudaError_t e;
     prof_end(ctx);
