@@ -30,6 +30,7 @@
 #include <climits>
 #include <cmath>
 
+#include "decode_schedule.h"
 #include "internal.h"
 #include "wave.cuh"
 
@@ -75,14 +76,18 @@ __global__ void to_double_kernel(const float* __restrict__ in, double* __restric
 // them in the order of the tile diagonals D = J - I.  Tile (I, J) needs row
 // block I + 1 up to diagonal D - 1, which needed row block I + 2 up to D - 2,
 // and so on: a CTA publishes its row block's finished diagonals in a flag
-// (release) and waits for its neighbour's alone (acquire, bounded), not for a
-// grid barrier.  Row index r = k + 1 of the second factor:
+// (release) and waits for the flags of the row blocks it reads next (acquire,
+// bounded; decode_schedule.h), not for a grid barrier.  Row index r = k + 1 of
+// the second factor:
 //   * r in a block R strictly between I and J: both factors lie in finished
 //     tiles.  Sixteen groups of 64 threads take every sixteenth R; a thread
 //     keeps four cells of the tile and reads e(r, j) from L2 once for all four,
-//     a(i, .) from shared memory.  R = I + 1 and I + 2 may still be in the
-//     making when the CTA starts the tile, so they come after the wait and the
-//     rest before it;
+//     a(i, .) from shared memory.  R = I + 1 and I + 2 are usually still in the
+//     making when the CTA starts the tile, so they come after the wait for row
+//     block I + 1 and the rest before it, behind row block I + 3 up to diagonal
+//     D - 3.  That is usually long done, and one thread without cells has seen it
+//     during the tile before (a look by every warp at the start of the tile
+//     instead: 0.66 ms at L = 1,000);
 //   * r in I or J: the factors lie in the tile itself (and in the two diagonal
 //     tiles).  A thread per cell; the cells become final along the 31
 //     anti-diagonals from the lower left corner, and in every step each cell
@@ -91,7 +96,7 @@ __global__ void to_double_kernel(const float* __restrict__ in, double* __restric
 //     stores inside, a step took 530 cycles).
 // Bound by the chain of L/16 waits and 31 steps each; a wavefront with one
 // grid barrier per two diagonals of cells took 3.61 ms at L = 1,000, this takes
-// 0.60 ms.
+// 0.63 ms.
 // ---------------------------------------------------------------------------
 constexpr int kDT = 16;          // cells per tile side
 constexpr int kDThreads = 1024;  // 16 groups of 64 threads
@@ -105,29 +110,36 @@ struct DecodeSmem {
     float at[kDT][kDT + 2];      // a of the tile: column J*16 - 1 at 0
     float bv[kDGroups][kDT * kDT];
     int bk[kDGroups][kDT * kDT];
+    DecodeWait seen;             // a flag and its value, seen during the tile before
 };
 
-// Waits (whole CTA) until flag >= want; false once any CTA has given up
+// Waits (one thread) until the flag is raised; false once any CTA has given up
 // waiting (sync[2], the host's error flag).
-__device__ bool flag_wait(const unsigned int* flag, unsigned int want, unsigned int* sync)
+__device__ bool flag_look(const unsigned int* flags, DecodeWait w, unsigned int* sync)
+{
+    unsigned int spins = 0;
+    while (ld_acquire_u32(flags + w.block) < (unsigned)w.diagonals)
+        if (!keep_waiting(spins, sync)) return false;
+    return true;
+}
+
+// The whole CTA.
+__device__ bool flag_wait(const unsigned int* flags, DecodeWait w, unsigned int* sync)
 {
     __shared__ int s_ok;
     __syncthreads();
-    if (threadIdx.x == 0) {
-        unsigned int spins = 0;
-        bool ok = true;
-        while (ld_acquire_u32(flag) < want) {
-            if (++spins > kSpinLimit || ((spins & 1023u) == 0u && ld_acquire_u32(&sync[2]) != 0u)) {
-                atomicExch(&sync[2], 1u);
-                ok = false;
-                break;
-            }
-            if (spins > 64u) __nanosleep(32);
-        }
-        s_ok = ok;
-    }
+    if (threadIdx.x == 0) s_ok = flag_look(flags, w, sync);
     __syncthreads();
     return s_ok != 0;
+}
+
+// A warp, apart from the others.
+__device__ __forceinline__ bool flag_wait_warp(const unsigned int* flags, DecodeWait w, unsigned int* sync)
+{
+    bool ok = true;
+    if ((threadIdx.x & 31) == 0) ok = flag_look(flags, w, sync);
+    __syncwarp();  // the other lanes' reads behind lane 0's look
+    return __all_sync(0xffffffffu, ok);
 }
 
 __device__ __forceinline__ void flag_set(unsigned int* flag, unsigned int v)
@@ -205,6 +217,8 @@ __global__ void __launch_bounds__(kDThreads) decode_tile_kernel(const float* __r
     }
     // phase 1: this thread's cells are (a0 + 4m, b)
     const int grp = tid >> 6, b1 = tid & 15, a0 = (tid >> 4) & 3;
+    bool lost = false;  // this warp has given up waiting
+    DecodeWait seen{-1, 0};
     for (int D = 1; D < NB; D++) {
         for (int I = blockIdx.x; I + D < NB; I += gridDim.x) {
             const int J = I + D;
@@ -241,8 +255,13 @@ __global__ void __launch_bounds__(kDThreads) decode_tile_kernel(const float* __r
                                        r - 1 + (v[0] == best ? 0 : (v[1] == best ? 1 : (v[2] == best ? 2 : 3))));
                     }
             };
-            for (int R = I + 3 + grp; R < J; R += kDGroups) block(R * kDT, 4);
-            if (!flag_wait(flags + I + 1, (unsigned)D, sync)) return;
+            const int R0 = decode_early_first(I) + grp;
+            const DecodeWait early = decode_early_wait(I, D);
+            // (a warp that has given up goes on: the launch is marked as failed)
+            if (R0 < J && !(seen.block == early.block && seen.diagonals >= early.diagonals) && !lost)
+                lost = !flag_wait_warp(flags, early, sync);
+            for (int R = R0; R < J; R += kDGroups) block(R * kDT, 4);
+            if (!flag_wait(flags, decode_late_wait(I, D), sync)) return;
             // cell (a, b) of this thread in the tile, and what it needs from the neighbouring tiles
             const int a = tid >> 4, b = tid & 15, i = I * kDT + a, j = J * kDT + b;
             const int jc = min(j, L - 1);
@@ -312,8 +331,15 @@ __global__ void __launch_bounds__(kDThreads) decode_tile_kernel(const float* __r
                     A[(size_t)i * L + j] = e2;
                     if (ROWS) arow[a * astride + j + 1] = e2;
                 }
+            } else if (tid == 256) {
+                // what the CTA's next tile waits for first
+                const bool more = I + (int)gridDim.x + D < NB;
+                const int next = more ? I + (int)gridDim.x : (int)blockIdx.x;
+                const int block = min(decode_early_wait(next, more ? D : D + 1).block, NB - 1);
+                S.seen = DecodeWait{block, (int)ld_acquire_u32(flags + block)};
             }
             flag_set(flags + I, (unsigned)D + 1u);
+            seen = S.seen;  // (written again behind the next tile's barriers)
             // what no other tile reads, while the others' values arrive: the
             // column-major copy and the traceback codes
             if (tid < 256 && j < L) {
