@@ -5,6 +5,8 @@
 #include <cstdlib>
 #include <cstddef>
 #include <cstring>
+#include <map>
+#include <mutex>
 #include <new>
 
 #include "internal.h"
@@ -59,6 +61,17 @@ int ensure_pinned(messi_ctx* ctx, size_t bytes, void** p)
     }
     *p = ctx->pinned;
     return MESSI_OK;
+}
+
+cudaError_t allow_smem(int device, const void* kernel, size_t bytes)
+{
+    static std::mutex mu;
+    static std::map<std::pair<const void*, int>, size_t> most;
+    std::lock_guard<std::mutex> lock(mu);
+    size_t& m = most[std::make_pair(kernel, device)];
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)std::max(m, bytes));
+    if (e == cudaSuccess) m = std::max(m, bytes);
+    return e;
 }
 
 static cudaEvent_t prof_event(messi_ctx* ctx)

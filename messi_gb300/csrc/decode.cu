@@ -618,7 +618,7 @@ int run_posterior_decoding(messi_ctx* ctx, int L, const double* d_single, const 
         const bool rows = grid == NB && bytes <= (size_t)160 * 1024;
         const void* kernel = rows ? (const void*)decode_tile_kernel<true> : (const void*)decode_tile_kernel<false>;
         if (rows) {
-            e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+            e = allow_smem(ctx->device, kernel, bytes);
             if (e != cudaSuccess) return cuda_fail(ctx, e, "decode_tile_kernel attributes");
         }
         void* args[] = {(void*)&f_single, (void*)&f_pair, &Lv, (void*)&a, &erow, &ecol, &d_scol, &astride, &d_sync, &d_flags};

@@ -333,6 +333,11 @@ int fail(messi_ctx* ctx, int code, const std::string& msg);
 int cuda_fail(messi_ctx* ctx, cudaError_t e, const char* what);
 int ensure(messi_ctx* ctx, int slot, size_t bytes, void** p);
 int ensure_pinned(messi_ctx* ctx, size_t bytes, void** p);
+// Lets launches of `kernel` on the current device use that much dynamic shared
+// memory.  The limit belongs to the kernel on the device, whichever thread or
+// context set it, so it only grows: a smaller call of another thread between
+// this one's and its launch takes nothing away.
+cudaError_t allow_smem(int device, const void* kernel, size_t bytes);
 // Start of every entry point (device, counters) and its end (stream sync, status checks).
 int begin(messi_ctx* ctx);
 int finish(messi_ctx* ctx);

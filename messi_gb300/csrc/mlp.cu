@@ -890,7 +890,7 @@ static int fused_rows(messi_ctx* ctx, messi_mlp* m, int batch, bool grad)
 {
     const size_t smem = rows_layout(m->in, m->H, m->out, m->D, grad).total;
     const void* kernel = grad ? (const void*)mlp_rows_kernel<true> : (const void*)mlp_rows_kernel<false>;
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const cudaError_t e = allow_smem(ctx->device, kernel, smem);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "mlp_rows_kernel attributes");
     // the gradients' operands are whole groups of 32 rows
     const int grid = grad ? pad32(batch) / kRows : (batch + kRows - 1) / kRows;

@@ -1074,13 +1074,8 @@ static int launch_path(messi_ctx* ctx, const SegDev* d_segs, const int2* d_tiles
     const size_t smem = sizeof(float4) * ((size_t)(lv.max_nb + 1) * (1 + 8 * lv.pg) + (lv.max_steps + 1) / 2 +
                                           (size_t)warps * NP * lv.max_depth * 128) +
                         (ROOT == 2 && ctas == 1 ? sizeof(double) * 32 * (size_t)lv.pg * nc : 0);
-    static thread_local std::pair<int, size_t> granted{-1, 0};
-    if (granted.first != ctx->device || granted.second < smem) {
-        cudaError_t e = cudaFuncSetAttribute(prune_path_kernel<ROOT, NP, MAXT, MINB>,
-                                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return cuda_fail(ctx, e, "prune_path_kernel attributes");
-        granted = {ctx->device, smem};
-    }
+    const cudaError_t e = allow_smem(ctx->device, (const void*)prune_path_kernel<ROOT, NP, MAXT, MINB>, smem);
+    if (e != cudaSuccess) return cuda_fail(ctx, e, "prune_path_kernel attributes");
     prune_path_kernel<ROOT, NP, MAXT, MINB><<<dim3(lv.tile_cnt, ctas), 32 * warps, smem, ctx->stream>>>(
         d_segs, d_tiles + lv.tile_off, d_P, numnodes, c0, nc, C, d_pi16, d_logw, d_lam, per_lambda ? 1 : 0, cs,
         lv.max_steps, lv.max_nb, lv.max_depth, shared_values);

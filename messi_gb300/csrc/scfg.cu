@@ -714,17 +714,6 @@ static int suffix_batch_window(const BandBatch& bb)
     return win;
 }
 
-static cudaError_t suffix_smem_attr(int win)
-{
-    const int bytes = 2 * win * (int)sizeof(float);
-    cudaError_t e = cudaFuncSetAttribute(inside_suffix_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         std::max(bytes, 0));
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(inside_suffix_batch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 std::max(bytes, 0));
-    return e;
-}
-
 __global__ void finish_Z_kernel(Band t)
 {
     if (threadIdx.x == 0 && blockIdx.x == 0)
@@ -1843,7 +1832,7 @@ int run_inside(messi_ctx* ctx, const Band& t, double B)
     if (t.L - 1 > t.Wb) {
         prof_begin(ctx, 2, (double)(t.L - 1 - t.Wb));
         const int win = suffix_launch_window(t.Wb);
-        cudaError_t e = suffix_smem_attr(win);
+        const cudaError_t e = allow_smem(ctx->device, (const void*)inside_suffix_kernel, (size_t)2 * win * sizeof(float));
         if (e != cudaSuccess) return cuda_fail(ctx, e, "inside_suffix_kernel attributes");
         inside_suffix_kernel<<<1, kSuffixThreads, (size_t)2 * win * sizeof(float), ctx->stream>>>(t, R, win);
         LAUNCH_CHECK(ctx, "inside_suffix_kernel");
@@ -1985,7 +1974,7 @@ int run_inside_batch(messi_ctx* ctx, const BandBatch& bb, double B)
     prof_end(ctx);
     prof_begin(ctx, 2, 0.0);
     const int win = suffix_batch_window(bb);
-    e = suffix_smem_attr(win);
+    e = allow_smem(ctx->device, (const void*)inside_suffix_batch_kernel, (size_t)2 * win * sizeof(float));
     if (e != cudaSuccess) return cuda_fail(ctx, e, "inside_suffix_batch_kernel attributes");
     inside_suffix_batch_kernel<<<n, kSuffixThreads, (size_t)2 * win * sizeof(float), ctx->stream>>>(bands, R, win);
     LAUNCH_CHECK(ctx, "inside_suffix_batch_kernel");
@@ -2193,8 +2182,7 @@ int run_outside(messi_ctx* ctx, const Band& t, double B)
     Rules R = make_rules(B);
     if (t.L - 1 > t.Wb) {
         const int win = suffix_launch_window(t.Wb);
-        cudaError_t e = cudaFuncSetAttribute(outside_suffix_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             2 * win * (int)sizeof(float));
+        const cudaError_t e = allow_smem(ctx->device, (const void*)outside_suffix_kernel, (size_t)2 * win * sizeof(float));
         if (e != cudaSuccess) return cuda_fail(ctx, e, "outside_suffix_kernel attributes");
         outside_suffix_kernel<<<1, kSuffixThreads, (size_t)2 * win * sizeof(float), ctx->stream>>>(t, R, win);
         LAUNCH_CHECK(ctx, "outside_suffix_kernel");
