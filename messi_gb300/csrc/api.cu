@@ -486,6 +486,8 @@ int messi_ctx_create(int device, messi_ctx** out)
             ctx->wave_threads = std::atoi(wt);
             ctx->fixed_wave = true;
         }
+        const char* sw = std::getenv("MESSI_SUFFIX_WINDOW");
+        if (sw) ctx->suffix_window = std::max(0, std::min(std::atoi(sw), kSuffixMaxWindow));
         const char* gr = std::getenv("MESSI_GRAPHS");
         if (gr && std::atoi(gr) == 0) ctx->graphs = false;
         const char* ps = std::getenv("MESSI_PRUNE_SHAPE");

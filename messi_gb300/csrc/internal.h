@@ -21,6 +21,7 @@ constexpr int kTile = 128;          // unique pairs per CTA in the pruning kerne
 constexpr int kSyncWords = 4;
 constexpr int kMaxLambda = 8;       // per-lambda conditionals kept in registers
 constexpr int kMaxStack = 512;      // tree height limit
+constexpr int kSuffixMaxWindow = 24576;  // cells of the suffix kernels' shared-memory window (192 KB)
 constexpr int kSlotUnpaired = 20;   // scratch slot of the per-site unpaired log-likelihoods
 constexpr int kSlotPlan = 26;       // of the plan of one structure's pairs
 constexpr int kSlotPlanRows = 27;   // of its message arena: rows, then exponents
@@ -237,6 +238,9 @@ struct messi_ctx {
     // sequences) and their size (256, 512 or 1024 threads; 0 = by band size)
     int wave_ctas = 0;
     int wave_threads = 0;
+    // largest shared-memory window of the suffix kernels, cells (env
+    // MESSI_SUFFIX_WINDOW: less, down to 0); wider bands take their pull form
+    int suffix_window = messi::kSuffixMaxWindow;
     // pruning launch shape: 0 = 32 pairs per warp, 20 warps/SM, 1 = 16
     // warps/SM, 2 = 64 pairs per warp, 12 warps/SM, 3 = tcgen05 form
     int prune_shape = 0;

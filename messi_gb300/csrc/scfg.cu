@@ -35,8 +35,8 @@
 // reduced by a group of G lanes (G grows with the number of split points) with
 // shuffle log-sum-exp; its middle split points, which do not read the diagonals
 // just finished, are summed one pair ahead.  The suffix recurrences run in one
-// CTA in blocks of 32 cells: the terms that reach outside the block are
-// summed by 32 warps in parallel, the in-block triangle by one warp.
+// CTA of 16 warps in blocks of 32 cells: the terms that reach outside the
+// block are summed by its warps in parallel, the in-block triangle by one warp.
 #include <algorithm>
 #include <cmath>
 
@@ -327,7 +327,6 @@ int launch_bandprep_from_dense(messi_ctx* ctx, const Band& t, const double* d_de
 // block's Wb+1 terms per cell from global memory after the block above was
 // final: 2.7 ms for the 8,199 suffix cells of a 9,000-column alignment with
 // span 800.)
-constexpr int kSuffixMaxWindow = 24576;  // cells of the shared-memory window (192 KB)
 // threads of a suffix CTA (16 warps: 128 registers each, so warp 0 keeps its
 // 32 prefetched terms in registers across the triangle)
 constexpr int kSuffixThreads = 512;
@@ -639,14 +638,15 @@ __device__ void inside_suffix_body(const Band& t, const Rules& R, float* am, flo
 __device__ void inside_suffix_body_pull(const Band& t, const Rules& R)
 {
     const int T = t.L - 1 - t.Wb;
-    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
     __shared__ float known[32];
     __shared__ float tri[32][33];  // Lrow[i0 - l][k], k < 32: the in-block terms, read by the serial warp
     for (int i0 = T - 1; i0 >= 0; i0 -= 32) {
         const int lo = max(0, i0 - 31);
-        const int i = i0 - w;
-        tri[w][lane] = (i >= lo && lane <= t.Wb) ? t.Lrow[(size_t)i * t.RS + lane] : -INFINITY;
-        if (i >= lo) {
+        for (int q = w; q < 32; q += nw) {  // a warp per cell i0 - q
+            const int i = i0 - q;
+            tri[q][lane] = (i >= lo && lane <= t.Wb) ? t.Lrow[(size_t)i * t.RS + lane] : -INFINITY;
+            if (i < lo) continue;
             float m = -INFINITY, s = 0.f;
             const float* lrow = t.Lrow + (size_t)i * t.RS;
             int k = (i0 - i) + lane;
@@ -655,7 +655,7 @@ __device__ void inside_suffix_body_pull(const Band& t, const Rules& R)
                          lrow[k + 64] + t.Ssuf[i + k + 65], lrow[k + 96] + t.Ssuf[i + k + 97]);
             for (; k <= t.Wb; k += 32) lse_add(m, s, lrow[k] + t.Ssuf[i + k + 1]);
             group_reduce<32>(m, s);
-            if (lane == 0) known[w] = lse_val(m, s);
+            if (lane == 0) known[q] = lse_val(m, s);
         }
         __syncthreads();
         if (w == 0) {
@@ -697,20 +697,20 @@ __global__ void __launch_bounds__(kSuffixThreads) inside_suffix_batch_kernel(con
 }
 
 // Window for the largest band that needs a suffix (0: none fits, the pull form runs).
-static int suffix_launch_window(int maxWb)
+static int suffix_launch_window(const messi_ctx* ctx, int maxWb)
 {
     const int win = suffix_window(maxWb);
-    return (win <= kSuffixMaxWindow) ? win : 0;
+    return (win <= ctx->suffix_window) ? win : 0;
 }
 
 // The window for a batch: the widest band among those that take the pushing
 // form (a band too wide for any window takes the pull form in a single call
 // too, so both paths give the same bits).
-static int suffix_batch_window(const BandBatch& bb)
+static int suffix_batch_window(const messi_ctx* ctx, const BandBatch& bb)
 {
     int win = 0;
     for (const Band& t : bb.host)
-        if (t.L - 1 > t.Wb && suffix_window(t.Wb) <= kSuffixMaxWindow) win = std::max(win, suffix_window(t.Wb));
+        if (t.L - 1 > t.Wb && suffix_window(t.Wb) <= ctx->suffix_window) win = std::max(win, suffix_window(t.Wb));
     return win;
 }
 
@@ -1831,7 +1831,7 @@ int run_inside(messi_ctx* ctx, const Band& t, double B)
     prof_end(ctx);
     if (t.L - 1 > t.Wb) {
         prof_begin(ctx, 2, (double)(t.L - 1 - t.Wb));
-        const int win = suffix_launch_window(t.Wb);
+        const int win = suffix_launch_window(ctx, t.Wb);
         const cudaError_t e = allow_smem(ctx->device, (const void*)inside_suffix_kernel, (size_t)2 * win * sizeof(float));
         if (e != cudaSuccess) return cuda_fail(ctx, e, "inside_suffix_kernel attributes");
         inside_suffix_kernel<<<1, kSuffixThreads, (size_t)2 * win * sizeof(float), ctx->stream>>>(t, R, win);
@@ -1973,7 +1973,7 @@ int run_inside_batch(messi_ctx* ctx, const BandBatch& bb, double B)
     cudaError_t e;
     prof_end(ctx);
     prof_begin(ctx, 2, 0.0);
-    const int win = suffix_batch_window(bb);
+    const int win = suffix_batch_window(ctx, bb);
     e = allow_smem(ctx->device, (const void*)inside_suffix_batch_kernel, (size_t)2 * win * sizeof(float));
     if (e != cudaSuccess) return cuda_fail(ctx, e, "inside_suffix_batch_kernel attributes");
     inside_suffix_batch_kernel<<<n, kSuffixThreads, (size_t)2 * win * sizeof(float), ctx->stream>>>(bands, R, win);
@@ -2131,14 +2131,15 @@ __device__ void outside_suffix_body(const Band& t, const Rules& R, float* am, fl
 __device__ void outside_suffix_body_pull(const Band& t, const Rules& R)
 {
     const int T = t.L - 1 - t.Wb;
-    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
     __shared__ float known[32];
     __shared__ float tri[32][33];  // Lcol[i0 + l - 1][k], k < 32: the in-block terms
     for (int i0 = 0; i0 < T; i0 += 32) {
         const int hi = min(T - 1, i0 + 31);
-        const int i = i0 + w;
-        tri[w][lane] = (i <= hi && i >= 1 && lane <= t.Wb) ? t.Lcol[(size_t)(i - 1) * t.RS + lane] : -INFINITY;
-        if (i <= hi) {
+        for (int q = w; q < 32; q += nw) {  // a warp per cell i0 + q
+            const int i = i0 + q;
+            tri[q][lane] = (i <= hi && i >= 1 && lane <= t.Wb) ? t.Lcol[(size_t)(i - 1) * t.RS + lane] : -INFINITY;
+            if (i > hi) continue;
             float m = -INFINITY, s = 0.f;
             if (i >= 1) {
                 const float* lcol = t.Lcol + (size_t)(i - 1) * t.RS;
@@ -2150,7 +2151,7 @@ __device__ void outside_suffix_body_pull(const Band& t, const Rules& R)
                 for (; k <= kmax; k += 32) lse_add(m, s, t.Osuf[i - k - 1] + lcol[k]);
             }
             group_reduce<32>(m, s);
-            if (lane == 0) known[w] = lse_val(m, s);
+            if (lane == 0) known[q] = lse_val(m, s);
         }
         __syncthreads();
         if (w == 0) {
@@ -2181,7 +2182,7 @@ int run_outside(messi_ctx* ctx, const Band& t, double B)
 {
     Rules R = make_rules(B);
     if (t.L - 1 > t.Wb) {
-        const int win = suffix_launch_window(t.Wb);
+        const int win = suffix_launch_window(ctx, t.Wb);
         const cudaError_t e = allow_smem(ctx->device, (const void*)outside_suffix_kernel, (size_t)2 * win * sizeof(float));
         if (e != cudaSuccess) return cuda_fail(ctx, e, "outside_suffix_kernel attributes");
         outside_suffix_kernel<<<1, kSuffixThreads, (size_t)2 * win * sizeof(float), ctx->stream>>>(t, R, win);
