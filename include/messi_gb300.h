@@ -100,8 +100,9 @@ int messi_ctx_launch_shapes(messi_ctx* ctx, int32_t* prune_shape, int32_t* wave_
 /* Text of the last error recorded on this context. */
 const char* messi_ctx_last_error(messi_ctx* ctx);
 /* Self-test of the bounded device waits (no counterpart in the reference):
- * launches a wait for a table cell that nothing writes, which gives up after
- * a few milliseconds and raises the error flag.
+ * launches a warp's wait for a table cell that nothing writes, which gives up
+ * after a few milliseconds and raises the error flag (MESSI_ESTATE if its
+ * lanes did not leave together).
  * *status receives the status such a wait produces (MESSI_ETIMEOUT when the
  * mechanism works); the call itself returns MESSI_OK and leaves the context
  * usable. */

@@ -570,12 +570,14 @@ int messi_selftest_bounded_wait(messi_ctx* ctx, int32_t* status)
     if (rc) return rc;
     if (!status) return fail(ctx, MESSI_EINVAL, "bounded-wait self-test: null argument");
     void* p;
-    if ((rc = ensure(ctx, kSlotVec, kSyncWords * sizeof(unsigned int), &p))) return rc;
-    unsigned int flag = 0;
+    if ((rc = ensure(ctx, kSlotVec, kSelftestWords * sizeof(unsigned int), &p))) return rc;
+    unsigned int words[kSelftestWords] = {};
     if ((rc = launch_wait_selftest(ctx, (unsigned int*)p))) return rc;
-    if ((rc = d2h(ctx, &flag, (unsigned int*)p + 2, sizeof(unsigned int)))) return rc;
+    if ((rc = d2h(ctx, words, p, sizeof(words)))) return rc;
     if ((rc = finish(ctx))) return rc;
-    *status = flag ? MESSI_ETIMEOUT : MESSI_OK;
+    *status = words[2] ? MESSI_ETIMEOUT : MESSI_OK;
+    for (int lane = 1; lane < 32; lane++)
+        if (words[2 * kSyncWords + lane] != words[2 * kSyncWords]) *status = MESSI_ESTATE;  // lanes left apart
     return MESSI_OK;
 }
 

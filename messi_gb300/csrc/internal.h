@@ -448,8 +448,10 @@ struct SideLaunches {
     ~SideLaunches() { ctx->stream = main; }
 };
 
-// Bounded-wait self-test (scfg.cu): a wait for a cell that nothing writes;
-// d_sync[2] becomes 1 when it gives up.
+// Bounded-wait self-test (scfg.cu): a warp's wait for a cell that nothing writes;
+// d_sync[2] becomes 1 when it gives up.  d_sync: two sets of status words, then the
+// looks that each of the 32 lanes took until one of them saw another's failure.
+constexpr int kSelftestWords = 2 * kSyncWords + 32;
 int launch_wait_selftest(messi_ctx* ctx, unsigned int* d_sync);
 // Dense L x L pair matrix: vals (nullable) of the unique root pairs, mixed with
 // addw + u[x] + u[y] when addw is finite (the factorised lambda categories).

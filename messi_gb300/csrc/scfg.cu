@@ -914,7 +914,7 @@ __device__ __forceinline__ bool outer_wait(const Band& t, int i, int d, bool min
         if (mine) outer_load<N>(t, i, d, o);
         mine = mine && !o.complete();
         if (!__any_sync(0xffffffffu, mine)) return true;
-        if (!keep_waiting(spins, sync)) return false;
+        if (!warp_keep_waiting(spins, sync)) return false;
     }
 }
 
@@ -1079,7 +1079,7 @@ __global__ void __launch_bounds__(MAXT) inside_pair_kernel(InsideBands<BATCH> ib
                      float& s) {
         unsigned int spins = 0;
         for (bool there = false; !there;) {
-            bad = __any_sync(0xffffffffu, !keep_waiting(spins, sync)) || bad;
+            bad = !warp_keep_waiting(spins, sync) || bad;
             if (bad) break;
             if (own_nan || (spins & 63u) == 0u) {
                 bool missing = false;
@@ -1575,7 +1575,7 @@ __global__ void __launch_bounds__(MAXT) outside_pair_kernel(Band t, Rules R, uns
                 c = outside_sum(g, 2 + x, valid, lane, G, R);
                 if (there || !__any_sync(0xffffffffu, valid && c.y != c.y)) break;
                 // a NaN: again, as in the inside pass
-                bad = __any_sync(0xffffffffu, !keep_waiting(spins, sync)) || bad;
+                bad = !warp_keep_waiting(spins, sync) || bad;
                 if (bad) break;
                 if (own_nan || (spins & 63u) == 0u) {
                     bool missing = false;
@@ -1597,7 +1597,7 @@ __global__ void __launch_bounds__(MAXT) outside_pair_kernel(Band t, Rules R, uns
             if (mine) load();
             mine = mine && !complete();
             if (!__any_sync(0xffffffffu, mine)) return;
-            if (!keep_waiting(spins, sync)) {
+            if (!warp_keep_waiting(spins, sync)) {
                 bad = true;
                 return;
             }
@@ -1765,23 +1765,31 @@ static int launch_inside(messi_ctx* ctx, const void* kernel, const void* many, v
     return e == cudaSuccess ? MESSI_OK : cuda_fail(ctx, e, "inside_pair_kernel");
 }
 
-// Self-test of the bounded wait: one thread waits for a cell (sync[3]) that
-// nothing writes, gives up after `limit` looks, raises the error flag (sync[2])
-// and returns.  Nothing faults and nothing waits unboundedly; the context stays
-// usable.
-__global__ void wait_selftest_kernel(unsigned int* sync, unsigned int limit)
+// Self-test of the bounded wait: a warp waits for a cell (sync[3]) that nothing
+// writes.  First lane 0 alone sees an error flag that is up (its status words are
+// the second set): all lanes have to leave at the look that finds it; the looks
+// of every lane are left behind the two sets.  Then the wait gives up after
+// `limit` looks and raises the flag of the first set.  Nothing faults and nothing
+// waits unboundedly; the context stays usable.
+__global__ void __launch_bounds__(32) wait_selftest_kernel(unsigned int* sync, unsigned int limit)
 {
+    const float* cell = reinterpret_cast<const float*>(sync + 3);
     unsigned int spins = 0;
-    while (unwritten(ld_cell(reinterpret_cast<const float*>(sync + 3))))
-        if (!keep_waiting(spins, sync, limit)) return;
+    while (unwritten(ld_cell(cell)))
+        if (!warp_keep_waiting(spins, threadIdx.x == 0 ? sync + kSyncWords : sync, limit)) break;
+    sync[2 * kSyncWords + threadIdx.x] = spins;
+    spins = 0;
+    while (unwritten(ld_cell(cell)))
+        if (!warp_keep_waiting(spins, sync, limit)) return;
 }
 
 int launch_wait_selftest(messi_ctx* ctx, unsigned int* d_sync)
 {
-    cudaError_t e = cudaMemsetAsync(d_sync, 0, kSyncWords * sizeof(unsigned int), ctx->stream);
+    cudaError_t e = cudaMemsetAsync(d_sync, 0, kSelftestWords * sizeof(unsigned int), ctx->stream);
     if (e == cudaSuccess) e = cudaMemsetAsync(d_sync + 3, 0xff, sizeof(unsigned int), ctx->stream);
+    if (e == cudaSuccess) e = cudaMemsetAsync(d_sync + kSyncWords + 2, 0xff, sizeof(unsigned int), ctx->stream);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "wait self-test reset");
-    wait_selftest_kernel<<<1, 1, 0, ctx->stream>>>(d_sync, 1u << 12);
+    wait_selftest_kernel<<<1, 32, 0, ctx->stream>>>(d_sync, 1u << 12);
     LAUNCH_CHECK(ctx, "wait_selftest_kernel");
     return MESSI_OK;
 }

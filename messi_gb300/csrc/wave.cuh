@@ -53,6 +53,15 @@ static __device__ __forceinline__ bool keep_waiting(unsigned int& spins, unsigne
     return true;
 }
 
+// The same for a whole warp that waits together: one decision for all 32 lanes.
+// Their own looks at sync[2] may differ, and a lane that left alone would leave
+// the others in the warp's votes for ever.
+static __device__ __forceinline__ bool warp_keep_waiting(unsigned int& spins, unsigned int* sync,
+                                                         unsigned int limit = kSpinLimit)
+{
+    return __all_sync(0xffffffffu, keep_waiting(spins, sync, limit));
+}
+
 // Lanes per cell for a split sum of `nterms` terms: at most 8 terms per lane
 // up to 256 terms, so a lane's loads are issued together and the sum costs
 // one L2 round trip; longer sums use the whole warp.
