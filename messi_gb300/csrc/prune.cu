@@ -1381,7 +1381,9 @@ int launch_bandprep_from_mix(messi_ctx* ctx, messi_dataset* ds, const Band& t, c
 //     the lanes, each lane a running log-sum-exp, merged at the end.
 // FP64 throughout; bound by the FP64 pipe (one exp per pair and category).  A
 // term more than 45 nats below its maximum is below 2^-64 of the sum and its
-// exp is not formed.  (One thread per (column, category) walking every partner
+// exp is not formed.  A NaN term, or infinities that meet, make the sum NaN (the
+// comparisons with the limit are written so that a NaN takes the exp); an
+// infinite pair posterior enters all ns * nl categories of its pair.  (One thread per (column, category) walking every partner
 // and category with a log1p(exp) each took 16.6 ms at 64 x 600, span 300.)
 // ---------------------------------------------------------------------------
 constexpr double kNegligible = -45.0;
@@ -1405,7 +1407,7 @@ __global__ void __launch_bounds__(256) siterate_pairs_kernel(const double* __res
             for (int l = 0; l < nl; l++) {
                 const int c = (side ? o * ns + s : s * ns + o) * nl + l;
                 const double d = logw[c] + catll[(size_t)c * nroot + b] - m;
-                if (d >= kNegligible) acc += exp(d);
+                if (!(d < kNegligible)) acc += exp(d);
             }
     out[(size_t)blockIdx.y * nroot + b] = (m == -INFINITY) ? -INFINITY : m + log(acc);
 }
@@ -1415,19 +1417,21 @@ struct LogSum {
     double m = -INFINITY, s = 0.0;
     __device__ __forceinline__ void add(double v, double w = 1.0)  // w e^v
     {
-        if (v == -INFINITY) return;
-        if (v > m) {
-            s = (m - v >= kNegligible) ? s * exp(m - v) + w : w;
+        if (v == -INFINITY) {
+            s += 0.0 * w;  // (another sum's NaN)
+        } else if (v > m) {
+            s = s * ((m - v >= kNegligible) ? exp(m - v) : 0.0) + w;
             m = v;
-        } else if (v - m >= kNegligible) {
+        } else if (!(v - m < kNegligible)) {
             s += w * exp(v - m);
         }
     }
-    __device__ __forceinline__ double value() const { return (m == -INFINITY) ? -INFINITY : m + log(s); }
+    __device__ __forceinline__ double value() const { return (m == -INFINITY && s == 0.0) ? -INFINITY : m + log(s); }
 };
 
 __global__ void __launch_bounds__(128) siterate_cols_kernel(const int* __restrict__ bandidx, int L, int W,
                                                             const double* __restrict__ pairll, long long nroot, int ns,
+                                                            int nl,
                                                             const double* __restrict__ single,
                                                             const double* __restrict__ pair,
                                                             const double* __restrict__ ull,
@@ -1440,6 +1444,9 @@ __global__ void __launch_bounds__(128) siterate_cols_kernel(const int* __restric
     const double* first = pairll + (size_t)s * nroot;
     const double* second = pairll + (size_t)(ns + s) * nroot;
     LogSum acc;
+    auto partner = [&](double pp, double ll) {
+        if (pp > 0.0) acc.add((pp == INFINITY && ns * nl > 1) ? (double)NAN : log(pp) + ll);
+    };
     if (lane == 0) {
         const double us = ull[(size_t)s * L + x];
         if (us != -INFINITY) acc.add(logw_site[s] + log(single[x]) + us);
@@ -1447,14 +1454,12 @@ __global__ void __launch_bounds__(128) siterate_cols_kernel(const int* __restric
     for (int k = 1 + lane; k <= W && x + k < L; k += 32) {
         const int b = bandidx[(size_t)x * (W + 1) + k];
         if (b < 0) continue;
-        const double pp = pair[(size_t)x + (size_t)(x + k) * L];
-        if (pp > 0.0) acc.add(log(pp) + first[b]);
+        partner(pair[(size_t)x + (size_t)(x + k) * L], first[b]);
     }
     for (int k = 1 + lane; k <= W && k <= x; k += 32) {
         const int b = bandidx[(size_t)(x - k) * (W + 1) + k];
         if (b < 0) continue;
-        const double pp = pair[(size_t)(x - k) + (size_t)x * L];
-        if (pp > 0.0) acc.add(log(pp) + second[b]);
+        partner(pair[(size_t)(x - k) + (size_t)x * L], second[b]);
     }
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) {
@@ -1475,7 +1480,7 @@ int launch_siterate_conditionals(messi_ctx* ctx, messi_dataset* ds, const double
         LAUNCH_CHECK(ctx, "siterate_pairs_kernel");
     }
     siterate_cols_kernel<<<dim3((ds->L + 3) / 4, nsite), 128, 0, ctx->stream>>>(
-        ds->d_bandidx, ds->L, ds->W, d_pairll, ds->nroot, nsite, d_single, d_pair, d_ull, d_logw_site, d_out);
+        ds->d_bandidx, ds->L, ds->W, d_pairll, ds->nroot, nsite, nlam, d_single, d_pair, d_ull, d_logw_site, d_out);
     LAUNCH_CHECK(ctx, "siterate_cols_kernel");
     return MESSI_OK;
 }
