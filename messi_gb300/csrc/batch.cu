@@ -443,6 +443,7 @@ int messi_batch_create(messi_ctx* ctx, int32_t n, const messi_alignment* alns, c
             }
         if (e == cudaSuccess) e = cudaMalloc((void**)&b->d_leafrows, R * sizeof(int2));
         if (e == cudaSuccess) e = cudaMemcpy(b->d_leafrows, rows.data(), R * sizeof(int2), cudaMemcpyHostToDevice);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(0);  // the context's stream does not wait for the default stream
     }
     if (e != cudaSuccess) {
         destroy_batch(b);

@@ -1037,9 +1037,10 @@ int messi_mlp_create(messi_ctx* ctx, int32_t in_dim, int32_t width, int32_t ncom
     if (e == cudaSuccess) e = cudaMalloc((void**)&m->grad, sizeof(float) * (m->nparam + 16));
     if (e == cudaSuccess) e = cudaMalloc((void**)&m->m1, sizeof(float) * m->nparam);
     if (e == cudaSuccess) e = cudaMalloc((void**)&m->m2, sizeof(float) * m->nparam);
-    if (e == cudaSuccess) e = cudaMemcpy(m->p32, p.data(), sizeof(float) * m->nparam, cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) e = cudaMemset(m->m1, 0, sizeof(float) * m->nparam);
-    if (e == cudaSuccess) e = cudaMemset(m->m2, 0, sizeof(float) * m->nparam);
+    if (e == cudaSuccess)
+        e = cudaMemcpyAsync(m->p32, p.data(), sizeof(float) * m->nparam, cudaMemcpyHostToDevice, ctx->stream);
+    if (e == cudaSuccess) e = cudaMemsetAsync(m->m1, 0, sizeof(float) * m->nparam, ctx->stream);
+    if (e == cudaSuccess) e = cudaMemsetAsync(m->m2, 0, sizeof(float) * m->nparam, ctx->stream);
     if (e != cudaSuccess) {
         messi_mlp_destroy(m);
         return cuda_fail(ctx, e, "mlp parameters");
@@ -1097,7 +1098,7 @@ int messi_mlp_set_params(messi_ctx* ctx, messi_mlp* m, const float* host)
 {
     if (!ctx || !m || !host) return MESSI_EINVAL;
     cudaSetDevice(ctx->device);
-    cudaError_t e = cudaMemcpy(m->p32, host, sizeof(float) * m->nparam, cudaMemcpyHostToDevice);
+    cudaError_t e = cudaMemcpyAsync(m->p32, host, sizeof(float) * m->nparam, cudaMemcpyHostToDevice, ctx->stream);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "mlp set params");
     to_bf16_kernel<<<blocks(m->nparam), 256, 0, ctx->stream>>>(m->p32, m->p16, m->nparam);
     const int rc = fused_pack(ctx, m);

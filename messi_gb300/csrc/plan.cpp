@@ -734,10 +734,9 @@ int allocate_arena(messi_dataset* ds, int C, std::string* err)
     ds->steps_host.assign((size_t)ds->nsteps, StepDev{});
     fill_descriptors(ds, ds->d_arena_f, ds->d_arena_e, 0, ds->arena_rows, (int64_t)ds->chunk * ds->arena_rows,
                      leaf_rows, 0, 0, ds->d_steps, ds->segs_host.data(), ds->steps_host.data());
-    // (a lent plan's in the stream's order, behind the last user of its scratch)
+    // in the stream's order: behind the last reader, before the next
     auto upload = [&](void* dst, const void* src, size_t bytes) {
-        return ds->lent ? cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, ds->ctx->stream)
-                        : cudaMemcpy(dst, src, bytes, cudaMemcpyHostToDevice);
+        return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, ds->ctx->stream);
     };
     cudaError_t e = upload(ds->d_segs, ds->segs_host.data(), sizeof(SegDev) * ds->segs.size());
     if (e == cudaSuccess) e = upload(ds->d_steps, ds->steps_host.data(), sizeof(StepDev) * (size_t)ds->nsteps);

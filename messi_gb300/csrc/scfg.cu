@@ -1938,6 +1938,7 @@ int bandbatch_alloc(const std::vector<int>& L, const std::vector<int>& Wb, BandB
     e = cudaMemcpy(bb->d_bands, bb->host.data(), (size_t)n * sizeof(Band), cudaMemcpyHostToDevice);
     if (e == cudaSuccess) e = cudaMemcpy(bb->d_cumL, cum.data(), (size_t)(n + 1) * sizeof(long long), cudaMemcpyHostToDevice);
     if (e == cudaSuccess) e = cudaMemcpy(bb->d_wbs, wbs.data(), (size_t)n * sizeof(int), cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(0);  // the contexts' streams do not wait for the default stream
     if (e != cudaSuccess) {
         *err = std::string("batch band descriptors: ") + cudaGetErrorString(e);
         return MESSI_ECUDA;
