@@ -41,7 +41,7 @@ struct messi_mlp {
     // parameters: W1[H][in] b1[H] W2[H][H] b2[H] W3[out][H] b3[out]
     int nparam = 0;
     float* p32 = nullptr;              // FP32 master
-    __nv_bfloat16* p16 = nullptr;      // BF16 copy
+    __nv_bfloat16* p16 = nullptr;      // BF16 copy (GEMM per layer only)
     float* grad = nullptr;
     float* m1 = nullptr;               // Adam moments
     float* m2 = nullptr;
@@ -333,7 +333,7 @@ __global__ void adam_kernel(float* __restrict__ p, const float* __restrict__ gr,
     m2[i] = b;
     const float v = p[i] - lr * (a / c1) / (sqrtf(b / c2) + eps);
     p[i] = v;
-    p16[i] = __float2bfloat16(v);
+    if (p16) p16[i] = __float2bfloat16(v);
 }
 
 __global__ void sumsq_kernel(const float* __restrict__ g, int n, float* __restrict__ out)
@@ -846,10 +846,9 @@ static int mlp_reserve(messi_ctx* ctx, messi_mlp* m, int batch)
 static inline unsigned blocks(long long n) { return (unsigned)((n + 255) / 256); }
 
 // ---- two-kernel form, host side ----
-// Repacks the BF16 weights from the FP32 master copy (queued on the stream).
+// The packed BF16 weights from the FP32 master copy (queued on the stream).
 static int fused_pack(messi_ctx* ctx, messi_mlp* m)
 {
-    if (!m->fused) return MESSI_OK;
     pack_weights_kernel<<<152, 256, 0, ctx->stream>>>(m->p32, m->w16, m->in, m->H, m->out);
     LAUNCH_CHECK(ctx, "pack_weights_kernel");
     return MESSI_OK;
@@ -913,6 +912,15 @@ static int fused_gradients(messi_ctx* ctx, messi_mlp* m, int batch, const float*
     const int jobs = tH * tH + tO * tH + tH * tI + (m->out + 2 * m->H + 127) / 128;
     mlp_wgrad_kernel<<<jobs, 128, 0, ctx->stream>>>(w);
     LAUNCH_CHECK(ctx, "mlp_wgrad_kernel");
+    return MESSI_OK;
+}
+
+// The weights as the network's form reads them, from the FP32 master copy.
+static int refresh_weights(messi_ctx* ctx, messi_mlp* m)
+{
+    if (m->fused) return fused_pack(ctx, m);
+    to_bf16_kernel<<<blocks(m->nparam), 256, 0, ctx->stream>>>(m->p32, m->p16, m->nparam);
+    LAUNCH_CHECK(ctx, "to_bf16_kernel");
     return MESSI_OK;
 }
 
@@ -1033,7 +1041,6 @@ int messi_mlp_create(messi_ctx* ctx, int32_t in_dim, int32_t width, int32_t ncom
     fill(off[2], (size_t)m->H * m->H, std::sqrt(3.0 / m->H));
     fill(off[4], (size_t)m->out * m->H, 0.1 * std::sqrt(3.0 / m->H));
     cudaError_t e = cudaMalloc((void**)&m->p32, sizeof(float) * m->nparam);
-    if (e == cudaSuccess) e = cudaMalloc((void**)&m->p16, sizeof(__nv_bfloat16) * m->nparam);
     if (e == cudaSuccess) e = cudaMalloc((void**)&m->grad, sizeof(float) * (m->nparam + 16));
     if (e == cudaSuccess) e = cudaMalloc((void**)&m->m1, sizeof(float) * m->nparam);
     if (e == cudaSuccess) e = cudaMalloc((void**)&m->m2, sizeof(float) * m->nparam);
@@ -1047,16 +1054,15 @@ int messi_mlp_create(messi_ctx* ctx, int32_t in_dim, int32_t width, int32_t ncom
     }
     // two-kernel form where 16 rows of activations fit half an SM's shared memory
     m->fused = rows_layout(in_dim, width, m->out, dim, true).total <= kRowsMaxSmem;
-    if (m->fused) {
-        const size_t n = packed_layout(in_dim, width, m->out).total;
-        e = cudaMalloc((void**)&m->w16, sizeof(__nv_bfloat16) * n);
-        if (e != cudaSuccess) {
-            messi_mlp_destroy(m);
-            return cuda_fail(ctx, e, "mlp packed weights");
-        }
+    if (m->fused)
+        e = cudaMalloc((void**)&m->w16, sizeof(__nv_bfloat16) * packed_layout(in_dim, width, m->out).total);
+    else
+        e = cudaMalloc((void**)&m->p16, sizeof(__nv_bfloat16) * m->nparam);
+    if (e != cudaSuccess) {
+        messi_mlp_destroy(m);
+        return cuda_fail(ctx, e, "mlp weights");
     }
-    to_bf16_kernel<<<blocks(m->nparam), 256, 0, ctx->stream>>>(m->p32, m->p16, m->nparam);
-    const int prc = fused_pack(ctx, m);
+    const int prc = refresh_weights(ctx, m);
     e = cudaStreamSynchronize(ctx->stream);
     if (prc || e != cudaSuccess) {
         messi_mlp_destroy(m);
@@ -1100,8 +1106,7 @@ int messi_mlp_set_params(messi_ctx* ctx, messi_mlp* m, const float* host)
     cudaSetDevice(ctx->device);
     cudaError_t e = cudaMemcpyAsync(m->p32, host, sizeof(float) * m->nparam, cudaMemcpyHostToDevice, ctx->stream);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "mlp set params");
-    to_bf16_kernel<<<blocks(m->nparam), 256, 0, ctx->stream>>>(m->p32, m->p16, m->nparam);
-    const int rc = fused_pack(ctx, m);
+    const int rc = refresh_weights(ctx, m);
     e = cudaStreamSynchronize(ctx->stream);
     return rc ? rc : ((e == cudaSuccess) ? MESSI_OK : cuda_fail(ctx, e, "mlp set params"));
 }
@@ -1180,7 +1185,7 @@ int messi_mlp_train_step(messi_ctx* ctx, messi_mlp* m, int32_t batch, const floa
     adam_kernel<<<blocks(m->nparam), 256, 0, ctx->stream>>>(m->p32, m->grad, m->m1, m->m2, m->p16, m->nparam, lr, b1,
                                                             b2, c1, c2, 1e-8f, clip);
     LAUNCH_CHECK(ctx, "adam_kernel");
-    if ((rc = fused_pack(ctx, m))) return rc;
+    if (m->fused && (rc = fused_pack(ctx, m))) return rc;
     e = cudaStreamSynchronize(ctx->stream);
     return (e == cudaSuccess) ? MESSI_OK : cuda_fail(ctx, e, "adam");
 }
