@@ -71,9 +71,10 @@ __global__ void __launch_bounds__(256) build_P16_kernel(const double* __restrict
                                                        const int* __restrict__ nodegrp, int numnodes, int C,
                                                        float* __restrict__ P)
 {
-    const int c = blockIdx.x, t = threadIdx.x;
+    // one grid dimension: a batch may have more runs of nodes than the second one takes
+    const int c = (int)(blockIdx.x % (unsigned)C), t = threadIdx.x;
     const int a = t >> 4, d = t & 15;
-    const int v0 = blockIdx.y * kP16Nodes, v1 = min(numnodes, v0 + kP16Nodes);
+    const int v0 = (int)(blockIdx.x / (unsigned)C) * kP16Nodes, v1 = min(numnodes, v0 + kP16Nodes);
     __shared__ double U[256], W[2][256], R[256], ex[kP16Nodes][16];
     auto group = [&](int v) { return nodegrp ? nodegrp[v] : (v == 0 ? -1 : 0); };  // the same in every thread
     if (t < 16 * kP16Nodes && v0 + a < v1) {
@@ -149,8 +150,8 @@ __global__ void build_P4_kernel(const double* __restrict__ eig4, const double* _
 int launch_build_P16(messi_ctx* ctx, const double* d_eig, const double* d_bl, const int* d_nodegrp, int numnodes,
                      int C, float* d_P)
 {
-    build_P16_kernel<<<dim3(C, (numnodes + kP16Nodes - 1) / kP16Nodes), 256, 0, ctx->stream>>>(d_eig, d_bl, d_nodegrp,
-                                                                                              numnodes, C, d_P);
+    const unsigned runs = (unsigned)(numnodes + kP16Nodes - 1) / kP16Nodes;
+    build_P16_kernel<<<(unsigned)C * runs, 256, 0, ctx->stream>>>(d_eig, d_bl, d_nodegrp, numnodes, C, d_P);
     LAUNCH_CHECK(ctx, "build_P16_kernel");
     return MESSI_OK;
 }
