@@ -414,7 +414,7 @@ int messi_batch_create(messi_ctx* ctx, int32_t n, const messi_alignment* alns, c
         for (int lv = 1; lv <= gr.H; lv++)
             for (int root = 0; root < 2; root++) {
                 SegLevel& sl = root ? gr.roots[lv] : gr.levels[lv];
-                level_shape(&sl, ctx->prune_shape != 3);
+                level_shape(&sl, ctx->prune_shape != 3, ctx->num_sms);
                 sl.tile_off = (int)tiles.size();
                 for (int a = gr.a0; a < gr.a1; a++) {
                     const messi_dataset* d = b->ds[a];

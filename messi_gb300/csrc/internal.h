@@ -87,9 +87,8 @@ struct SegDev {
     double* mixlam;    // root only: [kMaxLambda][n] per-lambda mixtures (nullable)
     double* catll;     // root only: [C][n] per-category log-likelihoods (nullable)
     int n;             // unique pairs of the segment's top node
-    int nsteps, nb, nmat;  // steps, gather slots, mat-vecs
+    int nsteps, nb;    // steps, gather slots
     int grp;           // model group (index of the category tables pi16/logw)
-    int pad;
 };
 
 // A segment as the plan holds it (steps in program order; `child` = the node
@@ -381,7 +380,7 @@ void fill_descriptors(const messi_dataset* ds, float* rows, int* exps, int64_t r
                       SegDev* segs, StepDev* steps);
 // Adds a segment to a level's launch, and picks the level's tile shape once all are in.
 void level_add(SegLevel* lv, const Segment& sg);
-void level_shape(SegLevel* lv, bool fuse);
+void level_shape(SegLevel* lv, bool fuse, int num_sms);
 // Gather indices of every segment from the per-node child lists (prune.cu):
 // ops = for each segment [op_off[s], op_off[s+1]) in parent-before-child order.
 struct IdxOp {

@@ -184,15 +184,18 @@ void level_add(SegLevel* lv, const Segment& sg)
 }
 
 // Four pair groups per CTA, all categories in turn, where the level's pairs alone
-// give the GPU's 152 SMs twelve warps each; below that one pair group per CTA,
+// give every SM twelve warps (GB300: 1,824); below that one pair group per CTA,
 // whose warps share the categories (launch_prune_level).  With the line at 4,096
 // warps a level of 3,803 took 171 us and takes 118, one of 3,344 (a batch) 341 ->
 // 251, the 1,872 of a root segment of 100 sequences 2,107 -> 1,517 (warps that
 // share the categories do not share their matrices in L1); below the line 1,807
 // take 475 us as they are and would take 505, 1,672 399 and 530.
-constexpr int64_t kGroupWarps = 12 * 152;
+constexpr int64_t kGroupWarpsPerSm = 12;
 
-void level_shape(SegLevel* lv, bool fuse) { lv->pg = (lv->warps >= kGroupWarps || !fuse) ? 4 : 1; }
+void level_shape(SegLevel* lv, bool fuse, int num_sms)
+{
+    lv->pg = (lv->warps >= kGroupWarpsPerSm * num_sms || !fuse) ? 4 : 1;
+}
 
 int build_plan(messi_dataset* ds, const messi_alignment* aln, int W, const uint8_t* pairmask, std::string* err,
                const std::vector<int2>* pairs, std::vector<int32_t>* pair_unique)
@@ -456,7 +459,7 @@ int build_plan(messi_dataset* ds, const messi_alignment* aln, int W, const uint8
     ds->SH = ds->segs[0].level;
     ds->seg_levels.assign(ds->SH + 1, SegLevel{});
     for (const Segment& sg : ds->segs) level_add(&ds->seg_levels[sg.level], sg);
-    for (SegLevel& lv : ds->seg_levels) level_shape(&lv, ds->fuse);
+    for (SegLevel& lv : ds->seg_levels) level_shape(&lv, ds->fuse, ds->ctx->num_sms);
     ds->executed = 0;
     for (const SegLevel& lv : ds->seg_levels) ds->executed += (int64_t)lv.units;
     ds->naive = ds->band_pairs * (int64_t)(N - 1);
@@ -653,7 +656,6 @@ void fill_descriptors(const messi_dataset* ds, float* rows, int* exps, int64_t r
         d.n = (int)sg.n;
         d.nsteps = (int)sg.steps.size();
         d.nb = sg.nb;
-        d.nmat = sg.nmat;
         d.grp = grp;
         if (sg.root != 0) {
             d.out = (unsigned)(row_base + sg.row_off);
