@@ -215,7 +215,8 @@ struct LikelihoodKey {
 constexpr int kTuneCalls = 4;
 constexpr int kPruneShapes = 3;
 constexpr int kWaveCands = 4;
-constexpr int kWaveThreadCands[kWaveCands] = {0, 256, 512, 1024};  // 0: chosen by band size
+constexpr int kWaveThreadCands[kWaveCands] = {0, 256, 512, 1024};  // 0: by the cells per CTA; the
+// inside kernel takes at most 512 (768 by its own rule), so the larger ones may launch alike
 struct TuneSlot {
     int k = 0;                       // evaluations timed so far
     bool done = false;

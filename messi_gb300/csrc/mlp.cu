@@ -573,7 +573,7 @@ __global__ void __launch_bounds__(kRowThreads) mlp_rows_kernel(const RowsArgs A)
         xs[r * R.ldx + kpos(k)] =
             __float2bfloat16((row0 + r < A.B && k < A.in) ? A.x[(size_t)(row0 + r) * A.in + k] : 0.f);
     }
-    float* tgt = comp + kRows * 17;  // [32][D]
+    float* tgt = comp + kRows * 17;  // [16][D]
     if (GRAD)
         for (int e = tid; e < kRows * A.D; e += kRowThreads)
             tgt[e] = (row0 + e / A.D < A.B) ? A.target[(size_t)row0 * A.D + e] : 0.f;

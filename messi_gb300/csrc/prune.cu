@@ -366,7 +366,7 @@ __device__ __forceinline__ void pow2_scale(float m, int& ex, float& sc)
 // states 4t..4t+3 of its pairs, which is the A layout of the next product:
 // column g of tile nt is state 4(g/2) + 2nt + g%2.
 // Measured (GB300, 64 x 1,000 columns, span 500, 36 categories): 2.96e8
-// distinct updates in 7.5 ms before; 3.6e8 (some recomputed) in 5.2 ms now,
+// distinct updates in 7.5 ms before; 3.6e8 (some recomputed) in 4.9 ms now,
 // DRAM traffic 35 GB -> ~7 GB.  What bounds it: about 245 instructions per 32
 // updates at half of the issue slots, the tensor pipe 41% busy (24 MMAs of 8.5
 // cycles a step), with the 20 warps per SM the registers allow: 16 took 13%

@@ -27,8 +27,8 @@
 //
 // Schedule.  One persistent cooperative launch walks the band diagonals (a
 // wavefront): all cells of a span are independent, so each diagonal is spread
-// over the whole grid, two diagonals at a time (a CTA owns a block of rows and
-// the second diagonal of a pair reads the first only at the CTA's own rows).
+// over the whole grid, two diagonals at a time (the rows of a pair are dealt to
+// the CTAs, and the second diagonal reads the first only at the CTA's own rows).
 // The CTAs wait for one another's cells; the waits have a bounded
 // iteration count: on timeout an error flag is raised, every CTA leaves, Z
 // becomes NaN and the host returns MESSI_ETIMEOUT.  A cell's split sum is
