@@ -234,9 +234,18 @@ int finish(messi_ctx* ctx)
     if (!ctx->prof_pending.empty()) prof_collect(ctx);
     e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_fail(ctx, e, "kernel execution");
-    if (ctx->status_host && *ctx->status_host != 0u)
-        return fail(ctx, MESSI_ETIMEOUT, "wavefront kernel gave up waiting (bounded spin)");
+    for (int k = 0; ctx->status_host && k < kStatusWords; k++)
+        if (ctx->status_host[k] != 0u)
+            return fail(ctx, MESSI_ETIMEOUT, "wavefront kernel gave up waiting (bounded spin)");
     return MESSI_OK;
+}
+
+int queue_status(messi_ctx* ctx, const unsigned int* d_flag)
+{
+    if (!ctx->status_host) return MESSI_OK;
+    unsigned int* word = ctx->status_host + ctx->status_used++ % kStatusWords;
+    const cudaError_t e = cudaMemcpyAsync(word, d_flag, sizeof(unsigned int), cudaMemcpyDeviceToHost, ctx->stream);
+    return (e == cudaSuccess) ? MESSI_OK : cuda_fail(ctx, e, "status readback");
 }
 
 void tune_begin(messi_ctx* ctx, const void* key, int C)
@@ -304,7 +313,8 @@ int begin(messi_ctx* ctx)
     if (!ctx) return MESSI_EINVAL;
     ctx->launches = 0;
     ctx->last_error.clear();
-    if (ctx->status_host) *ctx->status_host = 0u;
+    if (ctx->status_host) std::fill_n(ctx->status_host, kStatusWords, 0u);
+    ctx->status_used = 0;
     cudaError_t e = cudaSetDevice(ctx->device);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "cudaSetDevice");
     return MESSI_OK;
@@ -469,7 +479,7 @@ int messi_ctx_create(int device, messi_ctx** out)
         delete ctx;
         return MESSI_ECUDA;
     }
-    if (cudaMallocHost((void**)&ctx->status_host, 64) != cudaSuccess) {
+    if (cudaMallocHost((void**)&ctx->status_host, kStatusWords * sizeof(unsigned int)) != cudaSuccess) {
         cudaEventDestroy(ctx->fork_ev);
         cudaEventDestroy(ctx->join_ev);
         cudaStreamDestroy(ctx->side);
@@ -477,7 +487,7 @@ int messi_ctx_create(int device, messi_ctx** out)
         delete ctx;
         return MESSI_ENOMEM;
     }
-    *ctx->status_host = 0u;
+    std::fill_n(ctx->status_host, kStatusWords, 0u);
     {
         const char* w = std::getenv("MESSI_WAVE_CTAS");
         if (w) ctx->wave_ctas = std::max(0, std::atoi(w));
@@ -574,8 +584,13 @@ int messi_selftest_bounded_wait(messi_ctx* ctx, int32_t* status)
     unsigned int words[kSelftestWords] = {};
     if ((rc = launch_wait_selftest(ctx, (unsigned int*)p))) return rc;
     if ((rc = d2h(ctx, words, p, sizeof(words)))) return rc;
-    if ((rc = finish(ctx))) return rc;
-    *status = words[2] ? MESSI_ETIMEOUT : MESSI_OK;
+    // the failed wait's flag, then that of a pass without a failure
+    if ((rc = queue_status(ctx, (unsigned int*)p + 2))) return rc;
+    if ((rc = queue_status(ctx, (unsigned int*)p))) return rc;
+    rc = finish(ctx);
+    if (rc && rc != MESSI_ETIMEOUT) return rc;
+    ctx->last_error.clear();
+    *status = (rc == MESSI_ETIMEOUT && words[2]) ? MESSI_ETIMEOUT : MESSI_OK;
     for (int lane = 1; lane < 32; lane++)
         if (words[2 * kSyncWords + lane] != words[2 * kSyncWords]) *status = MESSI_ESTATE;  // lanes left apart
     return MESSI_OK;

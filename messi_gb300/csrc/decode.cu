@@ -635,11 +635,7 @@ int run_posterior_decoding(messi_ctx* ctx, int L, const double* d_single, const 
         to_double_kernel<<<(unsigned)((LL + bs - 1) / bs), bs, 0, ctx->stream>>>(ecol, d_eout, LL);
         LAUNCH_CHECK(ctx, "to_double_kernel");
     }
-    if (ctx->status_host) {
-        e = cudaMemcpyAsync(ctx->status_host, d_sync + 2, sizeof(unsigned int), cudaMemcpyDeviceToHost, ctx->stream);
-        if (e != cudaSuccess) return cuda_fail(ctx, e, "status readback");
-    }
-    return MESSI_OK;
+    return queue_status(ctx, d_sync + 2);
 }
 
 int run_sample_structures(messi_ctx* ctx, const Band& t, double B, int nstruct, unsigned long long seed,

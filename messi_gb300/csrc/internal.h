@@ -263,7 +263,9 @@ struct messi_ctx {
     messi::DevBuf scratch[32];
     void* pinned = nullptr;
     size_t pinned_bytes = 0;
-    unsigned int* status_host = nullptr;  // pinned word: wavefront wait status of the last call
+    // pinned words: wait status of each wavefront of the current call (nullptr: not read back)
+    unsigned int* status_host = nullptr;
+    int status_used = 0;
     // device buffers are reallocated only when they grow; every reallocation
     // bumps the epoch, so a captured launch sequence knows its pointers are stale
     uint64_t alloc_epoch = 0;
@@ -449,8 +451,9 @@ struct SideLaunches {
 };
 
 // Bounded-wait self-test (scfg.cu): a warp's wait for a cell that nothing writes;
-// d_sync[2] becomes 1 when it gives up.  d_sync: two sets of status words, then the
-// looks that each of the 32 lanes took until one of them saw another's failure.
+// d_sync[2] becomes 1 when it gives up, d_sync[0] stays 0.  d_sync: two sets of
+// status words, then the looks that each of the 32 lanes took until one of them saw
+// another's failure.
 constexpr int kSelftestWords = 2 * kSyncWords + 32;
 int launch_wait_selftest(messi_ctx* ctx, unsigned int* d_sync);
 // Dense L x L pair matrix: vals (nullable) of the unique root pairs, mixed with
@@ -510,7 +513,10 @@ void tune_begin(messi_ctx* ctx, const void* key, int C);
 void tune_mark(messi_ctx* ctx, int i);
 void tune_end(messi_ctx* ctx, const void* key, int C);
 void tune_forget(messi_ctx* ctx, const void* key);
-// Queue a copy of the wavefront wait status into ctx->status_host.
-int queue_status_readback(messi_ctx* ctx, const Band& t);
+// Queues a copy of a wavefront's error flag into the call's next status word: a
+// call has up to three wavefronts (inside, outside, decoding), and the end of the
+// call looks at all of them.
+constexpr int kStatusWords = 16;
+int queue_status(messi_ctx* ctx, const unsigned int* d_flag);
 
 }  // namespace messi

@@ -733,7 +733,7 @@ int launch_finish_Z(messi_ctx* ctx, const Band& t)
 {
     finish_Z_kernel<<<1, 32, 0, ctx->stream>>>(t);
     LAUNCH_CHECK(ctx, "finish_Z_kernel");
-    return queue_status_readback(ctx, t);
+    return queue_status(ctx, t.sync + 2);
 }
 
 
@@ -1794,14 +1794,6 @@ int launch_wait_selftest(messi_ctx* ctx, unsigned int* d_sync)
     return MESSI_OK;
 }
 
-int queue_status_readback(messi_ctx* ctx, const Band& t)
-{
-    if (!ctx->status_host) return MESSI_OK;
-    cudaError_t e = cudaMemcpyAsync(ctx->status_host, t.sync + 2, sizeof(unsigned int), cudaMemcpyDeviceToHost,
-                                    ctx->stream);
-    return (e == cudaSuccess) ? MESSI_OK : cuda_fail(ctx, e, "status readback");
-}
-
 // The outside kernel (cooperative), one CTA per SM, after its tables are filled
 // with kUnwritten.  More rows per CTA want more warps for their sums, although
 // fewer registers a thread then spill: 512, 768, 1,024 threads took 308, 366, 433
@@ -1990,9 +1982,7 @@ int run_inside_batch(messi_ctx* ctx, const BandBatch& bb, double B)
     prof_end(ctx);
     finish_Z_batch_kernel<<<(n + 127) / 128, 128, 0, ctx->stream>>>(bands, n, sync, bb.d_Z);
     LAUNCH_CHECK(ctx, "finish_Z_batch_kernel");
-    if (!ctx->status_host) return MESSI_OK;
-    e = cudaMemcpyAsync(ctx->status_host, sync + 2, sizeof(unsigned int), cudaMemcpyDeviceToHost, ctx->stream);
-    return (e == cudaSuccess) ? MESSI_OK : cuda_fail(ctx, e, "status readback");
+    return queue_status(ctx, sync + 2);
 }
 
 // ---------------------------------------------------------------------------
@@ -2211,7 +2201,7 @@ int run_outside(messi_ctx* ctx, const Band& t, double B)
     int rc = launch_outside(ctx, tt, args, sync);
     if (rc) return rc;
     prof_end(ctx);
-    return queue_status_readback(ctx, t);
+    return queue_status(ctx, t.sync + 2);
 }
 
 // ---------------------------------------------------------------------------
