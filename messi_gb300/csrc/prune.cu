@@ -1423,8 +1423,8 @@ struct LogSum {
         } else if (v > m) {
             s = s * ((m - v >= kNegligible) ? exp(m - v) : 0.0) + w;
             m = v;
-        } else if (!(v - m < kNegligible)) {
-            s += w * exp(v - m);
+        } else {
+            s += w * ((v - m < kNegligible) ? 0.0 : exp(v - m));  // (a negligible sum's NaN, too)
         }
     }
     __device__ __forceinline__ double value() const { return (m == -INFINITY && s == 0.0) ? -INFINITY : m + log(s); }

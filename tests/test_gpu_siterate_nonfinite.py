@@ -46,3 +46,24 @@ def test_non_finite_posteriors(where):
     assert np.isnan(got[:, bad]).all()
     rest = np.setdiff1d(np.arange(L), bad)
     np.testing.assert_array_equal(got[:, rest], clean[:, rest])
+
+
+@pytest.mark.parametrize("at", [(22, 46), (0, 88), (10, 11), (70, 99)])
+def test_infinite_pair_posteriors_far_below_their_columns_largest_term(at):
+    """The NaN of one partner meets sums of others that are hundreds of nats above
+    it (43 diverse sequences), in every lane of the column's warp."""
+    from messi_gb300 import api, synth
+    from messi_gb300 import model as M
+    L, W = 100, 88
+    s = synth.make_workload(dict(numseqs=43, numcols=L, W=W, paired=0.1, mean_bl=0.6), seed=9)
+    rng = np.random.default_rng(5)
+    pair = rng.random((L, L)) ** 8
+    pair = np.triu(pair, 1) + np.triu(pair, 1).T
+    single = rng.random(L)
+    params = M.getparams(s.params15, s.dataset.branchlengths, 3, 1)
+    clean = api.felsensteinposteriorsiterateconditionalscuda(single, pair, s.dataset, params, None, W)
+    pair[at] = np.inf
+    got = api.felsensteinposteriorsiterateconditionalscuda(single, pair, s.dataset, params, None, W)
+    assert np.isnan(got[:, list(at)]).all()
+    rest = np.setdiff1d(np.arange(L), at)
+    np.testing.assert_array_equal(got[:, rest], clean[:, rest])
