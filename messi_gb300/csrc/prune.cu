@@ -331,9 +331,13 @@ __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commi
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N)); }
 
-// Exact power-of-two rescale of a row max m > 0: m * 2^-ex in [0.5, 1).
-__device__ __forceinline__ void pow2_scale(float m, int& ex, float& sc)
+// Exact power-of-two rescale of a row max m > 0: m * 2^-ex in [0.5, 1), as two
+// factors: a denormal m needs more than the largest power of two.
+__device__ __forceinline__ void pow2_scale(float m, int& ex, float& pre, float& sc)
 {
+    const bool denormal = m > 0.f && m < 0x1p-126f;
+    pre = denormal ? 0x1p126f : 1.f;
+    m *= pre;
     const unsigned bits = __float_as_uint(m);
     const int E = (int)((bits >> 23) & 0xffu);
     if (E >= 1 && E <= 252) {  // normal, and 2^-ex representable
@@ -346,6 +350,7 @@ __device__ __forceinline__ void pow2_scale(float m, int& ex, float& sc)
         ex = 0;
         sc = 1.f;
     }
+    if (denormal) ex -= 126;
 }
 
 // ---------------------------------------------------------------------------
@@ -611,8 +616,8 @@ __global__ void __launch_bounds__(MAXT, MINB) prune_path_kernel(
                         mx[k] = max4(M[h][k]);
                     }
                     // Exact power-of-two rescale by the pair's largest state m to
-                    // [0.5, 1): 2^(126 - E), E the exponent field of m (E = 0, a
-                    // zero or denormal m, scales by 2^126, which is exact too).
+                    // [0.5, 1): 2^(126 - E), E the exponent field of m; E = 0, a
+                    // zero or denormal m, scales by 2^126 first.
                     const unsigned mb = __float_as_uint(quad_reduce(mx, t, [](float a, float b) { return fmaxf(a, b); }));
                     e[h] += (int)(mb >> 23) - 126;
                     const float sc = __uint_as_float((253u << 23) - (mb & 0x7f800000u));
@@ -620,6 +625,20 @@ __global__ void __launch_bounds__(MAXT, MINB) prune_path_kernel(
                     for (int k = 0; k < 4; k++) {
                         const float sk = __shfl_sync(0xffffffffu, sc, (lane & 28) + k);
                         M[h][k] = mul4(M[h][k], make_float4(sk, sk, sk, sk));
+                    }
+                    // a denormal m: the rest of its way, or the next product would
+                    // lose digits that a full row keeps (next to never: the vote costs
+                    // less than the runs of one side differ)
+                    const bool rest = mb - 1u < 0x007fffffu;
+                    if (__any_sync(0xffffffffu, rest)) {
+                        const unsigned rb = rest ? __float_as_uint(__uint_as_float(mb) * 0x1p126f) : (126u << 23);
+                        e[h] += (int)(rb >> 23) - 126;
+                        const float s2 = __uint_as_float((253u << 23) - (rb & 0x7f800000u));
+#pragma unroll
+                        for (int k = 0; k < 4; k++) {
+                            const float sk = __shfl_sync(0xffffffffu, s2, (lane & 28) + k);
+                            M[h][k] = mul4(M[h][k], make_float4(sk, sk, sk, sk));
+                        }
                     }
                 }
                 if (op.y & kStepPush) {
@@ -971,8 +990,10 @@ __global__ void __launch_bounds__(kTile, 6) prune_tc_kernel(const SegDev* __rest
 #pragma unroll
         for (int c = 1; c < 16; c++) m = fmaxf(m, V[c]);
         int ex;
-        float sc;
-        pow2_scale(m, ex, sc);
+        float pre, sc;
+        pow2_scale(m, ex, pre, sc);
+#pragma unroll
+        for (int c = 0; c < 16; c++) V[c] *= pre;
         if (myvalid) {
             // the row as two 32-byte stores: whole sectors
             float* o = nd.rows + ((size_t)nd.out + (size_t)cf * nd.ocs + myu) * 16;
